@@ -129,6 +129,8 @@ __global__ void __launch_bounds__(256) k_spec_accept(int* __restrict__ sp, const
 }
 
 #define HP_TRY(x) do { const int rc_ = (x); if (rc_ != HP_OK) return rc_; } while (0)
+// rows r0.. of a quantised activation buffer (r0 a multiple of 8: whole column tiles)
+static XQ8F xq_rows(const XQ8F& x, int r0, int K) { return XQ8F{(char*)x.q + xq_q_bytes(r0, K), (char*)x.sc + xq_sc_floats(r0, K) * 4}; }
 // descriptor layout (ints)
 Engine::Engine(const hp_model_cfg& cfg) : c_(cfg) {}
 Engine::~Engine() {
@@ -137,6 +139,7 @@ Engine::~Engine() {
     for (auto& v : ep_segs_) for (EpSeg& sg : v) if (sg.g) cudaGraphExecDestroy(sg.g);
     for (void* p : allocs_) cudaFree(p);
     if (h_desc_) cudaFreeHost(h_desc_);
+    if (pf_hdesc_) cudaFreeHost(pf_hdesc_);
     if (h_spec_) cudaFreeHost(h_spec_);
     if (ev0_) cudaEventDestroy(ev0_); if (ev1_) cudaEventDestroy(ev1_);
     if (s_) cudaStreamDestroy(s_);
@@ -321,6 +324,24 @@ int Engine::init() {
         { const int w = std::max(1, c.ep_world); e_lo_ = (int)((long long)c.ep_rank * c.n_expert / w); e_hi_ = (int)((long long)(c.ep_rank + 1) * c.n_expert / w); }
     }
     nsplit_max_ = (c.max_ctx + ATTN_SPLIT - 1) / ATTN_SPLIT;
+    if (tiled_ && c.ep_world <= 1 && c.max_ctx > 8) {   // prompt chunks (the GEMM reads tile-major weights; expert shards exchange after every pass)
+        const int PR = pf_rows_ = std::min(PF_MAXR, (c.max_ctx + 7) & ~7);
+        size_t planes = 0;
+        auto need = [&](const Lin& l) { if (l.N) planes = std::max(planes, (size_t)l.P * l.N); };
+        for (const LayerW& L : layers_) { need(L.in_proj); need(L.out_proj); need(L.down); need(L.gate_up); }
+        need(eh_proj_); need(mtp_.in_proj);
+        HP_TRY(alloc((void**)&pf_.x, (size_t)PR * E * 4)); HP_TRY(alloc((void**)&pf_.emb, (size_t)PR * E * 4)); HP_TRY(alloc((void**)&pf_.h, (size_t)PR * E * 4));
+        HP_TRY(alloc((void**)&pf_hin_, (size_t)PR * E * 4)); HP_TRY(alloc((void**)&pf_.big, (size_t)PR * bigw * 4)); HP_TRY(alloc((void**)&pf_.yparts, (size_t)PR * planes * 4));
+        HP_TRY(alloc(&pf_.xq.q, xq_q_bytes(PR, (int)kmax))); HP_TRY(alloc(&pf_.xq.sc, xq_sc_floats(PR, (int)kmax) * 4));
+        HP_CUDA(cudaMemsetAsync(pf_.xq.q, 0, xq_q_bytes(PR, (int)kmax), s_)); HP_CUDA(cudaMemsetAsync(pf_.xq.sc, 0, xq_sc_floats(PR, (int)kmax) * 4, s_));
+        HP_TRY(alloc(&pf_pack_, gemm_pack_bytes(PR, (int)kmax)));
+        if (ngdn()) HP_TRY(alloc((void**)&pf_gdn_, gdn_prefill_floats(PR, nq, nv) * 4));
+        HP_TRY(alloc((void**)&pf_desc_, (size_t)PR * 8 * 4)); HP_CUDA(cudaMallocHost((void**)&pf_hdesc_, (size_t)PR * 8 * 4));
+        if (c.n_expert) {
+            const size_t pairs = (size_t)PR * (c.n_expert_used + 1);
+            HP_TRY(alloc((void**)&pf_.xn, (size_t)PR * E * 4)); HP_TRY(alloc((void**)&pf_.moe_v, pairs * E * 4)); HP_TRY(alloc((void**)&pf_.moe_w, pairs * 4)); HP_TRY(alloc((void**)&pf_.moe_ids, pairs * 4));
+        }
+    }
     const size_t np = attn_partial_floats(MAXR, c.n_head_kv, nsplit_max_);
     HP_TRY(alloc((void**)&pO_, np * 256 * 4)); HP_TRY(alloc((void**)&pm_, np * 4)); HP_TRY(alloc((void**)&pl_, np * 4));
     HP_TRY(alloc((void**)&d_desc_, D_INTS * 4)); HP_CUDA(cudaMallocHost((void**)&h_desc_, D_INTS * 4)); memset(h_desc_, 0, D_INTS * 4);
@@ -361,12 +382,21 @@ int Engine::upload_desc() { HP_CUDA(cudaMemcpyAsync(d_desc_, h_desc_, D_INTS * 4
 static int lin_class_bit(const Lin& l, const hp_model_cfg& c) {
     return l.N == 2 * c.n_ff ? 16 : l.K == c.n_ff ? 32 : l.N == c.n_vocab ? 64 : l.K == c.n_embd ? 128 : 256;
 }
+// A linear over the rows of a prompt chunk; both kernels give the same bits. Up to 32 rows are one pass of the GEMV over the
+// weights and it is the faster one (gate|up of 27B, 32 rows: 88 against 90 us; its down projection 52 against 76), at 64
+// rows its two passes take 183 and 103 us against the GEMM's 140 and 112.
+int Engine::prefill_lin(const Lin& l, float* out, int ld, size_t part_stride, int R) {
+    if (R <= 32) return gemv_q4k_q8_parts(l.wt, xq_, out, l.N, l.K, R, ld, part_stride, err_, s_, pdl_, true);
+    return gemm_q4k_q8_parts(l.wt, xq_, out, l.N, l.K, R, ld, part_stride, pf_pack_, err_, s_, pdl_);
+}
 int Engine::lin_parts(const Lin& l, int R) {
     if (prof_skip_ & lin_class_bit(l, c_)) return HP_OK;
+    if (pf_on_) return prefill_lin(l, yparts_, l.N, (size_t)R * l.N, R);
     return gemv_q4k_q8_parts(l.wt ? l.wt : l.w, xq_, yparts_, l.N, l.K, R, l.N, (size_t)R * l.N, err_, s_, pdl_, l.wt != nullptr);
 }
 int Engine::lin(const Lin& l, float* out, int ld, int R) {
     if (prof_skip_ & lin_class_bit(l, c_)) return HP_OK;
+    if (l.P == 1 && pf_on_) return prefill_lin(l, out, ld, 0, R);
     if (l.P == 1) return gemv_q4k_q8_parts(l.wt ? l.wt : l.w, xq_, out, l.N, l.K, R, ld, 0, err_, s_, pdl_, l.wt != nullptr);
     HP_TRY(lin_parts(l, R));
     HP_CUDA(launch_pdl<16>(k_reduce_planes, dim3((l.N + 255) / 256, R), dim3(256), 0, s_, yparts_, (size_t)R * l.N, l.P, out, l.N, ld));
@@ -381,6 +411,7 @@ int Engine::norm_in(const Lin* prev, bool have_y, const uint16_t* w, float* xn, 
 }
 // qwen35.cpp:247-276
 int Engine::attn_block(const LayerW& L, uint16_t* kc, uint16_t* vc, size_t kv_stride, int R, int ngroups, bool kv_only) {
+    if (pf_on_) return prefill_attn(L, kc, vc, kv_stride, R, kv_only);
     const int ld = L.in_proj.N;
     AttnParams p; p.qkv = big_;
     if (L.in_proj.P > 1 && !(prof_skip_ & 4) && !gemv_only_) {   // the rope kernel adds the K-part planes itself
@@ -408,16 +439,16 @@ int Engine::ffn_block(const LayerW& L, int R) {
 }
 
 // Qwen4Exp::moe_layer (qwen4exp.cpp:345-354): router -> route -> gate|up for the k+1 slots -> silu*mul+q8 -> down + in-order combine
-int Engine::moe_block(const LayerW& L, int R) {
+// for rows [row0, row0 + R) of the current buffers (R <= MAXR, row0 a multiple of 8)
+int Engine::moe_rows(const LayerW& L, int R, int row0, const int* tok, const int* pos, const int* slot, int* pushed) {
     const hp_model_cfg& c = c_; const int E = c.n_embd, F = c.expert_ff, ns = c.n_expert_used + 1;
-    if (gemv_only_) return HP_OK;
     // synthetic routing (see hp_model_cfg.synth_router_logits): the key of a layer's draws; 0 = the router's own logits
     const int lidx = &L == &mtp_ ? c.n_layer : (int)(&L - layers_.data());
     const uint64_t rkey = c.synth_router_logits ? (splitmix64(c.seed ^ 0x726F75746572ull ^ ((uint64_t)lidx << 40)) | 1ull) : 0ull;
     // the (replicated) shared expert is computed by one GPU per layer, in turn, so that no GPU carries all of them
     const int own_sh = c.ep_world > 1 ? (lidx % c.ep_world == c.ep_rank ? 1 : 0) : 1;
-    MoeRouteParams rp; rp.W = L.router; rp.x = xn_; rp.logits = rlogits_; rp.E = c.n_expert; rp.K = E; rp.k = c.n_expert_used; rp.T = R;
-    rp.ids = moe_ids_; rp.w = moe_w_; rp.ticket = route_cnt_; rp.row_tok = d_desc_ + D_TOK; rp.row_pos = d_desc_ + D_POS; rp.row_slot = d_desc_ + D_SLOT; rp.synth_key = rkey;
+    MoeRouteParams rp; rp.W = L.router; rp.x = xn_ + (size_t)row0 * E; rp.logits = rlogits_; rp.E = c.n_expert; rp.K = E; rp.k = c.n_expert_used; rp.T = R;
+    rp.ids = moe_ids_ + (size_t)row0 * ns; rp.w = moe_w_ + (size_t)row0 * ns; rp.ticket = route_cnt_; rp.row_tok = tok + row0; rp.row_pos = pos + row0; rp.row_slot = slot + row0; rp.synth_key = rkey;
     rp.e_lo = e_lo_; rp.e_hi = e_hi_; rp.own_shared = own_sh; rp.segs = moe_segs_; rp.ctl = moe_ctl_; rp.touched = moe_touched_; rp.err = err_;
     HP_TRY(moe_route_group(rp, s_));
     // per-(row, slot) outputs of the experts this GPU owns, grouped by expert so that each touched expert matrix is read
@@ -426,18 +457,24 @@ int Engine::moe_block(const LayerW& L, int R) {
     if (c.ep_world > 1) { HP_TRY(ep_ready()); if (!ep_peer_) HP_CUDA(cudaMemsetAsync(moe_v_, 0, (size_t)R * ns * E * 4, s_)); }
     MoeGroupParams g; g.w_gate_up = L.exp_gate_up.wt; g.w_down = L.exp_down.wt; g.sh_gate_up = L.sh_gate_up.wt; g.sh_down = L.sh_down.wt;
     g.E = E; g.F = F; g.nslot = ns; g.T = R; g.e_lo = e_lo_;
-    g.xq = xq_; g.xq2 = xq2_; g.v = moe_v_; g.segs = moe_segs_; g.ctl = moe_ctl_; g.err = err_;
-    int pushed = 0;
+    g.xq = xq_rows(xq_, row0, E); g.xq2 = xq2_; g.v = moe_v_ + (size_t)row0 * ns * E; g.segs = moe_segs_; g.ctl = moe_ctl_; g.err = err_;
     if (ep_peer_) { g.ep_world = c.ep_world; g.ep_rank = c.ep_rank; g.ep_half = ep_half_; for (int q = 0; q < 8; ++q) { g.ep_x[q] = ep_peer_x_[q]; g.ep_ctl[q] = ep_peer_ctl_[q]; } }
-    HP_TRY(moe_experts_grouped(g, s_, &pushed));
-    if (c.ep_world > 1) HP_TRY(ep_peer_ ? ep_exchange_peer(R, lidx % c.ep_world, pushed != 0) : ep_exchange(moe_v_, (size_t)R * ns * E));
+    return moe_experts_grouped(g, s_, pushed);
+}
+int Engine::moe_block(const LayerW& L, int R) {
+    if (gemv_only_) return HP_OK;
+    if (pf_on_) return prefill_moe(L, R);
+    const hp_model_cfg& c = c_; const int lidx = &L == &mtp_ ? c.n_layer : (int)(&L - layers_.data());
+    int pushed = 0;
+    HP_TRY(moe_rows(L, R, 0, d_desc_ + D_TOK, d_desc_ + D_POS, d_desc_ + D_SLOT, &pushed));
+    if (c.ep_world > 1) HP_TRY(ep_peer_ ? ep_exchange_peer(R, lidx % c.ep_world, pushed != 0) : ep_exchange(moe_v_, (size_t)R * (c.n_expert_used + 1) * c.n_embd));
     return HP_OK;   // combined in slot order by the norm that follows (norm_in)
 }
 
 // qwen35.cpp:309-376
 int Engine::run_pass(int R, int nseq, int ngroups) {
     const hp_model_cfg& c = c_;
-    if (!gemv_only_) HP_TRY(embed_bf16(d_desc_ + D_TOK, embed_, x_, R, c.n_embd, c.n_vocab, s_));
+    if (!gemv_only_) HP_TRY(embed_bf16(pf_on_ ? pf_desc_ : d_desc_ + D_TOK, embed_, x_, R, c.n_embd, c.n_vocab, s_));
     const Lin* prev = nullptr; int gi = 0, ai = 0;
     for (int il = 0; il < c.n_layer; ++il) {
         const LayerW& L = layers_[il];
@@ -450,7 +487,13 @@ int Engine::run_pass(int R, int nseq, int ngroups) {
             g.conv_w = L.conv_w; g.dt_bias = L.dt_bias; g.a_neg = L.a_neg; g.norm_w = L.ssm_norm;
             g.state = gdn_state_ + (size_t)gi * st_layer_; g.conv_state = conv_state_ + (size_t)gi * cs_layer_; g.state_stride = st_stride_; g.conv_stride = cs_stride_;
             g.seq = d_desc_ + D_SEQS; g.replay_n = replay_n_; g.out = nullptr; g.xq = xq_; g.snap = nullptr; g.snap_row_stride = 0; g.eps = c.rms_eps; g.sigmoid_gate = c.gdn_sigmoid_gate;
-            if (!gemv_only_ && !(prof_skip_ & 1)) HP_TRY(gdn_forward(g, nseq, s_));
+            if (pf_on_) {
+                const size_t slot = pf_slot_;
+                GdnPrefillParams q; q.rows = big_; q.ld = ld_in_; q.off_z = g.off_z; q.off_b = g.off_b; q.off_a = g.off_a; q.n_qk = g.n_qk; q.n_v = g.n_v; q.T = R;
+                q.conv_w = g.conv_w; q.dt_bias = g.dt_bias; q.a_neg = g.a_neg; q.norm_w = g.norm_w; q.state = g.state + slot * st_stride_; q.conv_state = g.conv_state + slot * cs_stride_;
+                q.xq = xq_; q.eps = g.eps; q.sigmoid_gate = g.sigmoid_gate;
+                HP_TRY(gdn_prefill(q, pf_gdn_, s_));
+            } else if (!gemv_only_ && !(prof_skip_ & 1)) HP_TRY(gdn_forward(g, nseq, s_));
             HP_TRY(lin_parts(L.out_proj, R));
             ++gi;
         } else {
@@ -462,6 +505,7 @@ int Engine::run_pass(int R, int nseq, int ngroups) {
         prev = c.n_expert ? &moe_out_ : &L.down;
     }
     HP_TRY(norm_in(prev, true, output_norm_, h_, R));      // h for all rows (+ q8 of all rows), qwen35.cpp:370
+    if (pf_on_) return HP_OK;                              // the head of a prompt chunk: prefill_rows
     HP_TRY(lin(lm_head_, logits_, c.n_vocab, R));
     if (gemv_only_) return HP_OK;
     return argmax_rows(logits_, R, c.n_vocab, c.n_vocab, d_ids_, d_vals_, am_scratch_, s_);
@@ -555,7 +599,7 @@ int Engine::accept(int slot, int m) {
 // nothing else: the next draft takes its hidden row from the trunk)
 int Engine::run_mtp(int R, int ngroups, const float* h_dev, int ldh, bool want_logits, bool kv_only) {
     const hp_model_cfg& c = c_;
-    HP_TRY(embed_bf16(d_desc_ + D_TOK, embed_, emb_, R, c.n_embd, c.n_vocab, s_));
+    HP_TRY(embed_bf16(pf_on_ ? pf_desc_ : d_desc_ + D_TOK, embed_, emb_, R, c.n_embd, c.n_vocab, s_));
     HP_TRY(norm2_concat_quant(emb_, mtp_enorm_, h_dev, ldh, mtp_hnorm_, nullptr, xq_, R, c.n_embd, c.rms_eps, s_));
     HP_TRY(lin_parts(eh_proj_, R));   // x = eh_proj(...) : the norm kernel adds the K-part planes itself
     HP_TRY(add_rmsnorm_quant(x_, yparts_, eh_proj_.P, (size_t)R * eh_proj_.N, eh_proj_.N, mtp_.attn_norm, nullptr, xq_, R, c.n_embd, c.rms_eps, s_, true));
@@ -610,11 +654,6 @@ int Engine::topk(int which, int T, int k, int* ids, float* vals) {
     return HP_OK;
 }
 
-// Prompt ingestion for one slot (Qwen4Exp::prefill + mtp_catchup, qwen4exp.h:57-60,72-74; Backend::prefill,
-// front/serve.cpp:29): n tokens at positions pos0.., committed. This build runs them through the verify path in chunks
-// of 8 rows; with_mtp also runs the MTP block over the same rows, row p paired with the trunk's hidden row of position
-// p - 1 (zeros at position 0; the last row of the previous chunk / call otherwise), so that the draft block's KV cache
-// covers the prompt (spec27b.cpp:62-71). Afterwards row 0 of logits / h_nextn / the arg-max ids holds the LAST prompt row.
 // ---- expert-parallel exchange over peer memory -------------------------------------------------------------------------
 // After the down projection a rank holds the output rows of the (row, slot) pairs whose expert it owns. k_ep_push copies
 // them into the other ranks' exchange buffers (plain stores through the NVLink mapping), makes them visible system-wide
@@ -693,12 +732,117 @@ __global__ void k_prefill_last(float* __restrict__ logits, float* __restrict__ h
     for (int i = blockIdx.x * 256 + threadIdx.x; i < V; i += gridDim.x * 256) logits[i] = logits[(size_t)last * V + i];
     if (blockIdx.x == 0) { for (int i = threadIdx.x; i < E; i += 256) h[i] = h[(size_t)last * E + i]; if (threadIdx.x == 0) { ids[0] = ids[last]; vals[0] = vals[last]; } }
 }
+// exchanges the pass buffers with those of the prompt chunks for its lifetime
+struct Engine::PrefillScope {
+    Engine& e;
+    void swap() {
+        std::swap(e.x_, e.pf_.x); std::swap(e.xn_, e.pf_.xn); std::swap(e.big_, e.pf_.big); std::swap(e.yparts_, e.pf_.yparts); std::swap(e.emb_, e.pf_.emb); std::swap(e.h_, e.pf_.h);
+        std::swap(e.moe_v_, e.pf_.moe_v); std::swap(e.moe_w_, e.pf_.moe_w); std::swap(e.moe_ids_, e.pf_.moe_ids); std::swap(e.xq_, e.pf_.xq);
+    }
+    explicit PrefillScope(Engine& en) : e(en) { swap(); e.pf_on_ = true; }
+    ~PrefillScope() { swap(); e.pf_on_ = false; }
+};
+// descriptor of a chunk (ints, device + pinned host copy): token, position, slot, row group (within its batch) per row, then {r0, T, slot, pos0} per group
+int Engine::prefill_attn(const LayerW& L, uint16_t* kc, uint16_t* vc, size_t kv_stride, int R, bool kv_only) {
+    const int ld = L.in_proj.N, PR = pf_rows_;
+    AttnParams p; p.qkv = big_;
+    if (L.in_proj.P > 1) { HP_TRY(lin_parts(L.in_proj, R)); p.planes = yparts_; p.P = L.in_proj.P; p.part_stride = (size_t)R * ld; }
+    else HP_TRY(lin(L.in_proj, big_, ld, R));
+    p.ld = ld; p.n_head = c_.n_head; p.n_kv = c_.n_head_kv; p.n_rot = c_.n_rot; p.q_norm = L.q_norm; p.k_norm = L.k_norm; p.rope = rope_;
+    p.row_pos = pf_desc_ + PR; p.row_slot = pf_desc_ + 2 * PR; p.row_group = pf_desc_ + 3 * PR; p.groups = pf_desc_ + 4 * PR;
+    p.kc = kc; p.vc = vc; p.kv_stride = kv_stride; p.max_ctx = c_.max_ctx; p.pO = pO_; p.pm = pm_; p.pl = pl_; p.nsplit_max = pf_nsplit_;
+    p.out = nullptr; p.xq = xq_; p.eps = c_.rms_eps;
+    HP_TRY(attn_rope_kv(p, R, s_));
+    if (kv_only) return HP_OK;
+    for (const PfBatch& b : pf_batches_) {
+        AttnParams q = p; q.planes = nullptr;
+        q.qkv = big_ + (size_t)b.row0 * ld; q.row_pos += b.row0; q.row_slot += b.row0; q.row_group += b.row0; q.groups += 4 * b.g0; q.xq = xq_rows(xq_, b.row0, c_.n_head * 256);
+        HP_TRY(attn_decode(q, b.rows, b.ng, s_));
+    }
+    return lin_parts(L.out_proj, R);
+}
+// the routed experts of a chunk, MAXR rows at a time: the pairs of 32 rows share the expert matrices they touch
+int Engine::prefill_moe(const LayerW& L, int R) {
+    const int PR = pf_rows_;
+    for (int r0 = 0; r0 < R; r0 += MAXR) HP_TRY(moe_rows(L, std::min((int)MAXR, R - r0), r0, pf_desc_, pf_desc_ + PR, pf_desc_ + 2 * PR, nullptr));
+    return HP_OK;
+}
+// Rows [pos0, pos0 + R) of a slot through the trunk (and the K/V rows of the MTP block), committed. tail > 0: the last chunk
+// of a prompt; the head, the hidden rows and the whole MTP block of its last `tail` rows (R - tail a multiple of 8) end up where a
+// pass over just these rows leaves them.
+int Engine::prefill_rows(int slot, const int* tokens, int R, int pos0, int with_mtp, int tail) {
+    const hp_model_cfg& c = c_; const int E = c.n_embd, PR = pf_rows_, gr = attn_rows_per_group();
+    int* d = pf_hdesc_;
+    // attention batches: as many rows as the split partials of a MAXR-row pass over the whole context hold at this depth
+    pf_nsplit_ = (pos0 + R + ATTN_SPLIT - 1) / ATTN_SPLIT;
+    const int brows = std::max((int)MAXR, (int)((long long)MAXR * nsplit_max_ / pf_nsplit_) * gr & ~7);
+    pf_batches_.clear(); int g0 = 0;
+    for (int r0 = 0; r0 < R; r0 += brows) {
+        PfBatch b{r0, std::min(brows, R - r0), g0, 0};
+        for (int t0 = 0; t0 < b.rows; t0 += gr) {
+            const int tn = std::min(gr, b.rows - t0); int* g = d + 4 * PR + 4 * g0;
+            g[0] = t0; g[1] = tn; g[2] = slot; g[3] = pos0 + r0 + t0;
+            for (int t = t0; t < t0 + tn; ++t) d[3 * PR + r0 + t] = b.ng;
+            ++b.ng; ++g0;
+        }
+        pf_batches_.push_back(b);
+    }
+    for (int t = 0; t < R; ++t) { d[t] = tokens[t]; d[PR + t] = pos0 + t; d[2 * PR + t] = slot; }
+    HP_CUDA(cudaEventRecord(ev0_, s_));
+    HP_CUDA(cudaMemcpyAsync(pf_desc_, d, (size_t)PR * 8 * 4, cudaMemcpyHostToDevice, s_));
+    float* hp = hprev_ + (size_t)slot * E;
+    {
+        PrefillScope scope(*this);
+        pf_slot_ = slot;
+        HP_TRY(run_pass(R, 1, 0));
+        if (with_mtp) {
+            k_prefill_shift<<<R, 256, 0, s_>>>(h_, hp, pf_hin_, E, pos0 == 0 ? 1 : 0);
+            k_prefill_remember<<<1, 256, 0, s_>>>(h_, hp, R, E);
+            HP_CUDA(cudaGetLastError());
+        }
+        if (tail) {
+            const int r0 = R - tail;
+            HP_CUDA(cudaMemcpyAsync(pf_.h, h_ + (size_t)r0 * E, (size_t)tail * E * 4, cudaMemcpyDeviceToDevice, s_));   // pf_ holds the pass buffers in here
+            const XQ8F x = xq_rows(xq_, r0, E);
+            const Lin& l = lm_head_;
+            if (l.P == 1) HP_TRY(gemv_q4k_q8_parts(l.wt, x, logits_, l.N, l.K, tail, c.n_vocab, 0, err_, s_, pdl_, true));
+            else {
+                HP_TRY(gemv_q4k_q8_parts(l.wt, x, pf_.yparts, l.N, l.K, tail, l.N, (size_t)tail * l.N, err_, s_, pdl_, true));
+                HP_CUDA(launch_pdl<16>(k_reduce_planes, dim3((l.N + 255) / 256, tail), dim3(256), 0, s_, pf_.yparts, (size_t)tail * l.N, l.P, logits_, l.N, c.n_vocab));
+            }
+            HP_TRY(argmax_rows(logits_, tail, c.n_vocab, c.n_vocab, d_ids_, d_vals_, am_scratch_, s_));
+        }
+        if (with_mtp) HP_TRY(run_mtp(R, 0, pf_hin_, E, false, true));
+    }
+    HP_CUDA(cudaEventRecord(ev1_, s_));
+    if (tail && with_mtp) {   // its hidden rows (hp_mtp_h_dev): the whole block, the K/V rows come out the same again
+        const hp_slot_req r{slot, tokens + R - tail, tail, pos0 + R - tail};
+        HP_TRY(mtp_forward_reqs(&r, 1, pf_hin_ + (size_t)(R - tail) * E, false));
+    }
+    HP_TRY(sync_stream());
+    HP_CUDA(cudaEventElapsedTime(&last_ms_, ev0_, ev1_));
+    return check_device_status();
+}
+// Prompt ingestion for one slot (Qwen4Exp::prefill + mtp_catchup, qwen4exp.h:57-60,72-74; Backend::prefill,
+// front/serve.cpp:29): n tokens at positions pos0.., committed; with_mtp also runs the MTP block over the same rows, row p
+// paired with the trunk's hidden row of position p - 1 (zeros at position 0; the last row of the previous chunk / call
+// otherwise), so that the draft block's KV cache covers the prompt (spec27b.cpp:62-71). Afterwards row 0 of logits /
+// h_nextn / the arg-max ids holds the LAST prompt row.
+// More than 8 tokens run as chunks (prefill_rows): 301 tokens of the 27B shape took 251 ms as 38 verify passes of 8 rows,
+// each of which streams all weights, and 96.5 ms as one chunk.
 int Engine::prefill(int slot, const int* tokens, int n, int pos0, int with_mtp) {
     HP_REQUIRE(slot >= 0 && slot < c_.n_slots && tokens && n >= 1 && pos0 >= 0 && pos0 + n <= c_.max_ctx, "prefill: bad arguments (slot %d, n %d, pos0 %d)", slot, n, pos0);
     HP_REQUIRE(!with_mtp || c_.has_mtp, "model has no MTP block");
     const int E = c_.n_embd;
     int T = 0;
-    for (int p = 0; p < n; p += T) {
+    if (n > 8 && pf_rows_) {
+        // More than one 8-row pass: chunks of nearly equal size, a multiple of 8 rows except for the last
+        if (pend_[slot]) HP_TRY(flush_commits());   // the chunks start from the committed state
+        HP_CUDA(cudaMemsetAsync(replay_n_ + slot, 0, 4, s_)); pend_[slot] = 0; last_T_[slot] = 0;
+        const int nch = (n + pf_rows_ - 1) / pf_rows_, size = std::min(pf_rows_, ((n + nch - 1) / nch + 7) & ~7);
+        T = (n - 1) % 8 + 1;
+        for (int p = 0; p < n; p += size) { const int R = std::min(size, n - p); HP_TRY(prefill_rows(slot, tokens + p, R, pos0 + p, with_mtp, p + R == n ? T : 0)); }
+    } else for (int p = 0; p < n; p += T) {
         T = std::min(8, n - p);
         const hp_slot_req r{slot, tokens + p, T, pos0 + p};
         HP_TRY(forward(&r, 1, nullptr));

@@ -32,7 +32,7 @@ enum TensorKind { TK_ATTN_NORM = 0, TK_POST_NORM, TK_IN_PROJ, TK_OUT_PROJ, TK_GA
 
 class Engine {
 public:
-    static constexpr int MAXR = 32, MAXS = 8;
+    static constexpr int MAXR = 32, MAXS = 8, PF_MAXR = 512;   // rows of a pass, slots, rows of a prompt chunk
     explicit Engine(const hp_model_cfg& cfg);
     ~Engine();
     int init();                                              // allocate + generate weights; HP_* status
@@ -75,6 +75,11 @@ private:
     int ep_exchange(float* buf, size_t n);
     int ep_allreduce(float* buf, size_t n);
     int run_pass(int R, int nseq, int ngroups);              // trunk over the rows described by desc_ (already uploaded)
+    int prefill_rows(int slot, const int* tokens, int R, int pos0, int with_mtp, int tail);   // a prompt chunk through the GEMM path
+    int prefill_attn(const LayerW& L, uint16_t* kc, uint16_t* vc, size_t kv_stride, int R, bool kv_only);
+    int prefill_lin(const Lin& l, float* out, int ld, size_t part_stride, int R);
+    int prefill_moe(const LayerW& L, int R);
+    int moe_rows(const LayerW& L, int R, int row0, const int* tok, const int* pos, const int* slot, int* pushed);
     int run_mtp(int R, int ngroups, const float* h_dev, int ldh, bool want_logits, bool kv_only = false);
     int upload_desc();
     int enqueue_round(int S, int n);
@@ -115,6 +120,12 @@ private:
     int* d_specin_ = nullptr;                                     // the round's inputs: slot list, seeded substitutions
     float *hpend_ = nullptr, *hstage_ = nullptr, *hprev_ = nullptr;   // per-slot pending h rows; gathered MTP inputs; per-slot last prompt h (prefill catch-up)
     std::vector<int> spec_pos_, spec_on_;
+    // Prompt chunks of up to pf_rows_ rows: buffers of their own, exchanged with the pass buffers while a chunk runs (PrefillScope)
+    struct PassBuf { float *x = nullptr, *xn = nullptr, *big = nullptr, *yparts = nullptr, *emb = nullptr, *h = nullptr, *moe_v = nullptr, *moe_w = nullptr; int* moe_ids = nullptr; XQ8F xq{nullptr, nullptr}; } pf_;
+    struct PrefillScope;
+    struct PfBatch { int row0, rows, g0, ng; };                   // rows of a chunk that one attention launch takes
+    int pf_rows_ = 0, pf_slot_ = 0; bool pf_on_ = false; float *pf_gdn_ = nullptr, *pf_hin_ = nullptr; void* pf_pack_ = nullptr; int *pf_desc_ = nullptr, *pf_hdesc_ = nullptr;
+    std::vector<PfBatch> pf_batches_; int pf_nsplit_ = 0;
     void* topk_scratch_ = nullptr; int *d_topk_ids_ = nullptr; float* d_topk_vals_ = nullptr;
     uint16_t* prof_kv_ = nullptr;                                 // K/V rows saved around profile_pass
     // a round that carries collectives: the stretches between two exchanges as graphs, the exchanges enqueued by the host

@@ -1,0 +1,490 @@
+// Q4_K x int8 GEMM for prompt chunks (many rows) on the 5th-generation tensor cores: tcgen05.mma kind::i8 with the
+// accumulator in TMEM.
+//
+// The arithmetic is that of the verify GEMV (gemv_q4k.cu) operation by operation: the exact int32 dot of every 32-element
+// sub-block, then acc = fmaf((d*sc) * xd, (float)idot, acc); acc = fmaf(-(dmin*mn), xs, acc) in block order, with the
+// sums of a 16-row tile cut where the GEMV's partition cuts them (K parts, warp boundaries of the tile's CTA) and added
+// in the same order. A row therefore has the same bits whichever of the two kernels computed it.
+//
+// What bounds it: the fp32 update, 3 packed fp32 instructions per two outputs and sub-block: 16 register operand reads, 8
+// clocks per SM sub-partition with their shared-memory loads, 9.8 with the TMEM loads (the int -> float conversions run
+// beside them). The int8 mma.sync of the GEMV takes 14.7 clocks per 16x8x32 on this chip and does not overlap with the
+// fp32 pipe. Hence:
+//   * one CTA per SM, M = 128 weight rows (8 tiles of 16), N = 32..128 pass rows, one tcgen05.mma (K = 32) per sub-block,
+//     never accumulating: TMEM only hands the int32 dots over to the update, in slots of 2 or 4 sub-blocks;
+//   * 16 update warps (4 TMEM lane quadrants x 4 column ranges) read the dots with 16x256b loads, which leave a lane two
+//     rows x two adjacent columns per 16 lanes: one 16-byte read of the scales of the activations serves 4 rows. A step of a
+//     warp is 3 or 4 (column tile, sub-block) pairs whatever N is, all loads in front; four warps share a sub-partition and
+//     hide each other's waits;
+//   * 4 conversion warps split the nibbles into u8 (the high ones stay shifted by 4, the scale carries the exact 1/16) in
+//     the K-major, 64-byte-swizzled layout of the tensor core. Rows 2, 3, 6, 7 of a group store their high nibbles first, so
+//     that the 16 lanes of a store phase hit distinct banks;
+//   * the activations are brought into that layout once per call by k_tc_pack (a few microseconds), so that a half-block of
+//     a column range is one bulk copy (8-byte asynchronous copies by two warps took 2800 clocks per half-block);
+//   * one warp streams the weights (2304-byte tile chunks, ring of 4 blocks, primed before the dependency wait), one the
+//     activations, one thread issues the MMAs.
+// Registers: 768 threads x 80 at launch; the update warps take 96 (16 x 32 threads) from the conversion warps (56) and the
+// last four warps (40): 61440 in all.
+// Every wait is bounded and reports through the device status word.
+#include "hp_common.cuh"
+#include "kernels.h"
+
+namespace hp {
+namespace {
+
+constexpr int TC_EPI = 16, TC_CNV = 4, TC_THREADS = (TC_EPI + TC_CNV + 4) * 32, TC_RAWS = 4, TC_CNVS = 3;
+constexpr int TC_W_CNV = TC_EPI, TC_W_LD = TC_W_CNV + TC_CNV, TC_W_TMA = TC_W_LD + 1, TC_W_MMA = TC_W_TMA + 1;   // first warp of each role
+constexpr int TC_RAW_BYTES = 8 * 2304, TC_A_BYTES = 2 * 128 * 64;   // weights of one block; converted weights of half a block
+template <int NTC> struct TcGeom {
+    static constexpr int N = NTC * 8, GS = NTC <= 8 ? 4 : 2, SLOT = GS * N <= 128 ? 128 : 256, SLOTS = 512 / SLOT;   // GS sub-blocks per TMEM slot
+    static constexpr int BST = NTC <= 8 ? 6 : 3, SCS = NTC <= 8 ? 4 : 3, B_BYTES = 2 * N * 64;   // rings: half-blocks of activations, blocks of scales
+    static constexpr int PACK = 2 * B_BYTES + NTC * 512;                                         // packed activations of a block: two half-blocks, scales
+    static constexpr int SC_BYTES = 8 * 128 * 8 + NTC * 512;
+    static constexpr int OFF_A = TC_RAWS * TC_RAW_BYTES, OFF_B = OFF_A + TC_CNVS * TC_A_BYTES, OFF_SC = OFF_B + BST * B_BYTES, OFF_BAR = OFF_SC + SCS * SC_BYTES;
+    static constexpr int SMEM = OFF_BAR + 512 + 1024;   // + slack to align the ring to 1024 bytes
+};
+static_assert(TcGeom<16>::SMEM <= GEMV_SMEM_LIMIT && TcGeom<8>::SMEM <= GEMV_SMEM_LIMIT, "shared memory of the widest tiles");
+
+// Bounded wait that lets the hardware park the warp: up to 2^20 attempts of up to a microsecond
+__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, int* err) {
+    for (uint32_t it = 0; it < (1u << 20); ++it) {
+        uint32_t ok;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(bar), "r"(parity), "r"(1000u) : "memory");
+        if (ok) return true;
+    }
+    if (err) atomicExch(err, HP_ETIMEOUT);
+    return false;
+}
+// one lane of a converged warp; unlike lane == 0 the compiler knows that a single thread issues what follows
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {   // K-major operand, 64-byte swizzle: 8-row groups 512 bytes apart
+    return (uint64_t)((addr >> 4) & 0x3FFF) | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61);
+}
+__device__ __forceinline__ void tc_mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc) {   // D = A * B (no accumulation)
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, 0, 0;\ntcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}" ::"r"(d), "l"(a), "l"(b), "r"(idesc) : "memory");
+}
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void tc_reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void tc_reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;"); }
+__device__ __forceinline__ void tc_after_wait(uint32_t& v) { asm volatile("" : "+r"(v)); }   // orders the use of a loaded register behind tc_wait_ld
+// W column tiles of 8 for 16 TMEM lanes: v[4 i ..] = {row g: cols 2t, 2t+1; row g + 8: cols 2t, 2t+1} of tile i
+template <int W, int OFF = 0> __device__ __forceinline__ void tc_ld(uint32_t (&v)[W * 4], uint32_t addr) {
+    constexpr int o = OFF * 4;
+    if constexpr (W - OFF >= 4) {
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                     : "=r"(v[o]), "=r"(v[o + 1]), "=r"(v[o + 2]), "=r"(v[o + 3]), "=r"(v[o + 4]), "=r"(v[o + 5]), "=r"(v[o + 6]), "=r"(v[o + 7]), "=r"(v[o + 8]),
+                       "=r"(v[o + 9]), "=r"(v[o + 10]), "=r"(v[o + 11]), "=r"(v[o + 12]), "=r"(v[o + 13]), "=r"(v[o + 14]), "=r"(v[o + 15]) : "r"(addr + OFF * 8));
+        if constexpr (W - OFF > 4) tc_ld<W, OFF + 4>(v, addr);
+    } else if constexpr (W - OFF >= 2) {
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(v[o]), "=r"(v[o + 1]), "=r"(v[o + 2]), "=r"(v[o + 3]), "=r"(v[o + 4]), "=r"(v[o + 5]), "=r"(v[o + 6]), "=r"(v[o + 7]) : "r"(addr + OFF * 8));
+        if constexpr (W - OFF > 2) tc_ld<W, OFF + 2>(v, addr);
+    } else
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[o]), "=r"(v[o + 1]), "=r"(v[o + 2]), "=r"(v[o + 3]) : "r"(addr + OFF * 8));
+}
+
+struct TcArgs {
+    const uint8_t* W; const uint8_t* xp; float* y;   // xp: packed activations
+    int N, nb, P, R, ldy; size_t part_stride;
+    int G, ngrp, ncg;        // tiles of 16 rows per work item (8, or 4 with every second tile position empty), items along M, along the pass rows
+    int* err;
+};
+// Units of tile `tile` after which the GEMV's partition closes a partial sum: bit c of the result = after unit c (CB blocks) of the K part
+__device__ __forceinline__ uint64_t tc_cuts(int N, int nb, int P, int tile, int lane) {
+    const int tiles = (N + 15) / 16, gc = GEMV_NCTA / P, nbp = nb / P, C = nbp % 2 == 0 ? nbp / 2 : nbp;
+    const int cg = (int)(((long long)(tile + 1) * gc - 1) / tiles);
+    const int t0 = (int)((long long)cg * tiles / gc), t1 = (int)((long long)(cg + 1) * tiles / gc);
+    const int cu = (t1 - t0) * C, weff = cu < GEMV_WARPS ? cu : GEMV_WARPS;
+    uint64_t m = 0;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int c = lane + 32 * half, u = (tile - t0) * C + c + 1;
+        bool cut = false;
+        if (c < C) { const int w = (u * weff + cu - 1) / cu; cut = c == C - 1 || (w < weff && gemv_warp_start(cu, weff, w) == u); }
+        m |= (uint64_t)__ballot_sync(0xffffffffu, cut) << (32 * half);
+    }
+    return m;
+}
+
+// One step of an update warp: its W column tiles over GB sub-blocks (row scales 128 float2 apart, one 64-byte group of
+// activation scales per sub-block). H1: the quadrant's second tile exists.
+template <int W, int GB, bool H1>
+__device__ __forceinline__ void tc_update(float2 (&acc)[4][W], uint32_t ta, uint32_t sb_cols, const float4* xs, const float2* rs) {
+    uint32_t v0[GB][W * 4], v1[H1 ? GB : 1][W * 4];
+#pragma unroll
+    for (int b = 0; b < GB; ++b) {
+        tc_ld<W>(v0[b], ta + b * sb_cols);
+        if constexpr (H1) tc_ld<W>(v1[b], ta + b * sb_cols + (16u << 16));
+    }
+    float2 r[GB][H1 ? 4 : 2];
+#pragma unroll
+    for (int b = 0; b < GB; ++b)
+#pragma unroll
+        for (int i = 0; i < (H1 ? 4 : 2); ++i) r[b][i] = rs[b * 128 + 8 * i];
+    tc_wait_ld();
+#pragma unroll
+    for (int b = 0; b < GB; ++b)
+#pragma unroll
+        for (int i = 0; i < W * 4; ++i) { tc_after_wait(v0[b][i]); if constexpr (H1) tc_after_wait(v1[b][i]); }
+    auto upd = [&](float2& a, float2 sc, float4 xv, uint32_t i0, uint32_t i1) {
+        fma2(a, mul2(make_float2(sc.x, sc.x), make_float2(xv.x, xv.y)), make_float2(__int2float_rn((int)i0), __int2float_rn((int)i1)));
+        fma2(a, make_float2(sc.y, sc.y), make_float2(xv.z, xv.w));
+    };
+#pragma unroll
+    for (int b = 0; b < GB; ++b)
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+            const float4 x = xs[i * 32 + b * 4];
+            upd(acc[0][i], r[b][0], x, v0[b][4 * i], v0[b][4 * i + 1]);
+            upd(acc[1][i], r[b][1], x, v0[b][4 * i + 2], v0[b][4 * i + 3]);
+            if constexpr (H1) {
+                upd(acc[2][i], r[b][2], x, v1[b][4 * i], v1[b][4 * i + 1]);
+                upd(acc[3][i], r[b][3], x, v1[b][4 * i + 2], v1[b][4 * i + 3]);
+            }
+        }
+}
+
+template <int NTC>
+__global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
+    using Geo = TcGeom<NTC>;
+    constexpr int W = NTC / 4, GB = W == 1 ? 4 : W == 2 ? 2 : 1, GS = Geo::GS, SLOTS = Geo::SLOTS, BST = Geo::BST;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint32_t tmem_ptr;
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const uint32_t bars = smem_u32(smem + Geo::OFF_BAR);
+    const uint32_t raw_full = bars, raw_empty = bars + 64, a_full = bars + 128, a_empty = bars + 160, sc_full = bars + 192, sc_empty = bars + 224,
+                   tm_full = bars + 256, tm_empty = bars + 288, b_full = bars + 320, b_empty = bars + 384, fin = bars + 448;
+    pdl_launch_dependents();
+    if (tid == 0) {
+        for (int i = 0; i < TC_RAWS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, TC_CNV); }
+        for (int i = 0; i < TC_CNVS; ++i) { mbar_init(a_full + 8 * i, TC_CNV); mbar_init(a_empty + 8 * i, 1); }
+        for (int i = 0; i < Geo::SCS; ++i) { mbar_init(sc_full + 8 * i, TC_CNV + 1); mbar_init(sc_empty + 8 * i, TC_EPI); }
+        for (int i = 0; i < 4; ++i) { mbar_init(tm_full + 8 * i, 1); mbar_init(tm_empty + 8 * i, TC_EPI); }
+        for (int i = 0; i < BST; ++i) { mbar_init(b_full + 8 * i, 1); mbar_init(b_empty + 8 * i, 1); }
+        mbar_init(fin, 1);
+        fence_barrier_init();
+    }
+    if (warp == TC_W_MMA) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_ptr)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_ptr;
+    const int nb = a.nb, nbp = nb / a.P, tiles = (a.N + 15) / 16, G = a.G, items = a.ncg * a.ngrp * a.P;
+    // 8 bytes of lane (g, t) in a swizzled group of 8 rows x 64 bytes: first store (low half of the 64 elements, high half
+    // for odd row pairs); the other half is at sw ^ 32
+    const bool sel = (g >> 1) & 1;
+    const uint32_t sw = (uint32_t)(((((sel ? 2 : 0) + (t >> 1)) ^ ((g >> 1) & 3)) << 4) + (t & 1) * 8 + g * 64);
+
+    if (warp >= TC_W_LD) {
+        tc_reg_dec<40>();
+        if (warp == TC_W_TMA) {   // ---- weight stream: one 2304-byte chunk per tile and block
+            int k = 0; bool ok = true;
+            for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+                const int rest = it / a.ncg, grp = rest % a.ngrp, part = rest / a.ngrp, nt = min(G, tiles - grp * G);
+                const uint8_t* src = a.W + ((size_t)(grp * G) * nb + (size_t)part * nbp) * 2304;
+                for (int b = 0; b < nbp; ++b, ++k) {
+                    const int s = k % TC_RAWS;
+                    ok = tc_wait(raw_empty + 8 * s, ((k / TC_RAWS) & 1) ^ 1, a.err);
+                    if (!ok) break;
+                    if (tc_elect()) {
+                        mbar_expect_tx(raw_full + 8 * s, (uint32_t)nt * 2304u);
+                        const uint32_t d = smem_u32(smem + s * TC_RAW_BYTES);
+                        for (int i = 0; i < nt; ++i) bulk_g2s(d + i * 2304, src + ((size_t)i * nb + b) * 2304, 2304u, raw_full + 8 * s);
+                    }
+                    __syncwarp();
+                }
+            }
+            for (int i = k > TC_RAWS ? k - TC_RAWS : 0; i < k; ++i) tc_wait(raw_full + 8 * (i % TC_RAWS), (i / TC_RAWS) & 1, a.err);   // no copy outlives the CTA
+        } else if (warp == TC_W_MMA) {   // ---- MMA issue
+            const uint32_t idesc = (2u << 4) | (1u << 10) | ((uint32_t)(Geo::N / 8) << 17) | (8u << 24);   // s32 = u8 x s8, M = 128
+            int hb = 0, gr = 0; bool ok = true;
+            for (int it = blockIdx.x; it < items && ok; it += gridDim.x)
+                for (int h = 0; h < 2 * nbp && ok; ++h, ++hb) {
+                    const int as = hb % TC_CNVS, bs = hb % BST;
+                    ok = tc_wait(b_full + 8 * bs, (hb / BST) & 1, a.err) && tc_wait(a_full + 8 * as, (hb / TC_CNVS) & 1, a.err);
+                    const uint32_t abase = smem_u32(smem + Geo::OFF_A + as * TC_A_BYTES), bbase = smem_u32(smem + Geo::OFF_B + bs * Geo::B_BYTES);
+#pragma unroll
+                    for (int q = 0; q < 4 && ok; q += GS, ++gr) {
+                        const int slot = gr % SLOTS;
+                        ok = tc_wait(tm_empty + 8 * slot, ((gr / SLOTS) & 1) ^ 1, a.err);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (tc_elect()) {
+#pragma unroll
+                            for (int v = q; v < q + GS; ++v)
+                                tc_mma_i8(tmem + slot * Geo::SLOT + (v - q) * Geo::N, tc_desc(abase + (v >> 1) * 8192 + (v & 1) * 32),
+                                          tc_desc(bbase + (v >> 1) * (Geo::N * 64) + (v & 1) * 32), idesc);
+                            tc_commit(tm_full + 8 * slot);
+                            if (q + GS == 4) { tc_commit(a_empty + 8 * as); tc_commit(b_empty + 8 * bs); }
+                        }
+                        __syncwarp();
+                    }
+                }
+            if (tc_elect()) tc_commit(fin);
+            __syncwarp();
+            tc_wait(fin, 0, a.err);   // nothing in flight when the accumulator memory is given back
+        } else if (warp == TC_W_LD) {   // ---- activations and their scales
+            pdl_wait();
+            int hb = 0, k = 0; bool ok = true;
+            for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+                const int cg = it % a.ncg, part = it / a.ncg / a.ngrp;
+                const uint8_t* src = a.xp + ((size_t)cg * nb + (size_t)part * nbp) * Geo::PACK;
+                for (int b = 0; b < nbp && ok; ++b, ++k, src += Geo::PACK) {
+                    const int ss = k % Geo::SCS;
+                    ok = tc_wait(sc_empty + 8 * ss, ((k / Geo::SCS) & 1) ^ 1, a.err);
+                    if (!ok) break;
+                    if (tc_elect()) {
+                        mbar_expect_tx(sc_full + 8 * ss, NTC * 512);
+                        bulk_g2s(smem_u32(smem + Geo::OFF_SC + ss * Geo::SC_BYTES + 8192), src + 2 * Geo::B_BYTES, NTC * 512, sc_full + 8 * ss);
+                    }
+                    __syncwarp();
+                    for (int h = 0; h < 2 && ok; ++h, ++hb) {
+                        const int bs = hb % BST;
+                        ok = tc_wait(b_empty + 8 * bs, ((hb / BST) & 1) ^ 1, a.err);
+                        if (ok && tc_elect()) {
+                            mbar_expect_tx(b_full + 8 * bs, Geo::B_BYTES);
+                            bulk_g2s(smem_u32(smem + Geo::OFF_B + bs * Geo::B_BYTES), src + h * Geo::B_BYTES, Geo::B_BYTES, b_full + 8 * bs);
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+            // no copy outlives the CTA (the scales of a block are issued before its activations)
+            const int nh = ok ? hb : hb ? hb - 1 : 0;
+            for (int i = nh > BST ? nh - BST : 0; i < nh; ++i) tc_wait(b_full + 8 * (i % BST), (i / BST) & 1, a.err);
+            if (k) { const int i = k - 1; tc_wait(sc_full + 8 * (i % Geo::SCS), (i / Geo::SCS) & 1, a.err); }
+        }
+    } else if (warp >= TC_W_CNV) {   // ---- weights: row scales, nibbles -> u8
+        tc_reg_dec<56>();
+        const int cw = warp - TC_W_CNV, ct = cw * 32 + lane;
+        const uint32_t m_a = sel ? 0xF0F0F0F0u : 0x0F0F0F0Fu;   // nibbles of the first store; the second takes the others
+        int k = 0, hb = 0; bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+            const int grp = it / a.ncg % a.ngrp, nt = min(G, tiles - grp * G);
+            for (int b = 0; b < nbp && ok; ++b, ++k) {
+                const int s = k % TC_RAWS, ss = k % Geo::SCS;
+                const uint8_t* raw = smem + s * TC_RAW_BYTES;
+                ok = tc_wait(raw_full + 8 * s, (k / TC_RAWS) & 1, a.err);
+#pragma unroll 1
+                for (int h = 0; h < 2 && ok; ++h, ++hb) {
+                    const int as = hb % TC_CNVS;
+                    ok = tc_wait(a_empty + 8 * as, ((hb / TC_CNVS) & 1) ^ 1, a.err);
+                    if (!ok) break;
+                    uint8_t* A = smem + Geo::OFF_A + as * TC_A_BYTES;
+                    const uint8_t* rp = raw + 256 + 2 * h * 512 + lane * 16;
+                    uint4 w[4];   // unit u = cw + 4 i: tile u / 2, 64-element group u % 2 of the half-block
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) { const int u = cw + 4 * i; if ((u >> 1) < nt) w[i] = *reinterpret_cast<const uint4*>(rp + (u >> 1) * 2304 + (u & 1) * 512); }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int u = cw + 4 * i;
+                        if ((u >> 1) < nt) {
+                            uint8_t* d = A + (u & 1) * 8192 + (G == 8 ? (u >> 1) : (u & ~1)) * 1024;
+                            *reinterpret_cast<uint2*>(d + sw) = make_uint2(w[i].x & m_a, w[i].y & m_a);
+                            *reinterpret_cast<uint2*>(d + (sw ^ 32)) = make_uint2(w[i].x & ~m_a, w[i].y & ~m_a);
+                            *reinterpret_cast<uint2*>(d + 512 + sw) = make_uint2(w[i].z & m_a, w[i].w & m_a);
+                            *reinterpret_cast<uint2*>(d + 512 + (sw ^ 32)) = make_uint2(w[i].z & ~m_a, w[i].w & ~m_a);
+                        }
+                    }
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(a_full + 8 * as);
+                    if (h == 0) {   // scales of tile position ct / 16, row ct % 16: (d * sc, -(dmin * mn)) of the 8 sub-blocks
+                        ok = tc_wait(sc_empty + 8 * ss, ((k / Geo::SCS) & 1) ^ 1, a.err);
+                        if (!ok) break;
+                        const int pos = ct >> 4, ti = G == 8 ? pos : pos >> 1;
+                        if (ti < nt && (G == 8 || !(pos & 1))) {
+                            const RowScales rs = decode_scales(*reinterpret_cast<const uint4*>(raw + ti * 2304 + (ct & 15) * 16));
+                            float2* sp = reinterpret_cast<float2*>(smem + Geo::OFF_SC + ss * Geo::SC_BYTES) + ct;
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) { const float4 v = rs.get(q); sp[q * 128] = make_float2(v.x, v.z); }
+                        }
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(sc_full + 8 * ss);
+                    }
+                }
+                if (ok && lane == 0) mbar_arrive(raw_empty + 8 * s);
+            }
+        }
+    } else {   // ---- fp32 update: warp = (lane quadrant q, column quarter); half h of the quadrant holds one tile of 16 rows
+        tc_reg_inc<96>();
+        const int q = warp & 3, n0 = (warp >> 2) * W;
+        pdl_wait();
+        int k = 0, gr = 0; bool ok = true;
+        const int CB = nbp % 2 == 0 ? 2 : 1;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+            const int cg = it % a.ncg, rest = it / a.ncg, grp = rest % a.ngrp, part = rest / a.ngrp, tile0 = grp * G, tend = min(tiles, tile0 + G);
+            const int tl[2] = {tile0 + (G == 8 ? 2 * q : q), G == 8 ? tile0 + 2 * q + 1 : tiles};
+            const bool has0 = tl[0] < tend, has1 = tl[1] < tend;
+            const uint64_t cut[2] = {has0 ? tc_cuts(a.N, nb, a.P, tl[0], lane) : 0, has1 ? tc_cuts(a.N, nb, a.P, tl[1], lane) : 0};
+            float* y = a.y + (size_t)part * a.part_stride;
+            constexpr bool VREG = W <= 2;   // running sum of the closed pieces in registers, else in the output plane
+            float2 acc[4][W], sum[VREG ? 4 : 1][VREG ? W : 1];
+            bool first[2] = {true, true};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int w = 0; w < W; ++w) acc[i][w] = make_float2(0.f, 0.f);
+            for (int b = 0; b < nbp && ok; ++b, ++k) {
+                const int ss = k % Geo::SCS;
+                const uint8_t* scp = smem + Geo::OFF_SC + ss * Geo::SC_BYTES;
+                ok = tc_wait(sc_full + 8 * ss, (k / Geo::SCS) & 1, a.err);
+                if (!ok) break;
+                const float2* rsp = reinterpret_cast<const float2*>(scp) + q * 32 + g;
+                const float4* xsp = reinterpret_cast<const float4*>(scp + 8192) + n0 * 32 + t;
+#pragma unroll 1
+                for (int u = 0; u < 8 / GS && ok; ++u, ++gr) {
+                    const int slot = gr % SLOTS;
+                    ok = tc_wait(tm_full + 8 * slot, (gr / SLOTS) & 1, a.err);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (has0) {
+#pragma unroll 1
+                        for (int v = 0; v < GS; v += GB) {
+                            const int sb = u * GS + v;
+                            const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + slot * Geo::SLOT + v * Geo::N + n0 * 8;
+                            if (has1) tc_update<W, GB, true>(acc, ta, Geo::N, xsp + sb * 4, rsp + sb * 128);
+                            else tc_update<W, GB, false>(acc, ta, Geo::N, xsp + sb * 4, rsp + sb * 128);
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(tm_empty + 8 * slot);
+                }
+                if (!ok) break;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sc_empty + 8 * ss);
+                // partial sums that end with this block
+                if ((b + 1) % CB == 0) {
+                    const int c = (b + 1) / CB - 1;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (!((cut[h] >> c) & 1)) continue;
+                        const bool last = b + 1 == nbp;
+                        int ldy = a.ldy;
+                        asm volatile("" : "+r"(ldy));   // keeps the addresses of this rare path out of the registers of the loop
+                        float* yt = y + (size_t)((cg * NTC + n0) * 8 + 2 * t) * ldy + tl[h] * 16 + g;
+                        auto live = [&](int i, int w, int e) { return tl[h] * 16 + g + 8 * i < a.N && (cg * NTC + n0 + w) * 8 + 2 * t + e < a.R; };
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            float2 v[W];
+#pragma unroll
+                            for (int w = 0; w < W; ++w) { v[w] = acc[2 * h + i][w]; acc[2 * h + i][w] = make_float2(0.f, 0.f); }
+                            if (!first[h]) {
+                                float2 p[W];   // all loads in flight at once
+#pragma unroll
+                                for (int w = 0; w < W; ++w) {
+                                    if constexpr (VREG) p[w] = sum[2 * h + i][w];
+                                    else p[w] = make_float2(live(i, w, 0) ? yt[(size_t)(8 * w) * ldy + 8 * i] : 0.f, live(i, w, 1) ? yt[(size_t)(8 * w + 1) * ldy + 8 * i] : 0.f);
+                                }
+#pragma unroll
+                                for (int w = 0; w < W; ++w) { v[w].x = p[w].x + v[w].x; v[w].y = p[w].y + v[w].y; }
+                            }
+                            if constexpr (VREG) {
+#pragma unroll
+                                for (int w = 0; w < W; ++w) sum[2 * h + i][w] = v[w];
+                            }
+                            if (!VREG || last)
+#pragma unroll
+                                for (int w = 0; w < W; ++w) {
+                                    if (live(i, w, 0)) yt[(size_t)(8 * w) * ldy + 8 * i] = v[w].x;
+                                    if (live(i, w, 1)) yt[(size_t)(8 * w + 1) * ldy + 8 * i] = v[w].y;
+                                }
+                        }
+                        first[h] = false;
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == TC_W_MMA)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+// Activations in the order the GEMM copies them: per column range of NTC tiles and block two half-blocks (per 64-element
+// group the swizzled K-major tile of all columns), then the scales. Tiles beyond the rows are zero.
+template <int NTC>
+__global__ void __launch_bounds__(256) k_tc_pack(const uint4* __restrict__ xq, const float4* __restrict__ xsc, uint8_t* __restrict__ xp, int nb, int tiles8) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int blk = blockIdx.x, cg = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    uint8_t* d = xp + ((size_t)cg * nb + blk) * TcGeom<NTC>::PACK;
+    const uint32_t lo = (uint32_t)((((t >> 1) ^ ((g >> 1) & 3)) << 4) + (t & 1) * 8 + g * 64);   // the low sub-block's 8 bytes; the high one's: lo ^ 32
+#pragma unroll
+    for (int u = warp; u < NTC * 4; u += 8) {
+        const int n = u >> 2, jj = u & 3, nt = cg * NTC + n;
+        const uint4 v = nt < tiles8 ? xq[((size_t)nt * nb * 4 + (size_t)blk * 4 + jj) * 32 + lane] : make_uint4(0, 0, 0, 0);
+        uint8_t* p = d + (jj >> 1) * TcGeom<NTC>::B_BYTES + (jj & 1) * (NTC * 512) + n * 512;
+        *reinterpret_cast<uint2*>(p + lo) = make_uint2(v.x, v.y);
+        *reinterpret_cast<uint2*>(p + (lo ^ 32)) = make_uint2(v.z, v.w);
+    }
+    for (int n = warp; n < NTC; n += 8) {
+        const int nt = cg * NTC + n;
+        reinterpret_cast<float4*>(d + 2 * TcGeom<NTC>::B_BYTES)[n * 32 + lane] = nt < tiles8 ? xsc[((size_t)nt * nb + blk) * 32 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
+template <int NTC>
+int launch_tc(const TcArgs& a, const XQ8F& x, int grid, cudaStream_t s, bool pdl) {
+    constexpr int smem = TcGeom<NTC>::SMEM;
+    static bool attr[MAX_DEVICES] = {};   // per device: the opt-in belongs to the device's copy of the kernel
+    const int dev = current_device(); if (dev < 0) return HP_ECUDA;
+    if (!attr[dev]) { HP_CUDA(cudaFuncSetAttribute(k_gemm_q4k_tc<NTC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); attr[dev] = true; }
+    k_tc_pack<NTC><<<dim3(a.nb, a.ncg), 256, 0, s>>>((const uint4*)x.q, (const float4*)x.sc, (uint8_t*)a.xp, a.nb, (a.R + 7) / 8);
+    HP_CUDA(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    cudaLaunchAttribute at[1]; at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = pdl && !(pdl_off_mask(s) & 64) ? 1 : 0;
+    HP_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_q4k_tc<NTC>, a));
+    return HP_OK;
+}
+
+}  // namespace
+
+size_t gemm_pack_bytes(int R, int K) { return (size_t)((R + 7) / 8 + 15) * (size_t)(K / 256) * 2560; }
+int gemm_q4k_q8_parts(const void* Wt, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, void* pack, int* err, cudaStream_t s, bool pdl) {
+    HP_REQUIRE(K > 0 && K % 256 == 0, "gemm_q4k_q8: K=%d must be a positive multiple of 256", K);
+    HP_REQUIRE(N > 0 && R >= 1 && ldy >= N, "gemm_q4k_q8: bad shape N=%d R=%d ldy=%d", N, R, ldy);
+    HP_REQUIRE(pack && ((uintptr_t)pack & 15) == 0 && ((uintptr_t)Wt & 15) == 0, "gemm_q4k_q8: the pack buffer and the weights must be 16-byte aligned");
+    TcArgs a; a.W = (const uint8_t*)Wt; a.xp = (const uint8_t*)pack; a.y = yparts;
+    a.N = N; a.nb = K / 256; a.P = gemv_num_parts(N, a.nb); a.R = R; a.ldy = ldy; a.part_stride = part_stride; a.err = err;
+    HP_REQUIRE(a.P > 0, "gemm_q4k_q8: K=%d is too large for the K-part partition", K);
+    const int t8 = (R + 7) / 8, tiles = (N + 15) / 16;
+    // Cut of the rows into ncg column ranges of ntc tiles of 8, and of the weight tiles into items of G = 8 or 4 (the
+    // latter leaves every second tile position empty). The time of an item goes with ntc plus a constant for
+    // conversion and waiting; the cut with the least time over the rounds of the SMs is taken.
+    constexpr int TC_COST = 6;
+    int ntc = 0; long best = 0;
+    for (int c = 4; c <= 16; c += 4)
+        for (int G = 8; G >= 4; G -= 4) {
+            const int ncg = (t8 + c - 1) / c;
+            const long cost = ((long)ncg * a.P * ((tiles + G - 1) / G) + GEMV_NCTA - 1) / GEMV_NCTA * (G == 8 ? (c + TC_COST) * 3 : (c + TC_COST) * 2);
+            if (!ntc || cost < best) { best = cost; ntc = c; a.ncg = ncg; a.G = G; }
+        }
+    a.ngrp = (tiles + a.G - 1) / a.G;
+    const int items = a.ncg * a.ngrp * a.P, grid = items < GEMV_NCTA ? items : GEMV_NCTA;
+    switch (ntc) {
+        case 4: return launch_tc<4>(a, x, grid, s, pdl);
+        case 8: return launch_tc<8>(a, x, grid, s, pdl);
+        case 12: return launch_tc<12>(a, x, grid, s, pdl);
+        default: return launch_tc<16>(a, x, grid, s, pdl);
+    }
+}
+
+}  // namespace hp

@@ -52,6 +52,10 @@ int gemv_parts(int N, int K);
 // tiled = true: W is in the tile-major layout produced by gemv_repack_tiled (gemv_tiled_bytes(N, K) bytes)
 int gemv_q4k_q8_parts(const void* W, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, int* err, cudaStream_t s, bool pdl, bool tiled);
 size_t gemv_tiled_bytes(size_t N, int K);
+// gemm_q4k.cu: the same planes, bit for bit, for any number of rows, on tcgen05 (tile-major weights only). pack: scratch of
+// gemm_pack_bytes(R, K) bytes, 16-byte aligned
+int gemm_q4k_q8_parts(const void* Wt, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, void* pack, int* err, cudaStream_t s, bool pdl);
+size_t gemm_pack_bytes(int R, int K);
 // interleave_half = F > 0: src is a stack of [gate F rows | up F rows] matrices; gate and up rows of a feature share a tile
 int gemv_repack_tiled(const void* src, void* dst, size_t N, int K, cudaStream_t s, int interleave_half = 0);
 int gemv_q4k_q8(const void* W, const XQ8F& x, float* y, int N, int K, int R, int ldy, const GemvWorkspace& ws, cudaStream_t s, bool pdl);
@@ -82,6 +86,17 @@ struct GdnParams {
     float* out; XQ8F xq; float* snap; size_t snap_row_stride; float eps; int sigmoid_gate;
 };
 int gdn_forward(const GdnParams& p, int nseq, cudaStream_t s);
+
+// gdn_prefill.cu: T consecutive rows of one sequence, all of them committed to the stored state and conv history. rows,
+// state and conv_state point at the sequence's own; scratch: gdn_prefill_floats(T, ...) floats, 16-byte aligned
+struct GdnPrefillParams {
+    const float* rows; int ld, off_z, off_b, off_a, n_qk, n_v, T;
+    const float* conv_w; const void* dt_bias; const void* a_neg; const void* norm_w;
+    float* state; float* conv_state; XQ8F xq; float eps; int sigmoid_gate;
+    float *qk = nullptr, *v = nullptr, *o = nullptr, *gate = nullptr;   // set by gdn_prefill
+};
+size_t gdn_prefill_floats(int rows, int n_qk, int n_v);
+int gdn_prefill(GdnPrefillParams p, float* scratch, cudaStream_t s);
 
 // ---- attn.cu ----
 constexpr int ATTN_SPLIT = 128, ATTN_MAX_PAIRS = 48;   // keys per split; (row, q-head) pairs per kv head and row group

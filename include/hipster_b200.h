@@ -178,8 +178,9 @@ int hp_topk(hp_engine* e, int which, int T, int k, int* ids_host, float* vals_ho
 /* Prompt ingestion for one slot: n tokens at positions pos0.., committed (no accept needed). with_mtp != 0 also runs the
  * MTP block over the same rows so that its KV cache covers the prompt; successive calls for one prompt must follow each
  * other. Afterwards row 0 of hp_logits_dev / hp_h_nextn_dev (and hp_topk(0, 1, ...)) is the LAST prompt row.
- * Replaces Qwen4Exp::prefill + mtp_catchup (qwen4exp.h:57-60,72-74) and Backend::prefill (front/serve.cpp:29); this
- * build feeds the prompt through the verify path in chunks of 8 rows (the GEMM prefill path is not part of it). */
+ * Replaces Qwen4Exp::prefill + mtp_catchup (qwen4exp.h:57-60,72-74) and Backend::prefill (front/serve.cpp:29). More than
+ * 8 tokens run in chunks of up to 512 rows (GEMM projections, one recurrence per layer and chunk), with the same bits as
+ * passes of 8 rows; up to 8 tokens, and every prompt of an expert-parallel shard, run through the verify path. */
 int hp_prefill(hp_engine* e, int slot, const int* tokens_host, int n, int pos0, int with_mtp);
 const float* hp_logits_dev(const hp_engine* e);            /* qwen35.h:82 */
 const float* hp_h_nextn_dev(const hp_engine* e);           /* qwen35.h:83 */
