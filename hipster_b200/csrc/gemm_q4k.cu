@@ -12,10 +12,11 @@
 // fp32 pipe. Hence:
 //   * one CTA per SM, M = 128 weight rows (8 tiles of 16), N = 32..128 pass rows, one tcgen05.mma (K = 32) per sub-block,
 //     never accumulating: TMEM only hands the int32 dots over to the update, in slots of 2 or 4 sub-blocks;
-//   * 16 update warps (4 TMEM lane quadrants x 4 column ranges) read the dots with 16x256b loads, which leave a lane two
+//   * 8 update warps (4 TMEM lane quadrants x 2 column halves) read the dots with 16x256b loads, which leave a lane two
 //     rows x two adjacent columns per 16 lanes: one 16-byte read of the scales of the activations serves 4 rows. A step of a
-//     warp is 3 or 4 (column tile, sub-block) pairs whatever N is, all loads in front; four warps share a sub-partition and
-//     hide each other's waits;
+//     warp is 6 or 8 (column tile, sub-block) pairs whatever N is, all loads in front. (16 warps with steps of half the size
+//     hide more latency but execute the loads and addresses of a step twice, and these compete with the update for the
+//     register ports.)
 //   * 4 conversion warps split the nibbles into u8 (the high ones stay shifted by 4, the scale carries the exact 1/16) in
 //     the K-major, 64-byte-swizzled layout of the tensor core. Rows 2, 3, 6, 7 of a group store their high nibbles first, so
 //     that the 16 lanes of a store phase hit distinct banks;
@@ -23,8 +24,8 @@
 //     a column range is one bulk copy (8-byte asynchronous copies by two warps took 2800 clocks per half-block);
 //   * one warp streams the weights (2304-byte tile chunks, ring of 4 blocks, primed before the dependency wait), one the
 //     activations, one thread issues the MMAs.
-// Registers: 768 threads x 80 at launch; the update warps take 96 (16 x 32 threads) from the conversion warps (56) and the
-// last four warps (40): 61440 in all.
+// Registers: 512 threads x 128 at launch; the update warps take 184 (8 x 32 threads) from the conversion warps (72) and the
+// last four warps (56): 63488 in all.
 // Every wait is bounded and reports through the device status word.
 #include "hp_common.cuh"
 #include "kernels.h"
@@ -32,7 +33,7 @@
 namespace hp {
 namespace {
 
-constexpr int TC_EPI = 16, TC_CNV = 4, TC_THREADS = (TC_EPI + TC_CNV + 4) * 32, TC_RAWS = 4, TC_CNVS = 3;
+constexpr int TC_EPI = 8, TC_CNV = 4, TC_THREADS = (TC_EPI + TC_CNV + 4) * 32, TC_RAWS = 4, TC_CNVS = 3;
 constexpr int TC_W_CNV = TC_EPI, TC_W_LD = TC_W_CNV + TC_CNV, TC_W_TMA = TC_W_LD + 1, TC_W_MMA = TC_W_TMA + 1;   // first warp of each role
 constexpr int TC_RAW_BYTES = 8 * 2304, TC_A_BYTES = 2 * 128 * 64;   // weights of one block; converted weights of half a block
 template <int NTC> struct TcGeom {
@@ -156,7 +157,7 @@ __device__ __forceinline__ void tc_update(float2 (&acc)[4][W], uint32_t ta, uint
 template <int NTC>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
     using Geo = TcGeom<NTC>;
-    constexpr int W = NTC / 4, GB = W == 1 ? 4 : W == 2 ? 2 : 1, GS = Geo::GS, SLOTS = Geo::SLOTS, BST = Geo::BST;
+    constexpr int W = NTC / 2, GB = W == 2 ? 4 : W <= 4 ? 2 : 1, GS = Geo::GS, SLOTS = Geo::SLOTS, BST = Geo::BST;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint32_t tmem_ptr;
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
     const uint32_t sw = (uint32_t)(((((sel ? 2 : 0) + (t >> 1)) ^ ((g >> 1) & 3)) << 4) + (t & 1) * 8 + g * 64);
 
     if (warp >= TC_W_LD) {
-        tc_reg_dec<40>();
+        tc_reg_dec<56>();
         if (warp == TC_W_TMA) {   // ---- weight stream: one 2304-byte chunk per tile and block
             int k = 0; bool ok = true;
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
             if (k) { const int i = k - 1; tc_wait(sc_full + 8 * (i % Geo::SCS), (i / Geo::SCS) & 1, a.err); }
         }
     } else if (warp >= TC_W_CNV) {   // ---- weights: row scales, nibbles -> u8
-        tc_reg_dec<56>();
+        tc_reg_dec<72>();
         const int cw = warp - TC_W_CNV, ct = cw * 32 + lane;
         const uint32_t m_a = sel ? 0xF0F0F0F0u : 0x0F0F0F0Fu;   // nibbles of the first store; the second takes the others
         int k = 0, hb = 0; bool ok = true;
@@ -319,19 +320,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
                 if (ok && lane == 0) mbar_arrive(raw_empty + 8 * s);
             }
         }
-    } else {   // ---- fp32 update: warp = (lane quadrant q, column quarter); half h of the quadrant holds one tile of 16 rows
-        tc_reg_inc<96>();
+    } else {   // ---- fp32 update: warp = (lane quadrant q, column half); half h of the quadrant holds one tile of 16 rows
+        tc_reg_inc<184>();
         const int q = warp & 3, n0 = (warp >> 2) * W;
         pdl_wait();
         int k = 0, gr = 0; bool ok = true;
-        const int CB = nbp % 2 == 0 ? 2 : 1;
+        const int cb1 = nbp % 2 == 0 ? 1 : 0;   // blocks per unit of the GEMV's partition, less 1
         for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
             const int cg = it % a.ncg, rest = it / a.ncg, grp = rest % a.ngrp, part = rest / a.ngrp, tile0 = grp * G, tend = min(tiles, tile0 + G);
             const int tl[2] = {tile0 + (G == 8 ? 2 * q : q), G == 8 ? tile0 + 2 * q + 1 : tiles};
             const bool has0 = tl[0] < tend, has1 = tl[1] < tend;
             const uint64_t cut[2] = {has0 ? tc_cuts(a.N, nb, a.P, tl[0], lane) : 0, has1 ? tc_cuts(a.N, nb, a.P, tl[1], lane) : 0};
             float* y = a.y + (size_t)part * a.part_stride;
-            constexpr bool VREG = W <= 2;   // running sum of the closed pieces in registers, else in the output plane
+            constexpr bool VREG = W <= 4;   // running sum of the closed pieces in registers, else in the output plane
             float2 acc[4][W], sum[VREG ? 4 : 1][VREG ? W : 1];
             bool first[2] = {true, true};
 #pragma unroll
@@ -368,8 +369,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
                 __syncwarp();
                 if (lane == 0) mbar_arrive(sc_empty + 8 * ss);
                 // partial sums that end with this block
-                if ((b + 1) % CB == 0) {
-                    const int c = (b + 1) / CB - 1;
+                if ((b & cb1) == cb1) {
+                    const int c = b >> cb1;
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         if (!((cut[h] >> c) & 1)) continue;
@@ -467,22 +468,21 @@ int gemm_q4k_q8_parts(const void* Wt, const XQ8F& x, float* yparts, int N, int K
     HP_REQUIRE(a.P > 0, "gemm_q4k_q8: K=%d is too large for the K-part partition", K);
     const int t8 = (R + 7) / 8, tiles = (N + 15) / 16;
     // Cut of the rows into ncg column ranges of ntc tiles of 8, and of the weight tiles into items of G = 8 or 4 (the
-    // latter leaves every second tile position empty). The time of an item goes with ntc plus a constant for
-    // conversion and waiting; the cut with the least time over the rounds of the SMs is taken.
-    constexpr int TC_COST = 6;
+    // latter leaves every second tile position empty). An item of 20 blocks takes 53, 71 and 89 us at ntc = 8, 12 and 16:
+    // 4.5 us per tile and what 4 tiles would take; the cut with the least time over the rounds of the SMs is taken.
     int ntc = 0; long best = 0;
-    for (int c = 4; c <= 16; c += 4)
+    for (int c = 4; c <= 16; c += 2)
         for (int G = 8; G >= 4; G -= 4) {
             const int ncg = (t8 + c - 1) / c;
-            const long cost = ((long)ncg * a.P * ((tiles + G - 1) / G) + GEMV_NCTA - 1) / GEMV_NCTA * (G == 8 ? (c + TC_COST) * 3 : (c + TC_COST) * 2);
+            const long cost = ((long)ncg * a.P * ((tiles + G - 1) / G) + GEMV_NCTA - 1) / GEMV_NCTA * (G == 8 ? (c + 4) * 3 : (c + 4) * 2);
             if (!ntc || cost < best) { best = cost; ntc = c; a.ncg = ncg; a.G = G; }
         }
     a.ngrp = (tiles + a.G - 1) / a.G;
     const int items = a.ncg * a.ngrp * a.P, grid = items < GEMV_NCTA ? items : GEMV_NCTA;
     switch (ntc) {
-        case 4: return launch_tc<4>(a, x, grid, s, pdl);
-        case 8: return launch_tc<8>(a, x, grid, s, pdl);
-        case 12: return launch_tc<12>(a, x, grid, s, pdl);
+        case 4: return launch_tc<4>(a, x, grid, s, pdl);   case 6: return launch_tc<6>(a, x, grid, s, pdl);
+        case 8: return launch_tc<8>(a, x, grid, s, pdl);   case 10: return launch_tc<10>(a, x, grid, s, pdl);
+        case 12: return launch_tc<12>(a, x, grid, s, pdl); case 14: return launch_tc<14>(a, x, grid, s, pdl);
         default: return launch_tc<16>(a, x, grid, s, pdl);
     }
 }
