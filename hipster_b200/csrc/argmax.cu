@@ -38,7 +38,13 @@ __global__ void __launch_bounds__(256) k_argmax_part(const float* __restrict__ x
     const int r = blockIdx.y, c0 = blockIdx.x * AM_CHUNK, c1 = min(n, c0 + AM_CHUNK);
     const float* xr = x + (size_t)r * ld;
     float bv = -INFINITY; int bi = -1;
-    for (int i = c0 + threadIdx.x; i < c1; i += 256) { const float v = xr[i]; if (v > bv) { bv = v; bi = i; } }
+    // bound by latency (a block reads 32 KB once): all loads of a thread in flight before the first comparison
+    constexpr int NV = AM_CHUNK / 256;
+    float v[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) { const int i = c0 + threadIdx.x + 256 * k; v[k] = i < c1 ? xr[i] : -INFINITY; }
+#pragma unroll
+    for (int k = 0; k < NV; ++k) if (v[k] > bv) { bv = v[k]; bi = c0 + threadIdx.x + 256 * k; }   // -inf (absent, or an entry) never wins
     am_block_reduce(bv, bi, sv, si);
     if (threadIdx.x == 0) { pv[(size_t)r * gridDim.x + blockIdx.x] = bv; pi[(size_t)r * gridDim.x + blockIdx.x] = bi; }
 }
@@ -94,6 +100,8 @@ __global__ void __launch_bounds__(256) k_topk_final(const float* __restrict__ pv
 }
 // out[0] = mm (accepted drafts), out[1] = bonus token ids[mm]
 __global__ void k_accept(const int* __restrict__ ids, const int* __restrict__ drafts, int n_draft, int* __restrict__ out) {
+    pdl_launch_dependents();
+    pdl_wait();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         int mm = 0; while (mm < n_draft && ids[mm] == drafts[mm]) ++mm;
         out[0] = mm; out[1] = ids[mm];
@@ -163,8 +171,7 @@ int argmax_rows_static(const float* logits, int R, int n, int ld, int* ids, floa
 
 int accept_greedy(const int* ids, const int* drafts, int n_draft, int* out, cudaStream_t s) {
     HP_REQUIRE(n_draft >= 0 && n_draft <= 31, "accept_greedy: n_draft=%d out of range", n_draft);
-    k_accept<<<1, 32, 0, s>>>(ids, drafts, n_draft, out);
-    HP_CUDA(cudaGetLastError());
+    HP_CUDA(launch_pdl<1>(k_accept, dim3(1), dim3(32), 0, s, ids, drafts, n_draft, out));
     return HP_OK;
 }
 

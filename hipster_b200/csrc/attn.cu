@@ -244,6 +244,8 @@ __global__ void __launch_bounds__(256) k_attn_merge(const float* __restrict__ qk
 
 // descriptors of one sequence of R consecutive rows at pos0.. (slot 0), cut into row groups of gr rows
 __global__ void k_attn_desc(int* __restrict__ d, int R, int pos0, int gr) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = threadIdx.x; if (t >= R) return;
     d[t] = pos0 + t; d[32 + t] = 0; d[64 + t] = t / gr;
     if (t % gr == 0) { int* g = d + 96 + 4 * (t / gr); g[0] = t; g[1] = min(gr, R - t); g[2] = 0; g[3] = pos0 + t; }
@@ -295,8 +297,7 @@ int attn_decode_seq(float* qkv, int ld, int R, int pos0, int n_head, int n_kv, i
     HP_REQUIRE(n_kv >= 1 && n_head % n_kv == 0 && n_head / n_kv <= ATTN_MAX_PAIRS && ld >= n_head * 512 + 2 * n_kv * HD, "attn_decode_seq: bad head geometry");
     const int gr = std::max(1, std::min(8, ATTN_MAX_PAIRS / (n_head / n_kv))), ng = attn_seq_groups(R, n_head, n_kv);
     int* d = (int*)workspace;
-    k_attn_desc<<<1, 32, 0, s>>>(d, R, pos0, gr);
-    HP_CUDA(cudaGetLastError());
+    HP_CUDA(launch_pdl<4>(k_attn_desc, dim3(1), dim3(32), 0, s, d, R, pos0, gr));
     AttnParams p; p.qkv = qkv; p.ld = ld; p.n_head = n_head; p.n_kv = n_kv; p.n_rot = n_rot; p.q_norm = q_norm; p.k_norm = k_norm; p.rope = rope;
     p.row_pos = d; p.row_slot = d + 32; p.row_group = d + 64; p.groups = d + 96;
     p.kc = kc; p.vc = vc; p.kv_stride = 0; p.max_ctx = max_ctx; p.nsplit_max = (max_ctx + ATTN_SPLIT - 1) / ATTN_SPLIT;

@@ -407,6 +407,8 @@ __global__ void __launch_bounds__(256) k_repack_tiled(const uint8_t* __restrict_
 
 // sum the K-part planes in part order: y[r][n] = ((p0 + p1) + p2) + p3
 __global__ void k_reduce_parts(const float* __restrict__ parts, size_t part_stride, int P, float* __restrict__ y, int N, int R, int ldp, int ldy) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int n = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
     if (n >= N || r >= R) return;
     float v = parts[(size_t)r * ldp + n];
@@ -464,8 +466,7 @@ int gemv_q4k_q8(const void* W, const XQ8F& x, float* y, int N, int K, int R, int
     const size_t stride = (size_t)R * N;
     const int rc = gemv_q4k_q8_parts(W, x, ws.part, N, K, R, N, stride, ws.err, s, pdl, false);
     if (rc != HP_OK) return rc;
-    k_reduce_parts<<<dim3((N + 255) / 256, R), 256, 0, s>>>(ws.part, stride, P, y, N, R, N, ldy);
-    HP_CUDA(cudaGetLastError());
+    HP_CUDA(launch_pdl<16>(k_reduce_parts, dim3((N + 255) / 256, R), dim3(256), 0, s, ws.part, stride, P, y, N, R, N, ldy));
     return HP_OK;
 }
 

@@ -9,6 +9,8 @@ namespace {
 
 // warp per 32-element sub-block; grid (ceil(K/32/8), R)
 __global__ void __launch_bounds__(256) k_quantize_x_q8(const float* __restrict__ x, int ldx, int8_t* __restrict__ q, float* __restrict__ sc, int K) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int r = blockIdx.y, sb = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (sb * 32 >= K) return;
     warp_quant32_store(x[(size_t)r * ldx + sb * 32 + lane], r, sb, K, q, sc, lane);
@@ -40,8 +42,7 @@ __global__ void __launch_bounds__(256) k_dequant_q4k(const uint8_t* __restrict__
 int quantize_x_q8(const float* x, int ldx, XQ8F out, int R, int K, cudaStream_t s) {
     HP_REQUIRE(K > 0 && K % 64 == 0 && R >= 1 && ldx >= K, "quantize_x_q8: bad shape R=%d K=%d ldx=%d", R, K, ldx);
     dim3 grid((K / 32 + 7) / 8, R);
-    k_quantize_x_q8<<<grid, 256, 0, s>>>(x, ldx, (int8_t*)out.q, (float*)out.sc, K);
-    HP_CUDA(cudaGetLastError());
+    HP_CUDA(launch_pdl<16>(k_quantize_x_q8, grid, dim3(256), 0, s, x, ldx, (int8_t*)out.q, (float*)out.sc, K));
     return HP_OK;
 }
 int xq8_unpack(XQ8F in, int R, int K, int8_t* q, float* d, float* sm, cudaStream_t s) {
