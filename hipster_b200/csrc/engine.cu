@@ -383,8 +383,9 @@ static int lin_class_bit(const Lin& l, const hp_model_cfg& c) {
     return l.N == 2 * c.n_ff ? 16 : l.K == c.n_ff ? 32 : l.N == c.n_vocab ? 64 : l.K == c.n_embd ? 128 : 256;
 }
 // A linear over the rows of a prompt chunk; both kernels give the same bits. Up to 32 rows are one pass of the GEMV over the
-// weights and it is the faster one (gate|up of 27B, 32 rows: 88 against 90 us; its down projection 52 against 76), at 64
-// rows its two passes take 183 and 103 us against the GEMM's 140 and 112.
+// weights; beyond that it streams them again. GEMV against GEMM of the 27B layer's in-, out-projection, gate|up and down (us):
+// 32 rows 42 + 20 + 87 + 52 = 199 against 43 + 31 + 76 + 66 = 217; 48 rows 62 + 33 + 127 + 74 = 296 against
+// 52 + 37 + 94 + 80 = 264.
 int Engine::prefill_lin(const Lin& l, float* out, int ld, size_t part_stride, int R) {
     if (R <= 32) return gemv_q4k_q8_parts(l.wt, xq_, out, l.N, l.K, R, ld, part_stride, err_, s_, pdl_, true);
     return gemm_q4k_q8_parts(l.wt, xq_, out, l.N, l.K, R, ld, part_stride, pf_pack_, err_, s_, pdl_);
@@ -829,7 +830,7 @@ int Engine::prefill_rows(int slot, const int* tokens, int R, int pos0, int with_
 // otherwise), so that the draft block's KV cache covers the prompt (spec27b.cpp:62-71). Afterwards row 0 of logits /
 // h_nextn / the arg-max ids holds the LAST prompt row.
 // More than 8 tokens run as chunks (prefill_rows): 301 tokens of the 27B shape took 251 ms as 38 verify passes of 8 rows,
-// each of which streams all weights, and 96.5 ms as one chunk.
+// each of which streams all weights, and take 86 ms as one chunk.
 int Engine::prefill(int slot, const int* tokens, int n, int pos0, int with_mtp) {
     HP_REQUIRE(slot >= 0 && slot < c_.n_slots && tokens && n >= 1 && pos0 >= 0 && pos0 + n <= c_.max_ctx, "prefill: bad arguments (slot %d, n %d, pos0 %d)", slot, n, pos0);
     HP_REQUIRE(!with_mtp || c_.has_mtp, "model has no MTP block");
