@@ -7,14 +7,14 @@
 // in the same order. A row therefore has the same bits whichever of the two kernels computed it.
 //
 // What bounds it: the fp32 update, 3 packed fp32 instructions per two outputs and sub-block: 16 register operand reads, 8
-// clocks per SM sub-partition with their shared-memory loads, 9.8 with the TMEM loads (the int -> float conversions run
+// clocks per SM sub-partition with their shared-memory loads, 10.4 with the TMEM loads (the int -> float conversions run
 // beside them). The int8 mma.sync of the GEMV takes 14.7 clocks per 16x8x32 on this chip and does not overlap with the
 // fp32 pipe. Hence:
 //   * one CTA per SM, M = 128 weight rows (8 tiles of 16), N = 32..128 pass rows, one tcgen05.mma (K = 32) per sub-block,
 //     never accumulating: TMEM only hands the int32 dots over to the update, in slots of 2 or 4 sub-blocks;
 //   * 8 update warps (4 TMEM lane quadrants x 2 column halves) read the dots with 16x256b loads, which leave a lane two
 //     rows x two adjacent columns per 16 lanes: one 16-byte read of the scales of the activations serves 4 rows. A step of a
-//     warp is 6 or 8 (column tile, sub-block) pairs whatever N is, all loads in front. (16 warps with steps of half the size
+//     warp is 5 to 8 (column tile, sub-block) pairs whatever N is, all loads in front. (16 warps with steps of half the size
 //     hide more latency but execute the loads and addresses of a step twice, and these compete with the update for the
 //     register ports.)
 //   * 4 conversion warps split the nibbles into u8 (the high ones stay shifted by 4, the scale carries the exact 1/16) in
