@@ -46,7 +46,7 @@ template <int CB, bool TILED> struct SkGeom {
 template <int NT, int CB, bool TILED, bool XG = false>
 __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __restrict__ W, const uint4* __restrict__ xq, const float4* __restrict__ xsc,
                                                                 float* __restrict__ y, int N, int nb, int P, int R, int ldy, size_t part_stride,
-                                                                int* __restrict__ err) {
+                                                                int* __restrict__ err, int late) {
     using Geo = SkGeom<CB, TILED>;
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* ring_all = smem;
@@ -99,7 +99,10 @@ __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __
             if (it_chunk == C) { it_chunk = 0; ++it_tile; it_src += (size_t)16 * row_bytes - (size_t)C * unit_bytes; }
         }
     };
-    // the weight stream does not depend on the previous kernel: prime the ring before waiting for it
+    // Constant weights do not depend on the previous kernel: prime the ring before waiting for it. Weights that a kernel
+    // earlier in the stream may have written (late) are complete and visible only behind the wait, whoever triggered the
+    // early launch of this one.
+    if (late) pdl_wait();
     for (int i = 0; i < SK_STAGES && i < nunits; ++i) issue();
 
     pdl_wait();
@@ -363,7 +366,7 @@ __global__ void __launch_bounds__(F32_THREADS) k_gemv_q4k_f32(const uint8_t* __r
 
 template <int NT, int CB, bool TILED, bool XG = false>
 int launch_sk2(const uint8_t* W, const void* xq, const void* xsc, float* y, int N, int nb, int P, int R, int ldy, size_t part_stride,
-               int* err, cudaStream_t s, bool pdl) {
+               int* err, cudaStream_t s, bool pdl, bool late) {
     const size_t smem = SkGeom<CB, TILED>::FIXED + (XG ? 0 : (size_t)NT * (nb / P) * 2560);
     static size_t attr_smem[MAX_DEVICES] = {};   // per device: the opt-in belongs to the device's copy of the kernel
     const int dev = current_device(); if (dev < 0) return HP_ECUDA;
@@ -372,17 +375,17 @@ int launch_sk2(const uint8_t* W, const void* xq, const void* xsc, float* y, int 
     cfg.gridDim = dim3(GEMV_NCTA); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = s;
     cudaLaunchAttribute at[1]; at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = pdl && !(pdl_off_mask(s) & 64) ? 1 : 0;
-    HP_CUDA(cudaLaunchKernelEx(&cfg, k_gemv_q4k_sk<NT, CB, TILED, XG>, W, (const uint4*)xq, (const float4*)xsc, y, N, nb, P, R, ldy, part_stride, err));
+    HP_CUDA(cudaLaunchKernelEx(&cfg, k_gemv_q4k_sk<NT, CB, TILED, XG>, W, (const uint4*)xq, (const float4*)xsc, y, N, nb, P, R, ldy, part_stride, err, late ? 1 : 0));
     return HP_OK;
 }
 template <int NT, bool XG = false>
 int launch_sk(const uint8_t* W, bool tiled, const void* xq, const void* xsc, float* y, int N, int nb, int P, int R, int ldy, size_t part_stride,
-              int* err, cudaStream_t s, bool pdl) {
+              int* err, cudaStream_t s, bool pdl, bool late) {
     const bool cb2 = (nb / P) % 2 == 0;
-    if (tiled) return cb2 ? launch_sk2<NT, 2, true, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl)
-                          : launch_sk2<NT, 1, true, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl);
-    return cb2 ? launch_sk2<NT, 2, false, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl)
-               : launch_sk2<NT, 1, false, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl);
+    if (tiled) return cb2 ? launch_sk2<NT, 2, true, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late)
+                          : launch_sk2<NT, 1, true, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late);
+    return cb2 ? launch_sk2<NT, 2, false, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late)
+               : launch_sk2<NT, 1, false, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late);
 }
 
 // row-major ggml blocks -> tile-major chunks (see SkGeom); rows beyond N are zero (they contribute nothing).
@@ -428,7 +431,7 @@ int gemv_repack_tiled(const void* src, void* dst, size_t N, int K, cudaStream_t 
     HP_CUDA(cudaGetLastError()); return HP_OK;
 }
 
-int gemv_q4k_q8_parts(const void* W, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, int* err, cudaStream_t s, bool pdl, bool tiled) {
+int gemv_q4k_q8_parts(const void* W, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, int* err, cudaStream_t s, bool pdl, bool tiled, bool late) {
     HP_REQUIRE(K > 0 && K % 256 == 0, "gemv_q4k_q8: K=%d must be a positive multiple of 256", K);
     HP_REQUIRE(N > 0 && R >= 1 && R <= 32 && ldy >= N, "gemv_q4k_q8: bad shape N=%d R=%d ldy=%d", N, R, ldy);
     const int nb = K / 256, P = gemv_num_parts(N, nb);
@@ -442,29 +445,29 @@ int gemv_q4k_q8_parts(const void* W, const XQ8F& x, float* yparts, int N, int K,
     int rc;
     if (staged) {
         switch (ntile) {
-            case 1: rc = launch_sk<1>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl); break;
-            case 2: rc = launch_sk<2>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl); break;
-            case 3: rc = launch_sk<3>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl); break;
-            default: rc = launch_sk<4>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl); break;
+            case 1: rc = launch_sk<1>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl, late); break;
+            case 2: rc = launch_sk<2>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl, late); break;
+            case 3: rc = launch_sk<3>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl, late); break;
+            default: rc = launch_sk<4>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl, late); break;
         }
     } else {
         switch (ntile) {
-            case 2: rc = launch_sk<2, true>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl); break;
-            case 3: rc = launch_sk<3, true>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl); break;
-            default: rc = launch_sk<4, true>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl); break;
+            case 2: rc = launch_sk<2, true>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl, late); break;
+            case 3: rc = launch_sk<3, true>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl, late); break;
+            default: rc = launch_sk<4, true>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl, late); break;
         }
     }
     if (rc != HP_OK) return rc;
     return HP_OK;
 }
 
-int gemv_q4k_q8(const void* W, const XQ8F& x, float* y, int N, int K, int R, int ldy, const GemvWorkspace& ws, cudaStream_t s, bool pdl) {
+int gemv_q4k_q8(const void* W, const XQ8F& x, float* y, int N, int K, int R, int ldy, const GemvWorkspace& ws, cudaStream_t s, bool pdl, bool late) {
     HP_REQUIRE(K > 0 && K % 256 == 0 && N > 0, "gemv_q4k_q8: bad shape N=%d K=%d", N, K);
     const int P = gemv_num_parts(N, K / 256);
-    if (P == 1) return gemv_q4k_q8_parts(W, x, y, N, K, R, ldy, 0, ws.err, s, pdl, false);
+    if (P == 1) return gemv_q4k_q8_parts(W, x, y, N, K, R, ldy, 0, ws.err, s, pdl, false, late);
     HP_REQUIRE(ws.part && (size_t)P * R * N * sizeof(float) <= ws.part_bytes, "gemv_q4k_q8: workspace too small for %d K-part planes of %d x %d", P, R, N);
     const size_t stride = (size_t)R * N;
-    const int rc = gemv_q4k_q8_parts(W, x, ws.part, N, K, R, N, stride, ws.err, s, pdl, false);
+    const int rc = gemv_q4k_q8_parts(W, x, ws.part, N, K, R, N, stride, ws.err, s, pdl, false, late);
     if (rc != HP_OK) return rc;
     HP_CUDA(launch_pdl<16>(k_reduce_parts, dim3((N + 255) / 256, R), dim3(256), 0, s, ws.part, stride, P, y, N, R, N, ldy));
     return HP_OK;

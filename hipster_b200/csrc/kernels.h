@@ -50,7 +50,8 @@ struct GemvWorkspace { float* part; size_t part_bytes; int* err; };
 int gemv_parts(int N, int K);
 // raw form: part p of the K split writes plane yparts + p * part_stride ([R][ldy] each); the caller adds the planes in order
 // tiled = true: W is in the tile-major layout produced by gemv_repack_tiled (gemv_tiled_bytes(N, K) bytes)
-int gemv_q4k_q8_parts(const void* W, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, int* err, cudaStream_t s, bool pdl, bool tiled);
+// late = true: W is not constant, a kernel earlier in the stream may have written it (it is read behind the dependency wait only)
+int gemv_q4k_q8_parts(const void* W, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, int* err, cudaStream_t s, bool pdl, bool tiled, bool late = false);
 size_t gemv_tiled_bytes(size_t N, int K);
 // gemm_q4k.cu: the same planes, bit for bit, for any number of rows, on tcgen05 (tile-major weights only). pack: scratch of
 // gemm_pack_bytes(R, K) bytes, 16-byte aligned
@@ -58,7 +59,7 @@ int gemm_q4k_q8_parts(const void* Wt, const XQ8F& x, float* yparts, int N, int K
 size_t gemm_pack_bytes(int R, int K);
 // interleave_half = F > 0: src is a stack of [gate F rows | up F rows] matrices; gate and up rows of a feature share a tile
 int gemv_repack_tiled(const void* src, void* dst, size_t N, int K, cudaStream_t s, int interleave_half = 0);
-int gemv_q4k_q8(const void* W, const XQ8F& x, float* y, int N, int K, int R, int ldy, const GemvWorkspace& ws, cudaStream_t s, bool pdl);
+int gemv_q4k_q8(const void* W, const XQ8F& x, float* y, int N, int K, int R, int ldy, const GemvWorkspace& ws, cudaStream_t s, bool pdl, bool late);
 int gemv_q4k_f32(const void* W, const float* x, float* y, int N, int K, int R, int* err, cudaStream_t s);
 
 // ---- quant_ops.cu ----

@@ -128,3 +128,80 @@ def test_all_zero_and_tiny_activations():
     y = K_.gemv_q4k_q8(dev(W), xq, N, K).cpu().numpy()
     assert np.array_equal(bits(y), bits(orc.gemv_q4k_q8(W, oq, od, os_, N, K)))
     assert not y[1].any() and np.isfinite(y).all()
+
+
+# Weights written by a kernel right in front of the call: plain (a torch kernel), by a kernel of this library that triggers
+# early launches in its first instruction (its output taken as the next weights), and inside a captured graph.
+@pytest.mark.parametrize("N,K", [(4096, 5120), (4999, 512), (16, 256)])   # 4, 2 and 1 K parts; a ragged last tile
+def test_gemv_q8_weights_written_on_the_stream_right_before(N, K):
+    R = 3
+    Ws = [synth.q4k_matrix(N, K, seed=s) for s in (1, 2)]; x = synth.activations(R, K, seed=5)
+    q, d, s = orc.quantize_x_q8(x)
+    want = [bits(orc.gemv_q4k_q8(w, q, d, s, N, K)) for w in Ws]
+    key = dev(Ws[0].reshape(-1) ^ Ws[1].reshape(-1)); W = dev(Ws[1].reshape(-1)); xd = dev(x); xq = K_.XQ8(R, K)
+    ys = []
+    for _ in range(40):
+        W.bitwise_xor_(key)                              # the other matrix, written by a kernel
+        K_.quantize_x_q8(xd, xq)
+        ys.append(K_.gemv_q4k_q8(W, xq, N, K))
+    W.bitwise_xor_(key)
+    ys.append(K_.gemv_q4k_q8(W, xq, N, K))               # the writer is the kernel directly in front
+    for i, y in enumerate(ys):
+        assert np.array_equal(bits(y.cpu().numpy()), want[i % 2]), i
+    K_.device_status()
+
+
+def test_gemv_q8_weights_written_by_an_early_triggering_kernel():
+    xa, Wa = dev(synth.activations(32, 5120, seed=1)), [dev(synth.q4k_matrix(1152, 5120, seed=s)) for s in (2, 3)]
+    xb = K_.quantize_x_q8(dev(synth.activations(2, 256, seed=4))); qa, qb = K_.quantize_x_q8(xa), K_.XQ8(2, 256)
+    src = dev(synth.activations(2, 256, seed=4))
+    w = torch.empty((32, 1152), device="cuda")           # [1024] rows of one block: any bytes are a matrix
+    got = []
+    for i in range(20):
+        K_.gemv_q4k_q8(Wa[i % 2], qa, 1152, 5120, w)
+        K_.quantize_x_q8(src, qb)
+        got.append(K_.gemv_q4k_q8(w.view(torch.uint8), qb, 1024, 256))
+    for i in range(2):
+        K_.gemv_q4k_q8(Wa[i], qa, 1152, 5120, w)
+        torch.cuda.synchronize()
+        want = K_.gemv_q4k_q8(w.view(torch.uint8), xb, 1024, 256).view(torch.int32)
+        for y in got[i::2]:
+            assert torch.equal(y.view(torch.int32), want)
+
+
+@pytest.mark.parametrize("N,K", [(4096, 5120), (4999, 512)])
+def test_gemv_chain_captured_behind_copies_kernels_and_joins(N, K):
+    R = 3
+    Ws = [synth.q4k_matrix(N, K, seed=s) for s in (1, 2)]; x = synth.activations(R, K, seed=5)
+    q, d, s = orc.quantize_x_q8(x)
+    want = [bits(orc.gemv_q4k_q8(w, q, d, s, N, K)) for w in Ws]
+    Wd = [dev(w.reshape(-1)) for w in Ws]; src = Wd[0].clone(); W = torch.zeros_like(src); xd = dev(x); xq = K_.XQ8(R, K)
+    zero = torch.zeros_like(src); drafts = torch.zeros(R - 1, dtype=torch.int32, device="cuda")
+    K_.accept_greedy(K_.argmax(K_.gemv_q4k_q8(W, K_.quantize_x_q8(xd, xq), N, K))[0], drafts)   # workspaces exist before the capture
+    torch.cuda.synchronize()
+    for writer in ("kernel", "copy", "join"):
+        g, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(g):
+            main = torch.cuda.current_stream()
+            if writer == "join":
+                side.wait_stream(main)
+                with torch.cuda.stream(side):
+                    torch.bitwise_xor(src, zero, out=W)
+            K_.quantize_x_q8(xd, xq)
+            if writer == "kernel":
+                torch.bitwise_xor(src, zero, out=W)
+            elif writer == "copy":
+                W.copy_(src)
+            else:
+                main.wait_stream(side)
+            y = K_.gemv_q4k_q8(W, xq, N, K)
+            out = K_.accept_greedy(K_.argmax(y)[0], drafts)
+        for i in (0, 1, 0):
+            src.copy_(Wd[i]); y.zero_(); out.fill_(-1)
+            g.replay()
+            torch.cuda.synchronize()
+            assert np.array_equal(bits(y.cpu().numpy()), want[i]), (writer, i)
+            ids = orc.argmax(want[i].view(np.float32))[0]
+            mm = next((j for j in range(R - 1) if ids[j] != 0), R - 1)
+            assert out.cpu().tolist() == [mm, int(ids[mm])]
+    K_.device_status()
