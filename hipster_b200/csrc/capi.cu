@@ -128,7 +128,7 @@ int hp_accept_greedy(const int* ids_dev, const int* drafts_dev, int n_draft, int
 int hp_add_rmsnorm_quant(float* x_dev, const float* y_dev, int n_planes, size_t plane_stride, const void* w_bf16_dev, float* xn_dev, void* xq_q_dev, void* xq_sc_dev, int R, int n, float eps, void* stream) {
     HP_GUARD_BEGIN
     HP_REQUIRE(x_dev && w_bf16_dev && xq_q_dev && xq_sc_dev && (y_dev || n_planes == 0), "hp_add_rmsnorm_quant: null pointer");
-    return hp::add_rmsnorm_quant(x_dev, y_dev, n_planes, plane_stride, n, w_bf16_dev, xn_dev, hp::XQ8F{xq_q_dev, xq_sc_dev}, R, n, eps, (cudaStream_t)stream);
+    return hp::add_rmsnorm_quant(x_dev, y_dev, n_planes, plane_stride, n, w_bf16_dev, xn_dev, hp::XQ8F{xq_q_dev, xq_sc_dev}, R, n, eps, (cudaStream_t)stream, false, nullptr, 0, true);
     HP_GUARD_END
 }
 int hp_silu_mul_quant(const float* gate_up_dev, int ld, int F, void* xq_q_dev, void* xq_sc_dev, int R, void* stream) {
@@ -150,7 +150,7 @@ int hp_gdn_layer(const float* rows_dev, int ld, int T, int n_replay, int n_qk, i
     g.off_z = (2 * n_qk + n_v) * 128; g.off_b = g.off_z + n_v * 128; g.off_a = g.off_b + n_v;
     g.conv_w = conv_w_dev; g.dt_bias = dt_bias_bf16_dev; g.a_neg = a_neg_bf16_dev; g.norm_w = norm_w_bf16_dev;
     g.state = state_dev; g.conv_state = conv_state_dev; g.state_stride = 0; g.conv_stride = 0; g.seq = nullptr; g.replay_n = nullptr; g.imm_T = T; g.imm_replay = n_replay;   // one sequence, described by value
-    g.out = out_dev; g.xq = hp::XQ8F{xq_q_dev, xq_sc_dev}; g.snap = snap_dev; g.snap_row_stride = (size_t)n_v * 128 * 128; g.eps = eps; g.sigmoid_gate = sigmoid_gate;
+    g.out = out_dev; g.xq = hp::XQ8F{xq_q_dev, xq_sc_dev}; g.snap = snap_dev; g.snap_row_stride = (size_t)n_v * 128 * 128; g.eps = eps; g.sigmoid_gate = sigmoid_gate; g.late = true;
     return hp::gdn_forward(g, 1, (cudaStream_t)stream);
     HP_GUARD_END
 }
@@ -204,6 +204,7 @@ int hp_moe_layer(const float* xn_dev, const void* xq_q_dev, const void* xq_sc_de
     const MoeWs w = moe_ws(T, E, F, n_expert, k);
     char* ws = (char*)workspace_dev; const int ns = k + 1;
     float* logits = (float*)(ws + w.logits); int* cnt = (int*)(ws + w.cnt); float* v = (float*)(ws + w.v);
+    // the router kernel fetches its rows of router_dev in front of its dependency wait: the memsets keep its start behind all that the caller enqueued
     HP_CUDA(cudaMemsetAsync(cnt, 0, 32 * 4, s));
     HP_CUDA(cudaMemsetAsync(ws + w.q2, 0, w.total - w.q2, s));
     hp::MoeRouteParams rp; rp.W = router_dev; rp.x = xn_dev; rp.logits = logits; rp.E = n_expert; rp.K = E; rp.k = k; rp.T = T; rp.ids = ids_dev; rp.w = weights_dev; rp.ticket = cnt;

@@ -71,7 +71,7 @@ int dequant_q4k(const void* W, size_t nblk, float* out, cudaStream_t s);
 int embed_bf16(const int* tok, const void* table_bf16, float* out, int R, int E, int V, cudaStream_t s);
 // x += sum_p y_p (nullable y); xn = rmsnorm(x) * w; xq = q8(xn)   (reference add_rmsnorm_quant, ops.h:14)
 int add_rmsnorm_quant(float* x, const float* y, int P, size_t part_stride, int ldy, const void* w_bf16, float* xn, XQ8F xq, int R, int n, float eps, cudaStream_t s, bool assign = false,
-                      const float* slotw = nullptr, int nslot = 0);   // assign: x = sum_p y_p instead of x += ...; slotw: y = [R * nslot][ldy] expert outputs, x += sum_e fmaf(slotw, y) in slot order
+                      const float* slotw = nullptr, int nslot = 0, bool late = false);   // assign: x = sum_p y_p instead of x += ...; slotw: y = [R * nslot][ldy] expert outputs, x += sum_e fmaf(slotw, y) in slot order; late: w is read behind the dependency wait (as for the GEMV)
 // out[r] = [rmsnorm(a[r]) * wa | rmsnorm(b[r]) * wb] quantised   (reference norm2_concat_quant, ops.h:16)
 int norm2_concat_quant(const float* a, const void* wa, const float* b, int ldb, const void* wb, float* out, XQ8F xq, int R, int n, float eps, cudaStream_t s);
 // xq = q8(silu(gu[:, :F]) * gu[:, F:2F])   (reference silu_mul_quant, ops.h:25)
@@ -85,6 +85,7 @@ struct GdnParams {
     const int* seq; const int* replay_n;                 // device descriptors; seq == nullptr: one sequence {r0 = 0, T = imm_T, slot 0} with imm_replay rows to commit
     int imm_T = 0, imm_replay = 0;
     float* out; XQ8F xq; float* snap; size_t snap_row_stride; float eps; int sigmoid_gate;
+    bool late = false;                                   // conv_w and norm_w are read behind the dependency wait (as for the GEMV)
 };
 int gdn_forward(const GdnParams& p, int nseq, cudaStream_t s);
 

@@ -83,15 +83,16 @@ __device__ __forceinline__ void bf4(const uint16_t* w, float (&o)[4]) {
 template <int PT, int NG>   // PT > 0: the number of planes, known at compile time so that every load is in flight at once; 0: run-time P. NG: groups per thread
 __global__ void __cluster_dims__(NORM_CL, 1, 1) __launch_bounds__(NORM_TPB) k_add_rmsnorm_quant(float* __restrict__ x, const float* __restrict__ y, int P, size_t part_stride, int ldy,
                                                                      const uint16_t* __restrict__ w, float* __restrict__ xn, int8_t* __restrict__ q, float* __restrict__ sc,
-                                                                     int n, float eps, int assign, const float* __restrict__ slotw, int nslot) {
+                                                                     int n, float eps, int assign, const float* __restrict__ slotw, int nslot, int late) {
     __shared__ float tab[NORM_NW];
     pdl_launch_dependents();
     cluster_arrive_relaxed();   // matched by cluster_wait() before the first store into another CTA
     const int rank = blockIdx.x % NORM_CL, r = blockIdx.x / NORM_CL, lane = threadIdx.x & 31, t = rank * NORM_TPB + threadIdx.x;
     float* xr = x + (size_t)r * n;
     float wv[NG][4];
+    if (late) pdl_wait();   // the weights may have been written earlier in the stream; constant ones do not depend on the previous kernel
 #pragma unroll
-    for (int k = 0; k < NG; ++k) { const int i = 4 * (t + k * NORM_ROWT); if (i < n) bf4(w + i, wv[k]); }   // weights do not depend on the previous kernel
+    for (int k = 0; k < NG; ++k) { const int i = 4 * (t + k * NORM_ROWT); if (i < n) bf4(w + i, wv[k]); }
     pdl_wait();
     float4 v[NG];
 #pragma unroll
@@ -246,7 +247,7 @@ struct GdnArgs {
     int imm_T, imm_replay;                                        // used instead when seq == nullptr (a single sequence described by value)
     float* out; int8_t* oq; float* osc;                           // out f32 [rows][n_v*128] (nullable), quantised out
     float* snap; size_t snap_row_stride;                          // optional state snapshots after each new row
-    float eps; int sigmoid_gate;
+    float eps; int sigmoid_gate, late;
 };
 constexpr int GDN_MAXROWS = 16, GDN_CL = 4;   // replayed rows (<= 8) + new rows (<= 8) of one sequence; CTAs per head
 __device__ __forceinline__ float2 gdn_mul2(float2 a, float2 b) {
@@ -277,7 +278,7 @@ __global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, MINB) k_gd
     const int rank = blockIdx.x % GDN_CL, h = blockIdx.x / GDN_CL, hk = h % a.n_qk, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // Item e = tid + 256 k of this thread is (row index e / 96, local channel c = e % 96) both for the raw loads and for
     // the conv outputs. Local channel c: group c/32 = q, k, v; channel 32*rank + c%32 of the head. Its slot in a
-    // history / saved row, its column in a row of the merged projection, its conv taps (independent of the predecessor):
+    // history / saved row, its column in a row of the merged projection, its conv taps (the engine's are independent of the predecessor):
     int e_rr[NLD], e_c[NLD], e_slot[NLD], e_col[NLD];
     float4 cw[NCV];
 #pragma unroll
@@ -285,8 +286,10 @@ __global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, MINB) k_gd
         const int e = tid + 256 * k, rr = e / 96, c = e - rr * 96, g3 = c >> 5, cl = 32 * rank + (c & 31);
         e_rr[k] = rr; e_c[k] = c; e_slot[k] = g3 * D + cl;
         e_col[k] = g3 == 0 ? hk * D + cl : g3 == 1 ? a.n_qk * D + hk * D + cl : 2 * a.n_qk * D + h * D + cl;
-        if (k < NCV) cw[k] = *reinterpret_cast<const float4*>(a.conv_w + (size_t)e_col[k] * 4);
     }
+    if (a.late) pdl_wait();   // the taps and the norm weights may have been written earlier in the stream
+#pragma unroll
+    for (int k = 0; k < NCV; ++k) cw[k] = *reinterpret_cast<const float4*>(a.conv_w + (size_t)e_col[k] * 4);
     const float nw = bf2f(a.norm_w[32 * rank + lane]);
     pdl_wait();
     const int r0 = a.seq ? a.seq[blockIdx.y * 4 + 0] : 0, T = min(a.seq ? a.seq[blockIdx.y * 4 + 1] : a.imm_T, 8), slot = a.seq ? a.seq[blockIdx.y * 4 + 2] : 0;
@@ -447,7 +450,7 @@ int embed_bf16(const int* tok, const void* table, float* out, int R, int E, int 
     HP_CUDA(cudaGetLastError()); return HP_OK;
 }
 int add_rmsnorm_quant(float* x, const float* y, int P, size_t part_stride, int ldy, const void* w_bf16, float* xn, XQ8F xq, int R, int n, float eps, cudaStream_t s, bool assign,
-                      const float* slotw, int nslot) {
+                      const float* slotw, int nslot, bool late) {
     HP_REQUIRE(!assign || y, "add_rmsnorm_quant: assign needs planes");
     HP_REQUIRE(!slotw || (y && nslot >= 1), "add_rmsnorm_quant: the slot-weighted form needs the per-pair rows");
     HP_REQUIRE(R >= 1 && n > 0 && n % 64 == 0, "add_rmsnorm_quant: n=%d must be a positive multiple of 64", n);
@@ -459,7 +462,7 @@ int add_rmsnorm_quant(float* x, const float* y, int P, size_t part_stride, int l
         return pt == 1 ? k_add_rmsnorm_quant<1, NG> : pt == 2 ? k_add_rmsnorm_quant<2, NG> : pt == 4 ? k_add_rmsnorm_quant<4, NG> : k_add_rmsnorm_quant<0, NG>;
     };
     auto kern = n <= NORM_ROWT * 4 ? pick(std::integral_constant<int, 1>()) : pick(std::integral_constant<int, NORM_MAXG>());
-    HP_CUDA(launch_pdl(kern, dim3(R * NORM_CL), dim3(NORM_TPB), 0, s, x, y, P, part_stride, ldy, (const uint16_t*)w_bf16, xn, (int8_t*)xq.q, (float*)xq.sc, n, eps, assign ? 1 : 0, slotw, nslot));
+    HP_CUDA(launch_pdl(kern, dim3(R * NORM_CL), dim3(NORM_TPB), 0, s, x, y, P, part_stride, ldy, (const uint16_t*)w_bf16, xn, (int8_t*)xq.q, (float*)xq.sc, n, eps, assign ? 1 : 0, slotw, nslot, late ? 1 : 0));
     HP_CUDA(cudaGetLastError()); return HP_OK;
 }
 int norm2_concat_quant(const float* a, const void* wa, const float* b, int ldb, const void* wb, float* out, XQ8F xq, int R, int n, float eps, cudaStream_t s) {
@@ -482,7 +485,7 @@ int gdn_forward(const GdnParams& p, int nseq, cudaStream_t s) {
     a.n_qk = p.n_qk; a.n_v = p.n_v; a.conv_w = p.conv_w; a.dt_bias = (const uint16_t*)p.dt_bias; a.a_neg = (const uint16_t*)p.a_neg; a.norm_w = (const uint16_t*)p.norm_w;
     a.state = p.state; a.conv_state = p.conv_state; a.state_stride = p.state_stride; a.conv_stride = p.conv_stride;
     a.seq = p.seq; a.replay_n = p.replay_n; a.imm_T = p.imm_T; a.imm_replay = p.imm_replay; a.out = p.out; a.oq = (int8_t*)p.xq.q; a.osc = (float*)p.xq.sc;
-    a.snap = p.snap; a.snap_row_stride = p.snap_row_stride; a.eps = p.eps; a.sigmoid_gate = p.sigmoid_gate;
+    a.snap = p.snap; a.snap_row_stride = p.snap_row_stride; a.eps = p.eps; a.sigmoid_gate = p.sigmoid_gate; a.late = p.late;
     if (nseq >= 3) HP_CUDA(launch_pdl<128>(k_gdn<4>, dim3(p.n_v * GDN_CL, nseq), dim3(256), 0, s, a));
     else HP_CUDA(launch_pdl<128>(k_gdn<3>, dim3(p.n_v * GDN_CL, nseq), dim3(256), 0, s, a));
     HP_CUDA(cudaGetLastError()); return HP_OK;

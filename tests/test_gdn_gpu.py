@@ -155,3 +155,35 @@ def test_kernel_within_1e5_of_the_double_precision_transcription(gate):
     assert np.abs(o - out64).max() <= 1e-5 * np.abs(out64).max()
     assert np.abs(sn - snap64).max() <= 1e-5 * np.abs(snap64).max()
     assert np.abs(st - st64).max() <= 1e-5 * np.abs(st64).max()
+
+
+def test_weights_written_on_the_stream_right_before(setup):
+    """Conv taps and norm weights change between two calls, by kernels on the stream, with and without a quantiser (which
+    triggers early launches in its first instruction) in between. No rows are committed, so the state stays."""
+    from hipster_b200 import kernels as K_
+    T = 6
+    a, b = setup, Layer(seed=3)
+    d, e = a.dev(), b.dev()
+    cw, nw = [d["conv_w"].clone(), e["conv_w"].clone()], [d["nw"].clone(), e["nw"].clone()]
+    x = d["rows"][:, :512].contiguous(); xq = K_.XQ8(T, 512); s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def call(out):
+        L = hb.lib()
+        hb.check(L.hp_gdn_layer(hb.ptr(d["rows"]), LD, T, 0, NQK, NV, hb.ptr(d["conv_w"]), hb.ptr(d["dt"]), hb.ptr(d["an"]), hb.ptr(d["nw"]),
+                                hb.ptr(d["state"]), hb.ptr(d["conv"]), hb.ptr(d["saved"]), hb.ptr(out), ctypes.c_void_p(0), ctypes.c_void_p(0),
+                                ctypes.c_void_p(0), ctypes.c_float(a.eps), a.gate, s))
+        return out
+    new = lambda: torch.empty((T, NV * D), device="cuda")
+    want = []
+    for i in range(2):
+        d["conv_w"].copy_(cw[i]); d["nw"].copy_(nw[i]); torch.cuda.synchronize()
+        want.append(call(new())); torch.cuda.synchronize()
+    assert not torch.equal(want[0], want[1])
+    got = []
+    for i in range(40):
+        torch.mul(cw[i % 2], 1.0, out=d["conv_w"]); torch.bitwise_or(nw[i % 2], 0, out=d["nw"])
+        if i % 4 < 2:
+            K_.quantize_x_q8(x, xq)
+        got.append(call(new()))
+    for i, o in enumerate(got):
+        assert torch.equal(o.view(torch.int32), want[i % 2].view(torch.int32)), i

@@ -60,3 +60,29 @@ def test_silu_mul_quant_bit_exact(R, F):
     assert np.array_equal(q.cpu().numpy(), q_o)
     assert np.array_equal(d.cpu().numpy().view(np.uint32), d_o.view(np.uint32))
     assert np.array_equal(s.cpu().numpy().view(np.uint32), s_o.view(np.uint32))
+
+
+@pytest.mark.parametrize("n", [320, 5120, 10240])
+def test_add_rmsnorm_quant_weights_written_on_the_stream_right_before(n):
+    R, eps = 3, 1e-6
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((R, n)).astype(np.float32)
+    ws = [(rng.standard_normal(n).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16) for _ in range(2)]
+    want = []
+    for w in ws:
+        xn_o = np.empty((R, n), np.float32); q_o = np.empty((R, n), np.int8); d_o = np.empty((R, n // 32), np.float32); s_o = np.empty((R, n // 32), np.float32)
+        orc.lib().orc_add_rmsnorm_quant(_f(x), None, 0, ctypes.c_size_t(R * n), n, _f(w), _f(xn_o), _f(q_o), _f(d_o), _f(s_o), R, n, ctypes.c_float(eps))
+        want.append((xn_o.view(np.uint32), q_o))
+    key = torch.from_numpy((ws[0] ^ ws[1]).view(np.int16)).cuda(); wd = torch.from_numpy(ws[1].view(np.int16)).cuda()
+    xd = torch.from_numpy(x).cuda(); other = K_.XQ8(R, n)
+    got = []
+    for i in range(40):
+        wd.bitwise_xor_(key)
+        if i % 4 < 2:
+            K_.quantize_x_q8(xd, other)                          # triggers early launches in its first instruction
+        xn = torch.empty((R, n), dtype=torch.float32, device="cuda"); xq = K_.XQ8(R, n)
+        check(lib().hp_add_rmsnorm_quant(ptr(xd), None, 0, ctypes.c_size_t(0), ptr(wd), ptr(xn), ptr(xq.q), ptr(xq.sc), R, n, ctypes.c_float(eps), _stream()))
+        got.append((xn, xq))
+    for i, (xn, xq) in enumerate(got):
+        assert np.array_equal(xn.cpu().numpy().view(np.uint32), want[i % 2][0]), i
+        assert np.array_equal(xq.unpack()[0].cpu().numpy(), want[i % 2][1]), i
