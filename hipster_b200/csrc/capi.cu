@@ -6,6 +6,7 @@
 #include "../../include/hipster_b200.h"
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <string>
 #include <exception>
 
@@ -91,7 +92,8 @@ int hp_gemv_q4k_q8(const void* w_dev, const void* xq_q_dev, const void* xq_sc_de
     HP_REQUIRE(((uintptr_t)w_dev & 15) == 0, "hp_gemv_q4k_q8: weights must be 16-byte aligned");
     HP_REQUIRE(N > 0 && K > 0 && K % 256 == 0 && R >= 1 && R <= 32, "hp_gemv_q4k_q8: bad shape N=%d K=%d R=%d", N, K, R);
     hp::GemvWorkspace ws; { const int rc = hp::default_gemv_workspace(&ws, (size_t)4 * R * N * sizeof(float)); if (rc) return rc; }
-    return hp::gemv_q4k_q8(w_dev, hp::XQ8F{(void*)xq_q_dev, (void*)xq_sc_dev}, y_dev, N, K, R, ldy, ws, (cudaStream_t)stream, true, true);   // launched early, but the caller's weights are read behind the dependency wait
+    static const bool early = getenv("HIPSTER_B200_NO_PDL") == nullptr;
+    return hp::gemv_q4k_q8(w_dev, hp::XQ8F{(void*)xq_q_dev, (void*)xq_sc_dev}, y_dev, N, K, R, ldy, ws, (cudaStream_t)stream, early, true);   // launched early, but the caller's weights are read behind the dependency wait
     HP_GUARD_END
 }
 int hp_gemv_parts(int N, int K) { return (N > 0 && K > 0 && K % 256 == 0) ? hp::gemv_parts(N, K) : 0; }

@@ -1,5 +1,9 @@
 """Parity of the CUDA Q4_K GEMV path (through the C ABI) with the CPU oracle. Bit-exact for the quantised
 activations, the dequantised weights, the int8-activation GEMV, the f32-activation GEMV, argmax and acceptance."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -9,6 +13,7 @@ from hipster_b200 import kernels as K_, synth
 from oracle import orc
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.abspath(os.path.join(os.path.dirname(__file__), ".."))
 
 
 def dev(a):
@@ -205,3 +210,28 @@ def test_gemv_chain_captured_behind_copies_kernels_and_joins(N, K):
             mm = next((j for j in range(R - 1) if ids[j] != 0), R - 1)
             assert out.cpu().tolist() == [mm, int(ids[mm])]
     K_.device_status()
+
+
+_EDGES = """
+import torch
+from cuda.bindings import runtime as rt
+from hipster_b200 import kernels as K_
+w = torch.zeros(4096 * 144 * 2, dtype=torch.uint8, device="cuda"); x = torch.ones((3, 512), device="cuda"); xq = K_.XQ8(3, 512); y = torch.empty((3, 4096), device="cuda")
+K_.gemv_q4k_q8(w, K_.quantize_x_q8(x, xq), 4096, 512, y); torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph(keep_graph=True)
+with torch.cuda.graph(g):
+    K_.gemv_q4k_q8(w, K_.quantize_x_q8(x, xq), 4096, 512, y)
+err, src, dst, data, n = rt.cudaGraphGetEdges_v2(rt.cudaGraph_t(init_value=g.raw_cuda_graph()), 16)
+assert int(err) == 0 and n >= 1, (err, n)
+print("edges", sum(int(e.type) == int(rt.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic) for e in data[:n]))
+"""
+
+
+@pytest.mark.parametrize("env,want", [({}, 1), ({"HIPSTER_B200_NO_PDL": "1"}, 0), ({"HIPSTER_B200_PDL_OFF": "64"}, 0)])
+def test_public_gemv_honours_the_early_launch_switches(env, want):
+    """Programmatic edges of a captured quantise + GEMV call (one K part: two nodes, one edge between them)."""
+    pytest.importorskip("cuda.bindings.runtime")
+    clean = {k: v for k, v in os.environ.items() if not k.startswith("HIPSTER_B200_NO_PDL") and not k.startswith("HIPSTER_B200_PDL_OFF")}
+    r = subprocess.run([sys.executable, "-c", _EDGES], cwd=ROOT, env={**clean, **env}, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert r.stdout.split()[-1] == str(want), r.stdout
