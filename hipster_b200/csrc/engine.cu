@@ -144,6 +144,15 @@ Engine::~Engine() {
     if (ev0_) cudaEventDestroy(ev0_); if (ev1_) cudaEventDestroy(ev1_);
     if (s_) cudaStreamDestroy(s_);
 }
+// widest projection output of a pass, longest projection input
+size_t Engine::big_width() const {
+    const hp_model_cfg& c = c_; const int F = c.n_expert ? c.expert_ff : c.n_ff;
+    return std::max<size_t>({(size_t)ld_in_, (size_t)c.n_head * 512 + 2 * c.n_head_kv * 256, (size_t)2 * F, (size_t)2 * c.n_embd});
+}
+size_t Engine::k_max() const {
+    const hp_model_cfg& c = c_; const int F = c.n_expert ? c.expert_ff : c.n_ff;
+    return std::max<size_t>({(size_t)2 * c.n_embd, (size_t)F, (size_t)c.n_head * 256, (size_t)c.gdn_v_heads * 128});
+}
 int Engine::nattn() const { return c_.n_layer / c_.attn_every; }
 int Engine::ngdn() const { return c_.n_layer - nattn(); }
 
@@ -299,8 +308,7 @@ int Engine::init() {
     pend_.assign(c.n_slots, 0); last_r0_.assign(c.n_slots, 0); last_T_.assign(c.n_slots, 0);
     // work buffers
     const int F = c.n_expert ? c.expert_ff : c.n_ff;
-    const size_t bigw = std::max<size_t>({(size_t)gdn_in, (size_t)attn_in, (size_t)2 * F, (size_t)2 * E});
-    const size_t kmax = std::max<size_t>({(size_t)2 * E, (size_t)F, (size_t)c.n_head * 256, (size_t)nv * 128});
+    const size_t bigw = big_width(), kmax = k_max();
     HP_TRY(alloc((void**)&x_, (size_t)MAXR * E * 4)); HP_TRY(alloc((void**)&emb_, (size_t)MAXR * E * 4));
     HP_TRY(alloc((void**)&big_, (size_t)MAXR * bigw * 4));
     HP_TRY(alloc((void**)&yparts_, (size_t)4 * MAXR * std::max<size_t>(bigw, E) * 4));
@@ -324,24 +332,6 @@ int Engine::init() {
         { const int w = std::max(1, c.ep_world); e_lo_ = (int)((long long)c.ep_rank * c.n_expert / w); e_hi_ = (int)((long long)(c.ep_rank + 1) * c.n_expert / w); }
     }
     nsplit_max_ = (c.max_ctx + ATTN_SPLIT - 1) / ATTN_SPLIT;
-    if (tiled_ && c.ep_world <= 1 && c.max_ctx > 8) {   // prompt chunks (the GEMM reads tile-major weights; expert shards exchange after every pass)
-        const int PR = pf_rows_ = std::min(PF_MAXR, (c.max_ctx + 7) & ~7);
-        size_t planes = 0;
-        auto need = [&](const Lin& l) { if (l.N) planes = std::max(planes, (size_t)l.P * l.N); };
-        for (const LayerW& L : layers_) { need(L.in_proj); need(L.out_proj); need(L.down); need(L.gate_up); }
-        need(eh_proj_); need(mtp_.in_proj);
-        HP_TRY(alloc((void**)&pf_.x, (size_t)PR * E * 4)); HP_TRY(alloc((void**)&pf_.emb, (size_t)PR * E * 4)); HP_TRY(alloc((void**)&pf_.h, (size_t)PR * E * 4));
-        HP_TRY(alloc((void**)&pf_hin_, (size_t)PR * E * 4)); HP_TRY(alloc((void**)&pf_.big, (size_t)PR * bigw * 4)); HP_TRY(alloc((void**)&pf_.yparts, (size_t)PR * planes * 4));
-        HP_TRY(alloc(&pf_.xq.q, xq_q_bytes(PR, (int)kmax))); HP_TRY(alloc(&pf_.xq.sc, xq_sc_floats(PR, (int)kmax) * 4));
-        HP_CUDA(cudaMemsetAsync(pf_.xq.q, 0, xq_q_bytes(PR, (int)kmax), s_)); HP_CUDA(cudaMemsetAsync(pf_.xq.sc, 0, xq_sc_floats(PR, (int)kmax) * 4, s_));
-        HP_TRY(alloc(&pf_pack_, gemm_pack_bytes(PR, (int)kmax)));
-        if (ngdn()) HP_TRY(alloc((void**)&pf_gdn_, gdn_prefill_floats(PR, nq, nv) * 4));
-        HP_TRY(alloc((void**)&pf_desc_, (size_t)PR * 8 * 4)); HP_CUDA(cudaMallocHost((void**)&pf_hdesc_, (size_t)PR * 8 * 4));
-        if (c.n_expert) {
-            const size_t pairs = (size_t)PR * (c.n_expert_used + 1);
-            HP_TRY(alloc((void**)&pf_.xn, (size_t)PR * E * 4)); HP_TRY(alloc((void**)&pf_.moe_v, pairs * E * 4)); HP_TRY(alloc((void**)&pf_.moe_w, pairs * 4)); HP_TRY(alloc((void**)&pf_.moe_ids, pairs * 4));
-        }
-    }
     const size_t np = attn_partial_floats(MAXR, c.n_head_kv, nsplit_max_);
     HP_TRY(alloc((void**)&pO_, np * 256 * 4)); HP_TRY(alloc((void**)&pm_, np * 4)); HP_TRY(alloc((void**)&pl_, np * 4));
     HP_TRY(alloc((void**)&d_desc_, D_INTS * 4)); HP_CUDA(cudaMallocHost((void**)&h_desc_, D_INTS * 4)); memset(h_desc_, 0, D_INTS * 4);
@@ -824,6 +814,51 @@ int Engine::prefill_rows(int slot, const int* tokens, int R, int pos0, int with_
     HP_CUDA(cudaEventElapsedTime(&last_ms_, ev0_, ev1_));
     return check_device_status();
 }
+// Buffers of the prompt chunks (243 MB for the 27B shape), one block that the first prompt of more than 8 tokens takes and the
+// engine keeps: a model loads with what its passes need. They stay out, and prompts run as 8-row passes with the same results,
+// unless the device has twice their size free: what the caller and the captured rounds still allocate must not fail for
+// the sake of a faster prompt.
+int Engine::prefill_reserve() {
+    const hp_model_cfg& c = c_;
+    if (pf_rows_ || !tiled_ || c.ep_world > 1) return HP_OK;   // the GEMM reads tile-major weights; expert shards exchange after every pass
+    const int PR = std::min((int)PF_MAXR, (c.max_ctx + 7) & ~7), E = c.n_embd, nv = c.gdn_v_heads, nq = c.gdn_qk_heads;
+    const size_t bigw = big_width(), kmax = k_max();
+    size_t planes = 0;
+    auto need = [&](const Lin& l) { if (l.N) planes = std::max(planes, (size_t)l.P * l.N); };
+    for (const LayerW& L : layers_) { need(L.in_proj); need(L.out_proj); need(L.down); need(L.gate_up); }
+    need(eh_proj_); need(mtp_.in_proj);
+    PassBuf b; float *hin = nullptr, *gdn = nullptr; void* pack = nullptr; int* desc = nullptr;
+    std::vector<std::pair<void**, size_t>> at; size_t total = 0;
+    auto part = [&](void** p, size_t bytes) { at.emplace_back(p, total); total += (bytes + 255) & ~(size_t)255; };
+    part((void**)&b.x, (size_t)PR * E * 4); part((void**)&b.emb, (size_t)PR * E * 4); part((void**)&b.h, (size_t)PR * E * 4); part((void**)&hin, (size_t)PR * E * 4);
+    part((void**)&b.big, (size_t)PR * bigw * 4); part((void**)&b.yparts, (size_t)PR * planes * 4);
+    const size_t xq_at = total;
+    part(&b.xq.q, xq_q_bytes(PR, (int)kmax)); part(&b.xq.sc, xq_sc_floats(PR, (int)kmax) * 4);
+    const size_t xq_end = total;
+    part(&pack, gemm_pack_bytes(PR, (int)kmax));
+    if (ngdn()) part((void**)&gdn, gdn_prefill_floats(PR, nq, nv) * 4);
+    part((void**)&desc, (size_t)PR * 8 * 4);
+    if (c.n_expert) {
+        const size_t pairs = (size_t)PR * (c.n_expert_used + 1);
+        part((void**)&b.xn, (size_t)PR * E * 4); part((void**)&b.moe_v, pairs * E * 4); part((void**)&b.moe_w, pairs * 4); part((void**)&b.moe_ids, pairs * 4);
+    }
+    struct Relaxed {   // another thread's capture must not see an allocation of this one
+        cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
+        Relaxed() { cudaThreadExchangeStreamCaptureMode(&m); }
+        ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&m); }
+    } relaxed;
+    size_t avail = 0, all = 0;
+    HP_CUDA(cudaMemGetInfo(&avail, &all));
+    if (avail < 2 * total) return HP_OK;
+    if (!pf_hdesc_ && cudaMallocHost((void**)&pf_hdesc_, (size_t)PR * 8 * 4) != cudaSuccess) { pf_hdesc_ = nullptr; cudaGetLastError(); return HP_OK; }
+    char* block = nullptr;
+    if (cudaMalloc((void**)&block, total) != cudaSuccess) { cudaGetLastError(); return HP_OK; }
+    allocs_.push_back(block);
+    for (auto& [p, off] : at) *p = block + off;
+    HP_CUDA(cudaMemsetAsync(block + xq_at, 0, xq_end - xq_at, s_));
+    pf_ = b; pf_hin_ = hin; pf_gdn_ = gdn; pf_pack_ = pack; pf_desc_ = desc; pf_rows_ = PR;
+    return HP_OK;
+}
 // Prompt ingestion for one slot (Qwen4Exp::prefill + mtp_catchup, qwen4exp.h:57-60,72-74; Backend::prefill,
 // front/serve.cpp:29): n tokens at positions pos0.., committed; with_mtp also runs the MTP block over the same rows, row p
 // paired with the trunk's hidden row of position p - 1 (zeros at position 0; the last row of the previous chunk / call
@@ -836,6 +871,7 @@ int Engine::prefill(int slot, const int* tokens, int n, int pos0, int with_mtp) 
     HP_REQUIRE(!with_mtp || c_.has_mtp, "model has no MTP block");
     const int E = c_.n_embd;
     int T = 0;
+    if (n > 8) HP_TRY(prefill_reserve());
     if (n > 8 && pf_rows_) {
         // More than one 8-row pass: chunks of nearly equal size, a multiple of 8 rows except for the last
         if (pend_[slot]) HP_TRY(flush_commits());   // the chunks start from the committed state

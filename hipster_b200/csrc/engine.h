@@ -75,6 +75,8 @@ private:
     int ep_exchange(float* buf, size_t n);
     int ep_allreduce(float* buf, size_t n);
     int run_pass(int R, int nseq, int ngroups);              // trunk over the rows described by desc_ (already uploaded)
+    size_t big_width() const; size_t k_max() const;
+    int prefill_reserve();                                   // buffers of the prompt chunks, when they fit; sets pf_rows_
     int prefill_rows(int slot, const int* tokens, int R, int pos0, int with_mtp, int tail);   // a prompt chunk through the GEMM path
     int prefill_attn(const LayerW& L, uint16_t* kc, uint16_t* vc, size_t kv_stride, int R, bool kv_only);
     int prefill_lin(const Lin& l, float* out, int ld, size_t part_stride, int R);
@@ -120,7 +122,7 @@ private:
     int* d_specin_ = nullptr;                                     // the round's inputs: slot list, seeded substitutions
     float *hpend_ = nullptr, *hstage_ = nullptr, *hprev_ = nullptr;   // per-slot pending h rows; gathered MTP inputs; per-slot last prompt h (prefill catch-up)
     std::vector<int> spec_pos_, spec_on_;
-    // Prompt chunks of up to pf_rows_ rows: buffers of their own, exchanged with the pass buffers while a chunk runs (PrefillScope)
+    // Prompt chunks of up to pf_rows_ rows: buffers of their own, exchanged with the pass buffers while a chunk runs (PrefillScope); pf_rows_ = 0 until they exist
     struct PassBuf { float *x = nullptr, *xn = nullptr, *big = nullptr, *yparts = nullptr, *emb = nullptr, *h = nullptr, *moe_v = nullptr, *moe_w = nullptr; int* moe_ids = nullptr; XQ8F xq{nullptr, nullptr}; } pf_;
     struct PrefillScope;
     struct PfBatch { int row0, rows, g0, ng; };                   // rows of a chunk that one attention launch takes

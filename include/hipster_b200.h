@@ -180,7 +180,10 @@ int hp_topk(hp_engine* e, int which, int T, int k, int* ids_host, float* vals_ho
  * other. Afterwards row 0 of hp_logits_dev / hp_h_nextn_dev (and hp_topk(0, 1, ...)) is the LAST prompt row.
  * Replaces Qwen4Exp::prefill + mtp_catchup (qwen4exp.h:57-60,72-74) and Backend::prefill (front/serve.cpp:29). More than
  * 8 tokens run in chunks of up to 512 rows (GEMM projections, one recurrence per layer and chunk), with the same bits as
- * passes of 8 rows; up to 8 tokens, and every prompt of an expert-parallel shard, run through the verify path. */
+ * passes of 8 rows; up to 8 tokens, and every prompt of an expert-parallel shard or of a row-major engine
+ * (HIPSTER_B200_ROWMAJOR), run through the verify path. The first such prompt allocates the chunks' work buffers, which the
+ * engine keeps until hp_free (243 MB for the 27B shape, 252 MB for the flash-next preset); while less than twice their size is
+ * free on the device, prompts run through the verify path as well. hp_load does not need that memory. */
 int hp_prefill(hp_engine* e, int slot, const int* tokens_host, int n, int pos0, int with_mtp);
 const float* hp_logits_dev(const hp_engine* e);            /* qwen35.h:82 */
 const float* hp_h_nextn_dev(const hp_engine* e);           /* qwen35.h:83 */

@@ -61,3 +61,49 @@ def test_prefill_chunks_fill_the_draft_block(n):
     ref.mtp_forward(0, [tok], prev[None, :], n)
     assert np.array_equal(bits(eng.mtp_logits(1)), bits(ref.mtp_logits(1)))
     eng.close()
+
+
+def test_chunk_buffers_come_with_the_first_long_prompt_and_only_where_they_fit():
+    """A model loads with what its passes need, also where the buffers of the prompt chunks (about 170 MB for this shape)
+    would not fit beside it; prompts then run as 8-row passes with the same bits, and as chunks once there is room."""
+    import torch
+    MB = 1 << 20
+    cfg = hb.ModelCfg.preset("tiny", n_ff=17408)
+    free = lambda: torch.cuda.mem_get_info()[0]  # noqa: E731
+    rng = np.random.default_rng(5)
+    prompts = [[int(x) for x in rng.integers(0, cfg.n_vocab, size=n)] for n in (20, 21)]
+    ref = orc.Model(cfg)
+    warm = hb.Engine(cfg); warm.prefill(0, prompts[0], with_mtp=False); warm.prefill(1, prompts[0][:8]); warm.close()   # kernels loaded
+    torch.cuda.empty_cache()
+    f0 = free()
+    eng = hb.Engine(cfg)
+    weights = f0 - free()
+    eng.prefill(0, prompts[0][:8], with_mtp=False)
+    assert f0 - free() - weights <= 4 * MB                       # short prompts do not take them
+    eng.prefill(0, prompts[0], with_mtp=False)
+    chunks = f0 - free() - weights
+    assert 100 * MB < chunks < 200 * MB
+    eng.close()
+    assert free() >= f0 - 4 * MB
+    hog = torch.empty(free() - weights - chunks // 2, dtype=torch.uint8, device="cuda")
+    eng = hb.Engine(cfg)                                         # half of the buffers' size is left
+    left = free()
+    assert left < chunks
+
+    def check(slot, prompt):
+        eng.prefill(slot, prompt, with_mtp=False)
+        for p in range(0, len(prompt), 8):
+            T = min(8, len(prompt) - p)
+            ref.forward([(slot, prompt[p:p + T], p)]); ref.accept(slot, T)
+        assert np.array_equal(bits(eng.logits(1)[0]), bits(ref.logits(T)[T - 1]))
+        assert np.array_equal(bits(eng.h_nextn(T)[1:]), bits(ref.h_nextn(T)[1:]))
+
+    check(0, prompts[0])
+    assert free() >= left - 4 * MB                               # (a kernel used for the first time may take its code's page)
+    del hog
+    torch.cuda.empty_cache()
+    check(1, prompts[1])                                         # the other slot, as a chunk
+    for e in (eng, ref):                                         # both go on from their prompts
+        e.forward([(0, [3, 4], 20), (1, [5], 21)])
+    assert np.array_equal(bits(eng.logits(3)), bits(ref.logits(3)))
+    eng.close()
