@@ -459,25 +459,28 @@ int launch_tc(const TcArgs& a, const XQ8F& x, int grid, cudaStream_t s, bool pdl
 }  // namespace
 
 size_t gemm_pack_bytes(int R, int K) { return (size_t)((R + 7) / 8 + 15) * (size_t)(K / 256) * 2560; }
-int gemm_q4k_q8_parts(const void* Wt, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, void* pack, int* err, cudaStream_t s, bool pdl) {
+// The cut of the rows into column ranges of ntc tiles of 8, and of the weight tiles into items of G = 8 or 4 (the latter leaves
+// every second tile position empty). An item of 20 blocks takes 53, 71 and 89 us at ntc = 8, 12 and 16: 4.5 us per tile and
+// what 4 tiles would take; the cut with the least time over the rounds of the SMs is taken.
+void gemm_cut(int N, int K, int R, int* ntc, int* G) {
+    const int t8 = (R + 7) / 8, tiles = (N + 15) / 16, P = gemv_num_parts(N, K / 256);
+    long best = 0; *ntc = 0;
+    for (int c = 4; c <= 16; c += 2)
+        for (int g = 8; g >= 4; g -= 4) {
+            const int ncg = (t8 + c - 1) / c;
+            const long cost = ((long)ncg * P * ((tiles + g - 1) / g) + GEMV_NCTA - 1) / GEMV_NCTA * (g == 8 ? (c + 4) * 3 : (c + 4) * 2);
+            if (!*ntc || cost < best) { best = cost; *ntc = c; *G = g; }
+        }
+}
+int gemm_q4k_q8_cut(const void* Wt, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, void* pack, int* err, cudaStream_t s, bool pdl, int ntc, int G) {
     HP_REQUIRE(K > 0 && K % 256 == 0, "gemm_q4k_q8: K=%d must be a positive multiple of 256", K);
     HP_REQUIRE(N > 0 && R >= 1 && ldy >= N, "gemm_q4k_q8: bad shape N=%d R=%d ldy=%d", N, R, ldy);
     HP_REQUIRE(pack && ((uintptr_t)pack & 15) == 0 && ((uintptr_t)Wt & 15) == 0, "gemm_q4k_q8: the pack buffer and the weights must be 16-byte aligned");
+    HP_REQUIRE((G == 8 || G == 4) && ntc >= 4 && ntc <= 16 && ntc % 2 == 0, "gemm_q4k_q8: no cut of %d column tiles and %d weight tiles", ntc, G);
     TcArgs a; a.W = (const uint8_t*)Wt; a.xp = (const uint8_t*)pack; a.y = yparts;
     a.N = N; a.nb = K / 256; a.P = gemv_num_parts(N, a.nb); a.R = R; a.ldy = ldy; a.part_stride = part_stride; a.err = err;
     HP_REQUIRE(a.P > 0, "gemm_q4k_q8: K=%d is too large for the K-part partition", K);
-    const int t8 = (R + 7) / 8, tiles = (N + 15) / 16;
-    // Cut of the rows into ncg column ranges of ntc tiles of 8, and of the weight tiles into items of G = 8 or 4 (the
-    // latter leaves every second tile position empty). An item of 20 blocks takes 53, 71 and 89 us at ntc = 8, 12 and 16:
-    // 4.5 us per tile and what 4 tiles would take; the cut with the least time over the rounds of the SMs is taken.
-    int ntc = 0; long best = 0;
-    for (int c = 4; c <= 16; c += 2)
-        for (int G = 8; G >= 4; G -= 4) {
-            const int ncg = (t8 + c - 1) / c;
-            const long cost = ((long)ncg * a.P * ((tiles + G - 1) / G) + GEMV_NCTA - 1) / GEMV_NCTA * (G == 8 ? (c + 4) * 3 : (c + 4) * 2);
-            if (!ntc || cost < best) { best = cost; ntc = c; a.ncg = ncg; a.G = G; }
-        }
-    a.ngrp = (tiles + a.G - 1) / a.G;
+    a.G = G; a.ngrp = ((N + 15) / 16 + G - 1) / G; a.ncg = ((R + 7) / 8 + ntc - 1) / ntc;
     const int items = a.ncg * a.ngrp * a.P, grid = items < GEMV_NCTA ? items : GEMV_NCTA;
     switch (ntc) {
         case 4: return launch_tc<4>(a, x, grid, s, pdl);   case 6: return launch_tc<6>(a, x, grid, s, pdl);
@@ -485,6 +488,11 @@ int gemm_q4k_q8_parts(const void* Wt, const XQ8F& x, float* yparts, int N, int K
         case 12: return launch_tc<12>(a, x, grid, s, pdl); case 14: return launch_tc<14>(a, x, grid, s, pdl);
         default: return launch_tc<16>(a, x, grid, s, pdl);
     }
+}
+int gemm_q4k_q8_parts(const void* Wt, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, void* pack, int* err, cudaStream_t s, bool pdl) {
+    HP_REQUIRE(K > 0 && K % 256 == 0 && N > 0 && R >= 1 && gemv_num_parts(N, K / 256) > 0, "gemm_q4k_q8: bad shape N=%d K=%d R=%d", N, K, R);
+    int ntc, G; gemm_cut(N, K, R, &ntc, &G);
+    return gemm_q4k_q8_cut(Wt, x, yparts, N, K, R, ldy, part_stride, pack, err, s, pdl, ntc, G);
 }
 
 }  // namespace hp

@@ -1,0 +1,103 @@
+"""The prompt GEMM against the verify GEMV in pieces of 32 rows, plane by plane and bit for bit: every cut (column tiles per
+range, weight tiles per item) on shapes whose K parts are odd and even numbers of blocks, longer than the rings, whose CTAs
+take one and several items, with ragged last tiles, column ranges and rows. Both launchers are internal to the library
+(csrc/kernels.h), so they are called by their C++ names. Which cut a call takes is a rule on its sizes (gemm_cut)."""
+import ctypes
+
+import pytest
+import torch
+
+import hipster_b200 as hb
+from hipster_b200 import kernels as K_
+
+CUTS = [(ntc, G) for ntc in (4, 6, 8, 10, 12, 14, 16) for G in (8, 4)]
+SHAPES = [(100, 5120), (4999, 5120), (2100, 17408), (34816, 1024), (4096, 768), (40, 256)]
+
+
+class XQ8F(ctypes.Structure):
+    _fields_ = [("q", ctypes.c_void_p), ("sc", ctypes.c_void_p)]
+
+
+def sym(name, *argtypes):
+    f = getattr(hb.lib(), name)
+    f.argtypes = argtypes
+    return f
+
+
+CUT = "_ZN2hp15gemm_q4k_q8_cutEPKvRKNS_4XQ8FEPfiiiimPvPiP11CUstream_stbii"
+P, I, Z, B = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t, ctypes.c_bool
+
+
+def gemm_cut(N, K, R):
+    f = sym("_ZN2hp8gemm_cutEiiiPiS0_", I, I, I, P, P)
+    ntc, G = I(), I()
+    f(N, K, R, ctypes.addressof(ntc), ctypes.addressof(G))
+    return ntc.value, G.value
+
+
+def pack(R, K):
+    f = sym("_ZN2hp15gemm_pack_bytesEii", I, I)
+    f.restype = Z
+    return torch.full((f(R, K),), 0xA5, dtype=torch.uint8, device="cuda")
+
+
+def run_gemm(wt, xq, N, K, R, ldy, cut, err):
+    y = torch.full((hb.lib().hp_gemv_parts(N, K), R, ldy), float("nan"), device="cuda")
+    f = sym(CUT, P, P, P, I, I, I, I, Z, P, P, P, B, I, I)
+    x, pk = XQ8F(xq.q.data_ptr(), xq.sc.data_ptr()), pack(R, K)
+    hb.check(f(wt.data_ptr(), ctypes.addressof(x), y.data_ptr(), N, K, R, ldy, R * ldy, pk.data_ptr(), err.data_ptr(), torch.cuda.current_stream().cuda_stream, True, *cut))
+    return y
+
+
+def run_gemv(wt, xq, N, K, R, ldy, err):
+    L = hb.lib()
+    y = torch.full((L.hp_gemv_parts(N, K), R, ldy), float("nan"), device="cuda")
+    f = sym("_ZN2hp17gemv_q4k_q8_partsEPKvRKNS_4XQ8FEPfiiiimPiP11CUstream_stbbb", P, P, P, I, I, I, I, Z, P, P, B, B, B)
+    for r0 in range(0, R, 32):
+        x = XQ8F(xq.q.data_ptr() + L.hp_xq8_q_bytes(r0, K), xq.sc.data_ptr() + L.hp_xq8_sc_bytes(r0, K)) if r0 else XQ8F(xq.q.data_ptr(), xq.sc.data_ptr())
+        hb.check(f(wt.data_ptr(), ctypes.addressof(x), y.data_ptr() + 4 * r0 * ldy, N, K, min(32, R - r0), ldy, R * ldy, err.data_ptr(),
+                   torch.cuda.current_stream().cuda_stream, False, True, False))
+    return y
+
+
+@pytest.fixture(scope="module")
+def weights():
+    out = {}
+    for i, (N, K) in enumerate(SHAPES):
+        g = torch.Generator(device="cuda").manual_seed(i)
+        blk = torch.randint(0, 256, (N * (K // 256), 144), dtype=torch.uint8, device="cuda", generator=g)
+        blk[:, :4] = torch.randn((blk.shape[0], 2), device="cuda", generator=g).mul_(0.01).abs_().half().view(torch.uint8)
+        out[N, K] = K_.repack_tiled(blk.reshape(-1), N, K, 0)
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ntc,G", CUTS)
+def test_every_cut_gives_the_bits_of_the_gemv(weights, ntc, G):
+    for N, K in SHAPES:
+        for R in {8 * ntc - 3, 8 * ntc + 1, 16 * ntc + 5} if N < 30000 else {8 * ntc + 8}:
+            ldy = N + 5
+            x = torch.randn((R, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(R))
+            xq = K_.quantize_x_q8(x); err = torch.zeros(1, dtype=torch.int32, device="cuda")
+            got, want = run_gemm(weights[N, K], xq, N, K, R, ldy, (ntc, G), err), run_gemv(weights[N, K], xq, N, K, R, ldy, err)
+            assert err.item() == 0
+            assert not torch.isnan(want[:, :, :N]).any()
+            assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (N, K, R)   # and nothing beyond column N
+
+
+@pytest.mark.parametrize("ntc,G", [(5, 8), (0, 8), (18, 8), (2, 8), (-4, 8), (8, 2), (8, 16), (8, 0)])
+def test_cuts_that_do_not_exist_are_refused(ntc, G):
+    f = sym(CUT, P, P, P, I, I, I, I, Z, P, P, P, B, I, I)       # refused on the host, before any pointer is used
+    x = XQ8F(4096, 4096)
+    assert f(4096, ctypes.addressof(x), 4096, 40, 256, 8, 40, 320, 4096, 4096, None, False, ntc, G) == 1
+    assert b"no cut" in hb.lib().hp_last_error()
+
+
+def test_the_rule_takes_tested_cuts_only_and_all_widths_occur():
+    seen = set()
+    for E, F, heads, kv in ((5120, 17408, 24, 4), (2048, 0, 24, 2), (512, 1024, 4, 2)):
+        lins = [(16480 if E > 512 else 1544, E), (heads * 512 + kv * 512, E), (E, heads * 256), (E, 2 * E)] + ([(2 * F, E), (E, F)] if F else [])
+        for N, K in lins:
+            seen |= {gemm_cut(N, K, R) for R in range(33, 513)}
+    assert seen <= set(CUTS)
+    assert {c[0] for c in seen} == {4, 6, 8, 10, 12, 14, 16}
