@@ -41,7 +41,7 @@ def test_prefill_equals_chunked_forward_and_oracle():
     eng.prefill(0, prompt[:10], pos0=0, with_mtp=True)          # two calls for one prompt: the second continues the first
     eng.prefill(0, prompt[10:], pos0=10, with_mtp=True)
     prev = np.zeros(cfg.n_embd, dtype=np.float32)
-    for p0, p1 in [(0, 8), (8, 10), (10, 18), (18, 21)]:         # the chunks hp_prefill used
+    for p0, p1 in [(0, 8), (8, 10), (10, 18), (18, 21)]:         # the 8-row passes whose bits hp_prefill reproduces
         toks = prompt[p0:p1]; T = len(toks)
         ref.forward([(0, toks, p0)]); ref.accept(0, T)
         h = ref.h_nextn(T)

@@ -1,6 +1,7 @@
 """hp_prefill over more than one 8-row pass (the chunked GEMM path) against the CPU oracle's 8-row passes, bit for bit: sizes
-around the edges of its row tiles (8), of the GEMV / GEMM rule (32), of the column ranges (32, 64, 128) and of a chunk (512);
-the tail rows, the draft block's cache and hidden rows, and the recurrent state (through the pass that follows)."""
+around the edges of its row tiles (8), of the GEMV / GEMM rule (32) and of a chunk (512), one and several attention batches per
+chunk and several chunks per prompt; the tail rows, the draft block's cache and hidden rows, the recurrent state (through the
+pass that follows) and pending accepts. (The GEMM's column ranges: test_gemm_gpu.py.)"""
 import numpy as np
 import pytest
 
@@ -63,6 +64,79 @@ def test_prefill_chunks_fill_the_draft_block(n):
     eng.close()
 
 
+def oracle_prefill(ref, slot, prompt, pos0, prev, with_mtp):
+    """hp_prefill as 8-row passes of the oracle; prev: hidden row in front of the prompt -> rows of the last pass, its last row."""
+    for p in range(0, len(prompt), 8):
+        T = min(8, len(prompt) - p)
+        ref.forward([(slot, prompt[p:p + T], pos0 + p)]); ref.accept(slot, T)
+        h = ref.h_nextn(T)
+        if with_mtp:
+            ref.mtp_forward(slot, prompt[p:p + T], np.vstack([prev[None, :], h[:T - 1]]), pos0 + p)
+        prev = h[T - 1].copy()
+    return T, prev
+
+
+@pytest.mark.parametrize("over,n0,n,batches", [(dict(n_head=24, n_head_kv=2, max_ctx=1024), 400, 501, 4),    # 4 rows per group: batches of 128, 128, 128, 117
+                                               (dict(max_ctx=1024), 500, 512, 2),                            # 8 rows per group
+                                               (dict(n_head=24, n_head_kv=2, max_ctx=700), 150, 515, 2)])    # chunks of 264 and 251 rows, two batches each
+def test_prefill_attention_in_several_batches(over, n0, n, batches):
+    cfg = hb.ModelCfg.preset("tiny", **over)
+    gr = min(8, 48 // (cfg.n_head // cfg.n_head_kv))             # rows per attention row group
+    size = n if n <= 512 else (-(-n // 2) + 7) & ~7
+    rows, end = n - (n > 512) * size, n0 + n                     # the last chunk
+    per = max(32, (32 * -(-cfg.max_ctx // 128) // -(-end // 128)) * gr & ~7)
+    assert -(-rows // per) == batches
+    eng = hb.Engine(cfg); ref = orc.Model(cfg)
+    prompt = [int(x) for x in np.random.default_rng(n).integers(0, cfg.n_vocab, size=n0 + n)]
+    eng.prefill(0, prompt[:n0], with_mtp=False); eng.prefill(0, prompt[n0:], pos0=n0, with_mtp=False)
+    _, prev = oracle_prefill(ref, 0, prompt[:n0], 0, None, False)
+    T, prev = oracle_prefill(ref, 0, prompt[n0:], n0, prev, False)
+    assert np.array_equal(bits(eng.logits(1)[0]), bits(ref.logits(T)[T - 1]))
+    assert np.array_equal(bits(eng.h_nextn(T)[1:]), bits(ref.h_nextn(T)[1:]))
+    for e in (eng, ref):
+        e.forward([(0, [9, 8, 7], n0 + n)])
+    assert np.array_equal(bits(eng.logits(3)), bits(ref.logits(3)))
+    eng.close()
+
+
+def test_prefill_several_chunks_fill_the_draft_block():
+    cfg = hb.ModelCfg.preset("tiny", max_ctx=1100)
+    eng = hb.Engine(cfg); ref = orc.Model(cfg)
+    n = 1030                                                     # chunks of 344, 344 and 342 rows
+    prompt = [int(x) for x in np.random.default_rng(n).integers(0, cfg.n_vocab, size=n)]
+    eng.prefill(1, prompt, with_mtp=True)
+    T, prev = oracle_prefill(ref, 1, prompt, 0, np.zeros(cfg.n_embd, dtype=np.float32), True)
+    assert np.array_equal(bits(eng.logits(1)[0]), bits(ref.logits(T)[T - 1]))
+    assert np.array_equal(bits(eng.mtp_h(T)), bits(ref.mtp_h(T)))
+    tok = int(eng.topk(0, 1)[0][0])
+    eng.mtp_forward(1, [tok], eng.h_nextn_ptr(), n)              # attends over the draft block's K/V rows of every chunk
+    ref.mtp_forward(1, [tok], prev[None, :], n)
+    assert np.array_equal(bits(eng.mtp_logits(1)), bits(ref.mtp_logits(1)))
+    eng.close()
+
+
+@pytest.mark.parametrize("decide", ["before", "after"])
+def test_prefill_with_other_slots_rows_pending(decide):
+    """Slot 1 has rows of which a prefix is accepted before or after the prompt of slot 0, whose own pending rows make the
+    prompt commit every slot's."""
+    cfg = hb.ModelCfg.preset("tiny", max_ctx=128)
+    eng = hb.Engine(cfg); ref = orc.Model(cfg)
+    a, b, c, prompt = [[int(x) for x in np.random.default_rng(i).integers(0, cfg.n_vocab, size=n)] for i, n in enumerate((4, 5, 6, 37))]
+    for e in (eng, ref):
+        e.forward([(0, a, 0), (1, b, 0)])
+        e.accept(0, 3)
+        if decide == "before" or e is ref:                       # the oracle keeps one pass' rows only
+            e.accept(1, 2)
+    eng.prefill(0, prompt, pos0=3, with_mtp=False)
+    oracle_prefill(ref, 0, prompt, 3, None, False)
+    if decide == "after":
+        eng.accept(1, 2)
+    for e in (eng, ref):
+        e.forward([(1, c, 2), (0, [1, 2], 40)])
+    assert np.array_equal(bits(eng.logits(8)), bits(ref.logits(8)))
+    eng.close()
+
+
 def test_chunk_buffers_come_with_the_first_long_prompt_and_only_where_they_fit():
     """A model loads with what its passes need, also where the buffers of the prompt chunks (about 170 MB for this shape)
     would not fit beside it; prompts then run as 8-row passes with the same bits, and as chunks once there is room."""
@@ -92,9 +166,7 @@ def test_chunk_buffers_come_with_the_first_long_prompt_and_only_where_they_fit()
 
     def check(slot, prompt):
         eng.prefill(slot, prompt, with_mtp=False)
-        for p in range(0, len(prompt), 8):
-            T = min(8, len(prompt) - p)
-            ref.forward([(slot, prompt[p:p + T], p)]); ref.accept(slot, T)
+        T, _ = oracle_prefill(ref, slot, prompt, 0, None, False)
         assert np.array_equal(bits(eng.logits(1)[0]), bits(ref.logits(T)[T - 1]))
         assert np.array_equal(bits(eng.h_nextn(T)[1:]), bits(ref.h_nextn(T)[1:]))
 
