@@ -38,7 +38,8 @@ __global__ void __launch_bounds__(256) k_argmax_part(const float* __restrict__ x
     const int r = blockIdx.y, c0 = blockIdx.x * AM_CHUNK, c1 = min(n, c0 + AM_CHUNK);
     const float* xr = x + (size_t)r * ld;
     float bv = -INFINITY; int bi = -1;
-    // bound by latency (a block reads 32 KB once): all loads of a thread in flight before the first comparison
+    // bound by latency (a block reads 32 KB once): all loads of a thread in flight before the first comparison (both launches, 1 x 248320:
+    // 3.54 us with a loop of load and compare, 3.29 so; 24 rows 5.54 and 5.49)
     constexpr int NV = AM_CHUNK / 256;
     float v[NV];
 #pragma unroll

@@ -373,9 +373,11 @@ static int lin_class_bit(const Lin& l, const hp_model_cfg& c) {
     return l.N == 2 * c.n_ff ? 16 : l.K == c.n_ff ? 32 : l.N == c.n_vocab ? 64 : l.K == c.n_embd ? 128 : 256;
 }
 // A linear over the rows of a prompt chunk; both kernels give the same bits. Up to 32 rows are one pass of the GEMV over the
-// weights; beyond that it streams them again. GEMV against GEMM of the 27B layer's in-, out-projection, gate|up and down (us):
-// 32 rows 42 + 20 + 87 + 52 = 199 against 43 + 31 + 76 + 66 = 217; 48 rows 62 + 33 + 127 + 74 = 296 against
-// 52 + 37 + 94 + 80 = 264.
+// weights; beyond that it streams them again. One line for all projections, where their sum over a 27B layer turns. GEMV against
+// GEMM (us), GDN in-, out-projection, gate|up and down: 24 rows 26 + 13 + 50 + 29 = 118 against 38 + 27 + 72 + 62 = 198;
+// 32 rows 42 + 16 + 86 + 55 = 198 against 38 + 27 + 72 + 62 = 198; 48 rows 60 + 27 + 120 + 77 = 283 against
+// 47 + 32 + 89 + 76 = 244. Single projections turn elsewhere: gate|up below 32 rows, the out-projection between 64 and 96; of
+// the 2048-wide model the in-projections near 48 (GDN) and 128 (attention), the out-projection between 96 and 128.
 int Engine::prefill_lin(const Lin& l, float* out, int ld, size_t part_stride, int R) {
     if (R <= 32) return gemv_q4k_q8_parts(l.wt, xq_, out, l.N, l.K, R, ld, part_stride, err_, s_, pdl_, true);
     return gemm_q4k_q8_parts(l.wt, xq_, out, l.N, l.K, R, ld, part_stride, pf_pack_, err_, s_, pdl_);

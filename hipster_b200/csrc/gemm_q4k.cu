@@ -6,10 +6,11 @@
 // sums of a 16-row tile cut where the GEMV's partition cuts them (K parts, warp boundaries of the tile's CTA) and added
 // in the same order. A row therefore has the same bits whichever of the two kernels computed it.
 //
-// What bounds it: the fp32 update, 3 packed fp32 instructions per two outputs and sub-block: 16 register operand reads, 8
-// clocks per SM sub-partition with their shared-memory loads, 10.4 with the TMEM loads (the int -> float conversions run
-// beside them). The int8 mma.sync of the GEMV takes 14.7 clocks per 16x8x32 on this chip and does not overlap with the
-// fp32 pipe. Hence:
+// What bounds it: the fp32 update, two conversions and three packed fp32 instructions per two outputs and sub-block. From
+// registers alone a 16x8x32 tile of it takes 15.3 clocks of an SM sub-partition; the int8 mma.sync of the GEMV takes 8.0 and
+// does not overlap with it (23.9 together). In place this kernel takes 36 to 47 clocks per tile at 512 rows (34816 x 5120: 690
+// us) and 60 at 32 (72 us), the GEMV 72 at 32 rows (86 us): the rest is TMEM and shared-memory loads, addresses and waits.
+// Hence:
 //   * one CTA per SM, M = 128 weight rows (8 tiles of 16), N = 32..128 pass rows, one tcgen05.mma (K = 32) per sub-block,
 //     never accumulating: TMEM only hands the int32 dots over to the update, in slots of 2 or 4 sub-blocks;
 //   * 8 update warps (4 TMEM lane quadrants x 2 column halves) read the dots with 16x256b loads, which leave a lane two
@@ -25,7 +26,7 @@
 //   * one warp streams the weights (2304-byte tile chunks, ring of 4 blocks, primed before the dependency wait), one the
 //     activations, one thread issues the MMAs.
 // Registers: 512 threads x 128 at launch; the update warps take 184 (8 x 32 threads) from the conversion warps (72) and the
-// last four warps (56): 63488 in all.
+// last four warps (56): 63488 in all. Only the form of 8 column tiles spills (68 bytes stored, 180 loaded).
 // Every wait is bounded and reports through the device status word.
 #include "hp_common.cuh"
 #include "kernels.h"
@@ -460,8 +461,8 @@ int launch_tc(const TcArgs& a, const XQ8F& x, int grid, cudaStream_t s, bool pdl
 
 size_t gemm_pack_bytes(int R, int K) { return (size_t)((R + 7) / 8 + 15) * (size_t)(K / 256) * 2560; }
 // The cut of the rows into column ranges of ntc tiles of 8, and of the weight tiles into items of G = 8 or 4 (the latter leaves
-// every second tile position empty). An item of 20 blocks takes 53, 71 and 89 us at ntc = 8, 12 and 16: 4.5 us per tile and
-// what 4 tiles would take; the cut with the least time over the rounds of the SMs is taken.
+// every second tile position empty). An item of 20 blocks takes 36, 56, 72 and 90 us at ntc = 4, 8, 12 and 16: 4.5 us
+// for each of ntc + 4; the cut with the least time over the rounds of the SMs is taken.
 void gemm_cut(int N, int K, int R, int* ntc, int* G) {
     const int t8 = (R + 7) / 8, tiles = (N + 15) / 16, P = gemv_num_parts(N, K / 256);
     long best = 0; *ntc = 0;

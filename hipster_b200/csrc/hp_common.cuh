@@ -171,7 +171,9 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // GEMV, the MoE kernels (work before the dependency wait: ring set-up, router rows), the SiLU kernel (-0.13 ms per dense
 // round: its CTAs sit beside the gate|up GEMV's and start the moment it ends) and attention gain, while programmatic
 // edges on the row norms and the GDN kernel cost ~0.1 ms per round each, so while a stream is being captured the default
-// mask switches those and the bookkeeping classes off. HIPSTER_B200_PDL_OFF=<mask> overrides both.
+// mask switches those and the bookkeeping classes off. HIPSTER_B200_PDL_OFF=<mask> overrides both. Work in front of the wait
+// may read only what nobody writes while the library runs: the engine's own weights. What a caller hands to a public entry
+// point is read behind it, since the kernels in front (and the caller's) may trigger before they have waited themselves.
 inline int pdl_off_mask(cudaStream_t s) {
     static const int env = [] { const char* e = getenv("HIPSTER_B200_PDL_OFF"); return e ? atoi(e) : -1; }();
     if (env >= 0) return env;
