@@ -173,7 +173,8 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // edges on the row norms and the GDN kernel cost ~0.1 ms per round each, so while a stream is being captured the default
 // mask switches those and the bookkeeping classes off. HIPSTER_B200_PDL_OFF=<mask> overrides both. Work in front of the wait
 // may read only what nobody writes while the library runs: the engine's own weights. What a caller hands to a public entry
-// point is read behind it, since the kernels in front (and the caller's) may trigger before they have waited themselves.
+// point is read behind it, since the kernels in front (and the caller's) may trigger before they have waited themselves
+// (or behind a memset: hp_moe_layer's router rows).
 inline int pdl_off_mask(cudaStream_t s) {
     static const int env = [] { const char* e = getenv("HIPSTER_B200_PDL_OFF"); return e ? atoi(e) : -1; }();
     if (env >= 0) return env;
