@@ -54,10 +54,11 @@ __global__ void __launch_bounds__(D) k_gdn_pf_conv(GdnPrefillParams a) {
 }
 
 // grid (8, v heads), 128 threads: 16 rows of the head's state, thread = 16 columns of one row (k_gdn's layout), in registers
-// for the whole chunk. Bound by the dependent chain of a row. One pass over the 16 columns carries two chains: the output of
-// row r (m . q) and, with the next decay applied, the first product of row r + 1 (m . k), so that a row costs 16 dependent
-// steps and one round of shuffles instead of two of each (301 rows: 124 us before). q, k, v and gates arrive by asynchronous
-// copies, 16 rows ahead. 8 CTAs of a head instead of 4: the chain is the same and the 384 CTAs of 48 heads spread over all SMs.
+// for the whole chunk. Bound by the dependent chain of a row (16 fmaf, 3 shuffles, 16 fmaf): q, k, v and gates arrive by
+// asynchronous copies, 16 rows ahead. 8 CTAs of a head instead of 4: the chain is the same and the 384 CTAs of 48 heads
+// spread over all SMs. 301 rows: 124 us under ncu. (One pass over the columns for the output of a row and the first product of
+// the next one, so half the dependent steps per row, took 141: its extra registers, moves and branches cost more. Prefill of
+// 301 tokens of the 27B shape 85.0 ms so, 85.8 with the shared pass; 512 tokens 123.3 and 124.4.)
 __global__ void __launch_bounds__(D) k_gdn_pf_scan(GdnPrefillParams a) {
     __shared__ __align__(16) float sqk[2][PF_CH][PF_STR];
     __shared__ float sv[2][PF_CH][16];
@@ -80,57 +81,38 @@ __global__ void __launch_bounds__(D) k_gdn_pf_scan(GdnPrefillParams a) {
         for (int e = tid; e < n * 2; e += D) cp_async4(reinterpret_cast<float*>(&sg[s][e >> 1]) + (e & 1), a.gate + ((size_t)(r0 + (e >> 1)) * a.n_v + h) * 2 + (e & 1));
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto load16 = [](float2 (&d)[8], const float* p) {
-#pragma unroll
-        for (int i = 0; i < 8; i += 2) { const float4 v = *reinterpret_cast<const float4*>(p + 2 * i); d[i] = make_float2(v.x, v.y); d[i + 1] = make_float2(v.z, v.w); }
-    };
     stage(0, 0);
-    cp_async_wait_all();
-    __syncthreads();
-    float2 kr[8];
-    float dot = 0.f;
-    load16(kr, &sqk[0][0][160 + 20 * ck]);
-    {
-        const float d0 = sg[0][0].y; const float2 dc2 = make_float2(d0, d0);
+    for (int r0 = 0, s = 0; r0 < a.T; r0 += PF_CH, s ^= 1) {
+        if (r0 + PF_CH < a.T) { stage(r0 + PF_CH, s ^ 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+        else cp_async_wait_all();
+        __syncthreads();
+        const int n = min(PF_CH, a.T - r0);
+        for (int it = 0; it < n; ++it) {
+            const float beta = sg[s][it].x, decay = sg[s][it].y;
+            const float* kk = &sqk[s][it][160 + 20 * ck]; const float* qq = &sqk[s][it][20 * ck];
+            float2 kr[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { m[i] = mul2(m[i], dc2); dot = fmaf(m[i].x, kr[i].x, dot); dot = fmaf(m[i].y, kr[i].y, dot); }
-    }
-#pragma unroll 2
-    for (int r = 0; r < a.T; ++r) {
-        const int s = (r / PF_CH) & 1, it = r % PF_CH;
-        const bool more = r + 1 < a.T;
-        if (it == 0) {
-            if (r) __syncthreads();   // every thread has left the other stage
-            if (r + PF_CH < a.T) stage(r + PF_CH, s ^ 1);
-        }
-        if (it == PF_CH - 1 && more) { cp_async_wait_all(); __syncthreads(); }   // the next stage has landed
-        const int sn = ((r + 1) / PF_CH) & 1, in = (r + 1) % PF_CH;
-        float2 kn[8], q[8]; float dn = 0.f, decay = 1.f;
-        load16(q, &sqk[s][it][20 * ck]);
-        if (more) { load16(kn, &sqk[sn][in][160 + 20 * ck]); decay = sg[sn][in].y; }
-        const float beta = sg[s][it].x, vj = sv[s][it][jl];
+            for (int i = 0; i < 8; i += 2) { const float4 v = *reinterpret_cast<const float4*>(kk + 2 * i); kr[i] = make_float2(v.x, v.y); kr[i + 1] = make_float2(v.z, v.w); }
+            const float2 dc2 = make_float2(decay, decay);
+            float dot = 0.f;
 #pragma unroll
-        for (int off = 1; off < 8; off <<= 1) dot = dot + __shfl_xor_sync(0xffffffffu, dot, off);
-        const float delta = (vj - dot) * beta;
-        const float2 dl2 = make_float2(delta, delta), dc2 = make_float2(decay, decay);
-        float o = 0.f;
-        if (more) {
+            for (int i = 0; i < 8; ++i) { m[i] = mul2(m[i], dc2); dot = fmaf(m[i].x, kr[i].x, dot); dot = fmaf(m[i].y, kr[i].y, dot); }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                fma2(m[i], dl2, kr[i]); o = fmaf(m[i].x, q[i].x, o); o = fmaf(m[i].y, q[i].y, o);
-                m[i] = mul2(m[i], dc2); dn = fmaf(m[i].x, kn[i].x, dn); dn = fmaf(m[i].y, kn[i].y, dn);
+            for (int off = 1; off < 8; off <<= 1) dot = dot + __shfl_xor_sync(0xffffffffu, dot, off);
+            const float delta = (sv[s][it][jl] - dot) * beta;
+            const float2 dl2 = make_float2(delta, delta);
+            float o = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {
+                const float4 qv = *reinterpret_cast<const float4*>(qq + 2 * i);
+                fma2(m[i], dl2, kr[i]); o = fmaf(m[i].x, qv.x, o); o = fmaf(m[i].y, qv.y, o);
+                fma2(m[i + 1], dl2, kr[i + 1]); o = fmaf(m[i + 1].x, qv.z, o); o = fmaf(m[i + 1].y, qv.w, o);
             }
-        } else {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { fma2(m[i], dl2, kr[i]); o = fmaf(m[i].x, q[i].x, o); o = fmaf(m[i].y, q[i].y, o); }
+            for (int off = 1; off < 8; off <<= 1) o = o + __shfl_xor_sync(0xffffffffu, o, off);
+            if (ck == 0) a.o[((size_t)(r0 + it) * a.n_v + h) * D + j] = o * 0.08838834764831845f;
         }
-#pragma unroll
-        for (int off = 1; off < 8; off <<= 1) o = o + __shfl_xor_sync(0xffffffffu, o, off);
-        if (ck == 0) a.o[((size_t)r * a.n_v + h) * D + j] = o * 0.08838834764831845f;
-        dot = dn;
-        if (more)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) kr[i] = kn[i];
+        __syncthreads();   // the stage is free again
     }
 #pragma unroll
     for (int i = 0; i < 8; i += 2) *reinterpret_cast<float4*>(Mrow + 2 * i) = make_float4(m[i].x, m[i].y, m[i + 1].x, m[i + 1].y);
