@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(D) k_gdn_pf_conv(GdnPrefillParams a) {
 // grid (8, v heads), 128 threads: 16 rows of the head's state, thread = 16 columns of one row (k_gdn's layout), in registers
 // for the whole chunk. Bound by the dependent chain of a row (16 fmaf, 3 shuffles, 16 fmaf): q, k, v and gates arrive by
 // asynchronous copies, 16 rows ahead. 8 CTAs of a head instead of 4: the chain is the same and the 384 CTAs of 48 heads
-// spread over all SMs. 301 rows: 124 us under ncu. (One pass over the columns for the output of a row and the first product of
+// spread over all SMs. 301 rows: 127 us under ncu. (One pass over the columns for the output of a row and the first product of
 // the next one, so half the dependent steps per row, took 141: its extra registers, moves and branches cost more. Prefill of
 // 301 tokens of the 27B shape 85.0 ms so, 85.8 with the shared pass; 512 tokens 123.3 and 124.4.)
 __global__ void __launch_bounds__(D) k_gdn_pf_scan(GdnPrefillParams a) {
