@@ -16,6 +16,10 @@
 // the CTA's K part are staged once per CTA in shared memory by bulk copies. One fp32 update per sub-block follows, in
 // block order:
 //     acc = fmaf((d*sc) * xd, (float)idot, acc);  acc = fmaf(-(dmin*mn), xs, acc);
+// Besides HBM the inner loop is bound by the shared-memory pipe and by issue: per 16x256 block and column tile 64 clocks of weights, 64
+// of activations and, read 64 bits at a time, 64 of column scales (128 with 128-bit reads) at one warp instruction per 4 to 16
+// clocks. Up to 4 rows (decode, drafts, short verify passes) take the form FEW. Decode of the 27B shape 5.33 ms a pass with 128-bit
+// reads and the full tile, 4.76 with both changes.
 // A tile whose blocks are spread over several warps of the CTA is finished through shared memory: the partial sums
 // are added in warp order. Each K part writes its own output plane; the planes are added in part order by the
 // consumer (or by the small reduction kernel of the public entry point). No atomics, no cross-CTA traffic.
@@ -35,19 +39,22 @@ constexpr int SK_XG = 4;   // copy pairs per column tile of the activations; NT 
 // Tile-major (TILED = true, the engine repacks to it at load; same bytes, permuted): for every 16-row tile and block a
 // contiguous 2304-byte chunk = 16 headers (16 B each) + nibbles stored [j][lane][row g 8 B | row g+8 8 B], so a stage
 // is ONE bulk copy and every lane fetches its two rows of a 64-element group with one 128-bit shared-memory load.
-template <int CB, bool TILED> struct SkGeom {
-    static constexpr int ROW_STRIDE = CB == 2 ? 288 : 160;   // 288 = 2*128+32, 160 = 128+32: rows land on distinct 32-byte bank groups
-    static constexpr int STAGE_BYTES = TILED ? CB * 2304 : 16 * ROW_STRIDE;
+// SB: blocks per stage.
+template <int SB, bool TILED> struct SkGeom {
+    static constexpr int ROW_STRIDE = SB == 2 ? 288 : 160;   // 288 = 2*128+32, 160 = 128+32: rows land on distinct 32-byte bank groups
+    static constexpr int STAGE_BYTES = TILED ? SB * 2304 : 16 * ROW_STRIDE;
     static constexpr int FIXED = GEMV_WARPS * SK_STAGES * STAGE_BYTES + 1024;
 };
 
 // XG: the activations are read from global memory (L2) inside the loop instead of being staged in shared memory: the
 // form for several column tiles whose activations do not fit beside the rings (small matrices with a long K).
-template <int NT, int CB, bool TILED, bool XG = false>
+// CB: blocks per unit of the partition, SB: blocks per ring stage (1 or CB). FEW: at most 4 rows, see FewCols.
+template <int NT, int CB, int SB, bool TILED, bool XG = false, bool FEW = false>
 __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __restrict__ W, const uint4* __restrict__ xq, const float4* __restrict__ xsc,
                                                                 float* __restrict__ y, int N, int nb, int P, int R, int ldy, size_t part_stride,
                                                                 int* __restrict__ err, int late) {
-    using Geo = SkGeom<CB, TILED>;
+    using Geo = SkGeom<SB, TILED>;
+    constexpr int SPU = CB / SB;                           // stages per unit
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* ring_all = smem;
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + GEMV_WARPS * SK_STAGES * Geo::STAGE_BYTES);
@@ -58,16 +65,16 @@ __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const GemvCta ct = gemv_cta(N, nb, P, blockIdx.x);
-    const int C = nbp / CB, kb0 = ct.part * nbp;
+    const int C = nbp / CB, CS = nbp / SB, kb0 = ct.part * nbp;
     const int cu = (ct.t1 - ct.t0) * C;                    // units of this CTA
     const int weff = cu < GEMV_WARPS ? cu : GEMV_WARPS;
     const int u0 = warp < weff ? gemv_warp_start(cu, weff, warp) : 0, u1 = warp < weff ? gemv_warp_start(cu, weff, warp + 1) : 0;
-    const int nunits = u1 - u0;
+    const int nst = (u1 - u0) * SPU;                       // stages of this warp
     uint8_t* ring = ring_all + warp * SK_STAGES * Geo::STAGE_BYTES;
     const uint32_t bar0 = smem_u32(&bars[warp * SK_STAGES]);
     const uint32_t xbar = smem_u32(&bars[GEMV_WARPS * SK_STAGES]);
     const uint32_t row_bytes = (uint32_t)nb * 144u;
-    constexpr uint32_t unit_bytes = CB * 144u;
+    constexpr uint32_t piece_bytes = SB * 144u;            // of one row in a stage (row-major)
     y += (size_t)ct.part * part_stride;
     pdl_launch_dependents();   // the next kernel may be scheduled; it waits for this one to finish before using its output
     if (lane == 0) {
@@ -77,34 +84,33 @@ __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __
     }
     __syncthreads();
 
-    // issue cursor (tile, chunk) of the next unit to fetch; advanced incrementally, no divisions in the loop
-    const int first_tile = ct.t0 + (nunits ? u0 / C : 0);
-    int it_tile = first_tile, it_chunk = nunits ? u0 % C : 0, it_i = 0;
-    const uint8_t* it_src = TILED ? W + ((size_t)it_tile * nb + kb0 + it_chunk * CB) * 2304
-                                  : W + ((size_t)it_tile * 16 + (lane & 15)) * row_bytes + (size_t)(kb0 + it_chunk * CB) * 144;
+    // issue cursor (tile, stage of it) of the next stage to fetch; advanced incrementally, no divisions in the loop
+    const int first_tile = ct.t0 + (nst ? u0 / C : 0);
+    int it_tile = first_tile, it_chunk = nst ? u0 % C * SPU : 0, it_i = 0;
+    const uint8_t* it_src = TILED ? W + ((size_t)it_tile * nb + kb0 + it_chunk * SB) * 2304
+                                  : W + ((size_t)it_tile * 16 + (lane & 15)) * row_bytes + (size_t)(kb0 + it_chunk * SB) * 144;
     const uint32_t ring_lane = smem_u32(ring) + (TILED ? 0 : (lane & 15) * Geo::ROW_STRIDE);
     auto issue = [&]() {
         const int s = it_i % SK_STAGES;
         const uint32_t bar = bar0 + 8 * s;
         if constexpr (TILED) {
-            if (lane == 0) { mbar_expect_tx(bar, CB * 2304u); bulk_g2s(ring_lane + s * Geo::STAGE_BYTES, it_src, CB * 2304u, bar); }
-            ++it_i; ++it_chunk; it_src += CB * 2304;
-            if (it_chunk == C) { it_chunk = 0; ++it_tile; it_src += (size_t)(nb - C * CB) * 2304; }
+            if (lane == 0) { mbar_expect_tx(bar, SB * 2304u); bulk_g2s(ring_lane + s * Geo::STAGE_BYTES, it_src, SB * 2304u, bar); }
+            ++it_i; ++it_chunk; it_src += SB * 2304;
+            if (it_chunk == CS) { it_chunk = 0; ++it_tile; it_src += (size_t)(nb - nbp) * 2304; }
         } else {
             const int nrows = min(16, N - it_tile * 16);
-            if (lane == 0) mbar_expect_tx(bar, unit_bytes * (uint32_t)nrows);
+            if (lane == 0) mbar_expect_tx(bar, piece_bytes * (uint32_t)nrows);
             __syncwarp();
-            if (lane < nrows) bulk_g2s(ring_lane + s * Geo::STAGE_BYTES, it_src, unit_bytes, bar);
-            ++it_i; ++it_chunk; it_src += unit_bytes;
-            if (it_chunk == C) { it_chunk = 0; ++it_tile; it_src += (size_t)16 * row_bytes - (size_t)C * unit_bytes; }
+            if (lane < nrows) bulk_g2s(ring_lane + s * Geo::STAGE_BYTES, it_src, piece_bytes, bar);
+            ++it_i; ++it_chunk; it_src += piece_bytes;
+            if (it_chunk == CS) { it_chunk = 0; ++it_tile; it_src += (size_t)16 * row_bytes - (size_t)CS * piece_bytes; }
         }
     };
     // Constant weights do not depend on the previous kernel: prime the ring before waiting for it. Weights that a kernel
     // earlier in the stream may have written (late) are complete and visible only behind the wait, whoever triggered the
     // early launch of this one.
     if (late) pdl_wait();
-    for (int i = 0; i < SK_STAGES && i < nunits; ++i) issue();
-
+    for (int i = 0; i < SK_STAGES && i < nst; ++i) issue();
     pdl_wait();
 
     if (!XG && warp == 0) {   // quantised activations of blocks [kb0, kb0 + nbp), all NT column tiles, by bulk copies. Per column
@@ -124,62 +130,71 @@ __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __
         }
     }
 
-    float2 acc[NT][2];   // [n][0] = row g, cols 2t,2t+1 ; [n][1] = row g+8
+    static_assert(!FEW || (NT == 1 && !XG), "FEW is a form of the single column tile");
+    constexpr int NA = FEW ? 1 : 2, NV = 2 * NA;   // accumulator pairs and values of a lane per column tile
+    const FewCols few(lane);
+    float2 acc[NT][NA];   // [n][0] = row g, cols 2t,2t+1 ; [n][1] = row g+8 (FEW: [0] = the lane's row and columns)
     auto zero_acc = [&]() {
-#pragma unroll
-        for (int n = 0; n < NT; ++n) { acc[n][0] = make_float2(0.f, 0.f); acc[n][1] = make_float2(0.f, 0.f); }
-    };
-    zero_acc();
-    auto store_tile = [&](int tile, const float (&v)[NT][4]) {
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int row = tile * 16 + g + ((k & 2) ? 8 : 0), col = n * 8 + 2 * t + (k & 1);
+            for (int i = 0; i < NA; ++i) acc[n][i] = make_float2(0.f, 0.f);
+    };
+    zero_acc();
+    auto store_tile = [&](int tile, const float (&v)[NT][NV]) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                const int row = tile * 16 + (FEW ? few.row : g + ((k & 2) ? 8 : 0)), col = n * 8 + (FEW ? few.col : 2 * t) + (k & 1);
                 if (row < N && col < R) y[(size_t)col * ldy + row] = v[n][k];
             }
     };
     // a tile covered by this warp alone is stored at once; otherwise the partial sum goes to shared memory
     // (slot 0 = the warp's first tile, slot 1 = its last tile) and is combined after the CTA barrier
     float* red = reinterpret_cast<float*>(ring_all);   // reused after every warp has drained its ring
-    float part_v[2][NT][4]; bool part_on[2] = {false, false}; int part_tile[2] = {0, 0};
+    float part_v[2][NT][NV]; bool part_on[2] = {false, false}; int part_tile[2] = {0, 0};
     auto flush = [&](int tile, bool whole) {
-        float v[NT][4];
+        float v[NT][NV];
 #pragma unroll
-        for (int n = 0; n < NT; ++n) { v[n][0] = acc[n][0].x; v[n][1] = acc[n][0].y; v[n][2] = acc[n][1].x; v[n][3] = acc[n][1].y; }
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int i = 0; i < NA; ++i) { v[n][2 * i] = acc[n][i].x; v[n][2 * i + 1] = acc[n][i].y; }
         if (whole) { store_tile(tile, v); return; }
         const int slot = tile == first_tile ? 0 : 1;
         part_on[slot] = true; part_tile[slot] = tile;
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) part_v[slot][n][k] = v[n][k];
+            for (int k = 0; k < NV; ++k) part_v[slot][n][k] = v[n][k];
     };
 
     // per-lane constant offsets
     const uint32_t w_lane = TILED ? 256 + lane * 16 : g * Geo::ROW_STRIDE + 16 + 8 * t;   // weights: row g (+8 rows: + 8*ROW_STRIDE)
-    const uint32_t hdr_lane = TILED ? g * 16 : g * Geo::ROW_STRIDE;      // header of row g (+8 rows: + HDR8)
+    const uint32_t hdr_lane = (FEW ? few.row : g) * (TILED ? 16 : Geo::ROW_STRIDE);       // header of row g (+8 rows: + HDR8); FEW: of the lane's row
+    const int x_lane = FEW ? few.frag : lane, xs_lane = FEW ? few.col >> 1 : t;           // this lane's fragment and scales of the activations
     constexpr int HDR8 = TILED ? 128 : 8 * Geo::ROW_STRIDE;
     constexpr int BLK_STRIDE = TILED ? 2304 : 144;
 
-    int cur_tile = first_tile, chunk = nunits ? u0 % C : 0;
+    int cur_tile = first_tile, chunk = nst ? u0 % C * SPU : 0;
     bool cur_from_start = chunk == 0;
     bool ok = XG ? true : mbar_wait(xbar, 0, err);
-    for (int i = 0; i < nunits && ok; ++i) {
+    for (int i = 0; i < nst && ok; ++i) {
         const int s = i % SK_STAGES;
         ok = mbar_wait(bar0 + 8 * s, (i / SK_STAGES) & 1, err);
         if (!ok) break;
         const uint8_t* st = ring + s * Geo::STAGE_BYTES;
-        const uint4* xqp = xq_s + ((XG ? kb0 : 0) + chunk * CB) * 128 + lane;
-        const float4* xsp = xsc_s + ((XG ? kb0 : 0) + chunk * CB) * 32 + t;
+        const uint4* xqp = xq_s + ((XG ? kb0 : 0) + chunk * SB) * 128 + x_lane;
+        const float4* xsp = xsc_s + ((XG ? kb0 : 0) + chunk * SB) * 32 + xs_lane;
 #pragma unroll
-        for (int blk = 0; blk < CB; ++blk) {
+        for (int blk = 0; blk < SB; ++blk) {
             // Scales of this lane's two rows (g, g+8), decoded in registers from the 16-byte headers. A 6-bit value v
             // becomes the float 8388608 + v by a byte permute into the mantissa of 0x4B000000, and
             // fmaf(d, 8388608 + v, -(d * 8388608)) is exactly d * v (one rounding of an exactly representable
             // product). Odd sub-blocks take the high nibbles unshifted (16 * q): their d carries the exact 1/16.
-            const RowScales ra = decode_scales(*reinterpret_cast<const uint4*>(st + hdr_lane + blk * BLK_STRIDE));
-            const RowScales rb = decode_scales(*reinterpret_cast<const uint4*>(st + hdr_lane + HDR8 + blk * BLK_STRIDE));
+            const RowScales ra = decode_scales(lds_u4_halves(st + hdr_lane + blk * BLK_STRIDE));
+            RowScales rb;
+            if constexpr (!FEW) rb = decode_scales(lds_u4_halves(st + hdr_lane + HDR8 + blk * BLK_STRIDE));
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 uint2 w0, w1;
@@ -190,56 +205,45 @@ __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __
                     w0 = *reinterpret_cast<const uint2*>(st + w_lane + blk * 144 + 32 * j);
                     w1 = *reinterpret_cast<const uint2*>(st + w_lane + 8 * Geo::ROW_STRIDE + blk * 144 + 32 * j);
                 }
-                const uint32_t alo[4] = {w0.x & 0x0F0F0F0Fu, w1.x & 0x0F0F0F0Fu, w0.y & 0x0F0F0F0Fu, w1.y & 0x0F0F0F0Fu};
-                const uint32_t ahi[4] = {w0.x & 0xF0F0F0F0u, w1.x & 0xF0F0F0F0u, w0.y & 0xF0F0F0F0u, w1.y & 0xF0F0F0F0u};
-                const float4 sa0 = ra.get(2 * j), sb0 = rb.get(2 * j);           // low-nibble sub-block: rows g, g+8
-                const float4 sa1 = ra.get(2 * j + 1), sb1 = rb.get(2 * j + 1);   // high-nibble sub-block
+                const Q4kGroup wg(w0, w1);
+                if constexpr (FEW) {
+                    wg.dot_few(acc[0][0], ra, j, few, xqp[(blk * 4 + j) * 32], Q4kGroup::cols_smem(xsp + (blk * 8 + 2 * j) * 4), Q4kGroup::cols_smem(xsp + (blk * 8 + 2 * j + 1) * 4));
+                } else {
+                    const Q4kGroup::Scales sc(ra, rb, j);
 #pragma unroll
-                for (int n = 0; n < NT; ++n) {
-                    const uint4* xfp = xqp + n * xstride * 128 + (blk * 4 + j) * 32;
-                    const float4* x0p = xsp + n * xstride * 32 + (blk * 8 + 2 * j) * 4;
-                    const uint4 xf = XG ? __ldcg(xfp) : *xfp;
-                    const float4 x0 = XG ? __ldcg(x0p) : *x0p;
-                    const float4 x1 = XG ? __ldcg(x0p + 4) : x0p[4];
-                    // The accumulator input carries 0x4B400000: the int32 result, read as fp32, is 12582912 + idot
-                    // exactly (|idot| < 2^22), so the int -> float conversion is one exact packed subtraction.
-                    int c0[4], c1[4];
-                    mma_u8s8_magic(c0, alo, xf.x, xf.y);
-                    mma_u8s8_magic(c1, ahi, xf.z, xf.w);
-                    const float2 xd0 = make_float2(x0.x, x0.y), xs0 = make_float2(x0.z, x0.w);
-                    const float2 xd1 = make_float2(x1.x, x1.y), xs1 = make_float2(x1.z, x1.w);
-                    const float2 mg = make_float2(-12582912.f, -12582912.f);
-                    // low-nibble sub-block 2j, then high-nibble sub-block 2j+1 (block order)
-                    fma2(acc[n][0], mul2(make_float2(sa0.x, sa0.y), xd0), add2(make_float2(__int_as_float(c0[0]), __int_as_float(c0[1])), mg));
-                    fma2(acc[n][0], make_float2(sa0.z, sa0.w), xs0);
-                    fma2(acc[n][1], mul2(make_float2(sb0.x, sb0.y), xd0), add2(make_float2(__int_as_float(c0[2]), __int_as_float(c0[3])), mg));
-                    fma2(acc[n][1], make_float2(sb0.z, sb0.w), xs0);
-                    fma2(acc[n][0], mul2(make_float2(sa1.x, sa1.y), xd1), add2(make_float2(__int_as_float(c1[0]), __int_as_float(c1[1])), mg));
-                    fma2(acc[n][0], make_float2(sa1.z, sa1.w), xs1);
-                    fma2(acc[n][1], mul2(make_float2(sb1.x, sb1.y), xd1), add2(make_float2(__int_as_float(c1[2]), __int_as_float(c1[3])), mg));
-                    fma2(acc[n][1], make_float2(sb1.z, sb1.w), xs1);
+                    for (int n = 0; n < NT; ++n) {
+                        const uint4* xfp = xqp + n * xstride * 128 + (blk * 4 + j) * 32;
+                        const float4* x0p = xsp + n * xstride * 32 + (blk * 8 + 2 * j) * 4;
+                        const uint4 xf = XG ? __ldcg(xfp) : *xfp;
+                        Q4kGroup::ColScales x0, x1;
+                        if constexpr (XG) {
+                            const float4 v0 = __ldcg(x0p), v1 = __ldcg(x0p + 4);
+                            x0 = {make_float2(v0.x, v0.y), make_float2(v0.z, v0.w)}; x1 = {make_float2(v1.x, v1.y), make_float2(v1.z, v1.w)};
+                        } else { x0 = Q4kGroup::cols_smem(x0p); x1 = Q4kGroup::cols_smem(x0p + 4); }
+                        wg.dot(acc[n][0], acc[n][1], sc, xf, x0, x1);
+                    }
                 }
             }
         }
         __syncwarp();   // every lane has read the stage before it is refilled
-        if (it_i < nunits) issue();
-        if (++chunk == C) {
+        if (it_i < nst) issue();
+        if (++chunk == CS) {
             flush(cur_tile, cur_from_start);
             zero_acc();
             chunk = 0; ++cur_tile; cur_from_start = true;
-        } else if (i + 1 == nunits) {
+        } else if (i + 1 == nst) {
             flush(cur_tile, false);
         }
     }
     // ---------------- tiles shared by several warps of this CTA: combine through shared memory in warp order
-    __syncthreads();   // every ring is drained: its memory becomes the exchange buffer [warp][slot][NT*4][32]
+    __syncthreads();   // every ring is drained: its memory becomes the exchange buffer [warp][slot][NT * NV][32]
 #pragma unroll
     for (int sl = 0; sl < 2; ++sl)
         if (part_on[sl])
 #pragma unroll
             for (int n = 0; n < NT; ++n)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) red[((warp * 2 + sl) * NT * 4 + n * 4 + k) * 32 + lane] = part_v[sl][n][k];
+                for (int k = 0; k < NV; ++k) red[((warp * 2 + sl) * NT * NV + n * NV + k) * 32 + lane] = part_v[sl][n][k];
     __syncthreads();
     if (!ok) return;
 #pragma unroll
@@ -252,17 +256,17 @@ __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __
         int src[GEMV_WARPS];
 #pragma unroll
         for (int ww = 0; ww < GEMV_WARPS; ++ww)
-            src[ww] = (ww >= w_first && ww <= warp) ? (ww * 2 + ((gemv_warp_start(cu, weff, ww) / C == tl) ? 0 : 1)) * NT * 4 : -1;
-        float v[NT][4];
+            src[ww] = (ww >= w_first && ww <= warp) ? (ww * 2 + ((gemv_warp_start(cu, weff, ww) / C == tl) ? 0 : 1)) * NT * NV : -1;
+        float v[NT][NV];
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
+            for (int k = 0; k < NV; ++k) {
                 float a = 0.f;
 #pragma unroll
                 for (int ww = 0; ww < GEMV_WARPS; ++ww)
                     if (src[ww] >= 0) {
-                        const float pv = red[(src[ww] + n * 4 + k) * 32 + lane];
+                        const float pv = red[(src[ww] + n * NV + k) * 32 + lane];
                         a = ww == w_first ? pv : a + pv;
                     }
                 v[n][k] = a;
@@ -364,28 +368,35 @@ __global__ void __launch_bounds__(F32_THREADS) k_gemv_q4k_f32(const uint8_t* __r
     }
 }
 
-template <int NT, int CB, bool TILED, bool XG = false>
+template <int NT, int CB, int SB, bool TILED, bool XG, bool FEW>
 int launch_sk2(const uint8_t* W, const void* xq, const void* xsc, float* y, int N, int nb, int P, int R, int ldy, size_t part_stride,
                int* err, cudaStream_t s, bool pdl, bool late) {
-    const size_t smem = SkGeom<CB, TILED>::FIXED + (XG ? 0 : (size_t)NT * (nb / P) * 2560);
+    const size_t smem = SkGeom<SB, TILED>::FIXED + (XG ? 0 : (size_t)NT * (nb / P) * 2560);
     static size_t attr_smem[MAX_DEVICES] = {};   // per device: the opt-in belongs to the device's copy of the kernel
     const int dev = current_device(); if (dev < 0) return HP_ECUDA;
-    if (smem > attr_smem[dev]) { HP_CUDA(cudaFuncSetAttribute(k_gemv_q4k_sk<NT, CB, TILED, XG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr_smem[dev] = smem; }
+    if (smem > attr_smem[dev]) { HP_CUDA(cudaFuncSetAttribute(k_gemv_q4k_sk<NT, CB, SB, TILED, XG, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr_smem[dev] = smem; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(GEMV_NCTA); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = s;
     cudaLaunchAttribute at[1]; at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = pdl && !(pdl_off_mask(s) & 64) ? 1 : 0;
-    HP_CUDA(cudaLaunchKernelEx(&cfg, k_gemv_q4k_sk<NT, CB, TILED, XG>, W, (const uint4*)xq, (const float4*)xsc, y, N, nb, P, R, ldy, part_stride, err, late ? 1 : 0));
+    HP_CUDA(cudaLaunchKernelEx(&cfg, k_gemv_q4k_sk<NT, CB, SB, TILED, XG, FEW>, W, (const uint4*)xq, (const float4*)xsc, y, N, nb, P, R, ldy, part_stride, err, late ? 1 : 0));
     return HP_OK;
 }
-template <int NT, bool XG = false>
+// the activations of ntile column tiles fit in shared memory beside a ring of SB blocks per stage
+template <int SB, bool TILED> bool sk_fits(int ntile, int nbp) { return (size_t)SkGeom<SB, TILED>::FIXED + (size_t)ntile * nbp * 2560 <= (size_t)GEMV_SMEM_LIMIT; }
+template <int NT, bool XG = false, bool FEW = false>
 int launch_sk(const uint8_t* W, bool tiled, const void* xq, const void* xsc, float* y, int N, int nb, int P, int R, int ldy, size_t part_stride,
               int* err, cudaStream_t s, bool pdl, bool late) {
-    const bool cb2 = (nb / P) % 2 == 0;
-    if (tiled) return cb2 ? launch_sk2<NT, 2, true, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late)
-                          : launch_sk2<NT, 1, true, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late);
-    return cb2 ? launch_sk2<NT, 2, false, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late)
-               : launch_sk2<NT, 1, false, XG>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late);
+    const int nbp = nb / P;
+    const bool cb2 = nbp % 2 == 0;
+    if (tiled) {
+        if (!cb2) return launch_sk2<NT, 1, 1, true, XG, FEW>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late);
+        // stages of one block where the activations leave no room for longer ones
+        if constexpr (NT == 3 && !XG) { if (!sk_fits<2, true>(NT, nbp)) return launch_sk2<NT, 2, 1, true, XG, FEW>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late); }
+        return launch_sk2<NT, 2, 2, true, XG, FEW>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late);
+    }
+    return cb2 ? launch_sk2<NT, 2, 2, false, XG, FEW>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late)
+               : launch_sk2<NT, 1, 1, false, XG, FEW>(W, xq, xsc, y, N, nb, P, R, ldy, part_stride, err, s, pdl, late);
 }
 
 // row-major ggml blocks -> tile-major chunks (see SkGeom); rows beyond N are zero (they contribute nothing).
@@ -440,10 +451,12 @@ int gemv_q4k_q8_parts(const void* W, const XQ8F& x, float* yparts, int N, int K,
     // all column tiles in one launch: their activations staged in shared memory beside the rings when they fit, read
     // from L2 inside the loop otherwise (small matrices with a long K: one launch instead of one per tile of 8 columns;
     // same per-column arithmetic either way)
-    const bool staged = ntile == 1 || (size_t)SkGeom<2, false>::FIXED + (size_t)ntile * nbp * 2560 <= (size_t)GEMV_SMEM_LIMIT;
+    // (three tiles of 20 blocks: 34816 x 5120 at 24 rows took 48 us from L2)
+    const bool staged = ntile == 1 || (tiled ? (nbp % 2 || ntile == 3 ? sk_fits<1, true>(ntile, nbp) : sk_fits<2, true>(ntile, nbp)) : (nbp % 2 ? sk_fits<1, false>(ntile, nbp) : sk_fits<2, false>(ntile, nbp)));
     const uint8_t* w = (const uint8_t*)W;
     int rc;
-    if (staged) {
+    if (R <= 4) rc = launch_sk<1, false, true>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl, late);
+    else if (staged) {
         switch (ntile) {
             case 1: rc = launch_sk<1>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl, late); break;
             case 2: rc = launch_sk<2>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl, late); break;

@@ -191,6 +191,19 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// 64-bit shared-memory reads. A 128-bit read takes four passes of the shared-memory pipe however few distinct addresses the warp has (16
+// clocks per warp of a sub-partition, measured with 4, 8 and 32), a 64-bit one a single pass (4 clocks) as long as the addresses fit in
+// 128 bytes: what several lanes read alike is fetched in two of these. volatile keeps the compiler from joining them again.
+__device__ __forceinline__ float2 lds_f2(const void* p) {
+    float2 v; asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_u32(p))); return v;
+}
+__device__ __forceinline__ uint4 lds_u4_halves(const void* p) {
+    uint4 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(smem_u32(p)));
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2+8];" : "=r"(v.z), "=r"(v.w) : "r"(smem_u32(p)));
+    return v;
+}
+
 // ---- shared pieces of the Q4_K tensor-core GEMV inner loop (dense GEMV and routed-expert GEMV) ----
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     float2 r;
@@ -237,6 +250,50 @@ __device__ __forceinline__ RowScales decode_scales(const uint4 hdr) {
     r.mn[1] = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
     return r;
 }
+
+// A tile of at most 4 pass rows: the 8 columns of the tensor-core tile hold them twice. Lane (g, t) finds the dots of
+// weight rows g and g + 8 with pass rows 2 (t & 1), + 1 in its accumulators, and the lane whose t differs by 2 the same ones:
+// lanes t < 2 take row g, the others row g + 8, so that a lane decodes the scales of one row and updates one pair of outputs.
+struct FewCols {
+    bool upper; int row, col, frag;   // the lane's weight row in the tile, the first of its two columns, its activation fragment
+    __device__ __forceinline__ explicit FewCols(int lane) : upper((lane & 2) != 0), row((lane >> 2) + ((lane & 2) ? 8 : 0)), col(2 * (lane & 1)), frag(((lane >> 2) & 3) * 4 + (lane & 3)) {}
+};
+// The 64 elements (sub-blocks 2 j: low nibbles, 2 j + 1: high nibbles) of a 16-row tile that a lane holds for weight rows g (w0)
+// and g + 8 (w1), and their update of the lane's accumulators: acc = fmaf((d*sc) * xd, idot, acc); acc = fmaf(-(dmin*mn), xs,
+// acc) per sub-block, in order. The accumulator input of the tensor-core tile carries 0x4B400000: the int32 result, read as
+// fp32, is 12582912 + idot exactly (|idot| < 2^22), so the int -> float conversion is one exact packed subtraction.
+struct Q4kGroup {
+    uint32_t alo[4], ahi[4];
+    __device__ __forceinline__ Q4kGroup() {}
+    __device__ __forceinline__ Q4kGroup(uint2 w0, uint2 w1)
+        : alo{w0.x & 0x0F0F0F0Fu, w1.x & 0x0F0F0F0Fu, w0.y & 0x0F0F0F0Fu, w1.y & 0x0F0F0F0Fu}, ahi{w0.x & 0xF0F0F0F0u, w1.x & 0xF0F0F0F0u, w0.y & 0xF0F0F0F0u, w1.y & 0xF0F0F0F0u} {}
+    struct Scales {   // of both rows and both sub-blocks: shared by all column tiles
+        float4 a0, b0, a1, b1;
+        __device__ __forceinline__ Scales() {}
+        __device__ __forceinline__ Scales(const RowScales& ra, const RowScales& rb, int j) : a0(ra.get(2 * j)), b0(rb.get(2 * j)), a1(ra.get(2 * j + 1)), b1(rb.get(2 * j + 1)) {}
+    };
+    struct ColScales { float2 d, s; };   // of the lane's two columns in one sub-block
+    static __device__ __forceinline__ ColScales cols_smem(const float4* p) { ColScales c; c.d = lds_f2(p); c.s = lds_f2(reinterpret_cast<const float*>(p) + 2); return c; }
+    static __device__ __forceinline__ void update(float2& acc, const float4& s, const ColScales& x, int i0, int i1) {
+        fma2(acc, mul2(make_float2(s.x, s.y), x.d), add2(make_float2(__int_as_float(i0), __int_as_float(i1)), make_float2(-12582912.f, -12582912.f)));
+        fma2(acc, make_float2(s.z, s.w), x.s);
+    }
+    // xf: activation fragment; x0, x1: column scales of the two sub-blocks
+    __device__ __forceinline__ void dot(float2& acc_g, float2& acc_g8, const Scales& s, const uint4& xf, const ColScales& x0, const ColScales& x1) const {
+        int c0[4], c1[4];
+        mma_u8s8_magic(c0, alo, xf.x, xf.y);
+        mma_u8s8_magic(c1, ahi, xf.z, xf.w);
+        update(acc_g, s.a0, x0, c0[0], c0[1]); update(acc_g8, s.b0, x0, c0[2], c0[3]);
+        update(acc_g, s.a1, x1, c1[0], c1[1]); update(acc_g8, s.b1, x1, c1[2], c1[3]);
+    }
+    __device__ __forceinline__ void dot_few(float2& acc, const RowScales& r, int j, const FewCols& few, const uint4& xf, const ColScales& x0, const ColScales& x1) const {
+        int c0[4], c1[4];
+        mma_u8s8_magic(c0, alo, xf.x, xf.y);
+        mma_u8s8_magic(c1, ahi, xf.z, xf.w);
+        update(acc, r.get(2 * j), x0, few.upper ? c0[2] : c0[0], few.upper ? c0[3] : c0[1]);
+        update(acc, r.get(2 * j + 1), x1, few.upper ? c1[2] : c1[0], few.upper ? c1[3] : c1[1]);
+    }
+};
 
 // int8 tensor-core tile: D(16x8,s32) = A(16x32,u8 row) * B(32x8,s8 col) + 0
 __device__ __forceinline__ void mma_u8s8(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {

@@ -469,7 +469,9 @@ __global__ void __launch_bounds__(MQ_WARPS * 32, 1) k_moe_gemv_quad(MoeGArgs a) 
     };
     for (int i = 0; i < DEPTH; ++i) issue();
     int cseg = u_lo < u_hi ? u_lo / ups : 0, c_us = u_lo < u_hi ? u_lo % ups : 0, staged = -1, ccount = 0;
-    int c0 = -1, c1 = -1;   // pair indices of this lane's columns 2t, 2t + 1
+    const FewCols fc(lane);
+    bool few = false;       // the staged segment has at most 4 columns (see FewCols)
+    int c0 = -1, c1 = -1;   // pair indices of this lane's columns 2t, 2t + 1 (few: fc.col, fc.col + 1)
     const uint4* xq4 = reinterpret_cast<const uint4*>(a.xq);
     const int nsb = a.xK >> 5, nk64 = a.xK >> 6;
     for (int cu = u_lo; cu < u_hi; ++cu) {
@@ -491,7 +493,9 @@ __global__ void __launch_bounds__(MQ_WARPS * 32, 1) k_moe_gemv_quad(MoeGArgs a) 
 #pragma unroll 8
                 for (int sb = qtid >> 4; sb < nsb; sb += 8) xsc_s[sb * 16 + w] = ssrc ? __ldcg(ssrc + (size_t)sb * 16) : 0.f;
             }
-            c0 = 2 * t < ncols ? __ldcg(&sg->cols[2 * t]) : -1; c1 = 2 * t + 1 < ncols ? __ldcg(&sg->cols[2 * t + 1]) : -1;
+            few = ncols <= 4;
+            const int ca = few ? fc.col : 2 * t;
+            c0 = ca < ncols ? __ldcg(&sg->cols[ca]) : -1; c1 = ca + 1 < ncols ? __ldcg(&sg->cols[ca + 1]) : -1;
             staged = cseg;
             quad_barrier(quad);
         }
@@ -504,31 +508,26 @@ __global__ void __launch_bounds__(MQ_WARPS * 32, 1) k_moe_gemv_quad(MoeGArgs a) 
 #pragma unroll
                 for (int blk = 0; blk < SB; ++blk) {
                     const int b = st * SB + blk;
-                    const RowScales ra = decode_scales(*reinterpret_cast<const uint4*>(sp + g * 16 + blk * 2304));
-                    const RowScales rb = decode_scales(*reinterpret_cast<const uint4*>(sp + g * 16 + 128 + blk * 2304));
-                    const uint4* xqp = xq_s + (size_t)b * 128 + lane;
-                    const float4* xsp = reinterpret_cast<const float4*>(xsc_s) + (size_t)b * 32 + t;
+                    const uint8_t* wp = sp + blk * 2304 + 256 + lane * 16;
+                    if (few) {
+                        const RowScales r = decode_scales(lds_u4_halves(sp + fc.row * 16 + blk * 2304));
+                        const uint4* xqp = xq_s + (size_t)b * 128 + fc.frag;
+                        const float4* xsp = reinterpret_cast<const float4*>(xsc_s) + (size_t)b * 32 + (fc.col >> 1);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint4 ww = *reinterpret_cast<const uint4*>(sp + 256 + lane * 16 + blk * 2304 + 512 * j);
-                        const uint32_t alo[4] = {ww.x & 0x0F0F0F0Fu, ww.z & 0x0F0F0F0Fu, ww.y & 0x0F0F0F0Fu, ww.w & 0x0F0F0F0Fu};
-                        const uint32_t ahi[4] = {ww.x & 0xF0F0F0F0u, ww.z & 0xF0F0F0F0u, ww.y & 0xF0F0F0F0u, ww.w & 0xF0F0F0F0u};
-                        const float4 sa0 = ra.get(2 * j), sb0 = rb.get(2 * j), sa1 = ra.get(2 * j + 1), sb1 = rb.get(2 * j + 1);
-                        const uint4 xf = xqp[j * 32];
-                        const float4 x0 = xsp[(2 * j) * 4], x1 = xsp[(2 * j + 1) * 4];
-                        const float2 xd0 = make_float2(x0.x, x0.y), xs0v = make_float2(x0.z, x0.w), xd1 = make_float2(x1.x, x1.y), xs1v = make_float2(x1.z, x1.w);
-                        int m0[4], m1[4];
-                        mma_u8s8_magic(m0, alo, xf.x, xf.y);
-                        mma_u8s8_magic(m1, ahi, xf.z, xf.w);
-                        const float2 mg = make_float2(-12582912.f, -12582912.f);
-                        fma2(acc0, mul2(make_float2(sa0.x, sa0.y), xd0), add2(make_float2(__int_as_float(m0[0]), __int_as_float(m0[1])), mg));
-                        fma2(acc0, make_float2(sa0.z, sa0.w), xs0v);
-                        fma2(acc1, mul2(make_float2(sb0.x, sb0.y), xd0), add2(make_float2(__int_as_float(m0[2]), __int_as_float(m0[3])), mg));
-                        fma2(acc1, make_float2(sb0.z, sb0.w), xs0v);
-                        fma2(acc0, mul2(make_float2(sa1.x, sa1.y), xd1), add2(make_float2(__int_as_float(m1[0]), __int_as_float(m1[1])), mg));
-                        fma2(acc0, make_float2(sa1.z, sa1.w), xs1v);
-                        fma2(acc1, mul2(make_float2(sb1.x, sb1.y), xd1), add2(make_float2(__int_as_float(m1[2]), __int_as_float(m1[3])), mg));
-                        fma2(acc1, make_float2(sb1.z, sb1.w), xs1v);
+                        for (int j = 0; j < 4; ++j) {
+                            const uint4 ww = *reinterpret_cast<const uint4*>(wp + 512 * j);
+                            Q4kGroup(make_uint2(ww.x, ww.y), make_uint2(ww.z, ww.w)).dot_few(acc0, r, j, fc, xqp[j * 32], Q4kGroup::cols_smem(xsp + 8 * j), Q4kGroup::cols_smem(xsp + 8 * j + 4));
+                        }
+                    } else {
+                        const RowScales ra = decode_scales(lds_u4_halves(sp + g * 16 + blk * 2304));
+                        const RowScales rb = decode_scales(lds_u4_halves(sp + g * 16 + 128 + blk * 2304));
+                        const uint4* xqp = xq_s + (size_t)b * 128 + lane;
+                        const float4* xsp = reinterpret_cast<const float4*>(xsc_s) + (size_t)b * 32 + t;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const uint4 ww = *reinterpret_cast<const uint4*>(wp + 512 * j);
+                            Q4kGroup(make_uint2(ww.x, ww.y), make_uint2(ww.z, ww.w)).dot(acc0, acc1, Q4kGroup::Scales(ra, rb, j), xqp[j * 32], Q4kGroup::cols_smem(xsp + 8 * j), Q4kGroup::cols_smem(xsp + 8 * j + 4));
+                        }
                     }
                 }
             }
@@ -539,33 +538,46 @@ __global__ void __launch_bounds__(MQ_WARPS * 32, 1) k_moe_gemv_quad(MoeGArgs a) 
         const int tile = c_us * MOE_UNIT_TILES + w4;
         if constexpr (MODE == 1) {
             if (ok) {
-                if (c0 >= 0) { a.y[(size_t)c0 * a.N + tile * 16 + g] = acc0.x; a.y[(size_t)c0 * a.N + tile * 16 + g + 8] = acc1.x; }
-                if (c1 >= 0) { a.y[(size_t)c1 * a.N + tile * 16 + g] = acc0.y; a.y[(size_t)c1 * a.N + tile * 16 + g + 8] = acc1.y; }
+                auto store = [&](float* y) {
+                    y += tile * 16;
+                    if (few) {
+                        if (c0 >= 0) y[(size_t)c0 * a.N + fc.row] = acc0.x;
+                        if (c1 >= 0) y[(size_t)c1 * a.N + fc.row] = acc0.y;
+                    } else {
+                        if (c0 >= 0) { y[(size_t)c0 * a.N + g] = acc0.x; y[(size_t)c0 * a.N + g + 8] = acc1.x; }
+                        if (c1 >= 0) { y[(size_t)c1 * a.N + g] = acc0.y; y[(size_t)c1 * a.N + g + 8] = acc1.y; }
+                    }
+                };
+                store(a.y);
                 // the same values into every other rank's exchange buffer: the transfer rides on the stores, tile by tile
                 // (the 8 lanes that share t write 32 consecutive bytes of a pair's row)
                 for (int q = 0; q < a.ep_world; ++q) {
                     if (a.ep_world <= 1 || q == a.ep_rank) continue;
-                    float* py = a.ep_x[q] + ep_off;
-                    if (c0 >= 0) { py[(size_t)c0 * a.N + tile * 16 + g] = acc0.x; py[(size_t)c0 * a.N + tile * 16 + g + 8] = acc1.x; }
-                    if (c1 >= 0) { py[(size_t)c1 * a.N + tile * 16 + g] = acc0.y; py[(size_t)c1 * a.N + tile * 16 + g + 8] = acc1.y; }
+                    store(a.ep_x[q] + ep_off);
                 }
             }
         } else {
             // rows g = gate of feature 8 * tile + g, rows g + 8 = up of the same feature; the unit's 4 tiles (this quad's 4
             // warps) are one 32-feature quantisation group per column: amax / 127, q = rint(v * (127 / amax)),
             // s = d * sum(q) (gemv.hip:36-51)
+            if (few) {   // gate and up of a feature are in lanes whose t differs by 2: both get both, and only t < 2 stores
+                const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, acc0.x, 2), __shfl_xor_sync(0xffffffffu, acc0.y, 2));
+                acc1 = fc.upper ? acc0 : o; acc0 = fc.upper ? o : acc0;
+            }
+            const bool mine = ok && !(few && fc.upper);
+            const int te = few ? t & 1 : t;   // column pair in the exchange words
             const float act[2] = {silu_det(acc0.x) * acc1.x, silu_det(acc0.y) * acc1.y};
             float am[2] = {fabsf(act[0]), fabsf(act[1])};
 #pragma unroll
             for (int off = 4; off < 32; off <<= 1) { am[0] = fmaxf(am[0], __shfl_xor_sync(0xffffffffu, am[0], off)); am[1] = fmaxf(am[1], __shfl_xor_sync(0xffffffffu, am[1], off)); }
-            if (g == 0) { ex_amax[w4 * 8 + t * 2] = am[0]; ex_amax[w4 * 8 + t * 2 + 1] = am[1]; }
+            if (g == 0) { ex_amax[w4 * 8 + te * 2] = am[0]; ex_amax[w4 * 8 + te * 2 + 1] = am[1]; }
             quad_barrier(quad);
             int qs[2]; float dd[2];
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 float amax = 0.f;
 #pragma unroll
-                for (int w = 0; w < 4; ++w) amax = fmaxf(amax, ex_amax[w * 8 + t * 2 + c]);
+                for (int w = 0; w < 4; ++w) amax = fmaxf(amax, ex_amax[w * 8 + te * 2 + c]);
                 dd[c] = amax / 127.f;
                 const float id = amax > 0.f ? 127.f / amax : 0.f;
                 const int q = __float2int_rn(act[c] * id);
@@ -574,16 +586,16 @@ __global__ void __launch_bounds__(MQ_WARPS * 32, 1) k_moe_gemv_quad(MoeGArgs a) 
                 for (int off = 4; off < 32; off <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
                 qs[c] = sum;
                 const int pair = c ? c1 : c0;
-                if (pair >= 0 && ok) a.oq[xq_q_index(pair, c_us * 32 + 8 * w4 + g, a.F)] = (int8_t)q;
+                if (pair >= 0 && mine) a.oq[xq_q_index(pair, c_us * 32 + 8 * w4 + g, a.F)] = (int8_t)q;
             }
-            if (g == 0) { ex_sum[w4 * 8 + t * 2] = qs[0]; ex_sum[w4 * 8 + t * 2 + 1] = qs[1]; }
+            if (g == 0) { ex_sum[w4 * 8 + te * 2] = qs[0]; ex_sum[w4 * 8 + te * 2 + 1] = qs[1]; }
             quad_barrier(quad);
-            if (w4 == 0 && g == 0 && ok) {
+            if (w4 == 0 && g == 0 && mine) {
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
                     const int pair = c ? c1 : c0;
                     if (pair >= 0) {
-                        const int sum = ex_sum[t * 2 + c] + ex_sum[8 + t * 2 + c] + ex_sum[16 + t * 2 + c] + ex_sum[24 + t * 2 + c];
+                        const int sum = ex_sum[te * 2 + c] + ex_sum[8 + te * 2 + c] + ex_sum[16 + te * 2 + c] + ex_sum[24 + te * 2 + c];
                         const size_t di = xq_d_index(pair, c_us, a.F); a.osc[di] = dd[c]; a.osc[di + 2] = dd[c] * (float)sum;
                     }
                 }

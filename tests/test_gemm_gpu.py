@@ -85,6 +85,24 @@ def test_every_cut_gives_the_bits_of_the_gemv(weights, ntc, G):
             assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (N, K, R)   # and nothing beyond column N
 
 
+# the tile-major form of the GEMV on both sides of its row limits (4 rows; three column tiles whose activations leave room for one-block
+# stages only: 20 blocks), against the row-major one
+@pytest.mark.gpu
+@pytest.mark.parametrize("R", [1, 4, 5, 8, 16, 17, 24])
+@pytest.mark.parametrize("N,K", [(100, 5120), (16480, 5120), (4096, 768), (2100, 17408)])
+def test_tile_major_gemv_gives_the_bits_of_the_row_major_one(N, K, R):
+    g = torch.Generator(device="cuda").manual_seed(R)
+    blk = torch.randint(0, 256, (N * (K // 256), 144), dtype=torch.uint8, device="cuda", generator=g)
+    blk[:, :4] = torch.randn((blk.shape[0], 2), device="cuda", generator=g).mul_(0.01).abs_().half().view(torch.uint8)
+    xq = K_.quantize_x_q8(torch.randn((R, K), device="cuda", generator=g)); err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    planes = run_gemv(K_.repack_tiled(blk.reshape(-1), N, K, 0), xq, N, K, R, N, err)
+    got = planes[0].clone()
+    for p in planes[1:]:
+        got += p
+    assert err.item() == 0
+    assert torch.equal(got.view(torch.int32), K_.gemv_q4k_q8(blk, xq, N, K).view(torch.int32))
+
+
 @pytest.mark.parametrize("ntc,G", [(5, 8), (0, 8), (18, 8), (2, 8), (-4, 8), (8, 2), (8, 16), (8, 0)])
 def test_cuts_that_do_not_exist_are_refused(ntc, G):
     f = sym(CUT, P, P, P, I, I, I, I, Z, P, P, P, B, I, I)       # refused on the host, before any pointer is used

@@ -53,6 +53,16 @@ def test_gemv_q8_bit_exact_vs_oracle(N, K, R):
     assert np.array_equal(bits(y), bits(want))
 
 
+# up to 4 rows take the form that holds each column twice, 5 the full tile: one tile, a ragged last one, odd and even K parts, a tile shared by all warps
+@pytest.mark.parametrize("R", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("N,K", [(16, 256), (50, 768), (100, 5120), (7, 17408)])
+def test_gemv_q8_few_rows_bit_exact_vs_oracle(N, K, R):
+    W = synth.q4k_matrix(N, K, seed=N); x = synth.activations(R, K, seed=R)
+    y = K_.gemv_q4k_q8(dev(W), K_.quantize_x_q8(dev(x)), N, K).cpu().numpy()
+    K_.device_status()
+    assert np.array_equal(bits(y), bits(orc.gemv_q4k_q8(W, *orc.quantize_x_q8(x), N, K)))
+
+
 def test_gemv_q8_row_result_independent_of_row_count():
     # the reference's T-invariance contract (README.md:65: T>1 vs T=1 logit difference 0.0000)
     N, K = 256, 5120

@@ -36,6 +36,23 @@ def test_moe_layer_bit_exact_vs_oracle(n_expert, k, E, F, T):
     assert np.allclose(w_o, w64, rtol=1e-5, atol=0)
 
 
+@pytest.mark.parametrize("n_expert,k,T", [(8, 2, 24), (4, 1, 19), (16, 3, 7)])
+def test_experts_of_every_number_of_rows(n_expert, k, T):
+    """Segments of 1 to 8 columns: up to 4 take the form that holds each column twice, more the full tile, and an expert
+    of more than 8 rows both."""
+    E, F = 512, 256
+    rng = np.random.default_rng(T)
+    xn = rng.normal(0, 1, size=(T, E)).astype(np.float32)
+    router = (rng.normal(0, 1, size=(n_expert + 1, E)) / np.sqrt(E)).astype(np.float32)
+    egu = synth.q4k_matrix(n_expert * 2 * F, E, seed=1).reshape(-1); edn = synth.q4k_matrix(n_expert * E, F, seed=2).reshape(-1)
+    sgu = synth.q4k_matrix(2 * F, E, seed=3).reshape(-1); sdn = synth.q4k_matrix(E, F, seed=4).reshape(-1)
+    d = lambda a: torch.from_numpy(a).cuda()
+    ids, w, y = K_.moe_layer(d(xn), d(router), d(egu), d(edn), d(sgu), d(sdn), F, n_expert, k)
+    K_.device_status()
+    ids_o, _, y_o, _ = orc.moe_layer(xn, router, egu, edn, sgu, sdn, E, F, n_expert, k)
+    assert np.array_equal(ids.cpu().numpy(), ids_o) and np.array_equal(bits(y.cpu().numpy()), bits(y_o))
+
+
 def test_router_ties_go_to_the_lower_expert_id():
     """Two experts with identical router rows get identical probabilities: the lower id must be ranked first."""
     n_expert, k, E, F, T = 64, 4, 512, 256, 3
