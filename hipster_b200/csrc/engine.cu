@@ -412,7 +412,7 @@ int Engine::attn_block(const LayerW& L, uint16_t* kc, uint16_t* vc, size_t kv_st
         p.planes = yparts_; p.P = L.in_proj.P; p.part_stride = (size_t)R * ld;
     } else HP_TRY(lin(L.in_proj, big_, ld, R)); p.ld = ld; p.n_head = c_.n_head; p.n_kv = c_.n_head_kv; p.n_rot = c_.n_rot;
     p.q_norm = L.q_norm; p.k_norm = L.k_norm; p.rope = rope_; p.row_pos = d_desc_ + D_POS; p.row_slot = d_desc_ + D_SLOT; p.row_group = d_desc_ + D_RGROUP; p.groups = d_desc_ + D_GROUPS;
-    p.kc = kc; p.vc = vc; p.kv_stride = kv_stride; p.max_ctx = c_.max_ctx; p.pO = pO_; p.pm = pm_; p.pl = pl_; p.nsplit_max = nsplit_max_;
+    p.kc = kc; p.vc = vc; p.kv_stride = kv_stride; p.max_ctx = c_.max_ctx; p.pO = pO_; p.pm = pm_; p.pl = pl_; p.nsplit_max = nsplit_max_; p.group_rows = grp_rows_;
     p.out = nullptr; p.xq = xq_; p.eps = c_.rms_eps;
     if (kv_only) return attn_rope_kv(p, R, s_);   // only this layer's K/V rows are wanted
     if (!gemv_only_ && !(prof_skip_ & 4)) { HP_TRY(attn_rope_kv(p, R, s_)); HP_TRY(attn_decode(p, R, ngroups, s_)); }
@@ -532,6 +532,7 @@ int Engine::flush_commits() {
 int Engine::fill_desc(const hp_slot_req* reqs, int S, int* rows, int* ngroups, bool with_seqs) {
     int* d = h_desc_; int r0 = 0, ng = 0;
     const int gr = attn_rows_per_group();
+    grp_rows_ = 0;
     for (int i = 0; i < S; ++i) {
         const hp_slot_req& r = reqs[i];
         if (with_seqs) { d[D_SEQS + i * 4] = r0; d[D_SEQS + i * 4 + 1] = r.T; d[D_SEQS + i * 4 + 2] = r.slot; d[D_SEQS + i * 4 + 3] = 0; }
@@ -540,7 +541,7 @@ int Engine::fill_desc(const hp_slot_req* reqs, int S, int* rows, int* ngroups, b
             HP_REQUIRE(ng < MAXR, "pass needs more than %d attention row groups", MAXR);   // cannot happen while rows <= MAXR; keeps the table write in bounds
             d[D_GROUPS + ng * 4] = r0 + t0; d[D_GROUPS + ng * 4 + 1] = tn; d[D_GROUPS + ng * 4 + 2] = r.slot; d[D_GROUPS + ng * 4 + 3] = r.pos + t0;
             for (int t = t0; t < t0 + tn; ++t) d[D_RGROUP + r0 + t] = ng;
-            ++ng;
+            grp_rows_ = std::max(grp_rows_, tn); ++ng;
         }
         for (int t = 0; t < r.T; ++t) { d[D_TOK + r0 + t] = r.tokens[t]; d[D_POS + r0 + t] = r.pos + t; d[D_SLOT + r0 + t] = r.slot; }
         r0 += r.T;
@@ -749,7 +750,7 @@ int Engine::prefill_attn(const LayerW& L, uint16_t* kc, uint16_t* vc, size_t kv_
     if (kv_only) return HP_OK;
     for (const PfBatch& b : pf_batches_) {
         AttnParams q = p; q.planes = nullptr;
-        q.qkv = big_ + (size_t)b.row0 * ld; q.row_pos += b.row0; q.row_slot += b.row0; q.row_group += b.row0; q.groups += 4 * b.g0; q.xq = xq_rows(xq_, b.row0, c_.n_head * 256);
+        q.group_rows = attn_rows_per_group(); q.qkv = big_ + (size_t)b.row0 * ld; q.row_pos += b.row0; q.row_slot += b.row0; q.row_group += b.row0; q.groups += 4 * b.g0; q.xq = xq_rows(xq_, b.row0, c_.n_head * 256);
         HP_TRY(attn_decode(q, b.rows, b.ng, s_));
     }
     return lin_parts(L.out_proj, R);
@@ -1045,7 +1046,7 @@ int Engine::spec_begin(int slot, int id_last, int pos, const float* h_pending_de
 int Engine::attn_rows_per_group() const { return std::max(1, std::min(8, ATTN_MAX_PAIRS / (c_.n_head / c_.n_head_kv))); }
 int Engine::enqueue_round(int S, int n) {
     const int E = c_.n_embd, gr = attn_rows_per_group();
-    auto groups = [&](int Tm) { return S * ((Tm + gr - 1) / gr); };
+    auto groups = [&](int Tm) { grp_rows_ = std::min(gr, Tm); return S * ((Tm + gr - 1) / gr); };   // of a pass of Tm rows per slot
     HP_CUDA(cudaMemcpyAsync(d_specin_, h_spec_, SI_INTS * 4, cudaMemcpyHostToDevice, s_));
     for (int i = 0; i < n; ++i) {   // draft, chained on the MTP's own h (spec27b.cpp:81-85, batchfn.cpp:98-104)
         HP_CUDA(launch_pdl<2>(k_spec_setup, dim3(1), dim3(32), 0, s_, d_spec_, d_specin_, d_desc_, 0, i, n, S, gr));

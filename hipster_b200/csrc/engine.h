@@ -104,7 +104,7 @@ private:
     int* replay_n_ = nullptr; std::vector<int> pend_, last_r0_, last_T_;
     // work
     float *x_ = nullptr, *xn_ = nullptr, *big_ = nullptr, *yparts_ = nullptr, *logits_ = nullptr, *mlogits_ = nullptr, *h_ = nullptr, *mh_ = nullptr, *emb_ = nullptr;
-    float *pO_ = nullptr, *pm_ = nullptr, *pl_ = nullptr; int nsplit_max_ = 0;
+    float *pO_ = nullptr, *pm_ = nullptr, *pl_ = nullptr; int nsplit_max_ = 0, grp_rows_ = 0;   // split partials, splits of the whole context; most rows of an attention group of the current pass
     XQ8F xq_{nullptr, nullptr}, xq2_{nullptr, nullptr};
     float *rlogits_ = nullptr, *moe_w_ = nullptr, *moe_v_ = nullptr; void* moe_segs_ = nullptr; int* moe_ctl_ = nullptr; unsigned long long* moe_touched_ = nullptr; int* moe_ids_ = nullptr; int* route_cnt_ = nullptr; Lin moe_out_;
     int e_lo_ = 0, e_hi_ = 0, ep_world_ = 1; void* nccl_comm_ = nullptr; bool ep_failed_ = false;

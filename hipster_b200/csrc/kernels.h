@@ -108,12 +108,13 @@ struct AttnParams {
     float* qkv; int ld, n_head, n_kv, n_rot;            // rows [q_full n_head x 512 | k n_kv x 256 | v n_kv x 256]
     const float* planes = nullptr; int P = 0; size_t part_stride = 0;   // optional: the projection as K-part planes, summed by the rope kernel into qkv
     const void* q_norm; const void* k_norm; const void* rope;   // bf16 [256] x 2; float2 (cos, sin) [max_ctx][n_rot/2]
-    const int* row_pos; const int* row_slot; const int* row_group; const int* groups;   // device descriptors; group = {r0, T, slot, pos0}
+    const int* row_pos; const int* row_slot; const int* row_group; const int* groups;   // device descriptors; group = {r0, T, slot, pos0}; all nullptr: one sequence,
+    int imm_pos0 = 0, imm_gr = 1;                        // rows 0 .. of slot 0 at positions imm_pos0 .., imm_gr rows per group
+    int group_rows = 0;                                  // upper bound of the rows of a group (0: unknown)
     void* kc; void* vc; size_t kv_stride; int max_ctx;   // f16 [slot][n_kv][max_ctx][256] for this layer
     float* pO; float* pm; float* pl; int nsplit_max;     // split partials
     float* out; XQ8F xq; float eps;
 };
-size_t attn_smem_bytes();
 size_t attn_partial_floats(int ngroups, int n_kv, int nsplit_max);
 int attn_rope_kv(const AttnParams& p, int rows, cudaStream_t s);          // reference k_qk_norm_rope_kv (ops.hip:363-411)
 int attn_decode(const AttnParams& p, int rows, int ngroups, cudaStream_t s);   // reference attn_decode_mq (ops.h:72)
