@@ -178,7 +178,7 @@ int hp_q4k_repack_tiled(const void* w_dev, void* w_tiled_dev, size_t N, int K, i
     return hp::gemv_repack_tiled(w_dev, w_tiled_dev, N, K, (cudaStream_t)stream, interleave_half);
     HP_GUARD_END
 }
-// workspace of hp_moe_layer: router logits | ticket counters | per-pair outputs | quantised activations of the pairs | segments | control words
+// workspace of hp_moe_layer: router logits | per-pair outputs | ticket counters | quantised activations of the pairs | segments | control words
 namespace {
 struct MoeWs { size_t logits, cnt, v, q2, sc2, segs, ctl, total; };
 MoeWs moe_ws(int T, int E, int F, int n_expert, int k) {
@@ -186,8 +186,8 @@ MoeWs moe_ws(int T, int E, int F, int n_expert, int k) {
     const size_t pairs = (size_t)T * (k + 1);
     MoeWs w; size_t o = 0;
     w.logits = o; o += al((size_t)T * (n_expert + 1) * 4);
-    w.cnt = o; o += al(32 * 4);
     w.v = o; o += al(pairs * E * 4);
+    w.cnt = o; o += al(32 * 4);   // from here on: cleared at the start of a call
     w.q2 = o; o += al(hp::xq_q_bytes((int)pairs, F));
     w.sc2 = o; o += al(hp::xq_sc_floats((int)pairs, F) * 4);
     w.segs = o; o += al(hp::moe_seg_bytes());
@@ -206,9 +206,8 @@ int hp_moe_layer(const float* xn_dev, const void* xq_q_dev, const void* xq_sc_de
     const MoeWs w = moe_ws(T, E, F, n_expert, k);
     char* ws = (char*)workspace_dev; const int ns = k + 1;
     float* logits = (float*)(ws + w.logits); int* cnt = (int*)(ws + w.cnt); float* v = (float*)(ws + w.v);
-    // the router kernel fetches its rows of router_dev in front of its dependency wait: the memsets keep its start behind all that the caller enqueued
-    HP_CUDA(cudaMemsetAsync(cnt, 0, 32 * 4, s));
-    HP_CUDA(cudaMemsetAsync(ws + w.q2, 0, w.total - w.q2, s));
+    // the router kernel fetches its rows of router_dev in front of its dependency wait: the memset keeps its start behind all that the caller enqueued
+    HP_CUDA(cudaMemsetAsync(cnt, 0, w.total - w.cnt, s));
     hp::MoeRouteParams rp; rp.W = router_dev; rp.x = xn_dev; rp.logits = logits; rp.E = n_expert; rp.K = E; rp.k = k; rp.T = T; rp.ids = ids_dev; rp.w = weights_dev; rp.ticket = cnt;
     rp.e_lo = 0; rp.e_hi = n_expert; rp.own_shared = 1; rp.segs = ws + w.segs; rp.ctl = (int*)(ws + w.ctl); rp.err = hp::device_err_flag();
     { const int rc = hp::moe_route_group(rp, s); if (rc) return rc; }

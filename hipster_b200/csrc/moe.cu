@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 1) k_moe_gemv_grouped(MoeGArgs
 }
 
 // ---- the same GEMVs with the work cut by quads of warps ------------------------------------------------------------
-// A CTA is three quads of four warps. A quad owns a contiguous range of work units (segment, 4 tiles), i.e. mostly one
+// A CTA is four quads of four warps. A quad owns a contiguous range of work units (segment, 4 tiles), i.e. mostly one
 // or two segments: it gathers the segment's <= 8 activation columns ONCE into shared memory in the layout of the dense
 // kernel (so a lane fetches its int8 fragment and its columns' scales with three 128-bit shared loads per 64 weights
 // instead of nine global loads), and its warps take one tile of every unit each (warp w: tile w), streamed through a
@@ -419,7 +419,10 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 1) k_moe_gemv_grouped(MoeGArgs
 // the quantisation of the launch time to whole units. MODE 0: the 32-feature quantisation group spans the quad's four
 // tiles: amax (a maximum) and the integer sum of the quantised values go through shared memory between two quad
 // barriers. Per output element the arithmetic is unchanged: one warp, blocks in order along K, no split.
-constexpr int MQ_WARPS = 12, MQ_QUADS = 3, MQ_AUX = 2048;   // bytes after the rings: barriers + the quads' exchange words
+// Bound by the latency of a warp's serial chain (24 rows: DRAM 45 %, issue 38 %, no pipe above 33 % of its peak with three quads and rings
+// of 3 stages): four quads with rings of 2 hold fewer bytes per warp and as many per SM, and one layer of 24 rows takes 116 us instead
+// of 125.
+constexpr int MQ_WARPS = 16, MQ_QUADS = 4, MQ_AUX = 2048;   // bytes after the rings: barriers + the quads' exchange words
 __device__ __forceinline__ void quad_barrier(int quad) { asm volatile("bar.sync %0, 128;" ::"r"(quad + 1) : "memory"); }
 template <int MODE, int SB, int DEPTH>
 __global__ void __launch_bounds__(MQ_WARPS * 32, 1) k_moe_gemv_quad(MoeGArgs a) {
@@ -679,9 +682,9 @@ static int launch_quad(const MoeGArgs& a, size_t smem, cudaStream_t s) {
     HP_CUDA(launch_pdl<8>(k_moe_gemv_quad<MODE, SB, DEPTH>, dim3(GEMV_NCTA), dim3(MQ_WARPS * 32), smem, s, a));
     return HP_OK;
 }
-// the quad form when the three quads' activation buffers fit beside the rings (K <= 2048 for the gate|up projection),
+// the quad form when the four quads' activation buffers fit beside the rings (K <= 2048 for the gate|up projection),
 // the one-warp-per-unit form otherwise
-static size_t quad_smem(const MoeGArgs& a) { const int sb = a.nb % 2 == 0 ? 2 : 1, depth = sb == 2 ? 3 : 6; return (size_t)MQ_WARPS * depth * sb * 2304 + MQ_AUX + (size_t)MQ_QUADS * a.nb * 2560; }
+static size_t quad_smem(const MoeGArgs& a) { const int sb = a.nb % 2 == 0 ? 2 : 1, depth = sb == 2 ? 2 : 4; return (size_t)MQ_WARPS * depth * sb * 2304 + MQ_AUX + (size_t)MQ_QUADS * a.nb * 2560; }
 static bool quad_form(const MoeGArgs& a) {
     static const bool v1 = getenv("HIPSTER_B200_MOE_UNITS") != nullptr;
     return !v1 && quad_smem(a) <= 227 * 1024 && a.tiles % MOE_UNIT_TILES == 0;
@@ -691,7 +694,7 @@ static int launch_experts(const MoeGArgs& a, bool few, cudaStream_t s) {
     const int sb = a.nb % 2 == 0 ? 2 : 1;
     const size_t smem = quad_smem(a);
     if (!quad_form(a)) return launch_grouped_sb<MODE>(a, few, s);
-    return sb == 2 ? launch_quad<MODE, 2, 3>(a, smem, s) : launch_quad<MODE, 1, 6>(a, smem, s);
+    return sb == 2 ? launch_quad<MODE, 2, 2>(a, smem, s) : launch_quad<MODE, 1, 4>(a, smem, s);
 }
 int moe_experts_grouped(const MoeGroupParams& p, cudaStream_t s, int* pushed) {
     HP_REQUIRE(p.E % 256 == 0 && p.F % 256 == 0 && p.T >= 1 && p.nslot >= 1 && p.T * p.nslot <= MOE_MAX_PAIRS, "moe_experts_grouped: bad shape");
