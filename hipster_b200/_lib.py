@@ -8,6 +8,9 @@ LIB_PATH = os.environ.get("HIPSTER_B200_LIB") or os.path.join(HERE, "libhipster_
 HEADER = os.path.join(HERE, "..", "include", "hipster_b200.h")
 
 _lib = None
+# argument types of the calls whose latency counts (p pointer, i int, f float): integers then pass without a wrapper object
+_TYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "f": ctypes.c_float}
+_HOT = {"hp_quantize_x_q8": "piiippp", "hp_gemv_q4k_q8": "ppppiiiip", "hp_argmax": "piiipppp", "hp_accept_greedy": "ppipp", "hp_attn_decode": "piiiiiipppppipppfpp"}
 
 
 class HipsterError(RuntimeError):
@@ -32,8 +35,10 @@ def lib():
             raise HipsterError(-1, f"{LIB_PATH} is missing: build it with `python -m hipster_b200.build` (needs nvcc); no fallback path exists")
         _lib = ctypes.CDLL(LIB_PATH)
         _lib.hp_last_error.restype = ctypes.c_char_p
-        for name in ("hp_xq8_q_bytes", "hp_xq8_sc_bytes", "hp_argmax_scratch_bytes"):
+        for name in ("hp_xq8_q_bytes", "hp_xq8_sc_bytes", "hp_argmax_scratch_bytes", "hp_attn_workspace_bytes"):
             getattr(_lib, name).restype = ctypes.c_size_t
+        for name, types in _HOT.items():
+            getattr(_lib, name).argtypes = [_TYPES[t] for t in types]
     return _lib
 
 
@@ -47,6 +52,7 @@ def ptr(t):
     """Device (or host) pointer of a torch tensor / numpy array as c_void_p; None -> NULL."""
     if t is None:
         return ctypes.c_void_p(0)
-    if hasattr(t, "data_ptr"):
+    try:
         return ctypes.c_void_p(t.data_ptr())
-    return ctypes.c_void_p(t.ctypes.data)
+    except AttributeError:
+        return ctypes.c_void_p(t.ctypes.data)

@@ -168,7 +168,7 @@ size_t argmax_scratch_bytes(int R, int n);
 int topk_rows(const float* logits, int R, int n, int ld, int k, int* ids, float* vals, void* scratch, cudaStream_t s);
 size_t topk_scratch_bytes(int R, int n, int k);
 int topk_max_k();
-// allocation-free variant: partials in a static device array of fixed size (see argmax.cu)
+// variant without a scratch argument, for at most 32 rows of 524288 entries (limits of hp_argmax_noalloc)
 int argmax_rows_static(const float* logits, int R, int n, int ld, int* ids, float* vals, cudaStream_t s);
 int argmax_static_max_rows();
 int argmax_static_max_n();

@@ -6,9 +6,14 @@ import torch
 
 from ._lib import lib, check, ptr
 
+# The calls below are a few microseconds of device work, so what they spend in Python counts: the handle of the current stream
+# comes without a Stream object around it, and the short calls pass pointers as integers to declared argument types (_lib.py; to a
+# function without declared types an integer would pass as 32 bits, hence the wrapper of _stream).
+_raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(_raw_stream(_device()))
 
 
 class XQ8:
@@ -17,8 +22,8 @@ class XQ8:
     def __init__(self, R, K, device="cuda"):
         L = lib()
         self.R, self.K = R, K
-        self.q = torch.zeros(L.hp_xq8_q_bytes(R, K), dtype=torch.uint8, device=device)
-        self.sc = torch.zeros(L.hp_xq8_sc_bytes(R, K), dtype=torch.uint8, device=device)
+        nq, ns = L.hp_xq8_q_bytes(R, K), L.hp_xq8_sc_bytes(R, K)   # nq is a multiple of 512: the scales stay aligned
+        self.q, self.sc = torch.zeros(nq + ns, dtype=torch.uint8, device=device).split((nq, ns))
 
     def unpack(self):
         """-> (q int8 [R][K], d f32 [R][K/32], s f32 [R][K/32]) in the reference's row layout."""
@@ -34,7 +39,7 @@ def quantize_x_q8(x, xq=None):
     assert x.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1
     R, K = x.shape
     xq = xq or XQ8(R, K, x.device)
-    check(lib().hp_quantize_x_q8(ptr(x), x.stride(0), R, K, ptr(xq.q), ptr(xq.sc), _stream()))
+    check(lib().hp_quantize_x_q8(x.data_ptr(), x.stride(0), R, K, xq.q.data_ptr(), xq.sc.data_ptr(), _raw_stream(_device())))
     return xq
 
 
@@ -49,7 +54,7 @@ def gemv_q4k_q8(w, xq, N, K, y=None):
     R = xq.R
     if y is None:
         y = torch.empty((R, N), dtype=torch.float32, device=w.device)
-    check(lib().hp_gemv_q4k_q8(ptr(w), ptr(xq.q), ptr(xq.sc), ptr(y), N, K, R, y.stride(0), _stream()))
+    check(lib().hp_gemv_q4k_q8(w.data_ptr(), xq.q.data_ptr(), xq.sc.data_ptr(), y.data_ptr(), N, K, R, y.stride(0), _raw_stream(_device())))
     return y
 
 
@@ -67,14 +72,14 @@ def argmax(logits, n=None):
     n = n or logits.shape[1]
     ids = torch.empty(R, dtype=torch.int32, device=logits.device)
     vals = torch.empty(R, dtype=torch.float32, device=logits.device)
-    scratch = torch.empty(lib().hp_argmax_scratch_bytes(R, n), dtype=torch.uint8, device=logits.device)
-    check(lib().hp_argmax(ptr(logits), R, n, ld, ptr(ids), ptr(vals), ptr(scratch), _stream()))
+    # the kernel needs no scratch; the argument must not be null
+    check(lib().hp_argmax(logits.data_ptr(), R, n, ld, ids.data_ptr(), vals.data_ptr(), ids.data_ptr(), _raw_stream(_device())))
     return ids, vals
 
 
 def argmax_noalloc(logits, n=None):
-    """argmax() for callers that cannot allocate device memory: the library's built-in scratch holds the partial
-    results, so the call takes only the input and the two output tensors (created by the caller beforehand)."""
+    """argmax() through the entry point for callers that cannot allocate device memory: it takes only the input and the two
+    output tensors (a C caller creates these beforehand), for at most 32 rows of 524288 entries."""
     R, ld = logits.shape[0], logits.stride(0)
     n = n or logits.shape[1]
     ids = torch.empty(R, dtype=torch.int32, device=logits.device)
@@ -86,7 +91,7 @@ def argmax_noalloc(logits, n=None):
 def accept_greedy(ids, drafts):
     """-> int32 tensor [mm, bonus] on device (reference host loop, engine/bench/spec27b.cpp:92-97)."""
     out = torch.empty(2, dtype=torch.int32, device=ids.device)
-    check(lib().hp_accept_greedy(ptr(ids), ptr(drafts), int(drafts.numel()), ptr(out), _stream()))
+    check(lib().hp_accept_greedy(ids.data_ptr(), drafts.data_ptr(), drafts.numel(), out.data_ptr(), _raw_stream(_device())))
     return out
 
 
@@ -99,13 +104,12 @@ def attn_decode(qkv, pos0, n_head, n_kv, n_rot, q_norm, k_norm, rope, kc, vc, ma
     q_norm / k_norm bf16 [256] (int16 tensors), rope f32 [max_ctx][n_rot/2][2], kc / vc f16 [n_kv][max_ctx][256] (updated).
     -> (out f32 [R][n_head*256], XQ8 of it or None). Reference: qk_norm_rope_kv + attn_decode_mq (ops.h:71-72,96)."""
     L = lib()
-    L.hp_attn_workspace_bytes.restype = ctypes.c_size_t
     R, ld = qkv.shape[0], qkv.stride(0)
     ws = torch.empty(L.hp_attn_workspace_bytes(R, n_head, n_kv, max_ctx), dtype=torch.uint8, device=qkv.device)
     out = torch.empty((R, n_head * 256), dtype=torch.float32, device=qkv.device)
     xq = XQ8(R, n_head * 256, qkv.device) if want_q8 else None
-    check(L.hp_attn_decode(ptr(qkv), ld, R, int(pos0), n_head, n_kv, n_rot, ptr(q_norm), ptr(k_norm), ptr(rope), ptr(kc), ptr(vc), int(max_ctx), ptr(out),
-                           ptr(xq.q) if xq else None, ptr(xq.sc) if xq else None, ctypes.c_float(eps), ptr(ws), _stream()))
+    check(L.hp_attn_decode(qkv.data_ptr(), ld, R, int(pos0), n_head, n_kv, n_rot, q_norm.data_ptr(), k_norm.data_ptr(), rope.data_ptr(), kc.data_ptr(), vc.data_ptr(), int(max_ctx),
+                           out.data_ptr(), xq.q.data_ptr() if xq else None, xq.sc.data_ptr() if xq else None, eps, ws.data_ptr(), _raw_stream(_device())))
     return out, xq
 
 

@@ -51,20 +51,16 @@ int hp_gemv_parts(int N, int K);
 /* f32-activation baseline, R <= 8, y [R][N]. Replaces gemv_q4_K_f32 (gemv.h:57, gemv.hip:1177-1216). */
 int hp_gemv_q4k_f32(const void* w_dev, const float* x_dev, float* y_dev, int N, int K, int R, void* stream);
 /* Row-wise argmax (maximum value, lowest index on ties) of logits [R][ld] over n entries.
- * Replaces argmax_topk with k = 1 (ops.h:118, ops.hip:702-716). scratch_dev: hp_argmax_scratch_bytes(R, n) bytes. */
+ * Replaces argmax_topk with k = 1 (ops.h:118, ops.hip:702-716). scratch_dev: hp_argmax_scratch_bytes(R, n) bytes (must
+ * not be null; the present kernel leaves them alone). */
 size_t hp_argmax_scratch_bytes(int R, int n);
 int hp_argmax(const float* logits_dev, int R, int n, int ld, int* ids_dev, float* vals_dev, void* scratch_dev, void* stream);
 /* hp_argmax for callers that must not allocate. It has no counterpart in the reference. A serving loop that has sized
  * its weights, KV caches and state to fill the GPU, or that runs its decode steps on a latency-critical thread, cannot
  * afford a cudaMalloc per call: the allocation may fail, and it serialises against everything running on the device.
- * This variant needs no scratch from the caller: its partial results live in a fixed 16 KiB array inside the library
- * image (held by every GPU that loads the library until the process exits). It accepts at most
- * hp_argmax_noalloc_max_rows() rows of hp_argmax_noalloc_max_n() entries and rejects larger shapes with HP_EINVAL.
- * It calls no allocating routine. The first call on each device resolves the array's address; make that call before
- * any stream capture begins. All calls share the one array: nothing in it has to be cleared between calls (every
- * element read is written first by the same call), but two calls that overlap on the GPU race on it. The stream must
- * belong to the current device (a stream of another device is refused). Not thread-safe: the first call on a device
- * records the address without a lock, so it must not run concurrently with another host thread's call. */
+ * This variant takes no scratch and allocates nothing. It accepts at most hp_argmax_noalloc_max_rows() rows of
+ * hp_argmax_noalloc_max_n() entries and rejects larger shapes with HP_EINVAL. The stream must belong to the current
+ * device (a stream of another device is refused) and must not be capturing. */
 int hp_argmax_noalloc(const float* logits_dev, int R, int n, int ld, int* ids_dev, float* vals_dev, void* stream);
 int hp_argmax_noalloc_max_rows(void);
 int hp_argmax_noalloc_max_n(void);

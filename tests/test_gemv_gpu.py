@@ -96,6 +96,24 @@ def test_argmax_and_accept():
         assert tuple(out) == orc.accept(oi, drafts)
 
 
+# one CTA per row up to 4096 entries, a cluster of eight beyond; pieces that are empty, ragged and unaligned rows (odd ld), ties across pieces
+@pytest.mark.parametrize("n,ld", [(1, 1), (7, 9), (4095, 4096), (4096, 4096), (4097, 4097), (4100, 4100), (70001, 70003), (262147, 262148)])
+def test_argmax_at_the_edges_of_its_pieces(n, ld):
+    rng = np.random.default_rng(n)
+    a = rng.normal(size=(5, ld)).astype(np.float32)
+    a[:, n:] = 1e9                                                       # beyond the row: not looked at
+    a[0, n - 1] = 50.0
+    a[1, :n] = a[1, 0]                                                   # all equal: the lowest index
+    a[2, n // 2] = a[2, n - 1] = 50.0
+    a[3, :n] = -np.inf; a[3, n // 3] = -1.0
+    a[4, : n - 1] = np.nan if n > 1 else a[4, : n - 1]; a[4, n - 1] = -3.0   # NaN never wins
+    ids, vals = K_.argmax(dev(a), n)
+    want = [n - 1, 0, n // 2, n // 3, n - 1]
+    assert ids.cpu().tolist() == want and np.array_equal(bits(vals.cpu().numpy()), bits(a[range(5), want]))
+    none, v = K_.argmax(dev(np.full((1, n), -np.inf, np.float32)))
+    assert none.item() == -1 and v.item() == -np.inf
+
+
 def test_config1_kernel_check_full_size():
     """Benchmark configuration 1: N=17408 x K=5120 Q4_K, 3 f32 activation rows, seed 0 -> GEMV, per-row argmax, greedy
     acceptance against 2 seeded draft ids; CUDA vs the CPU restatement, plus the reference's own tolerance rule."""
