@@ -261,11 +261,9 @@ __device__ __forceinline__ float2 gdn_fma2(float2 a, float2 b, float2 c) {   // 
         : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)), "l"(reinterpret_cast<unsigned long long&>(c)));
     return r;
 }
-// MINB = resident CTAs per SM the register budget is cut for: 3 (80 registers) for one or two sequences (one wave either
-// way), 4 (64 registers, a few bytes of spills) for passes over several sequences, where the grid runs in several waves
-// of this latency-bound kernel and a fourth CTA per SM shortens them. Same instructions, same results.
-template <int MINB>
-__global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, MINB) k_gdn(GdnArgs a) {
+// Passes over one or two sequences: one wave of a latency-bound kernel (one sequence of 6 rows, 4 replayed: 16.4 us with 128-bit reads of q
+// and k in the recurrence, 15.3 with 64-bit ones, see lds_f2; 1 row, 1 replayed: 9.3 and 8.4).
+__global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, 3) k_gdn(GdnArgs a) {
     constexpr int D = 128, NLD = 8, NCV = 6;   // items per thread: (16 + 3) * 96 <= 8 * 256 raw values, 16 * 96 = 6 * 256 conv outputs
     // conv'ed, then normalised q | k of every row (filled by all four CTAs); 16-float chunks padded to 20 so that the
     // eight chunk owners of a state row read 128 bits each from distinct banks
@@ -390,9 +388,11 @@ __global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, MINB) k_gd
         if (it == nrep && nrep > 0) commit_state();
         const float beta = sbeta[it], decay = sdecay[it];
         const float* kk = &sqk[it][160 + 20 * ck]; const float* qq = &sqk[it][20 * ck];
-        float2 kr[8];
+        float2 kr[8], qr[8];
 #pragma unroll
-        for (int i = 0; i < 8; i += 2) { const float4 v = *reinterpret_cast<const float4*>(kk + 2 * i); kr[i] = make_float2(v.x, v.y); kr[i + 1] = make_float2(v.z, v.w); }
+        for (int i = 0; i < 8; ++i) kr[i] = lds_f2(kk + 2 * i);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) qr[i] = lds_f2(qq + 2 * i);
         const float2 dc2 = make_float2(decay, decay);
         float dot = 0.f;
 #pragma unroll
@@ -404,9 +404,8 @@ __global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, MINB) k_gd
         float o = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; i += 2) {
-            const float4 qv = *reinterpret_cast<const float4*>(qq + 2 * i);
-            m[i] = gdn_fma2(dl2, kr[i], m[i]); o = fmaf(m[i].x, qv.x, o); o = fmaf(m[i].y, qv.y, o);
-            m[i + 1] = gdn_fma2(dl2, kr[i + 1], m[i + 1]); o = fmaf(m[i + 1].x, qv.z, o); o = fmaf(m[i + 1].y, qv.w, o);
+            m[i] = gdn_fma2(dl2, kr[i], m[i]); o = fmaf(m[i].x, qr[i].x, o); o = fmaf(m[i].y, qr[i].y, o);
+            m[i + 1] = gdn_fma2(dl2, kr[i + 1], m[i + 1]); o = fmaf(m[i + 1].x, qr[i + 1].x, o); o = fmaf(m[i + 1].y, qr[i + 1].y, o);
         }
 #pragma unroll
         for (int off = 1; off < 8; off <<= 1) o = o + __shfl_xor_sync(0xffffffffu, o, off);
@@ -440,6 +439,200 @@ __global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, MINB) k_gd
         if (a.out) a.out[oi] = v;
         if (a.oq) warp_quant32_store(v, row, (h * D + c) >> 5, Z, a.oq, a.osc, lane);
     }
+}
+
+constexpr int GDN_WCL = 2;   // CTAs per head
+constexpr int GDN_RAWW = 320, GDN_STR = 320;   // floats of a raw row (q 128 | k 128 | own v 64) and of a q | k row (16-float chunks padded to 20)
+struct GdnWideSmem {
+    // conv'ed, then normalised q | k of every row; the eight chunk owners of a state row read 64 bits each from distinct banks
+    float sqk[GDN_MAXROWS][GDN_STR];
+    float raw[3 + GDN_MAXROWS][GDN_RAWW];   // 3 taps of history | 8 saved rows | 8 new rows
+    float sv[GDN_MAXROWS][64], sout[8][64];
+    float csum[GDN_MAXROWS][2][4], snrm[GDN_MAXROWS][2], sbeta[GDN_MAXROWS], sdecay[GDN_MAXROWS], cred[8][4];
+};
+// The same layer for passes over three or more sequences, whose CTAs run in several waves: a cluster of 2 CTAs per (v-head,
+// sequence), CTA `rank` owns value rows 64*rank .. +63, a thread 16 columns of two of them, so that a read of q and k serves two
+// state rows. Every CTA convolves and normalises the head's 128 q and 128 k channels itself (warp w: 32 q channels for w < 4, 32 k
+// channels otherwise) and its own 64 v channels, from raw inputs that arrive by asynchronous copies; both CTAs read the saved rows and
+// the history, so these are rewritten at the end, behind the cluster barrier of the output norm. Sums and their order are those of
+// k_gdn. Eight sequences of 3 rows, 2 replayed: 30.8 us a launch, k_gdn 38.5; one sequence of 6 rows, 4 replayed: 16.8 and 15.3, of 1
+// row, 1 replayed: 9.9 and 8.4.
+__global__ void __cluster_dims__(GDN_WCL, 1, 1) __launch_bounds__(256, 3) k_gdn_wide(GdnArgs a) {
+    constexpr int D = 128;
+    extern __shared__ __align__(16) uint8_t gdn_smem[];
+    GdnWideSmem& sm = *reinterpret_cast<GdnWideSmem*>(gdn_smem);
+    pdl_launch_dependents();
+    cluster_arrive_relaxed();   // matched by cluster_wait() before the first store into the other CTA: it has started by then
+    const int rank = blockIdx.x % GDN_WCL, h = blockIdx.x / GDN_WCL, hk = h % a.n_qk, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // this thread's q | k channel tid: column in a row of the merged projection (its slot in a history / saved row is tid); v channels
+    const int qk_col = tid < D ? hk * D + tid : a.n_qk * D + hk * D + (tid - D), v_col = 2 * a.n_qk * D + h * D + 64 * rank, v_slot = 2 * D + 64 * rank;
+    if (a.late) pdl_wait();   // the taps and the norm weights may have been written earlier in the stream
+    const float4 cw = *reinterpret_cast<const float4*>(a.conv_w + (size_t)qk_col * 4);
+    const float4 cv0 = *reinterpret_cast<const float4*>(a.conv_w + (size_t)(v_col + lane) * 4), cv1 = *reinterpret_cast<const float4*>(a.conv_w + (size_t)(v_col + 32 + lane) * 4);
+    const float nw0 = bf2f(a.norm_w[64 * rank + lane]), nw1 = bf2f(a.norm_w[64 * rank + 32 + lane]);
+    pdl_wait();
+    const int r0 = a.seq ? a.seq[blockIdx.y * 4 + 0] : 0, T = min(a.seq ? a.seq[blockIdx.y * 4 + 1] : a.imm_T, 8), slot = a.seq ? a.seq[blockIdx.y * 4 + 2] : 0;
+    const int nrep = min(a.seq ? (a.replay_n ? a.replay_n[slot] : 0) : a.imm_replay, 8), nrows = nrep + T;
+    float* sav = a.saved + (size_t)slot * a.saved_stride + (size_t)h * 8 * 388;   // [8][q 128 | k 128 | v 128 | beta | alpha | pad]
+    float* cst = a.conv_state + (size_t)slot * a.conv_stride + (size_t)h * 3 * 384;   // [3 taps][q 128 | k 128 | v 128]; private per v-head
+    const float* rows = a.rows + (size_t)r0 * a.ld;
+    // ---- raw inputs of all rows by asynchronous copies, the state into registers
+    const int vc = tid & 63;
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) cp_async4(&sm.raw[i][tid], cst + i * 384 + tid);
+    if (tid < 192) cp_async4(&sm.raw[tid >> 6][256 + vc], cst + (tid >> 6) * 384 + v_slot + vc);
+#pragma unroll 1
+    for (int i = 0; i < T; ++i) cp_async4(&sm.raw[11 + i][tid], rows + (size_t)i * a.ld + qk_col);
+#pragma unroll 1
+    for (int i = tid >> 6; i < T; i += 4) cp_async4(&sm.raw[11 + i][256 + vc], rows + (size_t)i * a.ld + v_col + vc);
+#pragma unroll 1
+    for (int i = 0; i < nrep; ++i) cp_async4(&sm.raw[3 + i][tid], sav + i * 388 + tid);
+#pragma unroll 1
+    for (int i = tid >> 6; i < nrep; i += 4) cp_async4(&sm.raw[3 + i][256 + vc], sav + i * 388 + v_slot + vc);
+    const int jl = tid >> 3, ck = tid & 7;
+    float* Mrow = a.state + (size_t)slot * a.state_stride + ((size_t)h * D + 64 * rank + jl) * D + 16 * ck;   // and + 32 rows
+    float2 m[2][8];
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) { const float4 v = *reinterpret_cast<const float4*>(Mrow + q * 32 * D + 2 * i); m[q][i] = make_float2(v.x, v.y); m[q][i + 1] = make_float2(v.z, v.w); }
+    auto commit_state = [&](float* dst) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) *reinterpret_cast<float4*>(dst + q * 32 * D + 2 * i) = make_float4(m[q][i].x, m[q][i].y, m[q][i + 1].x, m[q][i + 1].y);
+    };
+    // gate inputs z of this lane's channels for the row that warp `warp` finishes
+    const int Z = a.n_v * D, zc = h * D + 64 * rank + lane;
+    float z0 = 0.f, z1 = 0.f;
+    if (warp < T) { const float* zp = rows + (size_t)warp * a.ld + a.off_z + zc; z0 = zp[0]; z1 = zp[32]; }
+    // gates of every row (both CTAs compute them), by the last warp
+    float raw_b = 0.f, raw_a = 0.f;
+    if (warp == 7 && lane < nrows) {
+        const bool replay = lane < nrep;
+        const float* row = rows + (size_t)(replay ? 0 : lane - nrep) * a.ld;
+        raw_b = replay ? sav[lane * 388 + 384] : row[a.off_b + h];
+        raw_a = replay ? sav[lane * 388 + 385] : row[a.off_a + h];
+        sm.sbeta[lane] = sigmoid_det(raw_b);
+        sm.sdecay[lane] = expf_det(bf2f(a.a_neg[h]) * softplus_det(raw_a + bf2f(a.dt_bias[h])));
+    }
+    cp_async_wait_all();
+    __syncthreads();
+
+    // ---- conv + SiLU: logical raw row i is the history for i < 3, then the saved rows, then the new ones. Squared l2 norms of q
+    // and k: xor tree over the warp's 32 channels, the four warp sums added in channel order
+    auto raw_row = [&](int i) -> const float* { return sm.raw[i < 3 + nrep ? i : i + 8 - nrep]; };
+    auto conv = [](const float4& w, float x0, float x1, float x2, float x3) { float t = w.x * x0; t = fmaf(w.y, x1, t); t = fmaf(w.z, x2, t); t = fmaf(w.w, x3, t); return silu_det(t); };
+    {
+        const int g2 = tid >> 7, ch = tid & 127, off = g2 * 160 + (ch >> 4) * 20 + (ch & 15);
+        float x0 = sm.raw[0][tid], x1 = sm.raw[1][tid], x2 = sm.raw[2][tid];
+#pragma unroll 2
+        for (int it = 0; it < nrows; ++it) {
+            const float x3 = raw_row(it + 3)[tid];
+            const float v = conv(cw, x0, x1, x2, x3);
+            x0 = x1; x1 = x2; x2 = x3;
+            sm.sqk[it][off] = v;
+            float p = v * v;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) p = p + __shfl_xor_sync(0xffffffffu, p, o);
+            if (lane == 0) sm.csum[it][g2][warp & 3] = p;
+        }
+#pragma unroll 2
+        for (int item = warp; item < 2 * nrows; item += 8) {
+            const int it = item >> 1, c = (item & 1) * 32 + lane;
+            sm.sv[it][c] = conv(item & 1 ? cv1 : cv0, raw_row(it)[256 + c], raw_row(it + 1)[256 + c], raw_row(it + 2)[256 + c], raw_row(it + 3)[256 + c]);
+        }
+        __syncthreads();
+        if (tid < 2 * nrows) {
+            const float* cs = &sm.csum[tid >> 1][tid & 1][0];
+            float tot = cs[0]; tot = tot + cs[1]; tot = tot + cs[2]; tot = tot + cs[3];
+            sm.snrm[tid >> 1][tid & 1] = fmaxf(sqrtf(tot), a.eps);
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int it = 0; it < nrows; ++it) sm.sqk[it][off] = sm.sqk[it][off] / sm.snrm[it][g2];   // q | k normalised in place
+    }
+    __syncthreads();
+
+    // ---- the recurrence, row after row, state in registers; no block-wide synchronisation inside
+#pragma unroll 1
+    for (int it = 0; it < nrows; ++it) {
+        if (it == nrep && nrep > 0) commit_state(Mrow);
+        const float beta = sm.sbeta[it], decay = sm.sdecay[it], v0 = sm.sv[it][jl], v1 = sm.sv[it][jl + 32];
+        const float* kk = &sm.sqk[it][160 + 20 * ck]; const float* qq = &sm.sqk[it][20 * ck];
+        float2 kr[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) kr[i] = lds_f2(kk + 2 * i);
+        const float2 dc2 = make_float2(decay, decay);
+        float d0 = 0.f, d1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            m[0][i] = mul2(m[0][i], dc2); m[1][i] = mul2(m[1][i], dc2);
+            d0 = fmaf(m[0][i].x, kr[i].x, d0); d1 = fmaf(m[1][i].x, kr[i].x, d1);
+            d0 = fmaf(m[0][i].y, kr[i].y, d0); d1 = fmaf(m[1][i].y, kr[i].y, d1);
+        }
+#pragma unroll
+        for (int off = 1; off < 8; off <<= 1) { d0 = d0 + __shfl_xor_sync(0xffffffffu, d0, off); d1 = d1 + __shfl_xor_sync(0xffffffffu, d1, off); }
+        const float e0 = (v0 - d0) * beta, e1 = (v1 - d1) * beta;
+        const float2 dl0 = make_float2(e0, e0), dl1 = make_float2(e1, e1);
+        float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float2 qv = lds_f2(qq + 2 * i);
+            fma2(m[0][i], dl0, kr[i]); fma2(m[1][i], dl1, kr[i]);
+            o0 = fmaf(m[0][i].x, qv.x, o0); o1 = fmaf(m[1][i].x, qv.x, o1);
+            o0 = fmaf(m[0][i].y, qv.y, o0); o1 = fmaf(m[1][i].y, qv.y, o1);
+        }
+        if (it >= nrep) {
+#pragma unroll
+            for (int off = 1; off < 8; off <<= 1) { o0 = o0 + __shfl_xor_sync(0xffffffffu, o0, off); o1 = o1 + __shfl_xor_sync(0xffffffffu, o1, off); }
+            if (ck == 0) { sm.sout[it - nrep][jl] = o0 * 0.08838834764831845f; sm.sout[it - nrep][jl + 32] = o1 * 0.08838834764831845f; }
+            if (a.snap) commit_state(a.snap + (size_t)(it - nrep) * a.snap_row_stride + ((size_t)h * D + 64 * rank + jl) * D + 16 * ck);
+        }
+    }
+    if (T == 0 && nrep > 0) commit_state(Mrow);
+    __syncthreads();
+
+    // ---- per-head RMSNorm * w * gate(z) + quantisation of the new rows; warp t takes row t, lane = two channels. The sum of
+    // squares over the head's 128 channels: a CTA sends its two warp sums to both CTAs of the cluster.
+    float o0 = 0.f, o1 = 0.f;
+    if (warp < T) {
+        o0 = sm.sout[warp][lane]; o1 = sm.sout[warp][lane + 32];
+        float p0 = o0 * o0, p1 = o1 * o1;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) { p0 = p0 + __shfl_xor_sync(0xffffffffu, p0, off); p1 = p1 + __shfl_xor_sync(0xffffffffu, p1, off); }
+        cluster_wait();
+        if (lane < 2 * GDN_WCL) st_cluster_f32(&sm.cred[warp][2 * rank + (lane & 1)], (uint32_t)(lane >> 1), lane & 1 ? p1 : p0);
+    } else cluster_wait();
+    const float g0 = warp < T ? (a.sigmoid_gate ? sigmoid_det(z0) : silu_det(z0)) : 0.f, g1 = warp < T ? (a.sigmoid_gate ? sigmoid_det(z1) : silu_det(z1)) : 0.f;
+    cluster_sync_all();
+    if (warp < T) {
+        const float* cr = sm.cred[warp];
+        float ss = cr[0]; ss = ss + cr[1]; ss = ss + cr[2]; ss = ss + cr[3];
+        const int row = r0 + warp;
+        const size_t oi = (size_t)row * Z + zc;
+        const float sc = 1.0f / sqrtf(ss / (float)D + a.eps), v0 = ((o0 * sc) * nw0) * g0, v1 = ((o1 * sc) * nw1) * g1;
+        if (a.out) { a.out[oi] = v0; a.out[oi + 32] = v1; }
+        if (a.oq) { warp_quant32_store(v0, row, zc >> 5, Z, a.oq, a.osc, lane); warp_quant32_store(v1, row, (zc >> 5) + 1, Z, a.oq, a.osc, lane); }
+    }
+    // both CTAs have read the saved rows and the history: raw inputs of the new rows for a later commit, history after the
+    // accepted prefix. A CTA writes 64 channels of q, k and v each.
+    if (tid < 192) {
+        const int g = tid >> 6, slot_c = g * D + 64 * rank + vc, rc = g < 2 ? slot_c : 256 + vc;
+#pragma unroll 1
+        for (int t = 0; t < T; ++t) sav[t * 388 + slot_c] = sm.raw[11 + t][rc];
+        if (nrep > 0)
+#pragma unroll
+            for (int tap = 0; tap < 3; ++tap) cst[tap * 384 + slot_c] = raw_row(nrep + tap)[rc];
+    }
+    if (rank == 0 && warp == 7 && lane >= nrep && lane < nrows) { sav[(lane - nrep) * 388 + 384] = raw_b; sav[(lane - nrep) * 388 + 385] = raw_a; }
+}
+int launch_gdn_wide(const GdnArgs& a, int n_v, int nseq, cudaStream_t s) {
+    static bool attr[MAX_DEVICES] = {};   // per device: the opt-in belongs to the device's copy of the kernel
+    const int dev = current_device(); if (dev < 0) return HP_ECUDA;
+    if (!attr[dev]) { HP_CUDA(cudaFuncSetAttribute(k_gdn_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GdnWideSmem))); attr[dev] = true; }
+    HP_CUDA(launch_pdl<128>(k_gdn_wide, dim3(n_v * GDN_WCL, nseq), dim3(256), sizeof(GdnWideSmem), s, a));
+    return HP_OK;
 }
 
 }  // namespace
@@ -486,8 +679,8 @@ int gdn_forward(const GdnParams& p, int nseq, cudaStream_t s) {
     a.state = p.state; a.conv_state = p.conv_state; a.state_stride = p.state_stride; a.conv_stride = p.conv_stride;
     a.seq = p.seq; a.replay_n = p.replay_n; a.imm_T = p.imm_T; a.imm_replay = p.imm_replay; a.out = p.out; a.oq = (int8_t*)p.xq.q; a.osc = (float*)p.xq.sc;
     a.snap = p.snap; a.snap_row_stride = p.snap_row_stride; a.eps = p.eps; a.sigmoid_gate = p.sigmoid_gate; a.late = p.late;
-    if (nseq >= 3) HP_CUDA(launch_pdl<128>(k_gdn<4>, dim3(p.n_v * GDN_CL, nseq), dim3(256), 0, s, a));
-    else HP_CUDA(launch_pdl<128>(k_gdn<3>, dim3(p.n_v * GDN_CL, nseq), dim3(256), 0, s, a));
+    if (nseq >= 3) return launch_gdn_wide(a, p.n_v, nseq, s);
+    HP_CUDA(launch_pdl<128>(k_gdn, dim3(p.n_v * GDN_CL, nseq), dim3(256), 0, s, a));
     HP_CUDA(cudaGetLastError()); return HP_OK;
 }
 

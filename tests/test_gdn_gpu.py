@@ -187,3 +187,40 @@ def test_weights_written_on_the_stream_right_before(setup):
         got.append(call(new()))
     for i, o in enumerate(got):
         assert torch.equal(o.view(torch.int32), want[i % 2].view(torch.int32)), i
+
+
+class _Gdn(ctypes.Structure):   # struct GdnParams (csrc/kernels.h)
+    _fields_ = [(n, t) for t, names in ((ctypes.c_void_p, "rows saved"), (ctypes.c_size_t, "saved_stride"), (ctypes.c_int, "ld off_z off_b off_a n_qk n_v"),
+                                        (ctypes.c_void_p, "conv_w dt_bias a_neg norm_w state conv_state"), (ctypes.c_size_t, "state_stride conv_stride"),
+                                        (ctypes.c_void_p, "seq replay_n"), (ctypes.c_int, "imm_T imm_replay"), (ctypes.c_void_p, "out q sc snap"),
+                                        (ctypes.c_size_t, "snap_row_stride"), (ctypes.c_float, "eps"), (ctypes.c_int, "sigmoid_gate"), (ctypes.c_bool, "late")) for n in names.split()]
+
+
+@pytest.mark.parametrize("Ts,reps", [((1, 8, 3), (0, 8, 2)), ((8, 8, 8), (8, 1, 0)), ((0, 2, 5), (3, 0, 7)), ((0, 0, 0), (1, 8, 0)), ((4, 1, 2), (1, 2, 4))])
+@pytest.mark.parametrize("n_qk,n_v", [(2, 4), (1, 3)])
+def test_three_sequences_take_the_wide_kernel_and_match_one_at_a_time(Ts, reps, n_qk, n_v):
+    """Passes over three or more sequences run another kernel (csrc/ops.cu, k_gdn_wide) than one sequence by itself: outputs, state,
+    history and saved rows have the same bits, for rows and replayed rows at both ends of their range."""
+    f = getattr(hb.lib(), "_ZN2hp11gdn_forwardERKNS_9GdnParamsEiP11CUstream_st")
+    f.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
+    g = torch.Generator(device="cuda").manual_seed(sum(Ts) + n_v)
+    rnd = lambda *s, std=1.0, mean=0.0: torch.randn(s, device="cuda", generator=g) * std + mean  # noqa: E731
+    bf = lambda t: t.bfloat16().view(torch.int16)  # noqa: E731
+    ld, R, K = (2 * n_qk + 2 * n_v) * 128 + 2 * n_v, max(sum(Ts), 1), n_v * 128
+    w = dict(rows=rnd(R, ld), conv_w=rnd((2 * n_qk + n_v) * 128, 4, std=0.5), dt_bias=bf(rnd(n_v, std=0.5)), a_neg=bf(-rnd(n_v).abs()), norm_w=bf(rnd(128, std=0.3, mean=1.0)))
+    mut = dict(state=rnd(3, n_v, 128, 128, std=0.1), conv_state=rnd(3, n_v, 3, 384), saved=rnd(3, n_v, 8, 388))
+    res = []
+    for together in (True, False):
+        m = {k: v.clone() for k, v in mut.items()}
+        out, xq = torch.zeros((R, K), device="cuda"), hb.kernels.XQ8(R, K)
+        p = _Gdn(ld=ld, off_z=(2 * n_qk + n_v) * 128, off_b=(2 * n_qk + 2 * n_v) * 128, off_a=(2 * n_qk + 2 * n_v) * 128 + n_v, n_qk=n_qk, n_v=n_v, out=out.data_ptr(), q=xq.q.data_ptr(),
+                 sc=xq.sc.data_ptr(), saved_stride=n_v * 8 * 388, state_stride=n_v * 128 * 128, conv_stride=n_v * 3 * 384, eps=1e-6, **{k: v.data_ptr() for k, v in {**w, **m}.items()})
+        seq = torch.tensor([[sum(Ts[:i]), Ts[i], i, 0] for i in range(3)], dtype=torch.int32, device="cuda"); rep = torch.tensor(reps, dtype=torch.int32, device="cuda")
+        p.replay_n = rep.data_ptr()
+        for i in [None] if together else range(3):
+            p.seq = seq.data_ptr() + (16 * i if i else 0)
+            hb.check(f(ctypes.addressof(p), 3 if together else 1, torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        res.append([out, xq.q, xq.sc, m["state"], m["conv_state"], m["saved"]])
+    for a, b in zip(*res):
+        assert torch.equal(a.contiguous().view(torch.uint8), b.contiguous().view(torch.uint8))
