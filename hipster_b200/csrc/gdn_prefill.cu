@@ -53,13 +53,12 @@ __global__ void __launch_bounds__(D) k_gdn_pf_conv(GdnPrefillParams a) {
     a.qk[((size_t)r * 2 * a.n_qk + hd) * D + c] = v / fmaxf(sqrtf(tot), a.eps);
 }
 
-// grid (8, v heads), 128 threads: 16 rows of the head's state, thread = 16 columns of one row (k_gdn's layout), in registers
-// for the whole chunk. Bound by the dependent chain of a row (16 fmaf, 3 shuffles, 16 fmaf): q, k, v and gates arrive by
-// asynchronous copies, 16 rows ahead. 8 CTAs of a head instead of 4: the chain is the same and the 384 CTAs of 48 heads
-// spread over all SMs. 301 rows: 127 us under ncu. (One pass over the columns for the output of a row and the first product of
-// the next one, so half the dependent steps per row, took 141: its extra registers, moves and branches cost more. Prefill of
-// 301 tokens of the 27B shape 85.0 ms so, 85.8 with the shared pass; 512 tokens 123.3 and 124.4.)
-__global__ void __launch_bounds__(D) k_gdn_pf_scan(GdnPrefillParams a) {
+// grid (8, v heads), 64 threads: 16 rows of the head's state, thread = 16 columns of two rows (k_gdn's layout), in registers
+// for the whole chunk. Bound by the dependent chain of a row (16 fmaf, 3 shuffles, 16 fmaf) and by the shared-memory pipe: q and k
+// are read 64 bits at a time (see lds_f2) and serve two state rows (one row per thread and 128-bit reads: 127 us for 301 rows under
+// ncu). q, k, v and gates arrive by asynchronous copies, 16 rows ahead.
+constexpr int PF_ST = 64;   // threads of the scan
+__global__ void __launch_bounds__(PF_ST) k_gdn_pf_scan(GdnPrefillParams a) {
     __shared__ __align__(16) float sqk[2][PF_CH][PF_STR];
     __shared__ float sv[2][PF_CH][16];
     __shared__ float2 sg[2][PF_CH];
@@ -67,18 +66,20 @@ __global__ void __launch_bounds__(D) k_gdn_pf_scan(GdnPrefillParams a) {
     const int part = blockIdx.x, h = blockIdx.y, hk = h % a.n_qk, tid = threadIdx.x, jl = tid >> 3, ck = tid & 7, j = 16 * part + jl;
     pdl_wait();
     float* Mrow = a.state + ((size_t)h * D + j) * D + 16 * ck;
-    float2 m[8];
+    float2 m[2][8];   // rows j and j + 8
 #pragma unroll
-    for (int i = 0; i < 8; i += 2) { const float4 v = *reinterpret_cast<const float4*>(Mrow + 2 * i); m[i] = make_float2(v.x, v.y); m[i + 1] = make_float2(v.z, v.w); }
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) { const float4 v = *reinterpret_cast<const float4*>(Mrow + q * 8 * D + 2 * i); m[q][i] = make_float2(v.x, v.y); m[q][i + 1] = make_float2(v.z, v.w); }
     auto stage = [&](int r0, int s) {
         const int n = min(PF_CH, a.T - r0);
-        for (int e = tid; e < n * 64; e += D) {   // 16-byte pieces of q (32) and k (32) of every row
+        for (int e = tid; e < n * 64; e += PF_ST) {   // 16-byte pieces of q (32) and k (32) of every row
             const int r = e >> 6, i = e & 63, g = i >> 5, p = i & 31;
             const float* src = a.qk + ((size_t)(r0 + r) * 2 * a.n_qk + g * a.n_qk + hk) * D + p * 4;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&sqk[s][r][g * 160 + (p >> 2) * 20 + (p & 3) * 4])), "l"(src) : "memory");
         }
-        for (int e = tid; e < n * 16; e += D) cp_async4(&sv[s][e >> 4][e & 15], a.v + ((size_t)(r0 + (e >> 4)) * a.n_v + h) * D + 16 * part + (e & 15));
-        for (int e = tid; e < n * 2; e += D) cp_async4(reinterpret_cast<float*>(&sg[s][e >> 1]) + (e & 1), a.gate + ((size_t)(r0 + (e >> 1)) * a.n_v + h) * 2 + (e & 1));
+        for (int e = tid; e < n * 16; e += PF_ST) cp_async4(&sv[s][e >> 4][e & 15], a.v + ((size_t)(r0 + (e >> 4)) * a.n_v + h) * D + 16 * part + (e & 15));
+        for (int e = tid; e < n * 2; e += PF_ST) cp_async4(reinterpret_cast<float*>(&sg[s][e >> 1]) + (e & 1), a.gate + ((size_t)(r0 + (e >> 1)) * a.n_v + h) * 2 + (e & 1));
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     stage(0, 0);
@@ -92,32 +93,40 @@ __global__ void __launch_bounds__(D) k_gdn_pf_scan(GdnPrefillParams a) {
             const float* kk = &sqk[s][it][160 + 20 * ck]; const float* qq = &sqk[s][it][20 * ck];
             float2 kr[8];
 #pragma unroll
-            for (int i = 0; i < 8; i += 2) { const float4 v = *reinterpret_cast<const float4*>(kk + 2 * i); kr[i] = make_float2(v.x, v.y); kr[i + 1] = make_float2(v.z, v.w); }
+            for (int i = 0; i < 8; ++i) kr[i] = lds_f2(kk + 2 * i);
+            const float v0 = sv[s][it][jl], v1 = sv[s][it][jl + 8];
             const float2 dc2 = make_float2(decay, decay);
-            float dot = 0.f;
+            float d0 = 0.f, d1 = 0.f;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { m[i] = mul2(m[i], dc2); dot = fmaf(m[i].x, kr[i].x, dot); dot = fmaf(m[i].y, kr[i].y, dot); }
-#pragma unroll
-            for (int off = 1; off < 8; off <<= 1) dot = dot + __shfl_xor_sync(0xffffffffu, dot, off);
-            const float delta = (sv[s][it][jl] - dot) * beta;
-            const float2 dl2 = make_float2(delta, delta);
-            float o = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; i += 2) {
-                const float4 qv = *reinterpret_cast<const float4*>(qq + 2 * i);
-                fma2(m[i], dl2, kr[i]); o = fmaf(m[i].x, qv.x, o); o = fmaf(m[i].y, qv.y, o);
-                fma2(m[i + 1], dl2, kr[i + 1]); o = fmaf(m[i + 1].x, qv.z, o); o = fmaf(m[i + 1].y, qv.w, o);
+            for (int i = 0; i < 8; ++i) {
+                m[0][i] = mul2(m[0][i], dc2); m[1][i] = mul2(m[1][i], dc2);
+                d0 = fmaf(m[0][i].x, kr[i].x, d0); d1 = fmaf(m[1][i].x, kr[i].x, d1);
+                d0 = fmaf(m[0][i].y, kr[i].y, d0); d1 = fmaf(m[1][i].y, kr[i].y, d1);
             }
 #pragma unroll
-            for (int off = 1; off < 8; off <<= 1) o = o + __shfl_xor_sync(0xffffffffu, o, off);
-            if (ck == 0) a.o[((size_t)(r0 + it) * a.n_v + h) * D + j] = o * 0.08838834764831845f;
+            for (int off = 1; off < 8; off <<= 1) { d0 = d0 + __shfl_xor_sync(0xffffffffu, d0, off); d1 = d1 + __shfl_xor_sync(0xffffffffu, d1, off); }
+            const float e0 = (v0 - d0) * beta, e1 = (v1 - d1) * beta;
+            const float2 dl0 = make_float2(e0, e0), dl1 = make_float2(e1, e1);
+            float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float2 qv = lds_f2(qq + 2 * i);
+                fma2(m[0][i], dl0, kr[i]); fma2(m[1][i], dl1, kr[i]);
+                o0 = fmaf(m[0][i].x, qv.x, o0); o1 = fmaf(m[1][i].x, qv.x, o1);
+                o0 = fmaf(m[0][i].y, qv.y, o0); o1 = fmaf(m[1][i].y, qv.y, o1);
+            }
+#pragma unroll
+            for (int off = 1; off < 8; off <<= 1) { o0 = o0 + __shfl_xor_sync(0xffffffffu, o0, off); o1 = o1 + __shfl_xor_sync(0xffffffffu, o1, off); }
+            if (ck == 0) { float* o = a.o + ((size_t)(r0 + it) * a.n_v + h) * D + j; o[0] = o0 * 0.08838834764831845f; o[8] = o1 * 0.08838834764831845f; }
         }
         __syncthreads();   // the stage is free again
     }
 #pragma unroll
-    for (int i = 0; i < 8; i += 2) *reinterpret_cast<float4*>(Mrow + 2 * i) = make_float4(m[i].x, m[i].y, m[i + 1].x, m[i + 1].y);
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) *reinterpret_cast<float4*>(Mrow + q * 8 * D + 2 * i) = make_float4(m[q][i].x, m[q][i].y, m[q][i + 1].x, m[q][i + 1].y);
     if (part == 0)   // conv history after the chunk: ascending taps, so that a chunk of fewer than 3 rows shifts the old ones in place
-        for (int c = tid; c < 384; c += D) {
+        for (int c = tid; c < 384; c += PF_ST) {
             const int g = c >> 7, col = g == 0 ? hk * D + c : g == 1 ? a.n_qk * D + hk * D + (c - D) : 2 * a.n_qk * D + h * D + (c - 2 * D);
             float* cst = a.conv_state + (size_t)h * 3 * 384 + c;
             for (int tap = 0; tap < 3; ++tap) { const int rr = a.T - 3 + tap; cst[tap * 384] = rr < 0 ? cst[(rr + 3) * 384] : a.rows[(size_t)rr * a.ld + col]; }
@@ -149,7 +158,7 @@ int gdn_prefill(GdnPrefillParams p, float* scratch, cudaStream_t s) {
     HP_REQUIRE(p.T >= 1 && p.n_qk >= 1 && p.n_v >= p.n_qk && scratch && ((uintptr_t)scratch & 15) == 0, "gdn_prefill: bad arguments");
     p.qk = scratch; p.v = p.qk + (size_t)p.T * 2 * p.n_qk * D; p.o = p.v + (size_t)p.T * p.n_v * D; p.gate = p.o + (size_t)p.T * p.n_v * D;
     HP_CUDA(launch_pdl<128>(k_gdn_pf_conv, dim3(2 * p.n_qk + p.n_v, p.T), dim3(D), 0, s, p));
-    HP_CUDA(launch_pdl<128>(k_gdn_pf_scan, dim3(8, p.n_v), dim3(D), 0, s, p));
+    HP_CUDA(launch_pdl<128>(k_gdn_pf_scan, dim3(8, p.n_v), dim3(PF_ST), 0, s, p));
     HP_CUDA(launch_pdl<128>(k_gdn_pf_out, dim3(p.n_v, p.T), dim3(D), 0, s, p));
     HP_CUDA(cudaGetLastError()); return HP_OK;
 }
