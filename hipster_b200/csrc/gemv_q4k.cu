@@ -16,10 +16,10 @@
 // the CTA's K part are staged once per CTA in shared memory by bulk copies. One fp32 update per sub-block follows, in
 // block order:
 //     acc = fmaf((d*sc) * xd, (float)idot, acc);  acc = fmaf(-(dmin*mn), xs, acc);
-// Besides HBM the inner loop is bound by the shared-memory pipe and by issue: per 16x256 block and column tile 64 clocks of weights, 64
-// of activations and, read 64 bits at a time, 64 of column scales (128 with 128-bit reads) at one warp instruction per 4 to 16
-// clocks. Up to 4 rows (decode, drafts, short verify passes) take the form FEW. Decode of the 27B shape 5.33 ms a pass with 128-bit
-// reads and the full tile, 4.76 with both changes.
+// Besides HBM the inner loop is bound by issue: three warps per sub-partition, some 320 instructions per 16x256 block and column tile. Up to 4
+// rows (decode, drafts, short verify passes) take the form FEW with about two thirds of them: 34816 x 5120 22.7 -> 19.8 us, 16480 x 5120 12.6 ->
+// 11.0, decode of the 27B shape 5.33 -> 4.75 ms a pass. (Column scales and headers through 64-bit instead of 128-bit shared-memory reads
+// spare its pipe but cost instructions: 6 rows 22.7 -> 23.2 us, 16 rows 31.4 -> 32.8.)
 // A tile whose blocks are spread over several warps of the CTA is finished through shared memory: the partial sums
 // are added in warp order. Each K part writes its own output plane; the planes are added in part order by the
 // consumer (or by the small reduction kernel of the public entry point). No atomics, no cross-CTA traffic.
@@ -192,9 +192,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __
             // becomes the float 8388608 + v by a byte permute into the mantissa of 0x4B000000, and
             // fmaf(d, 8388608 + v, -(d * 8388608)) is exactly d * v (one rounding of an exactly representable
             // product). Odd sub-blocks take the high nibbles unshifted (16 * q): their d carries the exact 1/16.
-            const RowScales ra = decode_scales(lds_u4_halves(st + hdr_lane + blk * BLK_STRIDE));
+            const RowScales ra = decode_scales(*reinterpret_cast<const uint4*>(st + hdr_lane + blk * BLK_STRIDE));
             RowScales rb;
-            if constexpr (!FEW) rb = decode_scales(lds_u4_halves(st + hdr_lane + HDR8 + blk * BLK_STRIDE));
+            if constexpr (!FEW) rb = decode_scales(*reinterpret_cast<const uint4*>(st + hdr_lane + HDR8 + blk * BLK_STRIDE));
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 uint2 w0, w1;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __
                 }
                 const Q4kGroup wg(w0, w1);
                 if constexpr (FEW) {
-                    wg.dot_few(acc[0][0], ra, j, few, xqp[(blk * 4 + j) * 32], Q4kGroup::cols_smem(xsp + (blk * 8 + 2 * j) * 4), Q4kGroup::cols_smem(xsp + (blk * 8 + 2 * j + 1) * 4));
+                    wg.dot_few(acc[0][0], ra, j, few, xqp[(blk * 4 + j) * 32], Q4kGroup::cols(xsp[(blk * 8 + 2 * j) * 4]), Q4kGroup::cols(xsp[(blk * 8 + 2 * j + 1) * 4]));
                 } else {
                     const Q4kGroup::Scales sc(ra, rb, j);
 #pragma unroll
@@ -215,11 +215,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __
                         const uint4* xfp = xqp + n * xstride * 128 + (blk * 4 + j) * 32;
                         const float4* x0p = xsp + n * xstride * 32 + (blk * 8 + 2 * j) * 4;
                         const uint4 xf = XG ? __ldcg(xfp) : *xfp;
-                        Q4kGroup::ColScales x0, x1;
-                        if constexpr (XG) {
-                            const float4 v0 = __ldcg(x0p), v1 = __ldcg(x0p + 4);
-                            x0 = {make_float2(v0.x, v0.y), make_float2(v0.z, v0.w)}; x1 = {make_float2(v1.x, v1.y), make_float2(v1.z, v1.w)};
-                        } else { x0 = Q4kGroup::cols_smem(x0p); x1 = Q4kGroup::cols_smem(x0p + 4); }
+                        const Q4kGroup::ColScales x0 = Q4kGroup::cols(XG ? __ldcg(x0p) : *x0p), x1 = Q4kGroup::cols(XG ? __ldcg(x0p + 4) : x0p[4]);
                         wg.dot(acc[n][0], acc[n][1], sc, xf, x0, x1);
                     }
                 }
@@ -382,6 +378,7 @@ int launch_sk2(const uint8_t* W, const void* xq, const void* xsc, float* y, int 
     HP_CUDA(cudaLaunchKernelEx(&cfg, k_gemv_q4k_sk<NT, CB, SB, TILED, XG, FEW>, W, (const uint4*)xq, (const float4*)xsc, y, N, nb, P, R, ldy, part_stride, err, late ? 1 : 0));
     return HP_OK;
 }
+constexpr size_t SPLIT_BYTES = (size_t)16 << 20;
 // the activations of ntile column tiles fit in shared memory beside a ring of SB blocks per stage
 template <int SB, bool TILED> bool sk_fits(int ntile, int nbp) { return (size_t)SkGeom<SB, TILED>::FIXED + (size_t)ntile * nbp * 2560 <= (size_t)GEMV_SMEM_LIMIT; }
 template <int NT, bool XG = false, bool FEW = false>
@@ -451,8 +448,16 @@ int gemv_q4k_q8_parts(const void* W, const XQ8F& x, float* yparts, int N, int K,
     // all column tiles in one launch: their activations staged in shared memory beside the rings when they fit, read
     // from L2 inside the loop otherwise (small matrices with a long K: one launch instead of one per tile of 8 columns;
     // same per-column arithmetic either way)
-    // (three tiles of 20 blocks: 34816 x 5120 at 24 rows took 48 us from L2)
-    const bool staged = ntile == 1 || (tiled ? (nbp % 2 || ntile == 3 ? sk_fits<1, true>(ntile, nbp) : sk_fits<2, true>(ntile, nbp)) : (nbp % 2 ? sk_fits<1, false>(ntile, nbp) : sk_fits<2, false>(ntile, nbp)));
+    // (three tiles of 20 blocks beside one-block stages: 34816 x 5120 at 24 rows 44.5 us, from L2 50.8)
+    auto fits = [&](int nt) { return tiled ? (nbp % 2 || nt == 3 ? sk_fits<1, true>(nt, nbp) : sk_fits<2, true>(nt, nbp)) : (nbp % 2 ? sk_fits<1, false>(nt, nbp) : sk_fits<2, false>(nt, nbp)); };
+    const bool staged = ntile == 1 || fits(ntile);
+    // ... unless the matrix is large: two launches of column tiles that fit stream it twice in less time than one waits for L2 (32
+    // rows of 34816 x 5120: 86 -> 64 us, 16480 x 5120: 42 -> 35; 2048 x 6144, 7 MB: 11.0 -> 11.4)
+    if (!staged && R > 16 && fits(2) && (size_t)N * nb * 144 >= SPLIT_BYTES) {
+        const int rc1 = gemv_q4k_q8_parts(W, x, yparts, N, K, 16, ldy, part_stride, err, s, pdl, tiled, late);
+        if (rc1 != HP_OK) return rc1;
+        return gemv_q4k_q8_parts(W, XQ8F{(char*)x.q + xq_q_bytes(16, K), (char*)x.sc + xq_sc_floats(16, K) * 4}, yparts + (size_t)16 * ldy, N, K, R - 16, ldy, part_stride, err, s, pdl, tiled, late);
+    }
     const uint8_t* w = (const uint8_t*)W;
     int rc;
     if (R <= 4) rc = launch_sk<1, false, true>(w, tiled, x.q, x.sc, yparts, N, nb, P, R, ldy, part_stride, err, s, pdl, late);

@@ -273,7 +273,8 @@ struct Q4kGroup {
         __device__ __forceinline__ Scales(const RowScales& ra, const RowScales& rb, int j) : a0(ra.get(2 * j)), b0(rb.get(2 * j)), a1(ra.get(2 * j + 1)), b1(rb.get(2 * j + 1)) {}
     };
     struct ColScales { float2 d, s; };   // of the lane's two columns in one sub-block
-    static __device__ __forceinline__ ColScales cols_smem(const float4* p) { ColScales c; c.d = lds_f2(p); c.s = lds_f2(reinterpret_cast<const float*>(p) + 2); return c; }
+    static __device__ __forceinline__ ColScales cols(const float4& v) { return {make_float2(v.x, v.y), make_float2(v.z, v.w)}; }
+    static __device__ __forceinline__ ColScales cols_smem(const float4* p) { return {lds_f2(p), lds_f2(reinterpret_cast<const float*>(p) + 2)}; }   // see lds_f2
     static __device__ __forceinline__ void update(float2& acc, const float4& s, const ColScales& x, int i0, int i1) {
         fma2(acc, mul2(make_float2(s.x, s.y), x.d), add2(make_float2(__int_as_float(i0), __int_as_float(i1)), make_float2(-12582912.f, -12582912.f)));
         fma2(acc, make_float2(s.z, s.w), x.s);
