@@ -132,6 +132,13 @@ __device__ __forceinline__ void tc_update(float2 (&acc)[4][W], uint32_t ta, uint
     for (int b = 0; b < GB; ++b)
 #pragma unroll
         for (int i = 0; i < (H1 ? 4 : 2); ++i) r[b][i] = rs[b * 128 + 8 * i];
+    // column scales of up to 8 column tiles four (tile, sub-block) pairs ahead: the first under the accumulator loads, the others under
+    // the arithmetic (34816 x 5120: 32 rows 73 -> 67 us, 64 rows 113 -> 104; wider tiles have no registers for it: 512 rows 693 -> 752)
+    constexpr int NX = GB * W, XA = W > 4 ? 1 : 4;
+    auto xat = [&](int j) { return xs[(j % W) * 32 + (j / W) * 4]; };
+    float4 xb[XA];
+#pragma unroll
+    for (int j = 0; j < XA; ++j) if (W <= 4) xb[j] = xat(j);
     tc_wait_ld();
 #pragma unroll
     for (int b = 0; b < GB; ++b)
@@ -145,7 +152,9 @@ __device__ __forceinline__ void tc_update(float2 (&acc)[4][W], uint32_t ta, uint
     for (int b = 0; b < GB; ++b)
 #pragma unroll
         for (int i = 0; i < W; ++i) {
-            const float4 x = xs[i * 32 + b * 4];
+            const int j = b * W + i;
+            const float4 x = W <= 4 ? xb[j % XA] : xat(j);
+            if (W <= 4 && j + XA < NX) xb[j % XA] = xat(j + XA);
             upd(acc[0][i], r[b][0], x, v0[b][4 * i], v0[b][4 * i + 1]);
             upd(acc[1][i], r[b][1], x, v0[b][4 * i + 2], v0[b][4 * i + 3]);
             if constexpr (H1) {
