@@ -625,9 +625,18 @@ __global__ void __launch_bounds__(MQ_WARPS * 32, 1) k_moe_gemv_quad(MoeGArgs a) 
 // in-order weighted combine of the per-(row, slot) expert outputs (gemv.hip:1104-1112); used by the kernel-level entry
 // point (inside the engine the combine runs in the norm kernel that follows)
 __global__ void __launch_bounds__(256) k_moe_combine(const float* __restrict__ v, const float* __restrict__ slotw, float* __restrict__ y, int nslot, int E) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x; if (i >= E) return;
+    constexpr int EB = 12;   // expert rows in flight at once
     float acc = 0.f;
-    for (int e = 0; e < nslot; ++e) acc = fmaf(slotw[t * nslot + e], v[(size_t)(t * nslot + e) * E + i], acc);
+    for (int e0 = 0; e0 < nslot; e0 += EB) {
+        float w[EB], u[EB];
+#pragma unroll
+        for (int e = 0; e < EB; ++e) if (e0 + e < nslot) { w[e] = slotw[t * nslot + e0 + e]; u[e] = v[(size_t)(t * nslot + e0 + e) * E + i]; }
+#pragma unroll
+        for (int e = 0; e < EB; ++e) if (e0 + e < nslot) acc = fmaf(w[e], u[e], acc);
+    }
     y[(size_t)t * E + i] = acc;
 }
 
@@ -723,7 +732,7 @@ int moe_experts_grouped(const MoeGroupParams& p, cudaStream_t s, int* pushed) {
 }
 int moe_combine(const float* v, const float* slotw, float* y, int T, int nslot, int E, cudaStream_t s) {
     HP_REQUIRE(T >= 1 && nslot >= 1 && E >= 1, "moe_combine: bad shape");
-    k_moe_combine<<<dim3((E + 255) / 256, T), 256, 0, s>>>(v, slotw, y, nslot, E);
-    HP_CUDA(cudaGetLastError()); return HP_OK;
+    HP_CUDA(launch_pdl<8>(k_moe_combine, dim3((E + 255) / 256, T), dim3(256), 0, s, v, slotw, y, nslot, E));
+    return HP_OK;
 }
 }  // namespace hp

@@ -115,13 +115,24 @@ __global__ void __cluster_dims__(NORM_CL, 1, 1) __launch_bounds__(NORM_TPB) k_ad
             // MoE combine (gemv.hip:1104-1112): y holds one row per (row, slot) pair; acc = fmaf(weight, value, acc) in slot order
 #pragma unroll
             for (int k = 0; k < NG; ++k) s[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-            for (int e = 0; e < nslot; ++e) {
-                const float we = slotw[r * nslot + e];
+            constexpr int EB = 12;   // expert rows in flight at once (one L2 round trip for the 11 slots of top-10 routing and a shared expert)
+            for (int e0 = 0; e0 < nslot; e0 += EB) {
+                float we[EB]; float4 uu[EB][NG];
 #pragma unroll
-                for (int k = 0; k < NG; ++k) {
-                    const int i = 4 * (t + k * NORM_ROWT);
-                    if (i < n) { const float4 uu = *reinterpret_cast<const float4*>(y + (size_t)(r * nslot + e) * ldy + i); s[k].x = fmaf(we, uu.x, s[k].x); s[k].y = fmaf(we, uu.y, s[k].y); s[k].z = fmaf(we, uu.z, s[k].z); s[k].w = fmaf(we, uu.w, s[k].w); }
+                for (int e = 0; e < EB; ++e) {
+                    if (e0 + e >= nslot) continue;
+                    we[e] = slotw[r * nslot + e0 + e];
+#pragma unroll
+                    for (int k = 0; k < NG; ++k) { const int i = 4 * (t + k * NORM_ROWT); if (i < n) uu[e][k] = *reinterpret_cast<const float4*>(y + (size_t)(r * nslot + e0 + e) * ldy + i); }
+                }
+#pragma unroll
+                for (int e = 0; e < EB; ++e) {
+                    if (e0 + e >= nslot) continue;
+#pragma unroll
+                    for (int k = 0; k < NG; ++k) {
+                        if (4 * (t + k * NORM_ROWT) >= n) continue;
+                        s[k].x = fmaf(we[e], uu[e][k].x, s[k].x); s[k].y = fmaf(we[e], uu[e][k].y, s[k].y); s[k].z = fmaf(we[e], uu[e][k].z, s[k].z); s[k].w = fmaf(we[e], uu[e][k].w, s[k].w);
+                    }
                 }
             }
         } else {
