@@ -9,7 +9,7 @@
 // What bounds it: the fp32 update, two conversions and three packed fp32 instructions per two outputs and sub-block. From
 // registers alone a 16x8x32 tile of it takes 15.3 clocks of an SM sub-partition; the int8 mma.sync of the GEMV takes 8.0 and
 // does not overlap with it (23.9 together). In place this kernel takes 36 to 47 clocks per tile at 512 rows (34816 x 5120: 690
-// us) and 60 at 32 (72 us), the GEMV 72 at 32 rows (86 us): the rest is TMEM and shared-memory loads, addresses and waits.
+// us) and 56 at 32 (67 us), the GEMV 52 at 32 rows (62 us): the rest is TMEM and shared-memory loads, addresses and waits.
 // Hence:
 //   * one CTA per SM, M = 128 weight rows (8 tiles of 16), N = 32..128 pass rows, one tcgen05.mma (K = 32) per sub-block,
 //     never accumulating: TMEM only hands the int32 dots over to the update, in slots of 2 or 4 sub-blocks;
@@ -26,7 +26,7 @@
 //   * one warp streams the weights (2304-byte tile chunks, ring of 4 blocks, primed before the dependency wait), one the
 //     activations, one thread issues the MMAs.
 // Registers: 512 threads x 128 at launch; the update warps take 184 (8 x 32 threads) from the conversion warps (72) and the
-// last four warps (56): 63488 in all. Only the form of 8 column tiles spills (68 bytes stored, 180 loaded).
+// last four warps (56): 63488 in all.
 // Every wait is bounded and reports through the device status word.
 #include "hp_common.cuh"
 #include "kernels.h"
