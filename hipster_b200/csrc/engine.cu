@@ -372,15 +372,15 @@ int Engine::upload_desc() { HP_CUDA(cudaMemcpyAsync(d_desc_, h_desc_, D_INTS * 4
 static int lin_class_bit(const Lin& l, const hp_model_cfg& c) {
     return l.N == 2 * c.n_ff ? 16 : l.K == c.n_ff ? 32 : l.N == c.n_vocab ? 64 : l.K == c.n_embd ? 128 : 256;
 }
-// A linear over the rows of a prompt chunk; both kernels give the same bits. Up to 32 rows are one pass of the GEMV over the
-// weights; beyond that it streams them again. One line for all projections, where their sum over a 27B layer turns. GEMV against
-// GEMM (us), GDN in-, out-projection, gate|up and down: 24 rows 26 + 13 + 50 + 29 = 118 against 38 + 27 + 72 + 62 = 198;
-// 32 rows 42 + 16 + 86 + 55 = 198 against 38 + 27 + 72 + 62 = 198; 48 rows 60 + 27 + 120 + 77 = 283 against
-// 47 + 32 + 89 + 76 = 244. Single projections turn elsewhere: gate|up below 32 rows, the out-projection between 64 and 96; of
-// the 2048-wide model the in-projections near 48 (GDN) and 128 (attention), the out-projection between 96 and 128.
+// A linear over the rows of a prompt chunk; both kernels give the same bits. The GEMV streams the weights once per 32 rows. One line
+// for all projections, where their sum over a 27B layer turns. GEMV against GEMM (us), GDN in-, out-projection, gate|up and down: 32
+// rows 34 + 16 + 62 + 30 = 142 against 36 + 26 + 67 + 58 = 187; 40 rows 47 + 24 + 85 + 44 = 200 against 44 + 31 + 85 + 73 = 233; 48
+// rows 51 + 27 + 94 + 48 = 220 against about 235; 64 rows 68 + 33 + 124 + 60 = 285 against 54 + 36 + 104 + 84 = 278.
 int Engine::prefill_lin(const Lin& l, float* out, int ld, size_t part_stride, int R) {
-    if (R <= 32) return gemv_q4k_q8_parts(l.wt, xq_, out, l.N, l.K, R, ld, part_stride, err_, s_, pdl_, true);
-    return gemm_q4k_q8_parts(l.wt, xq_, out, l.N, l.K, R, ld, part_stride, pf_pack_, err_, s_, pdl_);
+    if (R > 48) return gemm_q4k_q8_parts(l.wt, xq_, out, l.N, l.K, R, ld, part_stride, pf_pack_, err_, s_, pdl_);
+    for (int r0 = 0; r0 < R; r0 += 32)
+        HP_TRY(gemv_q4k_q8_parts(l.wt, xq_rows(xq_, r0, l.K), out + (size_t)r0 * ld, l.N, l.K, std::min(32, R - r0), ld, part_stride, err_, s_, pdl_, true));
+    return HP_OK;
 }
 int Engine::lin_parts(const Lin& l, int R) {
     if (prof_skip_ & lin_class_bit(l, c_)) return HP_OK;

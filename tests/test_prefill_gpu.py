@@ -41,6 +41,11 @@ def test_prefill_chunks_bit_exact_vs_oracle(preset, n, over):
     eng.close()
 
 
+@pytest.mark.parametrize("n", [32, 40, 48, 49])   # projections in one and two GEMV launches, and in the GEMM
+def test_prefill_on_both_sides_of_the_gemm_line(n):
+    test_prefill_chunks_bit_exact_vs_oracle("tiny", n, {})
+
+
 @pytest.mark.parametrize("n", [17, 42])
 def test_prefill_chunks_fill_the_draft_block(n):
     cfg = hb.ModelCfg.preset("tiny", max_ctx=128)
