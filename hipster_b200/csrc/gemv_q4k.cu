@@ -368,9 +368,9 @@ template <int NT, int CB, int SB, bool TILED, bool XG, bool FEW>
 int launch_sk2(const uint8_t* W, const void* xq, const void* xsc, float* y, int N, int nb, int P, int R, int ldy, size_t part_stride,
                int* err, cudaStream_t s, bool pdl, bool late) {
     const size_t smem = SkGeom<SB, TILED>::FIXED + (XG ? 0 : (size_t)NT * (nb / P) * 2560);
-    static size_t attr_smem[MAX_DEVICES] = {};   // per device: the opt-in belongs to the device's copy of the kernel
+    static size_t attr_smem[MAX_DEVICES] = {};   // per device: the opt-in belongs to the device's copy of the kernel; once, for all sizes
     const int dev = current_device(); if (dev < 0) return HP_ECUDA;
-    if (smem > attr_smem[dev]) { HP_CUDA(cudaFuncSetAttribute(k_gemv_q4k_sk<NT, CB, SB, TILED, XG, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr_smem[dev] = smem; }
+    if (smem > attr_smem[dev]) { HP_CUDA(cudaFuncSetAttribute(k_gemv_q4k_sk<NT, CB, SB, TILED, XG, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMV_SMEM_LIMIT)); attr_smem[dev] = GEMV_SMEM_LIMIT; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(GEMV_NCTA); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = s;
     cudaLaunchAttribute at[1]; at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
