@@ -9,7 +9,10 @@ from ._lib import lib, check, ptr
 # The calls below are a few microseconds of device work, so what they spend in Python counts: the handle of the current stream
 # comes without a Stream object around it, and the short calls pass pointers as integers to declared argument types (_lib.py; to a
 # function without declared types an integer would pass as 32 bits, hence the wrapper of _stream).
-_raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+try:
+    _raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+except AttributeError:   # torch without CUDA: the package still imports, and a call raises torch's own error
+    _raw_stream, _device = (lambda _: torch.cuda.current_stream().cuda_stream), (lambda: 0)
 
 
 def _stream():

@@ -1,6 +1,9 @@
 """Host-side logic that needs no GPU: the K-part rule of the GEMV (library vs the oracle's mirror), model presets, the
 seeded draft substitution, the expected tokens per round, and the expert-parallel ownership map."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -51,3 +54,13 @@ def test_buffer_size_helpers():
     L.hp_argmax_scratch_bytes.restype = ctypes.c_size_t
     assert L.hp_xq8_q_bytes(1, 256) == 256 * 8 and L.hp_xq8_q_bytes(9, 256) == 2 * 256 * 8
     assert L.hp_argmax_scratch_bytes(6, 248320) > 0 and L.hp_argmax_scratch_bytes(0, 5) == 0
+
+
+def test_package_imports_on_a_torch_build_without_cuda():
+    code = ("import torch\n"
+            "for n in ('_cuda_getCurrentRawStream', '_cuda_getDevice'):\n"
+            "    delattr(torch._C, n)\n"                       # what a build without CUDA does not have
+            "import hipster_b200\n"
+            "print(hipster_b200.lib().hp_version())\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and int(r.stdout) >= 100, r.stderr[-2000:]
