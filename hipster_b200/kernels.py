@@ -19,6 +19,11 @@ def _stream():
     return ctypes.c_void_p(_raw_stream(_device()))
 
 
+def _ptr(t):
+    """Device pointer as an integer; None stays None (NULL), which the library refuses by its own error."""
+    return None if t is None else t.data_ptr()
+
+
 class XQ8:
     """Quantised activations (reference: struct XQ8, engine/kernels/gemv.h:8) in the library's private layout."""
 
@@ -57,7 +62,7 @@ def gemv_q4k_q8(w, xq, N, K, y=None):
     R = xq.R
     if y is None:
         y = torch.empty((R, N), dtype=torch.float32, device=w.device)
-    check(lib().hp_gemv_q4k_q8(w.data_ptr(), xq.q.data_ptr(), xq.sc.data_ptr(), y.data_ptr(), N, K, R, y.stride(0), _raw_stream(_device())))
+    check(lib().hp_gemv_q4k_q8(_ptr(w), xq.q.data_ptr(), xq.sc.data_ptr(), y.data_ptr(), N, K, R, y.stride(0), _raw_stream(_device())))
     return y
 
 
@@ -111,7 +116,7 @@ def attn_decode(qkv, pos0, n_head, n_kv, n_rot, q_norm, k_norm, rope, kc, vc, ma
     ws = torch.empty(L.hp_attn_workspace_bytes(R, n_head, n_kv, max_ctx), dtype=torch.uint8, device=qkv.device)
     out = torch.empty((R, n_head * 256), dtype=torch.float32, device=qkv.device)
     xq = XQ8(R, n_head * 256, qkv.device) if want_q8 else None
-    check(L.hp_attn_decode(qkv.data_ptr(), ld, R, int(pos0), n_head, n_kv, n_rot, q_norm.data_ptr(), k_norm.data_ptr(), rope.data_ptr(), kc.data_ptr(), vc.data_ptr(), int(max_ctx),
+    check(L.hp_attn_decode(qkv.data_ptr(), ld, R, int(pos0), n_head, n_kv, n_rot, _ptr(q_norm), _ptr(k_norm), _ptr(rope), _ptr(kc), _ptr(vc), int(max_ctx),
                            out.data_ptr(), xq.q.data_ptr() if xq else None, xq.sc.data_ptr() if xq else None, eps, ws.data_ptr(), _raw_stream(_device())))
     return out, xq
 

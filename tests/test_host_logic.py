@@ -7,9 +7,10 @@ import sys
 
 import numpy as np
 import pytest
+import torch
 
 import hipster_b200 as hb
-from hipster_b200 import ep, spec
+from hipster_b200 import ep, kernels as K_, spec
 from oracle import orc
 
 
@@ -64,3 +65,14 @@ def test_package_imports_on_a_torch_build_without_cuda():
             "print(hipster_b200.lib().hp_version())\n")
     r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and int(r.stdout) >= 100, r.stderr[-2000:]
+
+
+def test_absent_tensors_are_refused_by_the_library(monkeypatch):
+    monkeypatch.setattr(K_, "_raw_stream", lambda dev: 0); monkeypatch.setattr(K_, "_device", lambda: 0)   # refused before any CUDA call
+    t = lambda *s: torch.zeros(s)  # noqa: E731
+    with pytest.raises(hb.HipsterError, match="null pointer"):
+        K_.gemv_q4k_q8(None, K_.XQ8(1, 256, "cpu"), 16, 256, t(1, 16))
+    args = dict(q_norm=t(256), k_norm=t(256), rope=t(128, 32, 2), kc=t(1, 128, 256), vc=t(1, 128, 256))
+    for name in args:
+        with pytest.raises(hb.HipsterError, match="null pointer"):
+            K_.attn_decode(t(1, 2 * 512 + 512), 0, 2, 1, 64, max_ctx=128, **{**args, name: None})
