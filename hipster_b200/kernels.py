@@ -4,10 +4,10 @@ import ctypes
 
 import torch
 
-from ._lib import lib, check, ptr
+from ._lib import lib, hot, check, ptr
 
 # The calls below are a few microseconds of device work, so what they spend in Python counts: the handle of the current stream
-# comes without a Stream object around it, and the short calls pass pointers as integers to declared argument types (_lib.py; to a
+# comes without a Stream object around it, and the short calls pass pointers as integers to declared argument types (_lib.hot; to a
 # function without declared types an integer would pass as 32 bits, hence the wrapper of _stream).
 try:
     _raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
@@ -47,7 +47,7 @@ def quantize_x_q8(x, xq=None):
     assert x.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1
     R, K = x.shape
     xq = xq or XQ8(R, K, x.device)
-    check(lib().hp_quantize_x_q8(x.data_ptr(), x.stride(0), R, K, xq.q.data_ptr(), xq.sc.data_ptr(), _raw_stream(_device())))
+    check(hot().hp_quantize_x_q8(x.data_ptr(), x.stride(0), R, K, xq.q.data_ptr(), xq.sc.data_ptr(), _raw_stream(_device())))
     return xq
 
 
@@ -62,7 +62,7 @@ def gemv_q4k_q8(w, xq, N, K, y=None):
     R = xq.R
     if y is None:
         y = torch.empty((R, N), dtype=torch.float32, device=w.device)
-    check(lib().hp_gemv_q4k_q8(_ptr(w), xq.q.data_ptr(), xq.sc.data_ptr(), y.data_ptr(), N, K, R, y.stride(0), _raw_stream(_device())))
+    check(hot().hp_gemv_q4k_q8(_ptr(w), xq.q.data_ptr(), xq.sc.data_ptr(), y.data_ptr(), N, K, R, y.stride(0), _raw_stream(_device())))
     return y
 
 
@@ -81,7 +81,7 @@ def argmax(logits, n=None):
     ids = torch.empty(R, dtype=torch.int32, device=logits.device)
     vals = torch.empty(R, dtype=torch.float32, device=logits.device)
     # the kernel needs no scratch; the argument must not be null
-    check(lib().hp_argmax(logits.data_ptr(), R, n, ld, ids.data_ptr(), vals.data_ptr(), ids.data_ptr(), _raw_stream(_device())))
+    check(hot().hp_argmax(logits.data_ptr(), R, n, ld, ids.data_ptr(), vals.data_ptr(), ids.data_ptr(), _raw_stream(_device())))
     return ids, vals
 
 
@@ -99,7 +99,7 @@ def argmax_noalloc(logits, n=None):
 def accept_greedy(ids, drafts):
     """-> int32 tensor [mm, bonus] on device (reference host loop, engine/bench/spec27b.cpp:92-97)."""
     out = torch.empty(2, dtype=torch.int32, device=ids.device)
-    check(lib().hp_accept_greedy(ids.data_ptr(), drafts.data_ptr(), drafts.numel(), out.data_ptr(), _raw_stream(_device())))
+    check(hot().hp_accept_greedy(ids.data_ptr(), drafts.data_ptr(), drafts.numel(), out.data_ptr(), _raw_stream(_device())))
     return out
 
 
@@ -116,7 +116,7 @@ def attn_decode(qkv, pos0, n_head, n_kv, n_rot, q_norm, k_norm, rope, kc, vc, ma
     ws = torch.empty(L.hp_attn_workspace_bytes(R, n_head, n_kv, max_ctx), dtype=torch.uint8, device=qkv.device)
     out = torch.empty((R, n_head * 256), dtype=torch.float32, device=qkv.device)
     xq = XQ8(R, n_head * 256, qkv.device) if want_q8 else None
-    check(L.hp_attn_decode(qkv.data_ptr(), ld, R, int(pos0), n_head, n_kv, n_rot, _ptr(q_norm), _ptr(k_norm), _ptr(rope), _ptr(kc), _ptr(vc), int(max_ctx),
+    check(hot().hp_attn_decode(qkv.data_ptr(), ld, R, int(pos0), n_head, n_kv, n_rot, _ptr(q_norm), _ptr(k_norm), _ptr(rope), _ptr(kc), _ptr(vc), int(max_ctx),
                            out.data_ptr(), xq.q.data_ptr() if xq else None, xq.sc.data_ptr() if xq else None, eps, ws.data_ptr(), _raw_stream(_device())))
     return out, xq
 

@@ -76,3 +76,10 @@ def test_absent_tensors_are_refused_by_the_library(monkeypatch):
     for name in args:
         with pytest.raises(hb.HipsterError, match="null pointer"):
             K_.attn_decode(t(1, 2 * 512 + 512), 0, 2, 1, 64, max_ctx=128, **{**args, name: None})
+
+
+def test_library_functions_take_any_ctypes_object():
+    null = ctypes.c_size_t(0)   # an address as a size_t or an int64, as callers with their own bindings pass it
+    L = hb.lib()
+    assert L.hp_argmax(null, 1, ctypes.c_int64(1), 1, null, null, null, null) == 1 and b"null pointer" in L.hp_last_error()
+    assert L.hp_gemv_q4k_q8(null, null, null, null, 16, 256, 1, 16, ctypes.c_uint64(0)) == 1 and b"null pointer" in L.hp_last_error()
