@@ -482,8 +482,8 @@ __global__ void __cluster_dims__(GDN_WCL, 1, 1) __launch_bounds__(256, 3) k_gdn_
     const float4 cv0 = *reinterpret_cast<const float4*>(a.conv_w + (size_t)(v_col + lane) * 4), cv1 = *reinterpret_cast<const float4*>(a.conv_w + (size_t)(v_col + 32 + lane) * 4);
     const float nw0 = bf2f(a.norm_w[64 * rank + lane]), nw1 = bf2f(a.norm_w[64 * rank + 32 + lane]);
     pdl_wait();
-    const int r0 = a.seq ? a.seq[blockIdx.y * 4 + 0] : 0, T = min(a.seq ? a.seq[blockIdx.y * 4 + 1] : a.imm_T, 8), slot = a.seq ? a.seq[blockIdx.y * 4 + 2] : 0;
-    const int nrep = min(a.seq ? (a.replay_n ? a.replay_n[slot] : 0) : a.imm_replay, 8), nrows = nrep + T;
+    const int r0 = a.seq[blockIdx.y * 4 + 0], T = min(a.seq[blockIdx.y * 4 + 1], 8), slot = a.seq[blockIdx.y * 4 + 2];
+    const int nrep = min(a.replay_n ? a.replay_n[slot] : 0, 8), nrows = nrep + T;
     float* sav = a.saved + (size_t)slot * a.saved_stride + (size_t)h * 8 * 388;   // [8][q 128 | k 128 | v 128 | beta | alpha | pad]
     float* cst = a.conv_state + (size_t)slot * a.conv_stride + (size_t)h * 3 * 384;   // [3 taps][q 128 | k 128 | v 128]; private per v-head
     const float* rows = a.rows + (size_t)r0 * a.ld;
@@ -507,11 +507,11 @@ __global__ void __cluster_dims__(GDN_WCL, 1, 1) __launch_bounds__(256, 3) k_gdn_
     for (int q = 0; q < 2; ++q)
 #pragma unroll
         for (int i = 0; i < 8; i += 2) { const float4 v = *reinterpret_cast<const float4*>(Mrow + q * 32 * D + 2 * i); m[q][i] = make_float2(v.x, v.y); m[q][i + 1] = make_float2(v.z, v.w); }
-    auto commit_state = [&](float* dst) {
+    auto commit_state = [&]() {
 #pragma unroll
         for (int q = 0; q < 2; ++q)
 #pragma unroll
-            for (int i = 0; i < 8; i += 2) *reinterpret_cast<float4*>(dst + q * 32 * D + 2 * i) = make_float4(m[q][i].x, m[q][i].y, m[q][i + 1].x, m[q][i + 1].y);
+            for (int i = 0; i < 8; i += 2) *reinterpret_cast<float4*>(Mrow + q * 32 * D + 2 * i) = make_float4(m[q][i].x, m[q][i].y, m[q][i + 1].x, m[q][i + 1].y);
     };
     // gate inputs z of this lane's channels for the row that warp `warp` finishes
     const int Z = a.n_v * D, zc = h * D + 64 * rank + lane;
@@ -568,7 +568,7 @@ __global__ void __cluster_dims__(GDN_WCL, 1, 1) __launch_bounds__(256, 3) k_gdn_
     // ---- the recurrence, row after row, state in registers; no block-wide synchronisation inside
 #pragma unroll 1
     for (int it = 0; it < nrows; ++it) {
-        if (it == nrep && nrep > 0) commit_state(Mrow);
+        if (it == nrep && nrep > 0) commit_state();
         const float beta = sm.sbeta[it], decay = sm.sdecay[it], v0 = sm.sv[it][jl], v1 = sm.sv[it][jl + 32];
         const float* kk = &sm.sqk[it][160 + 20 * ck]; const float* qq = &sm.sqk[it][20 * ck];
         float2 kr[8];
@@ -598,10 +598,9 @@ __global__ void __cluster_dims__(GDN_WCL, 1, 1) __launch_bounds__(256, 3) k_gdn_
 #pragma unroll
             for (int off = 1; off < 8; off <<= 1) { o0 = o0 + __shfl_xor_sync(0xffffffffu, o0, off); o1 = o1 + __shfl_xor_sync(0xffffffffu, o1, off); }
             if (ck == 0) { sm.sout[it - nrep][jl] = o0 * 0.08838834764831845f; sm.sout[it - nrep][jl + 32] = o1 * 0.08838834764831845f; }
-            if (a.snap) commit_state(a.snap + (size_t)(it - nrep) * a.snap_row_stride + ((size_t)h * D + 64 * rank + jl) * D + 16 * ck);
         }
     }
-    if (T == 0 && nrep > 0) commit_state(Mrow);
+    if (T == 0 && nrep > 0) commit_state();
     __syncthreads();
 
     // ---- per-head RMSNorm * w * gate(z) + quantisation of the new rows; warp t takes row t, lane = two channels. The sum of
@@ -684,6 +683,8 @@ int silu_mul_quant(const float* gu, int ldg, int F, XQ8F xq, int R, cudaStream_t
 }
 int gdn_forward(const GdnParams& p, int nseq, cudaStream_t s) {
     HP_REQUIRE(nseq >= 1 && nseq <= 8 && p.n_qk >= 1 && p.n_v >= p.n_qk, "gdn_forward: bad shape");
+    // a sequence described by value, and snapshots, whose rows have no place for a second sequence, are forms of a single one
+    HP_REQUIRE(nseq == 1 || (p.seq && !p.snap), "gdn_forward: %d sequences need descriptors and take no snapshots", nseq);
     GdnArgs a;
     a.rows = p.rows; a.saved = p.saved; a.saved_stride = p.saved_stride; a.ld = p.ld; a.off_z = p.off_z; a.off_b = p.off_b; a.off_a = p.off_a;
     a.n_qk = p.n_qk; a.n_v = p.n_v; a.conv_w = p.conv_w; a.dt_bias = (const uint16_t*)p.dt_bias; a.a_neg = (const uint16_t*)p.a_neg; a.norm_w = (const uint16_t*)p.norm_w;

@@ -83,3 +83,13 @@ def test_library_functions_take_any_ctypes_object():
     L = hb.lib()
     assert L.hp_argmax(null, 1, ctypes.c_int64(1), 1, null, null, null, null) == 1 and b"null pointer" in L.hp_last_error()
     assert L.hp_gemv_q4k_q8(null, null, null, null, 16, 256, 1, 16, ctypes.c_uint64(0)) == 1 and b"null pointer" in L.hp_last_error()
+
+
+def test_gdn_pass_over_several_sequences_needs_descriptors_and_takes_no_snapshots():
+    """Several sequences would write the same snapshot rows, and without descriptors all would be the same sequence: refused before any CUDA call."""
+    from test_gdn_gpu import _Gdn
+    f = getattr(hb.lib(), "_ZN2hp11gdn_forwardERKNS_9GdnParamsEiP11CUstream_st")
+    for nseq in (2, 3, 8):
+        for fields in (dict(seq=4096, snap=4096), dict(seq=None, snap=None, imm_T=1)):
+            p = _Gdn(n_qk=1, n_v=2, **fields)
+            assert f(ctypes.byref(p), nseq, ctypes.c_void_p(0)) == 1 and b"descriptors" in hb.lib().hp_last_error()
