@@ -8,7 +8,7 @@
 namespace hp {
 namespace {
 
-constexpr int AM_CHUNK = 8192;   // elements per stage-1 block of the top-k
+constexpr int AM_CHUNK = 8192;   // elements per stage-1 block of the top-k and of the two-launch arg-max
 
 __device__ __forceinline__ void am_better(float& bv, int& bi, float v, int i) {
     if (v > bv || (v == bv && i < bi && i >= 0)) { bv = v; bi = i; }
@@ -31,40 +31,40 @@ __device__ __forceinline__ void am_block_reduce(float& bv, int& bi, float* sv, i
         }
     }
 }
-// One cluster of up to 8 CTAs per row, each with a contiguous piece of it; the CTAs' winners meet in the first one's shared memory.
-// Bound by latency: one launch instead of a partial and a final one, and no scratch (back to back, 248320 entries: 1 row 3.5 -> 3.9
-// us, 6 rows 3.9 and 3.9, 24 rows 5.5 -> 4.7; a caller saves a launch and an allocation).
-// -inf (an absent entry, or a real one) and NaN never win; a row of nothing else yields -1.
-constexpr int AM_CL = 8, AM_THREADS = 512;
-template <int CL>
-__global__ void __launch_bounds__(AM_THREADS) k_argmax(const float* __restrict__ x, int n, int ld, int* __restrict__ ids, float* __restrict__ vals) {
-    __shared__ float sv[AM_THREADS / 32]; __shared__ int si[AM_THREADS / 32];
+// One cluster of CL CTAs of NT threads per row, each with a contiguous piece of the 16-byte groups of the row; the CTAs' winners meet in
+// the first one's shared memory. Bound by latency: a thread's 16 loads are in flight before its first comparison (launch bounds of
+// one CTA per SM: left alone the compiler takes 32 registers, half the loads and 3.6 us for one row of 248320), the entries in front
+// of the first 16-byte boundary and behind the last one are read one by one. -inf (an absent entry, or a real one) and NaN never win; a
+// row of nothing else yields -1.
+template <int CL, int NT>
+__global__ void __launch_bounds__(NT, 1) k_argmax(const float* __restrict__ x, int n, int ld, int* __restrict__ ids, float* __restrict__ vals) {
+    __shared__ float sv[NT / 32]; __shared__ int si[NT / 32];
     __shared__ float cv[CL]; __shared__ int ci[CL];
     pdl_launch_dependents();
     if constexpr (CL > 1) cluster_arrive_relaxed();   // matched by cluster_wait(): every CTA has started before the first store into another one
     const int r = blockIdx.x / CL, rank = blockIdx.x % CL, tid = threadIdx.x;
-    const int per = (n + 4 * CL - 1) / (4 * CL) * 4, c0 = min(n, rank * per), c1 = min(n, c0 + per);
     const float* xr = x + (size_t)r * ld;
+    const int head = min(n, (int)((16 - (reinterpret_cast<uintptr_t>(xr) & 15)) & 15) / 4), nq = (n - head) / 4;   // whole 16-byte groups
+    const int per = (nq + CL - 1) / CL, q0 = min(nq, rank * per), q1 = min(nq, q0 + per);
+    const float4* xa = reinterpret_cast<const float4*>(xr + head);
     pdl_wait();
     float bv = -INFINITY; int bi = -1;
-    const bool vec = (reinterpret_cast<uintptr_t>(xr) & 15) == 0;
-    const int v1 = vec ? c0 + ((c1 - c0) & ~3) : c0;   // [c0, v1) by 128-bit loads, 16 of a thread in flight; the rest one by one
+    if (rank == 0 && tid < head) am_better(bv, bi, xr[tid], tid);
     constexpr int NV = 16;
-    for (int b = c0 + 4 * tid; b < v1; b += 4 * AM_THREADS * NV) {
+    for (int b = q0 + tid; b < q1; b += NT * NV) {
         float4 v[NV];
 #pragma unroll
-        for (int k = 0; k < NV; ++k) { const int i = b + 4 * AM_THREADS * k; v[k] = i < v1 ? *reinterpret_cast<const float4*>(xr + i) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY); }
+        for (int k = 0; k < NV; ++k) v[k] = b + NT * k < q1 ? xa[b + NT * k] : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
-            const int i = b + 4 * AM_THREADS * k;
+            const int i = head + 4 * (b + NT * k);
             if (v[k].x > bv) { bv = v[k].x; bi = i; }
             if (v[k].y > bv) { bv = v[k].y; bi = i + 1; }
             if (v[k].z > bv) { bv = v[k].z; bi = i + 2; }
             if (v[k].w > bv) { bv = v[k].w; bi = i + 3; }
         }
     }
-#pragma unroll 4
-    for (int i = v1 + tid; i < c1; i += AM_THREADS) am_better(bv, bi, xr[i], i);
+    if (rank == CL - 1) { const int i = head + 4 * nq + tid; if (i < n) am_better(bv, bi, xr[i], i); }
     am_block_reduce(bv, bi, sv, si);
     if constexpr (CL > 1) {
         cluster_wait();
@@ -77,6 +77,34 @@ __global__ void __launch_bounds__(AM_THREADS) k_argmax(const float* __restrict__
         }
     }
     if (rank == 0 && tid == 0) { ids[r] = bi; if (vals) vals[r] = bv; }
+}
+// The form of a few very long rows: one CTA per 8192 entries, whose winners meet in a second launch. All loads of a thread are in flight
+// before the first comparison.
+__global__ void __launch_bounds__(256) k_argmax_part(const float* __restrict__ x, int n, int ld, float* __restrict__ pv, int* __restrict__ pi) {
+    pdl_launch_dependents();
+    pdl_wait();
+    __shared__ float sv[8]; __shared__ int si[8];
+    const int r = blockIdx.y, c0 = blockIdx.x * AM_CHUNK, c1 = min(n, c0 + AM_CHUNK);
+    const float* xr = x + (size_t)r * ld;
+    float bv = -INFINITY; int bi = -1;
+    constexpr int NV = AM_CHUNK / 256;
+    float v[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) { const int i = c0 + threadIdx.x + 256 * k; v[k] = i < c1 ? xr[i] : -INFINITY; }
+#pragma unroll
+    for (int k = 0; k < NV; ++k) if (v[k] > bv) { bv = v[k]; bi = c0 + threadIdx.x + 256 * k; }
+    am_block_reduce(bv, bi, sv, si);
+    if (threadIdx.x == 0) { pv[(size_t)r * gridDim.x + blockIdx.x] = bv; pi[(size_t)r * gridDim.x + blockIdx.x] = bi; }
+}
+__global__ void __launch_bounds__(256) k_argmax_final(const float* __restrict__ pv, const int* __restrict__ pi, int np, int* __restrict__ ids, float* __restrict__ vals) {
+    pdl_launch_dependents();
+    pdl_wait();
+    __shared__ float sv[8]; __shared__ int si[8];
+    const int r = blockIdx.x;
+    float bv = -INFINITY; int bi = -1;
+    for (int i = threadIdx.x; i < np; i += 256) am_better(bv, bi, pv[(size_t)r * np + i], pi[(size_t)r * np + i]);
+    am_block_reduce(bv, bi, sv, si);
+    if (threadIdx.x == 0) { ids[r] = bi; if (vals) vals[r] = bv; }
 }
 // ---- top-k per row (k <= TOPK_MAX), values descending, ties -> lower index (reference k_topk, ops.hip:702-716: k rounds
 // of a masked arg-max). Stage 1: each block holds a chunk of the row in shared memory and extracts the chunk's own top k by
@@ -131,17 +159,30 @@ __global__ void k_accept(const int* __restrict__ ids, const int* __restrict__ dr
 // Limits of the allocation-free entry point: part of its interface
 constexpr int AM_STATIC_ROWS = 32, AM_STATIC_N = 64 * AM_CHUNK;
 
-// rows of up to 4096 entries take one CTA, longer ones a cluster
-int launch_argmax(const float* logits, int R, int n, int ld, int* ids, float* vals, cudaStream_t s) {
-    if (n <= 4096) { HP_CUDA(launch_pdl<1>(k_argmax<1>, dim3(R), dim3(AM_THREADS), 0, s, logits, n, ld, ids, vals)); return HP_OK; }
+template <int CL, int NT>
+int launch_argmax_cl(const float* logits, int R, int n, int ld, int* ids, float* vals, cudaStream_t s) {
+    if constexpr (CL > 8) {   // beyond the portable cluster size
+        static bool attr[MAX_DEVICES] = {};   // per device: the opt-in belongs to the device's copy of the kernel
+        const int dev = current_device(); if (dev < 0) return HP_ECUDA;
+        if (!attr[dev]) { HP_CUDA(cudaFuncSetAttribute(k_argmax<CL, NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)); attr[dev] = true; }
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(R * AM_CL); cfg.blockDim = dim3(AM_THREADS); cfg.stream = s;
+    cfg.gridDim = dim3(R * CL); cfg.blockDim = dim3(NT); cfg.stream = s;
     cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = AM_CL; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = CL; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = (pdl_off_mask(s) & 1) ? 1 : 2;
-    HP_CUDA(cudaLaunchKernelEx(&cfg, k_argmax<AM_CL>, logits, n, ld, ids, vals));
+    HP_CUDA(cudaLaunchKernelEx(&cfg, k_argmax<CL, NT>, logits, n, ld, ids, vals));
     return HP_OK;
+}
+// One launch, without scratch. us in a captured graph for rows of 1, 6 and 24 (two launches of 8192-entry pieces in brackets): one CTA
+// up to 32768 entries, 2.6 2.7 2.8 there (3.5 3.7 4.2); 8 small CTAs, 65536: 2.6 2.8 3.3 (3.5 3.6 4.4); 8 CTAs, 248320: 3.3 3.4 4.8
+// (3.9 3.9 5.8); 16 CTAs for up to 12 longer rows, 524288: 3.6 3.7 (4.0 4.9), where 8 take 4.3 4.4, and 24 rows 6.8 (16: 8.0).
+int launch_argmax(const float* logits, int R, int n, int ld, int* ids, float* vals, cudaStream_t s) {
+    if (n <= 32768) return launch_argmax_cl<1, 512>(logits, R, n, ld, ids, vals, s);
+    if (n <= 65536) return launch_argmax_cl<8, 256>(logits, R, n, ld, ids, vals, s);
+    if (n <= 262144 || R > 12) return launch_argmax_cl<8, 512>(logits, R, n, ld, ids, vals, s);
+    return launch_argmax_cl<16, 512>(logits, R, n, ld, ids, vals, s);
 }
 
 }  // namespace
@@ -150,7 +191,14 @@ size_t argmax_scratch_bytes(int R, int n) { return (size_t)R * ((n + AM_CHUNK - 
 
 int argmax_rows(const float* logits, int R, int n, int ld, int* ids, float* vals, void* scratch, cudaStream_t s) {
     HP_REQUIRE(R >= 1 && n >= 1 && ld >= n && scratch, "argmax_rows: bad arguments R=%d n=%d ld=%d", R, n, ld);
-    return launch_argmax(logits, R, n, ld, ids, vals, s);
+    // few rows longer than a cluster reads at once take two launches (one row of 1 M entries 4.0 us, 4.5 in one launch; 4 M 5.7 and 10.0;
+    // 24 rows of 1 M 16.2 and 11.3)
+    if (n <= 524288 || R > 5) return launch_argmax(logits, R, n, ld, ids, vals, s);
+    const int np = (n + AM_CHUNK - 1) / AM_CHUNK;
+    float* pv = (float*)scratch; int* pi = (int*)(pv + (size_t)R * np);
+    HP_CUDA(launch_pdl<1>(k_argmax_part, dim3(np, R), dim3(256), 0, s, logits, n, ld, pv, pi));
+    HP_CUDA(launch_pdl<1>(k_argmax_final, dim3(R), dim3(256), 0, s, (const float*)pv, (const int*)pi, np, ids, vals));
+    return HP_OK;
 }
 size_t topk_scratch_bytes(int R, int n, int k) { return (size_t)R * ((n + AM_CHUNK - 1) / AM_CHUNK) * k * 8; }
 int topk_max_k() { return TOPK_MAX; }
@@ -167,7 +215,7 @@ int topk_rows(const float* logits, int R, int n, int ld, int k, int* ids, float*
 int argmax_static_max_rows() { return AM_STATIC_ROWS; }
 int argmax_static_max_n() { return AM_STATIC_N; }
 
-// Same kernel as argmax_rows, for callers without any scratch.
+// For callers without any scratch: always one launch.
 int argmax_rows_static(const float* logits, int R, int n, int ld, int* ids, float* vals, cudaStream_t s) {
     HP_REQUIRE(R >= 1 && n >= 1 && ld >= n, "argmax_rows_static: bad arguments R=%d n=%d ld=%d", R, n, ld);
     HP_REQUIRE(R <= AM_STATIC_ROWS && n <= AM_STATIC_N, "argmax_rows_static: R=%d n=%d exceed the limits (at most %d rows of %d entries)", R, n, AM_STATIC_ROWS, AM_STATIC_N);

@@ -96,7 +96,7 @@ def test_argmax_and_accept():
         assert tuple(out) == orc.accept(oi, drafts)
 
 
-# one CTA per row up to 4096 entries, a cluster of eight beyond; pieces that are empty, ragged and unaligned rows (odd ld), ties across pieces
+# one CTA per row for short rows, clusters for longer ones; pieces that are empty, ragged and unaligned rows (odd ld), ties across pieces
 @pytest.mark.parametrize("n,ld", [(1, 1), (7, 9), (4095, 4096), (4096, 4096), (4097, 4097), (4100, 4100), (70001, 70003), (262147, 262148)])
 def test_argmax_at_the_edges_of_its_pieces(n, ld):
     rng = np.random.default_rng(n)
@@ -112,6 +112,21 @@ def test_argmax_at_the_edges_of_its_pieces(n, ld):
     assert ids.cpu().tolist() == want and np.array_equal(bits(vals.cpu().numpy()), bits(a[range(5), want]))
     none, v = K_.argmax(dev(np.full((1, n), -np.inf, np.float32)))
     assert none.item() == -1 and v.item() == -np.inf
+
+
+# both sides of every line between the forms (rows of one CTA, of 8 small ones, of 8, of 16 for up to 12 rows, two launches for up to 5),
+# rows that start at every offset from a 16-byte boundary; the maximum in front of the first whole group, behind the last, tied with the middle
+@pytest.mark.parametrize("R,n", [(2, 3), (2, 32768), (2, 32769), (3, 65536), (3, 65537), (2, 262144), (12, 262147), (13, 262147), (1, 524288), (5, 524289), (6, 524289), (1, 1 << 21)])
+def test_argmax_forms(R, n):
+    for off in (0, 1, 3):
+        buf = torch.randn((R, n + 4 + (off & 1)), device="cuda"); x = buf[:, off:off + n]
+        buf[:, :off] = 1e9; buf[:, off + n:] = 1e9
+        want = x.argmax(1).tolist()
+        for r, (hi, lo) in enumerate([(n - 1, n - 1), (n // 2, 0), (n - 1, n // 3), (1, 0)][:R]):
+            x[r, hi] = x[r, lo] = 50.0
+            want[r] = lo
+        ids, vals = K_.argmax(x)
+        assert ids.tolist() == want and torch.equal(vals, x[torch.arange(R), torch.tensor(want)])
 
 
 def test_config1_kernel_check_full_size():
