@@ -179,7 +179,7 @@ int launch_argmax_cl(const float* logits, int R, int n, int ld, int* ids, float*
 // up to 32768 entries, 2.6 2.7 2.8 there (3.5 3.7 4.2); 8 small CTAs, 65536: 2.6 2.8 3.3 (3.5 3.6 4.4); 8 CTAs, 248320: 3.3 3.4 4.8
 // (3.9 3.9 5.8); 16 CTAs for up to 12 longer rows, 524288: 3.6 3.7 (4.0 4.9), where 8 take 4.3 4.4, and 24 rows 6.8 (16: 8.0).
 int launch_argmax(const float* logits, int R, int n, int ld, int* ids, float* vals, cudaStream_t s) {
-    if (n <= 32768) return launch_argmax_cl<1, 512>(logits, R, n, ld, ids, vals, s);
+    if (n <= 32768) { HP_CUDA(launch_pdl<1>(k_argmax<1, 512>, dim3(R), dim3(512), 0, s, logits, n, ld, ids, vals)); return HP_OK; }
     if (n <= 65536) return launch_argmax_cl<8, 256>(logits, R, n, ld, ids, vals, s);
     if (n <= 262144 || R > 12) return launch_argmax_cl<8, 512>(logits, R, n, ld, ids, vals, s);
     return launch_argmax_cl<16, 512>(logits, R, n, ld, ids, vals, s);
@@ -187,10 +187,11 @@ int launch_argmax(const float* logits, int R, int n, int ld, int* ids, float* va
 
 }  // namespace
 
-size_t argmax_scratch_bytes(int R, int n) { return (size_t)R * ((n + AM_CHUNK - 1) / AM_CHUNK) * 8; }
+// winners of the pieces of a row; rows of up to 65536 entries take one launch whatever their number
+size_t argmax_scratch_bytes(int R, int n) { return n <= 65536 ? 0 : (size_t)R * ((n + AM_CHUNK - 1) / AM_CHUNK) * 8; }
 
 int argmax_rows(const float* logits, int R, int n, int ld, int* ids, float* vals, void* scratch, cudaStream_t s) {
-    HP_REQUIRE(R >= 1 && n >= 1 && ld >= n && scratch, "argmax_rows: bad arguments R=%d n=%d ld=%d", R, n, ld);
+    HP_REQUIRE(R >= 1 && n >= 1 && ld >= n && (scratch || argmax_scratch_bytes(R, n) == 0), "argmax_rows: bad arguments R=%d n=%d ld=%d", R, n, ld);
     // few rows longer than a cluster reads at once take two launches (one row of 1 M entries 4.0 us, 4.5 in one launch; 4 M 5.7 and 10.0;
     // 24 rows of 1 M 16.2 and 11.3)
     if (n <= 524288 || R > 5) return launch_argmax(logits, R, n, ld, ids, vals, s);

@@ -62,7 +62,7 @@ def gemv_q4k_q8(w, xq, N, K, y=None):
     R = xq.R
     if y is None:
         y = torch.empty((R, N), dtype=torch.float32, device=w.device)
-    check(hot().hp_gemv_q4k_q8(_ptr(w), xq.q.data_ptr(), xq.sc.data_ptr(), y.data_ptr(), N, K, R, y.stride(0), _raw_stream(_device())))
+    check(hot().hp_gemv_q4k_q8(None if w is None else w.data_ptr(), xq.q.data_ptr(), xq.sc.data_ptr(), y.data_ptr(), N, K, R, y.stride(0), _raw_stream(_device())))
     return y
 
 
@@ -78,10 +78,11 @@ def argmax(logits, n=None):
     """Row-wise argmax (max value, lowest index) -> (ids int32 [R], vals f32 [R]) (reference argmax_topk k=1, ops.h:118)."""
     R, ld = logits.shape[0], logits.stride(0)
     n = n or logits.shape[1]
-    ids = torch.empty(R, dtype=torch.int32, device=logits.device)
-    vals = torch.empty(R, dtype=torch.float32, device=logits.device)
-    # the kernel needs no scratch; the argument must not be null
-    check(hot().hp_argmax(logits.data_ptr(), R, n, ld, ids.data_ptr(), vals.data_ptr(), ids.data_ptr(), _raw_stream(_device())))
+    dev, nb = logits.device, lib().hp_argmax_scratch_bytes(R, n)
+    ids = torch.empty(R, dtype=torch.int32, device=dev)
+    vals = torch.empty(R, dtype=torch.float32, device=dev)
+    scratch = torch.empty(nb, dtype=torch.uint8, device=dev) if nb else None
+    check(hot().hp_argmax(logits.data_ptr(), R, n, ld, ids.data_ptr(), vals.data_ptr(), scratch.data_ptr() if nb else None, _raw_stream(_device())))
     return ids, vals
 
 

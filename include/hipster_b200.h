@@ -51,8 +51,8 @@ int hp_gemv_parts(int N, int K);
 /* f32-activation baseline, R <= 8, y [R][N]. Replaces gemv_q4_K_f32 (gemv.h:57, gemv.hip:1177-1216). */
 int hp_gemv_q4k_f32(const void* w_dev, const float* x_dev, float* y_dev, int N, int K, int R, void* stream);
 /* Row-wise argmax (maximum value, lowest index on ties) of logits [R][ld] over n entries.
- * Replaces argmax_topk with k = 1 (ops.h:118, ops.hip:702-716). scratch_dev: hp_argmax_scratch_bytes(R, n) bytes (must
- * not be null; the present kernel leaves them alone). */
+ * Replaces argmax_topk with k = 1 (ops.h:118, ops.hip:702-716). scratch_dev: hp_argmax_scratch_bytes(R, n) bytes of
+ * the caller's, which no other call may use meanwhile; rows of up to 65536 entries need none (0 bytes: may be null). */
 size_t hp_argmax_scratch_bytes(int R, int n);
 int hp_argmax(const float* logits_dev, int R, int n, int ld, int* ids_dev, float* vals_dev, void* scratch_dev, void* stream);
 /* hp_argmax for callers that must not allocate. It has no counterpart in the reference. A serving loop that has sized

@@ -93,3 +93,22 @@ def test_gdn_pass_over_several_sequences_needs_descriptors_and_takes_no_snapshot
         for fields in (dict(seq=4096, snap=4096), dict(seq=None, snap=None, imm_T=1)):
             p = _Gdn(n_qk=1, n_v=2, **fields)
             assert f(ctypes.byref(p), nseq, ctypes.c_void_p(0)) == 1 and b"descriptors" in hb.lib().hp_last_error()
+
+
+def test_argmax_hands_over_a_scratch_of_the_stated_size(monkeypatch):
+    """A buffer of hp_argmax_scratch_bytes of its own wherever the library asks for one, no buffer where it asks for none."""
+    L = hb.lib()
+    assert L.hp_argmax_scratch_bytes(32, 65536) == 0 and L.hp_argmax_scratch_bytes(1, 65537) >= 8
+    p = ctypes.c_void_p(4096)   # refused before any CUDA call
+    assert L.hp_argmax(p, 1, 65537, 65537, p, None, None, None) == 1 and b"bad arguments" in L.hp_last_error()
+    made, calls = [], []
+    empty = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: made.append(empty(*a, **k)) or made[-1])
+    monkeypatch.setattr(K_, "hot", lambda: type("Lib", (), {"hp_argmax": staticmethod(lambda *a: calls.append(a) or 0)}))
+    monkeypatch.setattr(K_, "_raw_stream", lambda dev: 0); monkeypatch.setattr(K_, "_device", lambda: 0)
+    for R, n in ((3, 17408), (6, 248320), (1, 65537)):
+        made.clear()
+        ids, vals = K_.argmax(torch.zeros((R, n)))
+        scratch, need = calls[-1][6], L.hp_argmax_scratch_bytes(R, n)
+        bufs = {t.data_ptr(): t.numel() * t.element_size() for t in made if t is not ids and t is not vals}
+        assert (scratch is None and not bufs) if need == 0 else bufs[scratch] >= need
