@@ -141,12 +141,17 @@ __global__ void __launch_bounds__(SK_THREADS, 1) k_gemv_q4k_sk(const uint8_t* __
             for (int i = 0; i < NA; ++i) acc[n][i] = make_float2(0.f, 0.f);
     };
     zero_acc();
+    // The order of the sum in store_tile decides what the compiler keeps in registers across the loop. From the left, 5 to 8 rows of
+    // 248320 x 2048 take 52.6 us (53.8 otherwise) and 17 to 24 of 34816 x 5120 43.5 (44.3); in the other order 13 and 25 rows of
+    // 248320 x 2048 74.5 and 121.7 (75.6 and 123.7), 17 row-major ones 112.5 (116.5).
+    constexpr bool LEFT = XG || SPU > 1 || (NT == 1 && CB == 2) || (NT == 4 && !TILED);
     auto store_tile = [&](int tile, const float (&v)[NT][NV]) {
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
             for (int k = 0; k < NV; ++k) {
-                const int row = tile * 16 + (FEW ? few.row : g + ((k & 2) ? 8 : 0)), col = n * 8 + (FEW ? few.col : 2 * t) + (k & 1);
+                const int g8 = (k & 2) ? 8 : 0, col = n * 8 + (FEW ? few.col : 2 * t) + (k & 1);
+                const int row = FEW ? tile * 16 + few.row : LEFT ? tile * 16 + g + g8 : tile * 16 + (g + g8);
                 if (row < N && col < R) y[(size_t)col * ldy + row] = v[n][k];
             }
     };
