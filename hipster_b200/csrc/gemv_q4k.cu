@@ -456,9 +456,10 @@ int gemv_q4k_q8_parts(const void* W, const XQ8F& x, float* yparts, int N, int K,
     // (three tiles of 20 blocks beside one-block stages: 34816 x 5120 at 24 rows 44.5 us, from L2 50.8)
     auto fits = [&](int nt) { return tiled ? (nbp % 2 || nt == 3 ? sk_fits<1, true>(nt, nbp) : sk_fits<2, true>(nt, nbp)) : (nbp % 2 ? sk_fits<1, false>(nt, nbp) : sk_fits<2, false>(nt, nbp)); };
     const bool staged = ntile == 1 || fits(ntile);
-    // ... unless the matrix is large: two launches of column tiles that fit stream it twice in less time than one waits for L2 (32
-    // rows of 34816 x 5120: 86 -> 64 us, 16480 x 5120: 42 -> 35; 2048 x 6144, 7 MB: 11.0 -> 11.4)
-    if (!staged && R > 16 && fits(2) && (size_t)N * nb * 144 >= SPLIT_BYTES) {
+    // ... unless there are four tiles and the matrix is large: two launches of two tiles each stream it twice in less time than one waits
+    // for L2 (32 rows of 34816 x 5120: 86 -> 62 us, row-major 103 -> 75; 2048 x 6144, 7 MB: 10.8 in one, 11.4 in two). Three tiles are
+    // better off in one (24 rows row-major, 16480 x 5120: 30 against 36 us, 34816 x 5120: 60 against 67).
+    if (!staged && R > 24 && fits(2) && (size_t)N * nb * 144 >= SPLIT_BYTES) {
         const int rc1 = gemv_q4k_q8_parts(W, x, yparts, N, K, 16, ldy, part_stride, err, s, pdl, tiled, late);
         if (rc1 != HP_OK) return rc1;
         return gemv_q4k_q8_parts(W, XQ8F{(char*)x.q + xq_q_bytes(16, K), (char*)x.sc + xq_sc_floats(16, K) * 4}, yparts + (size_t)16 * ldy, N, K, R - 16, ldy, part_stride, err, s, pdl, tiled, late);

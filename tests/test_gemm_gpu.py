@@ -88,7 +88,7 @@ def test_every_cut_gives_the_bits_of_the_gemv(weights, ntc, G):
 # the tile-major form of the GEMV on both sides of its row limits (4 rows; three column tiles whose activations leave room for one-block
 # stages only: 20 blocks), against the row-major one
 @pytest.mark.gpu
-@pytest.mark.parametrize("R", [1, 4, 5, 8, 16, 17, 24])
+@pytest.mark.parametrize("R", [1, 4, 5, 8, 16, 17, 24, 25, 32])
 @pytest.mark.parametrize("N,K", [(100, 5120), (16480, 5120), (4096, 768), (2100, 17408)])
 def test_tile_major_gemv_gives_the_bits_of_the_row_major_one(N, K, R):
     g = torch.Generator(device="cuda").manual_seed(R)
@@ -101,6 +101,26 @@ def test_tile_major_gemv_gives_the_bits_of_the_row_major_one(N, K, R):
         got += p
     assert err.item() == 0
     assert torch.equal(got.view(torch.int32), K_.gemv_q4k_q8(blk, xq, N, K).view(torch.int32))
+
+
+# rows 25 to 32 of a large matrix run as two launches in both layouts: against one launch per column tile, in one K part and in two, an
+# even and an odd number of blocks per part; three tiles stay in one
+@pytest.mark.gpu
+@pytest.mark.parametrize("R", [24, 25, 32])
+@pytest.mark.parametrize("N,K,parts", [(16480, 5120, 1), (8192, 10240, 2), (16480, 5888, 1)])
+def test_two_launches_give_the_bits_of_single_column_tiles(N, K, parts, R):
+    assert hb.lib().hp_gemv_parts(N, K) == parts
+    g = torch.Generator(device="cuda").manual_seed(R)
+    blk = torch.randint(0, 256, (N * (K // 256), 144), dtype=torch.uint8, device="cuda", generator=g)
+    blk[:, :4] = torch.randn((blk.shape[0], 2), device="cuda", generator=g).mul_(0.01).abs_().half().view(torch.uint8)
+    x = torch.randn((R, K), device="cuda", generator=g); xq = K_.quantize_x_q8(x); err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    tiled = K_.repack_tiled(blk.reshape(-1), N, K, 0)
+    planes, rows = run_gemv(tiled, xq, N, K, R, N, err), K_.gemv_q4k_q8(blk, xq, N, K)
+    for r0 in range(0, R, 8):
+        r1 = min(R, r0 + 8); x8 = K_.quantize_x_q8(x[r0:r1].contiguous())
+        assert torch.equal(planes[:, r0:r1].view(torch.int32), run_gemv(tiled, x8, N, K, r1 - r0, N, err).view(torch.int32))
+        assert torch.equal(rows[r0:r1].view(torch.int32), K_.gemv_q4k_q8(blk, x8, N, K).view(torch.int32))
+    assert err.item() == 0
 
 
 @pytest.mark.parametrize("ntc,G", [(5, 8), (0, 8), (18, 8), (2, 8), (-4, 8), (8, 2), (8, 16), (8, 0)])
