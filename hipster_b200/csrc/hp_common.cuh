@@ -191,16 +191,18 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
-// 64-bit shared-memory reads. A 128-bit read takes four passes of the shared-memory pipe however few distinct addresses the warp has (16
-// clocks per warp of a sub-partition, measured with 4, 8 and 32), a 64-bit one a single pass (4 clocks) as long as the addresses fit in
-// 128 bytes: what several lanes read alike is fetched in two of these. volatile keeps the compiler from joining them again.
+// 64-bit shared-memory reads. A 128-bit read of 4 to 32 distinct addresses takes four passes of the shared-memory pipe (16 clocks per warp of
+// a sub-partition; 8 with one address), a 64-bit one a single pass (4 clocks) as long as the addresses fit in 128 bytes: what several
+// lanes read alike is fetched in two of these. volatile keeps the compiler from joining them again, the memory clobber keeps them
+// behind the stores in front of them (it costs nothing measurable: expert layer of 24 rows 114.3 and 113.6 us, eight GDN sequences and
+// the prompt scan the same).
 __device__ __forceinline__ float2 lds_f2(const void* p) {
-    float2 v; asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_u32(p))); return v;
+    float2 v; asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(smem_u32(p)) : "memory"); return v;
 }
 __device__ __forceinline__ uint4 lds_u4_halves(const void* p) {
     uint4 v;
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(smem_u32(p)));
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2+8];" : "=r"(v.z), "=r"(v.w) : "r"(smem_u32(p)));
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(smem_u32(p)) : "memory");
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2+8];" : "=r"(v.z), "=r"(v.w) : "r"(smem_u32(p)) : "memory");
     return v;
 }
 
