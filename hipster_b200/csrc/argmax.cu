@@ -220,10 +220,15 @@ int argmax_static_max_n() { return AM_STATIC_N; }
 int argmax_rows_static(const float* logits, int R, int n, int ld, int* ids, float* vals, cudaStream_t s) {
     HP_REQUIRE(R >= 1 && n >= 1 && ld >= n, "argmax_rows_static: bad arguments R=%d n=%d ld=%d", R, n, ld);
     HP_REQUIRE(R <= AM_STATIC_ROWS && n <= AM_STATIC_N, "argmax_rows_static: R=%d n=%d exceed the limits (at most %d rows of %d entries)", R, n, AM_STATIC_ROWS, AM_STATIC_N);
-    // a kernel can only be launched into a stream of the current device
+    // a kernel can only be launched into a stream of the current device. A capturing stream may not be asked for its device (the question
+    // would end the capture): there the launch itself refuses
     const int cur = current_device();
     int dev = cur;
-    if (s != nullptr && s != cudaStreamLegacy && s != cudaStreamPerThread) HP_CUDA(cudaStreamGetDevice(s, &dev));
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (s != nullptr && s != cudaStreamLegacy && s != cudaStreamPerThread) {
+        HP_CUDA(cudaStreamIsCapturing(s, &cap));
+        if (cap == cudaStreamCaptureStatusNone) HP_CUDA(cudaStreamGetDevice(s, &dev));
+    }
     HP_REQUIRE(cur >= 0 && dev == cur, "argmax_rows_static: the stream belongs to device %d but device %d is current", dev, cur);
     return launch_argmax(logits, R, n, ld, ids, vals, s);
 }

@@ -60,7 +60,7 @@ int hp_argmax(const float* logits_dev, int R, int n, int ld, int* ids_dev, float
  * afford a cudaMalloc per call: the allocation may fail, and it serialises against everything running on the device.
  * This variant takes no scratch and allocates nothing. It accepts at most hp_argmax_noalloc_max_rows() rows of
  * hp_argmax_noalloc_max_n() entries and rejects larger shapes with HP_EINVAL. The stream must belong to the current
- * device (a stream of another device is refused) and must not be capturing. */
+ * device (a stream of another device is refused); it may be capturing. */
 int hp_argmax_noalloc(const float* logits_dev, int R, int n, int ld, int* ids_dev, float* vals_dev, void* stream);
 int hp_argmax_noalloc_max_rows(void);
 int hp_argmax_noalloc_max_n(void);
