@@ -318,12 +318,11 @@ int attn_decode(const AttnParams& p, int rows, int ngroups, cudaStream_t s) {
 }  // namespace hp
 
 namespace hp {
-// Kernel-level form for one sequence: rows r = 0..R-1 at positions pos0 + r, described by value. The workspace holds the split partials
-// behind 1024 unused bytes.
+// Kernel-level form for one sequence: rows r = 0..R-1 at positions pos0 + r, described by value. The workspace holds the split partials.
 static int attn_seq_groups(int R, int n_head, int n_kv) { const int gr = std::max(1, std::min(8, ATTN_MAX_PAIRS / (n_head / n_kv))); return (R + gr - 1) / gr; }
 size_t attn_seq_workspace_bytes(int R, int n_head, int n_kv, int max_ctx) {
     const size_t np = attn_partial_floats(attn_seq_groups(R, n_head, n_kv), n_kv, (max_ctx + ATTN_SPLIT - 1) / ATTN_SPLIT);
-    return 1024 + np * (HD + 2) * sizeof(float);
+    return np * (HD + 2) * sizeof(float);
 }
 int attn_decode_seq(float* qkv, int ld, int R, int pos0, int n_head, int n_kv, int n_rot, const void* q_norm, const void* k_norm, const void* rope, void* kc, void* vc, int max_ctx,
                     float* out, XQ8F xq, float eps, void* workspace, cudaStream_t s) {
@@ -334,7 +333,7 @@ int attn_decode_seq(float* qkv, int ld, int R, int pos0, int n_head, int n_kv, i
     p.row_pos = p.row_slot = p.row_group = p.groups = nullptr; p.imm_pos0 = pos0; p.imm_gr = gr; p.group_rows = std::min(gr, R);
     p.kc = kc; p.vc = vc; p.kv_stride = 0; p.max_ctx = max_ctx; p.nsplit_max = (max_ctx + ATTN_SPLIT - 1) / ATTN_SPLIT;
     const size_t np = attn_partial_floats(ng, n_kv, p.nsplit_max);
-    p.pO = (float*)((char*)workspace + 1024); p.pm = p.pO + np * HD; p.pl = p.pm + np;
+    p.pO = (float*)workspace; p.pm = p.pO + np * HD; p.pl = p.pm + np;
     p.out = out; p.xq = xq; p.eps = eps;
     const int rc = attn_rope_kv(p, R, s);
     return rc != HP_OK ? rc : attn_decode(p, R, ng, s);

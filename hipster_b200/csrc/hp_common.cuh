@@ -266,12 +266,10 @@ struct FewCols {
 // fp32, is 12582912 + idot exactly (|idot| < 2^22), so the int -> float conversion is one exact packed subtraction.
 struct Q4kGroup {
     uint32_t alo[4], ahi[4];
-    __device__ __forceinline__ Q4kGroup() {}
     __device__ __forceinline__ Q4kGroup(uint2 w0, uint2 w1)
         : alo{w0.x & 0x0F0F0F0Fu, w1.x & 0x0F0F0F0Fu, w0.y & 0x0F0F0F0Fu, w1.y & 0x0F0F0F0Fu}, ahi{w0.x & 0xF0F0F0F0u, w1.x & 0xF0F0F0F0u, w0.y & 0xF0F0F0F0u, w1.y & 0xF0F0F0F0u} {}
     struct Scales {   // of both rows and both sub-blocks: shared by all column tiles
         float4 a0, b0, a1, b1;
-        __device__ __forceinline__ Scales() {}
         __device__ __forceinline__ Scales(const RowScales& ra, const RowScales& rb, int j) : a0(ra.get(2 * j)), b0(rb.get(2 * j)), a1(ra.get(2 * j + 1)), b1(rb.get(2 * j + 1)) {}
     };
     struct ColScales { float2 d, s; };   // of the lane's two columns in one sub-block
