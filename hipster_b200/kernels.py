@@ -19,11 +19,6 @@ def _stream():
     return ctypes.c_void_p(_raw_stream(_device()))
 
 
-def _ptr(t):
-    """Device pointer as an integer; None stays None (NULL), which the library refuses by its own error."""
-    return None if t is None else t.data_ptr()
-
-
 class XQ8:
     """Quantised activations (reference: struct XQ8, engine/kernels/gemv.h:8) in the library's private layout."""
 
@@ -117,8 +112,10 @@ def attn_decode(qkv, pos0, n_head, n_kv, n_rot, q_norm, k_norm, rope, kc, vc, ma
     ws = torch.empty(L.hp_attn_workspace_bytes(R, n_head, n_kv, max_ctx), dtype=torch.uint8, device=qkv.device)
     out = torch.empty((R, n_head * 256), dtype=torch.float32, device=qkv.device)
     xq = XQ8(R, n_head * 256, qkv.device) if want_q8 else None
-    check(hot().hp_attn_decode(qkv.data_ptr(), ld, R, int(pos0), n_head, n_kv, n_rot, _ptr(q_norm), _ptr(k_norm), _ptr(rope), _ptr(kc), _ptr(vc), int(max_ctx),
-                           out.data_ptr(), xq.q.data_ptr() if xq else None, xq.sc.data_ptr() if xq else None, eps, ws.data_ptr(), _raw_stream(_device())))
+    check(hot().hp_attn_decode(qkv.data_ptr(), ld, R, int(pos0), n_head, n_kv, n_rot, None if q_norm is None else q_norm.data_ptr(),
+                               None if k_norm is None else k_norm.data_ptr(), None if rope is None else rope.data_ptr(), None if kc is None else kc.data_ptr(),
+                               None if vc is None else vc.data_ptr(), int(max_ctx), out.data_ptr(), xq.q.data_ptr() if xq else None, xq.sc.data_ptr() if xq else None,
+                               eps, ws.data_ptr(), _raw_stream(_device())))
     return out, xq
 
 
