@@ -272,12 +272,13 @@ __device__ __forceinline__ float2 gdn_fma2(float2 a, float2 b, float2 c) {   // 
         : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)), "l"(reinterpret_cast<unsigned long long&>(c)));
     return r;
 }
-// Passes over one or two sequences: one wave of a latency-bound kernel (one sequence of 6 rows, 4 replayed: 16.4 us with 128-bit reads of q
-// and k in the recurrence, 15.3 with 64-bit ones, see lds_f2; 1 row, 1 replayed: 9.3 and 8.4).
+// Passes over one or two sequences: one wave of a latency-bound kernel. One sequence of 6 rows, 4 replayed: 12.7 us in a captured graph,
+// of 1 row, 1 replayed 7.8, two sequences of 6 rows 16.9 (q and k of the recurrence by 64-bit reads, see lds_f2; by 128-bit ones 12.8, 7.9
+// and 17.0).
 __global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, 3) k_gdn(GdnArgs a) {
     constexpr int D = 128, NLD = 8, NCV = 6;   // items per thread: (16 + 3) * 96 <= 8 * 256 raw values, 16 * 96 = 6 * 256 conv outputs
     // conv'ed, then normalised q | k of every row (filled by all four CTAs); 16-float chunks padded to 20 so that the
-    // eight chunk owners of a state row read 128 bits each from distinct banks
+    // eight chunk owners of a state row read 64 bits each from distinct banks
     __shared__ __align__(16) float sqk[GDN_MAXROWS][2 * 160];
     __shared__ float raw[GDN_MAXROWS + 3][96], sv[GDN_MAXROWS][32], sout[8][32];
     __shared__ float csum[GDN_MAXROWS][2][GDN_CL], snrm[GDN_MAXROWS][2], sbeta[GDN_MAXROWS], sdecay[GDN_MAXROWS];
@@ -466,8 +467,8 @@ struct GdnWideSmem {
 // state rows. Every CTA convolves and normalises the head's 128 q and 128 k channels itself (warp w: 32 q channels for w < 4, 32 k
 // channels otherwise) and its own 64 v channels, from raw inputs that arrive by asynchronous copies; both CTAs read the saved rows and
 // the history, so these are rewritten at the end, behind the cluster barrier of the output norm. Sums and their order are those of
-// k_gdn. Eight sequences of 3 rows, 2 replayed: 30.8 us a launch, k_gdn 38.5; one sequence of 6 rows, 4 replayed: 16.8 and 15.3, of 1
-// row, 1 replayed: 9.9 and 8.4.
+// k_gdn. us in a captured graph, k_gdn in brackets: eight sequences of 3 rows, 2 replayed, 30.5 (43.6; 39.7 with registers for four CTAs per
+// SM), three of them 13.8 (21.7); two sequences of 6 rows, 4 replayed, 17.8 (16.9), one 13.1 (12.7).
 __global__ void __cluster_dims__(GDN_WCL, 1, 1) __launch_bounds__(256, 3) k_gdn_wide(GdnArgs a) {
     constexpr int D = 128;
     extern __shared__ __align__(16) uint8_t gdn_smem[];
@@ -482,7 +483,8 @@ __global__ void __cluster_dims__(GDN_WCL, 1, 1) __launch_bounds__(256, 3) k_gdn_
     const float4 cv0 = *reinterpret_cast<const float4*>(a.conv_w + (size_t)(v_col + lane) * 4), cv1 = *reinterpret_cast<const float4*>(a.conv_w + (size_t)(v_col + 32 + lane) * 4);
     const float nw0 = bf2f(a.norm_w[64 * rank + lane]), nw1 = bf2f(a.norm_w[64 * rank + 32 + lane]);
     pdl_wait();
-    const int r0 = a.seq[blockIdx.y * 4 + 0], T = min(a.seq[blockIdx.y * 4 + 1], 8), slot = a.seq[blockIdx.y * 4 + 2];
+    const int4 sq = reinterpret_cast<const int4*>(a.seq)[blockIdx.y];   // one read: three 32-bit ones cost 2 % (other registers)
+    const int r0 = sq.x, T = min(sq.y, 8), slot = sq.z;
     const int nrep = min(a.replay_n ? a.replay_n[slot] : 0, 8), nrows = nrep + T;
     float* sav = a.saved + (size_t)slot * a.saved_stride + (size_t)h * 8 * 388;   // [8][q 128 | k 128 | v 128 | beta | alpha | pad]
     float* cst = a.conv_state + (size_t)slot * a.conv_stride + (size_t)h * 3 * 384;   // [3 taps][q 128 | k 128 | v 128]; private per v-head
@@ -691,7 +693,10 @@ int gdn_forward(const GdnParams& p, int nseq, cudaStream_t s) {
     a.state = p.state; a.conv_state = p.conv_state; a.state_stride = p.state_stride; a.conv_stride = p.conv_stride;
     a.seq = p.seq; a.replay_n = p.replay_n; a.imm_T = p.imm_T; a.imm_replay = p.imm_replay; a.out = p.out; a.oq = (int8_t*)p.xq.q; a.osc = (float*)p.xq.sc;
     a.snap = p.snap; a.snap_row_stride = p.snap_row_stride; a.eps = p.eps; a.sigmoid_gate = p.sigmoid_gate; a.late = p.late;
-    if (nseq >= 3) return launch_gdn_wide(a, p.n_v, nseq, s);
+    if (nseq >= 3) {
+        HP_REQUIRE(((uintptr_t)p.seq & 15) == 0, "gdn_forward: misaligned descriptors");
+        return launch_gdn_wide(a, p.n_v, nseq, s);
+    }
     HP_CUDA(launch_pdl<128>(k_gdn, dim3(p.n_v * GDN_CL, nseq), dim3(256), 0, s, a));
     HP_CUDA(cudaGetLastError()); return HP_OK;
 }

@@ -90,7 +90,7 @@ def test_gdn_pass_over_several_sequences_needs_descriptors_and_takes_no_snapshot
     from test_gdn_gpu import _Gdn
     f = getattr(hb.lib(), "_ZN2hp11gdn_forwardERKNS_9GdnParamsEiP11CUstream_st")
     for nseq in (2, 3, 8):
-        for fields in (dict(seq=4096, snap=4096), dict(seq=None, snap=None, imm_T=1)):
+        for fields in (dict(seq=4096, snap=4096), dict(seq=None, snap=None, imm_T=1)) + ((dict(seq=4100, snap=None),) if nseq > 2 else ()):   # three and more: read as 16-byte groups
             p = _Gdn(n_qk=1, n_v=2, **fields)
             assert f(ctypes.byref(p), nseq, ctypes.c_void_p(0)) == 1 and b"descriptors" in hb.lib().hp_last_error()
 
