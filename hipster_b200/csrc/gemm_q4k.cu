@@ -8,8 +8,9 @@
 //
 // What bounds it: the fp32 update, two conversions and three packed fp32 instructions per two outputs and sub-block. From
 // registers alone a 16x8x32 tile of it takes 15.3 clocks of an SM sub-partition; the int8 mma.sync of the GEMV takes 8.0 and
-// does not overlap with it (23.9 together). In place this kernel takes 36 to 47 clocks per tile at 512 rows (34816 x 5120: 690
-// us) and 56 at 32 (67 us), the GEMV 52 at 32 rows (62 us): the rest is TMEM and shared-memory loads, addresses and waits.
+// does not overlap with it (23.9 together). In place, at 1965 MHz, this kernel takes 36 clocks per tile at 512 rows of 34816 x 5120 (687
+// us; 40 to 49 for the other projections) and 57 at 32 (68 us), the GEMV 54 at 32 rows (65 us): the rest is TMEM and shared-memory
+// loads, addresses and waits.
 // Hence:
 //   * one CTA per SM, M = 128 weight rows (8 tiles of 16), N = 32..128 pass rows, one tcgen05.mma (K = 32) per sub-block,
 //     never accumulating: TMEM only hands the int32 dots over to the update, in slots of 2 or 4 sub-blocks;

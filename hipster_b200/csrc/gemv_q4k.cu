@@ -453,7 +453,7 @@ int gemv_q4k_q8_parts(const void* W, const XQ8F& x, float* yparts, int N, int K,
     // all column tiles in one launch: their activations staged in shared memory beside the rings when they fit, read
     // from L2 inside the loop otherwise (small matrices with a long K: one launch instead of one per tile of 8 columns;
     // same per-column arithmetic either way)
-    // (three tiles of 20 blocks beside one-block stages: 34816 x 5120 at 24 rows 44.5 us, from L2 50.8)
+    // (three tiles of 20 blocks beside one-block stages: 34816 x 5120 at 24 rows 43.6 us, from L2 49.8)
     auto fits = [&](int nt) { return tiled ? (nbp % 2 || nt == 3 ? sk_fits<1, true>(nt, nbp) : sk_fits<2, true>(nt, nbp)) : (nbp % 2 ? sk_fits<1, false>(nt, nbp) : sk_fits<2, false>(nt, nbp)); };
     const bool staged = ntile == 1 || fits(ntile);
     // ... unless there are four tiles and the matrix is large: two launches of two tiles each stream it twice in less time than one waits

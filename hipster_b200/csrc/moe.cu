@@ -413,8 +413,8 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 1) k_moe_gemv_grouped(MoeGArgs
 // ---- the same GEMVs with the work cut by quads of warps ------------------------------------------------------------
 // A CTA is four quads of four warps. A quad owns a contiguous range of work units (segment, 4 tiles), i.e. mostly one
 // or two segments: it gathers the segment's <= 8 activation columns ONCE into shared memory in the layout of the dense
-// kernel (so a lane fetches its int8 fragment and its columns' scales with three 128-bit shared loads per 64 weights
-// instead of nine global loads), and its warps take one tile of every unit each (warp w: tile w), streamed through a
+// kernel (so a lane fetches its int8 fragment and its columns' scales with one 128-bit and four 64-bit shared loads per 64
+// weights instead of nine global loads), and its warps take one tile of every unit each (warp w: tile w), streamed through a
 // private ring. A warp's pipeline thus runs over ~7 tiles per launch instead of ~1.75 four-tile units, which removes
 // the quantisation of the launch time to whole units. MODE 0: the 32-feature quantisation group spans the quad's four
 // tiles: amax (a maximum) and the integer sum of the quantised values go through shared memory between two quad
