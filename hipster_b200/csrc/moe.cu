@@ -419,9 +419,9 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 1) k_moe_gemv_grouped(MoeGArgs
 // the quantisation of the launch time to whole units. MODE 0: the 32-feature quantisation group spans the quad's four
 // tiles: amax (a maximum) and the integer sum of the quantised values go through shared memory between two quad
 // barriers. Per output element the arithmetic is unchanged: one warp, blocks in order along K, no split.
-// Bound by the latency of a warp's serial chain (24 rows: DRAM 45 %, issue 38 %, no pipe above 33 % of its peak with three quads and rings
-// of 3 stages): four quads with rings of 2 hold fewer bytes per warp and as many per SM, and one layer of 24 rows takes 116 us instead
-// of 125.
+// Bound by the latency of a warp's serial chain (24 rows, three quads with rings of 3 stages: DRAM 45 and 41 %, issue 54 and 49 %): four quads
+// with rings of 2 hold fewer bytes per warp and as many per SM, and segments of up to 4 columns take fewer instructions: DRAM 48 and 42 %,
+// issue 42 and 34 %, one layer of 24 rows 114 us instead of 125.
 constexpr int MQ_WARPS = 16, MQ_QUADS = 4, MQ_AUX = 2048;   // bytes after the rings: barriers + the quads' exchange words
 __device__ __forceinline__ void quad_barrier(int quad) { asm volatile("bar.sync %0, 128;" ::"r"(quad + 1) : "memory"); }
 template <int MODE, int SB, int DEPTH>
