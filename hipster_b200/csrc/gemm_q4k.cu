@@ -31,22 +31,23 @@
 // Every wait is bounded and reports through the device status word.
 #include "hp_common.cuh"
 #include "kernels.h"
+#include <cuda_fp8.h>
 
 namespace hp {
 namespace {
 
-constexpr int TC_EPI = 8, TC_CNV = 4, TC_THREADS = (TC_EPI + TC_CNV + 4) * 32, TC_RAWS = 4, TC_CNVS = 3;
+constexpr int TC_EPI = 8, TC_CNV = 4, TC_THREADS = (TC_EPI + TC_CNV + 4) * 32, TC_RAWS = 3, TC_CNVS = 3;
 constexpr int TC_W_CNV = TC_EPI, TC_W_LD = TC_W_CNV + TC_CNV, TC_W_TMA = TC_W_LD + 1, TC_W_MMA = TC_W_TMA + 1;   // first warp of each role
 constexpr int TC_RAW_BYTES = 8 * 2304, TC_A_BYTES = 2 * 128 * 64;   // weights of one block; converted weights of half a block
 template <int NTC> struct TcGeom {
     static constexpr int N = NTC * 8, GS = NTC <= 8 ? 4 : 2, SLOT = GS * N <= 128 ? 128 : 256, SLOTS = 512 / SLOT;   // GS sub-blocks per TMEM slot
-    static constexpr int BST = NTC <= 8 ? 6 : 3, SCS = NTC <= 8 ? 4 : 3, B_BYTES = 2 * N * 64;   // rings: half-blocks of activations, blocks of scales
+    static constexpr int BST = NTC <= 8 ? 4 : NTC <= 12 ? 3 : 2, SCS = NTC <= 8 ? 4 : 3, B_BYTES = 4 * N * 64;   // rings: half-blocks of activations (two planes), blocks of scales
     static constexpr int PACK = 2 * B_BYTES + NTC * 512;                                         // packed activations of a block: two half-blocks, scales
     static constexpr int SC_BYTES = 8 * 128 * 8 + NTC * 512;
     static constexpr int OFF_A = TC_RAWS * TC_RAW_BYTES, OFF_B = OFF_A + TC_CNVS * TC_A_BYTES, OFF_SC = OFF_B + BST * B_BYTES, OFF_BAR = OFF_SC + SCS * SC_BYTES;
     static constexpr int SMEM = OFF_BAR + 512 + 1024;   // + slack to align the ring to 1024 bytes
 };
-static_assert(TcGeom<16>::SMEM <= GEMV_SMEM_LIMIT && TcGeom<8>::SMEM <= GEMV_SMEM_LIMIT, "shared memory of the widest tiles");
+static_assert(TcGeom<16>::SMEM <= GEMV_SMEM_LIMIT && TcGeom<12>::SMEM <= GEMV_SMEM_LIMIT && TcGeom<8>::SMEM <= GEMV_SMEM_LIMIT, "shared memory of the widest tiles");
 
 // Bounded wait that lets the hardware park the warp: up to 2^20 attempts of up to a microsecond
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, int* err) {
@@ -67,8 +68,8 @@ __device__ __forceinline__ bool tc_elect() {
 __device__ __forceinline__ uint64_t tc_desc(uint32_t addr) {   // K-major operand, 64-byte swizzle: 8-row groups 512 bytes apart
     return (uint64_t)((addr >> 4) & 0x3FFF) | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61);
 }
-__device__ __forceinline__ void tc_mma_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc) {   // D = A * B (no accumulation)
-    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, 0, 0;\ntcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}" ::"r"(d), "l"(a), "l"(b), "r"(idesc) : "memory");
+__device__ __forceinline__ void tc_mma_f8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, int add) {   // D = A * B (+ D)
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(add) : "memory");
 }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -146,7 +147,7 @@ __device__ __forceinline__ void tc_update(float2 (&acc)[4][W], uint32_t ta, uint
 #pragma unroll
         for (int i = 0; i < W * 4; ++i) { tc_after_wait(v0[b][i]); if constexpr (H1) tc_after_wait(v1[b][i]); }
     auto upd = [&](float2& a, float2 sc, float4 xv, uint32_t i0, uint32_t i1) {
-        fma2(a, mul2(make_float2(sc.x, sc.x), make_float2(xv.x, xv.y)), make_float2(__int2float_rn((int)i0), __int2float_rn((int)i1)));
+        fma2(a, mul2(make_float2(sc.x, sc.x), make_float2(xv.x, xv.y)), make_float2(__uint_as_float(i0), __uint_as_float(i1)));
         fma2(a, make_float2(sc.y, sc.y), make_float2(xv.z, xv.w));
     };
 #pragma unroll
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
             }
             for (int i = k > TC_RAWS ? k - TC_RAWS : 0; i < k; ++i) tc_wait(raw_full + 8 * (i % TC_RAWS), (i / TC_RAWS) & 1, a.err);   // no copy outlives the CTA
         } else if (warp == TC_W_MMA) {   // ---- MMA issue
-            const uint32_t idesc = (2u << 4) | (1u << 10) | ((uint32_t)(Geo::N / 8) << 17) | (8u << 24);   // s32 = u8 x s8, M = 128
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(Geo::N / 8) << 17) | (8u << 24);   // f32 = e4m3 x e4m3, M = 128
             int hb = 0, gr = 0; bool ok = true;
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x)
                 for (int h = 0; h < 2 * nbp && ok; ++h, ++hb) {
@@ -237,8 +238,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
                         if (tc_elect()) {
 #pragma unroll
                             for (int v = q; v < q + GS; ++v)
-                                tc_mma_i8(tmem + slot * Geo::SLOT + (v - q) * Geo::N, tc_desc(abase + (v >> 1) * 8192 + (v & 1) * 32),
-                                          tc_desc(bbase + (v >> 1) * (Geo::N * 64) + (v & 1) * 32), idesc);
+#pragma unroll
+                                for (int pl = 0; pl < 2; ++pl)
+                                    tc_mma_f8(tmem + slot * Geo::SLOT + (v - q) * Geo::N, tc_desc(abase + (v >> 1) * 8192 + (v & 1) * 32),
+                                              tc_desc(bbase + ((v >> 1) * 2 + pl) * (Geo::N * 64) + (v & 1) * 32), idesc, pl);
                             tc_commit(tm_full + 8 * slot);
                             if (q + GS == 4) { tc_commit(a_empty + 8 * as); tc_commit(b_empty + 8 * bs); }
                         }
@@ -282,7 +285,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
     } else if (warp >= TC_W_CNV) {   // ---- weights: row scales, nibbles -> u8
         tc_reg_dec<72>();
         const int cw = warp - TC_W_CNV, ct = cw * 32 + lane;
-        const uint32_t m_a = sel ? 0xF0F0F0F0u : 0x0F0F0F0Fu;   // nibbles of the first store; the second takes the others
+        const int sh_a = sel ? 4 : 0, sh_b = 4 - sh_a;   // nibbles of the first store; the second takes the others
+        auto nib = [](uint32_t v, int sh) { return (v >> sh) & 0x0F0F0F0Fu; };
         int k = 0, hb = 0; bool ok = true;
         for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
             const int grp = it / a.ncg % a.ngrp, nt = min(G, tiles - grp * G);
@@ -305,10 +309,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
                         const int u = cw + 4 * i;
                         if ((u >> 1) < nt) {
                             uint8_t* d = A + (u & 1) * 8192 + (G == 8 ? (u >> 1) : (u & ~1)) * 1024;
-                            *reinterpret_cast<uint2*>(d + sw) = make_uint2(w[i].x & m_a, w[i].y & m_a);
-                            *reinterpret_cast<uint2*>(d + (sw ^ 32)) = make_uint2(w[i].x & ~m_a, w[i].y & ~m_a);
-                            *reinterpret_cast<uint2*>(d + 512 + sw) = make_uint2(w[i].z & m_a, w[i].w & m_a);
-                            *reinterpret_cast<uint2*>(d + 512 + (sw ^ 32)) = make_uint2(w[i].z & ~m_a, w[i].w & ~m_a);
+                            *reinterpret_cast<uint2*>(d + sw) = make_uint2(nib(w[i].x, sh_a), nib(w[i].y, sh_a));
+                            *reinterpret_cast<uint2*>(d + (sw ^ 32)) = make_uint2(nib(w[i].x, sh_b), nib(w[i].y, sh_b));
+                            *reinterpret_cast<uint2*>(d + 512 + sw) = make_uint2(nib(w[i].z, sh_a), nib(w[i].w, sh_a));
+                            *reinterpret_cast<uint2*>(d + 512 + (sw ^ 32)) = make_uint2(nib(w[i].z, sh_b), nib(w[i].w, sh_b));
                         }
                     }
                     fence_proxy_async();
@@ -319,7 +323,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
                         if (!ok) break;
                         const int pos = ct >> 4, ti = G == 8 ? pos : pos >> 1;
                         if (ti < nt && (G == 8 || !(pos & 1))) {
-                            const RowScales rs = decode_scales(*reinterpret_cast<const uint4*>(raw + ti * 2304 + (ct & 15) * 16));
+                            RowScales rs = decode_scales(*reinterpret_cast<const uint4*>(raw + ti * 2304 + (ct & 15) * 16));
+                            rs.dq = rs.d = rs.d * 512.f; rs.cdq = rs.cd = -(rs.d * 8388608.f);   // the accumulators hold idot / 512
                             float2* sp = reinterpret_cast<float2*>(smem + Geo::OFF_SC + ss * Geo::SC_BYTES) + ct;
 #pragma unroll
                             for (int q = 0; q < 8; ++q) { const float4 v = rs.get(q); sp[q * 128] = make_float2(v.x, v.z); }
@@ -428,6 +433,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
+// four int8 as e4m3: x = 16 a + b with |a|, |b| <= 8; hi = 16 a, lo = b, both exact
+__device__ __forceinline__ void tc_split(uint32_t x, uint32_t& hi, uint32_t& lo) {
+    hi = lo = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+        const int v0 = (int)(int8_t)(x >> (8 * i)), v1 = (int)(int8_t)(x >> (8 * i + 8)), a0 = (v0 + 8) & ~15, a1 = (v1 + 8) & ~15;
+        hi |= (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2((float)a0, (float)a1), __NV_SATFINITE, __NV_E4M3) << (8 * i);
+        lo |= (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2((float)(v0 - a0), (float)(v1 - a1)), __NV_SATFINITE, __NV_E4M3) << (8 * i);
+    }
+}
 // Activations in the order the GEMM copies them: per column range of NTC tiles and block two half-blocks (per 64-element
 // group the swizzled K-major tile of all columns), then the scales. Tiles beyond the rows are zero.
 template <int NTC>
@@ -441,9 +456,12 @@ __global__ void __launch_bounds__(256) k_tc_pack(const uint4* __restrict__ xq, c
     for (int u = warp; u < NTC * 4; u += 8) {
         const int n = u >> 2, jj = u & 3, nt = cg * NTC + n;
         const uint4 v = nt < tiles8 ? xq[((size_t)nt * nb * 4 + (size_t)blk * 4 + jj) * 32 + lane] : make_uint4(0, 0, 0, 0);
-        uint8_t* p = d + (jj >> 1) * TcGeom<NTC>::B_BYTES + (jj & 1) * (NTC * 512) + n * 512;
-        *reinterpret_cast<uint2*>(p + lo) = make_uint2(v.x, v.y);
-        *reinterpret_cast<uint2*>(p + (lo ^ 32)) = make_uint2(v.z, v.w);
+        uint8_t* p = d + (jj >> 1) * TcGeom<NTC>::B_BYTES + (jj & 1) * (2 * NTC * 512) + n * 512;
+        uint2 h, l;
+        tc_split(v.x, h.x, l.x); tc_split(v.y, h.y, l.y);
+        *reinterpret_cast<uint2*>(p + lo) = h; *reinterpret_cast<uint2*>(p + NTC * 512 + lo) = l;
+        tc_split(v.z, h.x, l.x); tc_split(v.w, h.y, l.y);
+        *reinterpret_cast<uint2*>(p + (lo ^ 32)) = h; *reinterpret_cast<uint2*>(p + NTC * 512 + (lo ^ 32)) = l;
     }
     for (int n = warp; n < NTC; n += 8) {
         const int nt = cg * NTC + n;
@@ -469,7 +487,7 @@ int launch_tc(const TcArgs& a, const XQ8F& x, int grid, cudaStream_t s, bool pdl
 
 }  // namespace
 
-size_t gemm_pack_bytes(int R, int K) { return (size_t)((R + 7) / 8 + 15) * (size_t)(K / 256) * 2560; }
+size_t gemm_pack_bytes(int R, int K) { return (size_t)((R + 7) / 8 + 15) * (size_t)(K / 256) * 4608; }
 // The cut of the rows into column ranges of ntc tiles of 8, and of the weight tiles into items of G = 8 or 4 (the latter leaves
 // every second tile position empty). An item of 20 blocks takes 36, 56, 72 and 90 us at ntc = 4, 8, 12 and 16: 4.5 us
 // for each of ntc + 4; the cut with the least time over the rounds of the SMs is taken.
