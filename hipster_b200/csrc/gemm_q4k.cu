@@ -393,34 +393,53 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
                         const bool last = b + 1 == nbp;
                         int ldy = a.ldy;
                         asm volatile("" : "+r"(ldy));   // keeps the addresses of this rare path out of the registers of the loop
-                        float* yt = y + (size_t)((cg * NTC + n0) * 8 + 2 * t) * ldy + tl[h] * 16 + g;
-                        auto live = [&](int i, int w, int e) { return tl[h] * 16 + g + 8 * i < a.N && (cg * NTC + n0 + w) * 8 + 2 * t + e < a.R; };
+                        if constexpr (VREG) {
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            float2 v[W];
-#pragma unroll
-                            for (int w = 0; w < W; ++w) { v[w] = acc[2 * h + i][w]; acc[2 * h + i][w] = make_float2(0.f, 0.f); }
-                            if (!first[h]) {
-                                float2 p[W];   // all loads in flight at once
+                            for (int i = 0; i < 2; ++i)
 #pragma unroll
                                 for (int w = 0; w < W; ++w) {
-                                    if constexpr (VREG) p[w] = sum[2 * h + i][w];
-                                    else p[w] = make_float2(live(i, w, 0) ? yt[(size_t)(8 * w) * ldy + 8 * i] : 0.f, live(i, w, 1) ? yt[(size_t)(8 * w + 1) * ldy + 8 * i] : 0.f);
+                                    float2 v = acc[2 * h + i][w]; acc[2 * h + i][w] = make_float2(0.f, 0.f);
+                                    if (!first[h]) v = make_float2(sum[2 * h + i][w].x + v.x, sum[2 * h + i][w].y + v.y);
+                                    sum[2 * h + i][w] = v;
                                 }
-#pragma unroll
-                                for (int w = 0; w < W; ++w) { v[w].x = p[w].x + v[w].x; v[w].y = p[w].y + v[w].y; }
-                            }
-                            if constexpr (VREG) {
-#pragma unroll
-                                for (int w = 0; w < W; ++w) sum[2 * h + i][w] = v[w];
-                            }
-                            if (!VREG || last)
-#pragma unroll
-                                for (int w = 0; w < W; ++w) {
-                                    if (live(i, w, 0)) yt[(size_t)(8 * w) * ldy + 8 * i] = v[w].x;
-                                    if (live(i, w, 1)) yt[(size_t)(8 * w + 1) * ldy + 8 * i] = v[w].y;
-                                }
+                            if (!last) { first[h] = false; continue; }
                         }
+                        // element {i, w, e}: row + 8 i, column 2 t + 8 w + e. Other warps wait at the next slot for the one that closes a
+                        // tile: whole tiles and ranges without predicates, one pointer per column pair, all loads in front
+                        const int row = tl[h] * 16 + g, col = (cg * NTC + n0) * 8 + 2 * t;
+                        float* yt = y + (size_t)col * ldy + row;
+                        const size_t step = (size_t)8 * ldy;
+                        auto close = [&](auto live) {
+                            if constexpr (!VREG) {
+                                if (!first[h]) {
+                                    float p[W][4];
+                                    const float* yp = yt;
+#pragma unroll
+                                    for (int w = 0; w < W; ++w, yp += step) {
+                                        const float* yq = yp + ldy;
+                                        p[w][0] = live(0, w, 0) ? yp[0] : 0.f; p[w][1] = live(0, w, 1) ? yq[0] : 0.f; p[w][2] = live(1, w, 0) ? yp[8] : 0.f; p[w][3] = live(1, w, 1) ? yq[8] : 0.f;
+                                    }
+#pragma unroll
+                                    for (int w = 0; w < W; ++w)
+#pragma unroll
+                                        for (int i = 0; i < 2; ++i) { float2& v = acc[2 * h + i][w]; v.x = p[w][2 * i] + v.x; v.y = p[w][2 * i + 1] + v.y; }
+                                }
+                            }
+                            float* yp = yt;
+#pragma unroll
+                            for (int w = 0; w < W; ++w, yp += step) {
+                                float* yq = yp + ldy;
+#pragma unroll
+                                for (int i = 0; i < 2; ++i) {
+                                    const float2 v = VREG ? sum[VREG ? 2 * h + i : 0][VREG ? w : 0] : acc[2 * h + i][w];
+                                    if (live(i, w, 0)) yp[8 * i] = v.x;
+                                    if (live(i, w, 1)) yq[8 * i] = v.y;
+                                    if constexpr (!VREG) acc[2 * h + i][w] = make_float2(0.f, 0.f);
+                                }
+                            }
+                        };
+                        if (tl[h] * 16 + 16 <= a.N && (cg * NTC + n0 + W) * 8 <= a.R) close([](int, int, int) { return true; });
+                        else close([&](int i, int w, int e) { return row + 8 * i < a.N && col + 8 * w + e < a.R; });
                         first[h] = false;
                     }
                 }
