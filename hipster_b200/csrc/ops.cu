@@ -275,7 +275,8 @@ __device__ __forceinline__ float2 gdn_fma2(float2 a, float2 b, float2 c) {   // 
 // Passes over one or two sequences: one wave of a latency-bound kernel. One sequence of 6 rows, 4 replayed: 12.7 us in a captured graph,
 // of 1 row, 1 replayed 7.8, two sequences of 6 rows 16.9 (q and k of the recurrence by 64-bit reads, see lds_f2; by 128-bit ones 12.8, 7.9
 // and 17.0).
-__global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, 3) k_gdn(GdnArgs a) {
+template <int OCC>
+__global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, OCC) k_gdn(GdnArgs a) {
     constexpr int D = 128, NLD = 8, NCV = 6;   // items per thread: (16 + 3) * 96 <= 8 * 256 raw values, 16 * 96 = 6 * 256 conv outputs
     // conv'ed, then normalised q | k of every row (filled by all four CTAs); 16-float chunks padded to 20 so that the
     // eight chunk owners of a state row read 64 bits each from distinct banks
@@ -363,7 +364,7 @@ __global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, 3) k_gdn(G
 #pragma unroll
     for (int k = 0; k < NCV; ++k) {
         const int it = e_rr[k], c = e_c[k];
-        if (it < nrows) {   // warp-uniform: a warp covers one group of one row
+        if (it < nrows && (it >= nrep || c >= 32)) {   // warp-uniform: a warp covers one group of one row. A replayed row needs no q
             const float4 w = cw[k];
             float t = w.x * raw[it][c]; t = fmaf(w.y, raw[it + 1][c], t); t = fmaf(w.z, raw[it + 2][c], t); t = fmaf(w.w, raw[it + 3][c], t);
             const float v = silu_det(t);
@@ -391,46 +392,64 @@ __global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, 3) k_gdn(G
     {   // normalise q | k of every row in place: thread tid owns channel tid (q for tid < 128, k otherwise)
         const int off = (tid >> 7) * 160 + ((tid & 127) >> 4) * 20 + (tid & 15);
 #pragma unroll 4
-        for (int it = 0; it < nrows; ++it) sqk[it][off] = sqk[it][off] / snrm[it][tid >> 7];
+        for (int it = tid < 128 ? nrep : 0; it < nrows; ++it) sqk[it][off] = sqk[it][off] / snrm[it][tid >> 7];
     }
     __syncthreads();
 
-    // ---- phase 2: the recurrence, row after row, state in registers; no block-wide synchronisation inside
-    for (int it = 0; it < nrows; ++it) {
-        if (it == nrep && nrep > 0) commit_state();
-        const float beta = sbeta[it], decay = sdecay[it];
-        const float* kk = &sqk[it][160 + 20 * ck]; const float* qq = &sqk[it][20 * ck];
-        float2 kr[8], qr[8];
+    // ---- phase 2: the recurrence, row after row, state in registers; no block-wide synchronisation inside. The chain from row to row is
+    // decay, first product (16 dependent fmaf and three shuffles), update: the second product of a row runs beside the decay and the
+    // first product of the next one, its reduction beside that one's, and the reads of the next row's k are in flight under both.
+    float2 kr[8], kn[8];
+    float dot = 0.f, o = 0.f;
+    auto ld8 = [&](float2 (&r)[8], const float* p) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) kr[i] = lds_f2(kk + 2 * i);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) qr[i] = lds_f2(qq + 2 * i);
-        const float2 dc2 = make_float2(decay, decay);
-        float dot = 0.f;
+        for (int i = 0; i < 8; ++i) r[i] = lds_f2(p + 2 * i);
+    };
+    if (nrows > 0) {
+        ld8(kr, &sqk[0][160 + 20 * ck]);
+        const float2 dc2 = make_float2(sdecay[0], sdecay[0]);
 #pragma unroll
         for (int i = 0; i < 8; ++i) { m[i] = gdn_mul2(m[i], dc2); dot = fmaf(m[i].x, kr[i].x, dot); dot = fmaf(m[i].y, kr[i].y, dot); }
+    }
+    auto row_step = [&](int it, auto fresh_) {   // fresh: a new row, with output; otherwise a replayed one
+        constexpr bool fresh = decltype(fresh_)::value;
+        const bool more = it + 1 < nrows;
+        const float beta = sbeta[it], vj = sv[it][jl], decay = sdecay[more ? it + 1 : it];
+        float2 qr[8];
+        if constexpr (fresh) ld8(qr, &sqk[it][20 * ck]);
+        ld8(kn, &sqk[more ? it + 1 : it][160 + 20 * ck]);
 #pragma unroll
-        for (int off = 1; off < 8; off <<= 1) dot = dot + __shfl_xor_sync(0xffffffffu, dot, off);
-        const float delta = (sv[it][jl] - dot) * beta;
-        const float2 dl2 = make_float2(delta, delta);
-        float o = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; i += 2) {
-            m[i] = gdn_fma2(dl2, kr[i], m[i]); o = fmaf(m[i].x, qr[i].x, o); o = fmaf(m[i].y, qr[i].y, o);
-            m[i + 1] = gdn_fma2(dl2, kr[i + 1], m[i + 1]); o = fmaf(m[i + 1].x, qr[i + 1].x, o); o = fmaf(m[i + 1].y, qr[i + 1].y, o);
+        for (int off = 1; off < 8; off <<= 1) {
+            dot = dot + __shfl_xor_sync(0xffffffffu, dot, off);
+            if constexpr (fresh) o = o + __shfl_xor_sync(0xffffffffu, o, off);   // of the row in front
         }
+        const float delta = (vj - dot) * beta;
+        if constexpr (fresh) { if (it > nrep && ck == 0) sout[it - 1 - nrep][jl] = o * 0.08838834764831845f; }
+        const float2 dl2 = make_float2(delta, delta), dc2 = make_float2(decay, decay);
 #pragma unroll
-        for (int off = 1; off < 8; off <<= 1) o = o + __shfl_xor_sync(0xffffffffu, o, off);
-        if (it >= nrep) {
-            if (ck == 0) sout[it - nrep][jl] = o * 0.08838834764831845f;
+        for (int i = 0; i < 8; ++i) m[i] = gdn_fma2(dl2, kr[i], m[i]);
+        if constexpr (fresh) {
             if (a.snap) {
                 float* sp = a.snap + (size_t)(it - nrep) * a.snap_row_stride + ((size_t)h * D + j) * D + 16 * ck;
 #pragma unroll
                 for (int i = 0; i < 8; i += 2) *reinterpret_cast<float4*>(sp + 2 * i) = make_float4(m[i].x, m[i].y, m[i + 1].x, m[i + 1].y);
             }
+        } else { if (it + 1 == nrep) commit_state(); }
+        o = 0.f; dot = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if constexpr (fresh) { o = fmaf(m[i].x, qr[i].x, o); o = fmaf(m[i].y, qr[i].y, o); }
+            m[i] = gdn_mul2(m[i], dc2); dot = fmaf(m[i].x, kn[i].x, dot); dot = fmaf(m[i].y, kn[i].y, dot);
+            kr[i] = kn[i];
         }
+    };
+    for (int it = 0; it < nrep; ++it) row_step(it, std::false_type());
+    for (int it = nrep; it < nrows; ++it) row_step(it, std::true_type());
+    if (T > 0) {
+#pragma unroll
+        for (int off = 1; off < 8; off <<= 1) o = o + __shfl_xor_sync(0xffffffffu, o, off);
+        if (ck == 0) sout[T - 1][jl] = o * 0.08838834764831845f;
     }
-    if (T == 0 && nrep > 0) commit_state();
     __syncthreads();
 
     // ---- phase 3: per-head RMSNorm * w * gate(z) + quantisation of the new rows; warp t takes row t, lane = channel.
@@ -697,7 +716,7 @@ int gdn_forward(const GdnParams& p, int nseq, cudaStream_t s) {
         HP_REQUIRE(((uintptr_t)p.seq & 15) == 0, "gdn_forward: misaligned descriptors");
         return launch_gdn_wide(a, p.n_v, nseq, s);
     }
-    HP_CUDA(launch_pdl<128>(k_gdn, dim3(p.n_v * GDN_CL, nseq), dim3(256), 0, s, a));
+    HP_CUDA(nseq == 1 ? launch_pdl<128>(k_gdn<2>, dim3(p.n_v * GDN_CL, nseq), dim3(256), 0, s, a) : launch_pdl<128>(k_gdn<3>, dim3(p.n_v * GDN_CL, nseq), dim3(256), 0, s, a));
     HP_CUDA(cudaGetLastError()); return HP_OK;
 }
 
