@@ -557,9 +557,10 @@ __global__ void __cluster_dims__(GDN_WCL, 1, 1) __launch_bounds__(256, 3) k_gdn_
     auto conv = [](const float4& w, float x0, float x1, float x2, float x3) { float t = w.x * x0; t = fmaf(w.y, x1, t); t = fmaf(w.z, x2, t); t = fmaf(w.w, x3, t); return silu_det(t); };
     {
         const int g2 = tid >> 7, ch = tid & 127, off = g2 * 160 + (ch >> 4) * 20 + (ch & 15);
-        float x0 = sm.raw[0][tid], x1 = sm.raw[1][tid], x2 = sm.raw[2][tid];
+        const int it0 = g2 ? 0 : nrep;   // a replayed row needs no q
+        float x0 = raw_row(it0)[tid], x1 = raw_row(it0 + 1)[tid], x2 = raw_row(it0 + 2)[tid];
 #pragma unroll 2
-        for (int it = 0; it < nrows; ++it) {
+        for (int it = it0; it < nrows; ++it) {
             const float x3 = raw_row(it + 3)[tid];
             const float v = conv(cw, x0, x1, x2, x3);
             x0 = x1; x1 = x2; x2 = x3;
@@ -582,7 +583,7 @@ __global__ void __cluster_dims__(GDN_WCL, 1, 1) __launch_bounds__(256, 3) k_gdn_
         }
         __syncthreads();
 #pragma unroll 4
-        for (int it = 0; it < nrows; ++it) sm.sqk[it][off] = sm.sqk[it][off] / sm.snrm[it][g2];   // q | k normalised in place
+        for (int it = it0; it < nrows; ++it) sm.sqk[it][off] = sm.sqk[it][off] / sm.snrm[it][g2];   // q | k normalised in place
     }
     __syncthreads();
 
@@ -607,15 +608,16 @@ __global__ void __cluster_dims__(GDN_WCL, 1, 1) __launch_bounds__(256, 3) k_gdn_
         for (int off = 1; off < 8; off <<= 1) { d0 = d0 + __shfl_xor_sync(0xffffffffu, d0, off); d1 = d1 + __shfl_xor_sync(0xffffffffu, d1, off); }
         const float e0 = (v0 - d0) * beta, e1 = (v1 - d1) * beta;
         const float2 dl0 = make_float2(e0, e0), dl1 = make_float2(e1, e1);
-        float o0 = 0.f, o1 = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float2 qv = lds_f2(qq + 2 * i);
-            fma2(m[0][i], dl0, kr[i]); fma2(m[1][i], dl1, kr[i]);
-            o0 = fmaf(m[0][i].x, qv.x, o0); o1 = fmaf(m[1][i].x, qv.x, o1);
-            o0 = fmaf(m[0][i].y, qv.y, o0); o1 = fmaf(m[1][i].y, qv.y, o1);
-        }
+        for (int i = 0; i < 8; ++i) { fma2(m[0][i], dl0, kr[i]); fma2(m[1][i], dl1, kr[i]); }
         if (it >= nrep) {
+            float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float2 qv = lds_f2(qq + 2 * i);
+                o0 = fmaf(m[0][i].x, qv.x, o0); o1 = fmaf(m[1][i].x, qv.x, o1);
+                o0 = fmaf(m[0][i].y, qv.y, o0); o1 = fmaf(m[1][i].y, qv.y, o1);
+            }
 #pragma unroll
             for (int off = 1; off < 8; off <<= 1) { o0 = o0 + __shfl_xor_sync(0xffffffffu, o0, off); o1 = o1 + __shfl_xor_sync(0xffffffffu, o1, off); }
             if (ck == 0) { sm.sout[it - nrep][jl] = o0 * 0.08838834764831845f; sm.sout[it - nrep][jl + 32] = o1 * 0.08838834764831845f; }
