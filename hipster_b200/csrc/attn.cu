@@ -111,7 +111,9 @@ template <int PPT, int NT> struct AttnGeom {
 // 2 x 36 x 128 x 256 fmaf = 9.6 us at 128 a clock); every score and every output element is one fmaf chain (over d, over
 // the keys), two chains per packed instruction. Hence tiles that fit the pairs (12 per 128 threads: idle pairs cost as much as live ones),
 // 6 pairs x 2 keys per thread in the score phase (16 f16 -> f32 conversions and 8 broadcasts, which share the pipe and the issue slots
-// with the math, per 96 fmaf; 3 pairs x 4 keys needed 16 per 48), and the V tile in flight under the scores.
+// with the math, per 96 fmaf; 3 pairs x 4 keys needed 16 per 48), and the V tile in flight under the scores. 36 pairs, thousand clocks
+// of a CTA: staging 4.5 (6.0 with the scalar stores of q), scores 16.4, softmax 3.5 (4.3 a pair at a time), P.V 14.9 (16.7 with four dims x
+// half the pairs per thread: more duplicated operands).
 template <int PPT, int NT>
 __global__ void __launch_bounds__(NT, 1) k_attn_split(AttnArgs a) {
     using Geo = AttnGeom<PPT, NT>;
@@ -138,11 +140,13 @@ __global__ void __launch_bounds__(NT, 1) k_attn_split(AttnArgs a) {
     for (int i = tid; i < nkeys * (HD / 8); i += NT) cp_async16(sV + i * 8, Vg + (size_t)i * 8);
     asm volatile("cp.async.commit_group;" ::: "memory");
     // pair = t*G + hh -> row r0+t, head kh*G + hh
-    for (int i = tid; i < npairs * (HD / 4); i += NT) {
-        const int p = i / (HD / 4), d4 = i % (HD / 4), tr = p / G, hh = p % G;
-        const float4 q = reinterpret_cast<const float4*>(a.qkv + (size_t)(r0 + tr) * a.ld + (kh * G + hh) * 512)[d4];
-        float* dst = sQ + (size_t)(p >> 1) * 2 * HD + 8 * d4 + (p & 1);
-        dst[0] = q.x; dst[2] = q.y; dst[4] = q.z; dst[6] = q.w;
+    // two neighbouring pairs at once: 128-bit stores of interleaved dims (scalar ones of a single pair hit every bank eight times)
+#pragma unroll 3
+    for (int i = tid; i < (npairs + 1) / 2 * (HD / 4); i += NT) {
+        const int p = i / (HD / 4) * 2, d4 = i % (HD / 4), t0 = p / G, p1 = min(p + 1, npairs - 1), t1 = p1 / G;
+        const float4 q0 = reinterpret_cast<const float4*>(a.qkv + (size_t)(r0 + t0) * a.ld + (kh * G + p - t0 * G) * 512)[d4], q1 = reinterpret_cast<const float4*>(a.qkv + (size_t)(r0 + t1) * a.ld + (kh * G + p1 - t1 * G) * 512)[d4];
+        float4* dst = reinterpret_cast<float4*>(sQ + (size_t)p * HD + 8 * d4);
+        dst[0] = make_float4(q0.x, q1.x, q0.y, q1.y); dst[1] = make_float4(q0.z, q1.z, q0.w, q1.w);
     }
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
@@ -183,27 +187,52 @@ __global__ void __launch_bounds__(NT, 1) k_attn_split(AttnArgs a) {
         }
     }
     __syncthreads();
-    // softmax pieces per pair: warp w takes pairs w, w + NW, ...; lane l takes keys l, l+32, l+64, l+96. Row t of the group
-    // sees keys <= pos0 + t. Maximum: exact in any order. Sum: the lane's keys in ascending order, then the xor tree (16..1).
-    for (int p = warp; p < npairs; p += NW) {
-        const int tr = p / G;
-        const int nk = min(nkeys, pos0 + tr + 1 - k_lo);
-        float sc[4]; float mx = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { const int k = lane + 32 * i; sc[i] = k < nk ? sE[k * ESTR + p] : -INFINITY; mx = fmaxf(mx, sc[i]); }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        float l = 0.f;
+    // softmax pieces: a warp takes QP neighbouring pairs, lane l keys l, l+32, l+64, l+96. Row t of the group sees keys <= pos0 + t.
+    // Maximum: exact in any order. Sum: the lane's keys in ascending order, then the xor tree (16..1). Four pairs at once (one where there
+    // are as many warps as pairs): a 128-bit access per key, and their chains of reductions run side by side.
+    constexpr int QP = PPT == 2 ? 1 : 4;
+    static_assert(Geo::NP / QP <= NW, "one group of pairs per warp");
+    if (warp * QP < npairs) {
+        const int pq = warp * QP;
+        float sc[QP][4], mx[QP], l[QP]; int nk[QP];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int k = lane + 32 * i;
-            const float e = k < nk ? expf_det(sc[i] - mx) : 0.f;
-            if (k < nkeys) sE[k * ESTR + p] = e;
-            l = i == 0 ? e : l + e;
+            if constexpr (QP == 4) { const float4 v = *reinterpret_cast<const float4*>(sE + k * ESTR + pq); sc[0][i] = v.x; sc[1][i] = v.y; sc[2][i] = v.z; sc[3][i] = v.w; }
+            else sc[0][i] = sE[k * ESTR + pq];
         }
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) l = l + __shfl_xor_sync(0xffffffffu, l, off);
-        if (lane == 0) { a.pm[pbase + p] = mx; a.pl[pbase + p] = l; }   // nk <= 0: mx = -inf, l = 0 (the merge skips it)
+        for (int c = 0; c < QP; ++c) {
+            nk[c] = min(nkeys, pos0 + (pq + c) / G + 1 - k_lo); mx[c] = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { if (lane + 32 * i >= nk[c]) sc[c][i] = -INFINITY; mx[c] = fmaxf(mx[c], sc[c][i]); }
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+            for (int c = 0; c < QP; ++c) mx[c] = fmaxf(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], off));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k = lane + 32 * i;
+#pragma unroll
+            for (int c = 0; c < QP; ++c) {
+                const float e = k < nk[c] ? expf_det(sc[c][i] - mx[c]) : 0.f;
+                sc[c][i] = e;
+                l[c] = i == 0 ? e : l[c] + e;
+            }
+            if (k < nkeys) {
+                if constexpr (QP == 4) *reinterpret_cast<float4*>(sE + k * ESTR + pq) = make_float4(sc[0][i], sc[1][i], sc[2][i], sc[3][i]);
+                else sE[k * ESTR + pq] = sc[0][i];
+            }
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+            for (int c = 0; c < QP; ++c) l[c] = l[c] + __shfl_xor_sync(0xffffffffu, l[c], off);
+        if (lane == 0) {   // nk <= 0: mx = -inf, l = 0 (the merge skips it)
+#pragma unroll
+            for (int c = 0; c < QP; ++c) if (pq + c < npairs) { a.pm[pbase + pq + c] = mx[c]; a.pl[pbase + pq + c] = l[c]; }
+        }
     }
     cp_async_wait_all();
     __syncthreads();
@@ -240,7 +269,7 @@ __global__ void __launch_bounds__(NT, 1) k_attn_split(AttnArgs a) {
 }
 
 // merge the splits of one (row, q-head) in split order, gate, write f32 + q8. grid rows * n_head, 256 threads. Bound by latency: the
-// maxima, weights and sums of up to 256 splits are fetched by as many threads at once, the partial outputs 8 splits at a time.
+// maxima, weights and sums of up to 256 splits are fetched by as many threads at once, 16 partial outputs are in flight, the first under the weights.
 __global__ void __launch_bounds__(256) k_attn_merge(const float* __restrict__ qkv, int ld, int n_head, int n_kv, const int* __restrict__ groups, const int* __restrict__ row_group,
                                                      int imm_pos0, int imm_rows, int imm_gr, const float* __restrict__ pO, const float* __restrict__ pm, const float* __restrict__ pl, int nsplit_max,
                                                      float* __restrict__ out, int8_t* __restrict__ oq, float* __restrict__ osc) {
@@ -259,20 +288,26 @@ __global__ void __launch_bounds__(256) k_attn_merge(const float* __restrict__ qk
     for (int s = d + 256; s < nsplit; s += 256) mx = fmaxf(mx, pm[pb + (size_t)s * MAXP]);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    float o = 0.f, l = 0.f;
+    constexpr int PF = 16;   // partial outputs in flight; the first ones under the weights
+    float pv[PF];
+#pragma unroll
+    for (int i = 0; i < PF; ++i) pv[i] = i < nsplit ? po[(size_t)i * MAXP * HD] : 0.f;
     if (lane == 0) smx[d >> 5] = mx;
     __syncthreads();
 #pragma unroll
     for (int w = 0; w < 8; ++w) mx = fmaxf(mx, smx[w]);
-    float o = 0.f, l = 0.f;
     for (int s0 = 0; s0 < nsplit; s0 += 256) {
         const int n = min(256, nsplit - s0);
         if (s0) { __syncthreads(); if (d < n) m0 = pm[pb + (size_t)(s0 + d) * MAXP]; }
         if (d < n) { sw[d] = expf_det(m0 - mx); sl[d] = pl[pb + (size_t)(s0 + d) * MAXP]; }
         __syncthreads();
-#pragma unroll 8
-        for (int s = 0; s < n; ++s) {
-            o = fmaf(sw[s], po[(size_t)(s0 + s) * MAXP * HD], o);
-            l = fmaf(sw[s], sl[s], l);
+        for (int s = 0; s < n; s += PF) {
+#pragma unroll
+            for (int i = 0; i < PF; ++i) {
+                if (s + i < n) { o = fmaf(sw[s + i], pv[i], o); l = fmaf(sw[s + i], sl[s + i], l); }
+                pv[i] = s0 + s + PF + i < nsplit ? po[(size_t)(s0 + s + PF + i) * MAXP * HD] : 0.f;
+            }
         }
     }
     const float v = (o / l) * sigmoid_det(gate);
