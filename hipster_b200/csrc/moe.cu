@@ -288,10 +288,10 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 1) k_moe_gemv_grouped(MoeGArgs
     uint8_t* ring = smem + warp * MOE_DEPTH * STAGE;
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + MOE_WARPS * MOE_DEPTH * STAGE);
     const uint32_t bar0 = smem_u32(&bars[warp * MOE_DEPTH]);
-    pdl_launch_dependents();
     if (lane == 0) { for (int s = 0; s < MOE_DEPTH; ++s) mbar_init(bar0 + 8 * s, 1); fence_barrier_init(); }
     __syncwarp();
     pdl_wait();
+    pdl_launch_dependents();   // behind the wait: see k_moe_gemv_quad
     const int spt = a.nb / SB;                                 // stages per tile
     const int ups = a.tiles / MOE_UNIT_TILES, total = a.ctl[0] * ups, spu = MOE_UNIT_TILES * spt;   // units per segment, units, stages per unit
     auto grab = [&]() { int u = 0; if (lane == 0) u = atomicAdd(a.ctl + a.ticket, 1); return __shfl_sync(0xffffffffu, u, 0); };
@@ -437,15 +437,14 @@ __global__ void __launch_bounds__(MQ_WARPS * 32, 1) k_moe_gemv_quad(MoeGArgs a) 
     uint4* xq_s = reinterpret_cast<uint4*>(xbuf);
     float* xsc_s = reinterpret_cast<float*>(xbuf + (size_t)a.nb * 2048);
     const uint32_t bar0 = smem_u32(&bars[warp * DEPTH]);
-    pdl_launch_dependents();
     if (lane == 0) { for (int s = 0; s < DEPTH; ++s) mbar_init(bar0 + 8 * s, 1); fence_barrier_init(); }
     __syncwarp();
-    pdl_wait();
+    // gate|up lets the down projection start once the grouping in front of both is complete: its CTAs read the segments and prime their
+    // rings on the SMs that have finished gate|up, in front of their own wait (for the quantised activations).
+    if (MODE == 0) pdl_wait();
+    pdl_launch_dependents();
     const int spt = a.nb / SB, ups = a.tiles / MOE_UNIT_TILES;   // stages per tile, units per segment
-    // expert parallelism: number of the exchange this launch feeds, and the half of the peers' buffers it goes to
-    unsigned ep_e = 0u; size_t ep_off = 0;
-    if constexpr (MODE == 1) { if (a.ep_world > 1) { ep_e = __ldcg(a.ep_ctl[a.ep_rank] + 8) + 1u; ep_off = (size_t)(ep_e & 1u) * a.ep_half; } }
-    const int total = a.ctl[0] * ups, nquads = (int)gridDim.x * MQ_QUADS, gq = (int)blockIdx.x * MQ_QUADS + quad;
+    const int total = __ldcg(a.ctl) * ups, nquads = (int)gridDim.x * MQ_QUADS, gq = (int)blockIdx.x * MQ_QUADS + quad;
     const int u_lo = (int)((long long)gq * total / nquads), u_hi = (int)((long long)(gq + 1) * total / nquads);
     const size_t tile_bytes = (size_t)a.nb * 2304;
     auto seg_weights = [&](int seg) -> const uint8_t* {
@@ -477,28 +476,39 @@ __global__ void __launch_bounds__(MQ_WARPS * 32, 1) k_moe_gemv_quad(MoeGArgs a) 
     int c0 = -1, c1 = -1;   // pair indices of this lane's columns 2t, 2t + 1 (few: fc.col, fc.col + 1)
     const uint4* xq4 = reinterpret_cast<const uint4*>(a.xq);
     const int nsb = a.xK >> 5, nk64 = a.xK >> 6;
+    // this thread's columns of a segment, all read at once (entries beyond ncols hold anything): of its gather items and of its outputs
+    const int gg = (qtid & 31) >> 2, tt = qtid & 3, sw = qtid & 15, gs = (sw >> 2) * 2 + (sw & 1);
+    int ncols = 0, col_g = 0, col_s = 0, col_f = 0, col_f1 = 0, col_t = 0, col_t1 = 0;
+    auto read_seg = [&](int seg) {
+        const MoeSeg* sg = a.segs + seg;
+        ncols = __ldcg(&sg->ncols); col_g = __ldcg(&sg->cols[gg]); col_s = __ldcg(&sg->cols[gs]);
+        col_f = __ldcg(&sg->cols[fc.col]); col_f1 = __ldcg(&sg->cols[fc.col + 1]); col_t = __ldcg(&sg->cols[2 * t]); col_t1 = __ldcg(&sg->cols[2 * t + 1]);
+    };
+    if (u_lo < u_hi) read_seg(cseg);
+    if (MODE == 1) pdl_wait();
+    // expert parallelism: number of the exchange this launch feeds, and the half of the peers' buffers it goes to
+    unsigned ep_e = 0u; size_t ep_off = 0;
+    if constexpr (MODE == 1) { if (a.ep_world > 1) { ep_e = __ldcg(a.ep_ctl[a.ep_rank] + 8) + 1u; ep_off = (size_t)(ep_e & 1u) * a.ep_half; } }
     for (int cu = u_lo; cu < u_hi; ++cu) {
         if (cseg != staged) {
             // gather the segment's columns: fragment (k block of 64, column gg, quarter tt) and scales (sub-block, column)
+            if (staged >= 0) read_seg(cseg);
             quad_barrier(quad);   // everybody has finished with the previous segment's activations
-            const MoeSeg* sg = a.segs + cseg;
-            const int ncols = __ldcg(&sg->ncols);
             {   // a thread's column and quarter are the same for all its items (the items are 128 apart): the column's row
                 // is looked up once, and the item loads are independent of each other (one L2 round trip, not one per item)
-                const int gg = (qtid & 31) >> 2, tt = qtid & 3;
-                const int r = gg < ncols ? __ldcg(&sg->cols[gg]) / a.xdiv : -1;
+                const int r = gg < ncols ? col_g / a.xdiv : -1;
                 const uint4* src = r >= 0 ? xq4 + (size_t)(r >> 3) * nk64 * 32 + (r & 7) * 4 + tt : nullptr;
 #pragma unroll 8
                 for (int kb = qtid >> 5; kb < nk64; kb += 4) xq_s[kb * 32 + (qtid & 31)] = src ? __ldcg(src + (size_t)kb * 32) : make_uint4(0u, 0u, 0u, 0u);
-                const int w = qtid & 15, gs = (w >> 2) * 2 + (w & 1), is_s = (w >> 1) & 1;
-                const int rs = gs < ncols ? __ldcg(&sg->cols[gs]) / a.xdiv : -1;
+                const int w = sw, is_s = (w >> 1) & 1;
+                const int rs = gs < ncols ? col_s / a.xdiv : -1;
                 const float* ssrc = rs >= 0 ? a.xsc + (size_t)(rs >> 3) * nsb * 16 + ((rs & 7) >> 1) * 4 + (rs & 1) + 2 * is_s : nullptr;
 #pragma unroll 8
                 for (int sb = qtid >> 4; sb < nsb; sb += 8) xsc_s[sb * 16 + w] = ssrc ? __ldcg(ssrc + (size_t)sb * 16) : 0.f;
             }
             few = ncols <= 4;
             const int ca = few ? fc.col : 2 * t;
-            c0 = ca < ncols ? __ldcg(&sg->cols[ca]) : -1; c1 = ca + 1 < ncols ? __ldcg(&sg->cols[ca + 1]) : -1;
+            c0 = ca < ncols ? (few ? col_f : col_t) : -1; c1 = ca + 1 < ncols ? (few ? col_f1 : col_t1) : -1;
             staged = cseg;
             quad_barrier(quad);
         }
