@@ -41,8 +41,8 @@ __global__ void __launch_bounds__(256) k_qk_norm_rope_kv(float* __restrict__ qkv
                                                           int ld, int n_head, int n_kv, const uint16_t* __restrict__ qw, const uint16_t* __restrict__ kw,
                                                           const float2* __restrict__ rope, int n_rot, const int* __restrict__ row_pos, const int* __restrict__ row_slot, int imm_pos0,
                                                           uint16_t* __restrict__ kc, uint16_t* __restrict__ vc, size_t kv_stride, int max_ctx, float eps) {
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();   // behind the wait: all that was enqueued in front of this kernel is complete when k_attn_split starts
     __shared__ float sh[8]; __shared__ float buf[HD];
     const int t = threadIdx.x, hb = blockIdx.x % (n_head + n_kv), r = blockIdx.x / (n_head + n_kv);
     const int pos = row_pos ? row_pos[r] : imm_pos0 + r, slot = row_slot ? row_slot[r] : 0;
@@ -91,7 +91,7 @@ struct AttnArgs {
     const float* qkv; int ld, n_head, n_kv;
     const uint16_t* kc; const uint16_t* vc; size_t kv_stride; int max_ctx;
     const int* groups;        // device: per group {r0, T, slot, pos0}; nullptr: rows 0 .. imm_rows - 1 of slot 0 at imm_pos0 .., imm_gr rows per group
-    int imm_pos0, imm_rows, imm_gr;
+    int imm_pos0, imm_rows, imm_gr, rows;   // rows: of the launch
     float* pO; float* pm; float* pl; int nsplit_max;   // partials [group][kv head][split][MAXP] (x 256 for pO)
 };
 __device__ __forceinline__ int4 attn_group(const int* groups, int gi, int pos0, int rows, int gr) {   // {r0, T, slot, pos0}
@@ -118,8 +118,6 @@ template <int PPT, int NT>
 __global__ void __launch_bounds__(NT, 1) k_attn_split(AttnArgs a) {
     using Geo = AttnGeom<PPT, NT>;
     constexpr int NW = Geo::NW, KPL = Geo::KPL, KG = Geo::KG, PP = Geo::PP, ESTR = Geo::ESTR;
-    pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ __align__(16) uint8_t sm_raw[];
     float* sQ = reinterpret_cast<float*>(sm_raw);                                   // [NP / 2][256][2]: two pairs side by side
     float* sE = sQ + Geo::NP * HD;                                                  // [SPL][ESTR] scores, then weights
@@ -132,12 +130,20 @@ __global__ void __launch_bounds__(NT, 1) k_attn_split(AttnArgs a) {
     const int k_lo = split * SPL;
     const int nkeys = min(SPL, pos0 + T - k_lo);          // keys of this split visible to the last row of the group
     if (nkeys <= 0 || T <= 0) return;
+    // Keys in front of every row of this launch were written by earlier passes: they are fetched in front of the dependency wait, under the
+    // kernel that writes the new ones (it releases this one once its own predecessors are complete).
+    const int nold = max(0, min(nkeys, pos0 - a.rows - k_lo));
     const size_t pbase = (((size_t)gi * a.n_kv + kh) * a.nsplit_max + split) * MAXP;
     const uint16_t* Kg = a.kc + (size_t)slot * a.kv_stride + ((size_t)kh * a.max_ctx + k_lo) * HD;
     const uint16_t* Vg = a.vc + (size_t)slot * a.kv_stride + ((size_t)kh * a.max_ctx + k_lo) * HD;
-    for (int i = tid; i < nkeys * (HD / 8); i += NT) { const int k = i / (HD / 8), c = i % (HD / 8); cp_async16(sK + k * KSTR + c * 8, Kg + (size_t)k * HD + c * 8); }
+    auto fetch_k = [&](int k0, int k1) { for (int i = k0 * (HD / 8) + tid; i < k1 * (HD / 8); i += NT) { const int k = i / (HD / 8), c = i % (HD / 8); cp_async16(sK + k * KSTR + c * 8, Kg + (size_t)k * HD + c * 8); } };
+    auto fetch_v = [&](int k0, int k1) { for (int i = k0 * (HD / 8) + tid; i < k1 * (HD / 8); i += NT) cp_async16(sV + i * 8, Vg + (size_t)i * 8); };
+    fetch_k(0, nold); fetch_v(0, nold);
+    pdl_wait();
+    pdl_launch_dependents();   // behind the wait, for the splits of a further launch over the same rows (see nold)
+    fetch_k(nold, nkeys);
     asm volatile("cp.async.commit_group;" ::: "memory");
-    for (int i = tid; i < nkeys * (HD / 8); i += NT) cp_async16(sV + i * 8, Vg + (size_t)i * 8);
+    fetch_v(nold, nkeys);
     asm volatile("cp.async.commit_group;" ::: "memory");
     // pair = t*G + hh -> row r0+t, head kh*G + hh
     // two neighbouring pairs at once: 128-bit stores of interleaved dims (scalar ones of a single pair hit every bank eight times)
@@ -339,7 +345,7 @@ int attn_rope_kv(const AttnParams& p, int rows, cudaStream_t s) {
 int attn_decode(const AttnParams& p, int rows, int ngroups, cudaStream_t s) {
     HP_REQUIRE(rows >= 1 && ngroups >= 1 && p.n_head % p.n_kv == 0 && (p.n_head / p.n_kv) <= MAXP, "attn_decode: at most %d (row, head) pairs per kv head and group", MAXP);
     AttnArgs a; a.qkv = p.qkv; a.ld = p.ld; a.n_head = p.n_head; a.n_kv = p.n_kv; a.kc = (const uint16_t*)p.kc; a.vc = (const uint16_t*)p.vc;
-    a.kv_stride = p.kv_stride; a.max_ctx = p.max_ctx; a.groups = p.groups; a.imm_pos0 = p.imm_pos0; a.imm_rows = rows; a.imm_gr = p.imm_gr; a.pO = p.pO; a.pm = p.pm; a.pl = p.pl; a.nsplit_max = p.nsplit_max;
+    a.kv_stride = p.kv_stride; a.max_ctx = p.max_ctx; a.groups = p.groups; a.imm_pos0 = p.imm_pos0; a.imm_rows = a.rows = rows; a.imm_gr = p.imm_gr; a.pO = p.pO; a.pm = p.pm; a.pl = p.pl; a.nsplit_max = p.nsplit_max;
     // group sizes live on the device; group_rows bounds them. Up to 8 pairs (the rows of a draft or decode step) take 2 pairs per thread
     const int pairs = (p.group_rows > 0 && p.group_rows < rows ? p.group_rows : rows) * (p.n_head / p.n_kv);
     const dim3 grid(p.nsplit_max, p.n_kv, ngroups);
