@@ -8,10 +8,8 @@ LIB_PATH = os.environ.get("HIPSTER_B200_LIB") or os.path.join(HERE, "libhipster_
 HEADER = os.path.join(HERE, "..", "include", "hipster_b200.h")
 
 _lib = _hot = None
-# argument types of the calls whose latency counts (p pointer, i int, f float): integers then pass without a wrapper object. They are
-# declared on function objects of this package's own (hot()): those of lib() take whatever ctypes objects a caller passes.
-_TYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "f": ctypes.c_float}
-_HOT = {"hp_quantize_x_q8": "piiippp", "hp_gemv_q4k_q8": "ppppiiiip", "hp_argmax": "piiipppp", "hp_accept_greedy": "ppipp", "hp_attn_decode": "piiiiiipppppipppfpp"}
+# the calls whose latency counts go through csrc/pycalls.c, bound to the library that is loaded here
+_HOT = ("hp_quantize_x_q8", "hp_gemv_q4k_q8", "hp_argmax", "hp_accept_greedy", "hp_attn_decode")
 
 
 class HipsterError(RuntimeError):
@@ -30,7 +28,7 @@ def declared_symbols():
 
 
 def lib():
-    global _lib, _hot
+    global _lib
     if _lib is None:
         if not os.path.exists(LIB_PATH):
             raise HipsterError(-1, f"{LIB_PATH} is missing: build it with `python -m hipster_b200.build` (needs nvcc); no fallback path exists")
@@ -38,16 +36,21 @@ def lib():
         _lib.hp_last_error.restype = ctypes.c_char_p
         for name in ("hp_xq8_q_bytes", "hp_xq8_sc_bytes", "hp_argmax_scratch_bytes", "hp_attn_workspace_bytes"):
             getattr(_lib, name).restype = ctypes.c_size_t
-        _hot = ctypes.CDLL(LIB_PATH)
-        for name, types in _HOT.items():
-            getattr(_hot, name).argtypes = [_TYPES[t] for t in types]
     return _lib
 
 
 def hot():
-    """The library with declared argument types on the calls of _HOT."""
+    """The calls of _HOT with integers (None: absent) for every argument, without ctypes in between."""
+    global _hot
     if _hot is None:
-        lib()
+        L = lib()
+        try:
+            from . import _calls
+        except ImportError as e:
+            raise HipsterError(-1, f"{os.path.join(HERE, '_calls')} is missing: build it with `python -m hipster_b200.build` ({e})") from e
+        for name in _HOT:
+            _calls.bind(name, ctypes.cast(getattr(L, name), ctypes.c_void_p).value)
+        _hot = _calls
     return _hot
 
 

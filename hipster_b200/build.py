@@ -7,6 +7,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -61,8 +62,24 @@ def build(verbose=False, force=False):
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    build_calls(force)
     build_driver(force)
     return LIB
+
+
+CALLS_SRC = os.path.join(CSRC, "pycalls.c")
+CALLS = os.path.join(HERE, "_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def build_calls(force=False):
+    """The CPython entry points of the short calls: no torch, no CUDA, not linked with the library."""
+    if force or _stale(CALLS, [CALLS_SRC]):
+        cmd = [shutil.which("gcc") or "gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], CALLS_SRC, "-o", CALLS]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError("building the CPython entry points failed")
+    return CALLS
 
 
 DRIVER_SRC = os.path.join(HERE, "driver", "spec_driver.cpp")

@@ -1,14 +1,15 @@
 """Kernel-level host API: the Python mirror of the reference's free kernel launchers
 (engine/kernels/gemv.h, ops.h). Arguments are torch CUDA tensors; every call goes through the C ABI."""
 import ctypes
+import functools
 
 import torch
 
 from ._lib import lib, hot, check, ptr
 
 # The calls below are a few microseconds of device work, so what they spend in Python counts: the handle of the current stream
-# comes without a Stream object around it, and the short calls pass pointers as integers to declared argument types (_lib.hot; to a
-# function without declared types an integer would pass as 32 bits, hence the wrapper of _stream).
+# comes without a Stream object around it, the short calls go through native entry points that take addresses as integers (_lib.hot; to
+# a ctypes function an integer would pass as 32 bits, hence the wrapper of _stream), and sizes that depend on shapes alone are computed once.
 try:
     _raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
 except AttributeError:   # torch without CUDA: the package still imports, and a call raises torch's own error
@@ -19,13 +20,27 @@ def _stream():
     return ctypes.c_void_p(_raw_stream(_device()))
 
 
+@functools.lru_cache(maxsize=256)
+def _xq8_bytes(R, K):
+    return lib().hp_xq8_q_bytes(R, K), lib().hp_xq8_sc_bytes(R, K)
+
+
+@functools.lru_cache(maxsize=256)
+def _argmax_scratch_bytes(R, n):
+    return lib().hp_argmax_scratch_bytes(R, n)
+
+
+@functools.lru_cache(maxsize=256)
+def _attn_workspace_bytes(R, n_head, n_kv, max_ctx):
+    return lib().hp_attn_workspace_bytes(R, n_head, n_kv, max_ctx)
+
+
 class XQ8:
     """Quantised activations (reference: struct XQ8, engine/kernels/gemv.h:8) in the library's private layout."""
 
     def __init__(self, R, K, device="cuda"):
-        L = lib()
         self.R, self.K = R, K
-        nq, ns = L.hp_xq8_q_bytes(R, K), L.hp_xq8_sc_bytes(R, K)   # nq is a multiple of 512: the scales stay aligned
+        nq, ns = _xq8_bytes(R, K)   # nq is a multiple of 512: the scales stay aligned
         self.q, self.sc = torch.zeros(nq + ns, dtype=torch.uint8, device=device).split((nq, ns))
 
     def unpack(self):
@@ -39,10 +54,11 @@ class XQ8:
 
 def quantize_x_q8(x, xq=None):
     """x f32 [R][K] -> XQ8 (reference quantize_x_q8, gemv.h:9)."""
-    assert x.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1
+    stride = x.stride()
+    assert x.dtype == torch.float32 and len(stride) == 2 and stride[1] == 1
     R, K = x.shape
     xq = xq or XQ8(R, K, x.device)
-    check(hot().hp_quantize_x_q8(x.data_ptr(), x.stride(0), R, K, xq.q.data_ptr(), xq.sc.data_ptr(), _raw_stream(_device())))
+    check(hot().hp_quantize_x_q8(x.data_ptr(), stride[0], R, K, xq.q.data_ptr(), xq.sc.data_ptr(), _raw_stream(_device())))
     return xq
 
 
@@ -73,7 +89,7 @@ def argmax(logits, n=None):
     """Row-wise argmax (max value, lowest index) -> (ids int32 [R], vals f32 [R]) (reference argmax_topk k=1, ops.h:118)."""
     R, ld = logits.shape[0], logits.stride(0)
     n = n or logits.shape[1]
-    dev, nb = logits.device, lib().hp_argmax_scratch_bytes(R, n)
+    dev, nb = logits.device, _argmax_scratch_bytes(R, n)
     ids = torch.empty(R, dtype=torch.int32, device=dev)
     vals = torch.empty(R, dtype=torch.float32, device=dev)
     scratch = torch.empty(nb, dtype=torch.uint8, device=dev) if nb else None
@@ -107,9 +123,8 @@ def attn_decode(qkv, pos0, n_head, n_kv, n_rot, q_norm, k_norm, rope, kc, vc, ma
     """GQA decode attention of one sequence: qkv f32 [R][ld] (normalised / rotated in place), rows at positions pos0 + r;
     q_norm / k_norm bf16 [256] (int16 tensors), rope f32 [max_ctx][n_rot/2][2], kc / vc f16 [n_kv][max_ctx][256] (updated).
     -> (out f32 [R][n_head*256], XQ8 of it or None). Reference: qk_norm_rope_kv + attn_decode_mq (ops.h:71-72,96)."""
-    L = lib()
     R, ld = qkv.shape[0], qkv.stride(0)
-    ws = torch.empty(L.hp_attn_workspace_bytes(R, n_head, n_kv, max_ctx), dtype=torch.uint8, device=qkv.device)
+    ws = torch.empty(_attn_workspace_bytes(R, n_head, n_kv, int(max_ctx)), dtype=torch.uint8, device=qkv.device)
     out = torch.empty((R, n_head * 256), dtype=torch.float32, device=qkv.device)
     xq = XQ8(R, n_head * 256, qkv.device) if want_q8 else None
     check(hot().hp_attn_decode(qkv.data_ptr(), ld, R, int(pos0), n_head, n_kv, n_rot, None if q_norm is None else q_norm.data_ptr(),
