@@ -35,6 +35,9 @@ struct RouteArgs {
     int e_lo, e_hi, own_shared; MoeSeg* segs; int* ctl; unsigned long long* touched;   // grouping (segs == nullptr: skipped)
     int stage_w, stage_x; int* err;                               // router rows / pass rows staged in shared memory; status word for the bounded waits
 };
+// orders this thread's accesses, and those that a block barrier put in front of them, against another CTA's behind a counter (all that a
+// ticket needs; __threadfence by every thread is sequentially consistent and takes longer)
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 constexpr int RG_THREADS = 512;
 constexpr int RG_ROUTE_SMEM = 8 * 1024 * 4;   // routing scratch: the probabilities of 8 rows x up to 1024 experts
 __global__ void __launch_bounds__(RG_THREADS) k_route_group(RouteArgs a) {
@@ -114,12 +117,10 @@ __global__ void __launch_bounds__(RG_THREADS) k_route_group(RouteArgs a) {
     // the groups are routed on different SMs at the same time: warps 2 r and 2 r + 1 route row 8 by + r. This code runs once per
     // launch on an SM that has not executed it before, so it is written for a small instruction footprint (rolled loops
     // over values kept in shared memory): unrolled over 32 register values it was bound by instruction fetch.
-    __threadfence();
     __syncthreads();
-    if (tid == 0) s_last = atomicAdd(a.ticket + blockIdx.y, 1) == (int)gridDim.x - 1;
+    if (tid == 0) { fence_gpu(); s_last = atomicAdd(a.ticket + blockIdx.y, 1) == (int)gridDim.x - 1; fence_gpu(); }
     __syncthreads();
     if (!s_last) return;
-    __threadfence();
     const int ns = a.k + 1;
     if (t < a.T) {
         const float* lg = a.y + (size_t)t * a.N;
@@ -198,14 +199,14 @@ __global__ void __launch_bounds__(RG_THREADS) k_route_group(RouteArgs a) {
     }
     if (tid == 0) a.ticket[blockIdx.y] = 0;   // ready for the next launch
     if (!a.segs) return;
-    // ---- grouping, by the CTA that routes last (second-level ticket): bucket b = expert e_lo + b (b < nown), then the
-    // shared expert; segments in bucket order, the pairs of a bucket in increasing pair index
-    __threadfence();
+    // ---- grouping, by the CTA that routes last (second-level ticket where there are several groups: 1.4 us): bucket b = expert e_lo + b
+    // (b < nown), then the shared expert; segments in bucket order, the pairs of a bucket in increasing pair index
     __syncthreads();
-    if (tid == 0) s_last = atomicAdd(a.ticket + 4, 1) == (int)gridDim.y - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
+    if (gridDim.y > 1) {
+        if (tid == 0) { fence_gpu(); s_last = atomicAdd(a.ticket + 4, 1) == (int)gridDim.y - 1; fence_gpu(); }
+        __syncthreads();
+        if (!s_last) return;
+    }
     const int nown = a.e_hi - a.e_lo, nb = nown + (a.own_shared ? 1 : 0), np = a.T * ns;
     // scnt[b] = bit mask of the rows that picked bucket b (a row picks an expert at most once, T <= 32): a pair's place in
     // its bucket is the number of lower rows in the mask
