@@ -25,7 +25,6 @@ namespace {
 // position, expert) instead of the GEMV's (benchmark input control: with random-init weights every row's hidden state is
 // nearly the same vector, so a linear router would send all rows to the same experts); the shared expert's gate keeps its logit.
 struct MoeSeg { int expert, ncols, cols[8]; int pad[6]; };   // 64 bytes; cols = pair indices t * nslot + e
-__device__ __forceinline__ void better(float& bv, int& bi, float v, int i) { if (v > bv || (v == bv && i < bi)) { bv = v; bi = i; } }
 __device__ __forceinline__ void row_barrier(int row) { asm volatile("bar.sync %0, 64;" ::"r"(row + 1) : "memory"); }   // the two warps of a row
 struct RouteArgs {
     const float* W; const float* x; float* y; int N, K, T;       // router [N = E + 1][K], rows x [T][K], logits y [T][N]
@@ -38,13 +37,13 @@ struct RouteArgs {
 // orders this thread's accesses, and those that a block barrier put in front of them, against another CTA's behind a counter (all that a
 // ticket needs; __threadfence by every thread is sequentially consistent and takes longer)
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-constexpr int RG_THREADS = 512;
+constexpr int RG_THREADS = 512, RG_CAND = 64;   // threads; candidates that are ranked at once
 constexpr int RG_ROUTE_SMEM = 8 * 1024 * 4;   // routing scratch: the probabilities of 8 rows x up to 1024 experts
 __global__ void __launch_bounds__(RG_THREADS) k_route_group(RouteArgs a) {
     pdl_launch_dependents();
     __shared__ int scnt[1026]; __shared__ int soff[1026]; __shared__ int swt[RG_THREADS / 32]; __shared__ int s_last;
     __shared__ __align__(8) unsigned long long wbar, xbar;
-    __shared__ float s_max[8][2], s_gsum[8][32], s_sel[8][16]; __shared__ uint32_t s_ck[8][32]; __shared__ int s_ci[8][32];
+    __shared__ float s_max[8][2], s_gsum[8][32], s_sel[8][16]; __shared__ uint32_t s_ck[8][RG_CAND], s_lane[RG_THREADS / 32][32], s_thr[8][2]; __shared__ int s_ci[8][RG_CAND], s_ncand[8];
     // dynamic shared memory: the CTA's 16 router rows [16][K] f32 (a.stage_w), then its 8 pass rows [8][K] f32 (a.stage_x);
     // the routing phase reuses the front of it
     extern __shared__ __align__(128) uint8_t rg_smem[];
@@ -154,42 +153,53 @@ __global__ void __launch_bounds__(RG_THREADS) k_route_group(RouteArgs a) {
         row_barrier(row);
         float sum = s_gsum[row][0];
         for (int q = 1; q < nq; ++q) sum = sum + s_gsum[row][q];
-        // Selection keys: a probability is a non-negative float, so its bit pattern orders like an unsigned integer;
-        // key = bits + 1, 0 = no entry (padding, or already taken). The warp's own k best by (key desc, index asc): one
-        // integer max and one integer min across the warp per winner; every global winner is among the 2 k candidates.
-        uint32_t lk = 0u; int li = 0x7fffffff;
+        // Selection keys: a probability is a non-negative float, so its bit pattern orders like an unsigned integer; key = bits + 1, 0 = no
+        // entry. At least k entries of a warp are no smaller than the k-th largest of its 32 lane maxima, so the row's k best are among
+        // the entries that reach the larger of its two warps' bounds: some 20 candidates of 512, each ranked by counting those in front of
+        // it (key desc, index asc). More than RG_CAND of them (many equal probabilities): k rounds of arg-max over the row.
+        uint32_t lk = 0u;
 #pragma unroll 4
         for (int q = qa; q < qb; ++q) {
             const int i = 32 * q + lane;
             const uint32_t key = i < a.E ? __float_as_uint(sv[i] / sum) + 1u : 0u;
-            sk[i] = key;
-            if (key > lk) { lk = key; li = i; }
+            sk[i] = key; lk = max(lk, key);
         }
-        uint32_t myk = 0u; int myi = 0x7fffffff;
-        for (int r = 0; r < a.k; ++r) {
-            const uint32_t m = __reduce_max_sync(0xffffffffu, lk);
-            const int wi = (int)__reduce_min_sync(0xffffffffu, lk == m ? (uint32_t)li : 0x7fffffffu);
-            if (lane == r) { myk = m; myi = wi; }
-            if (m != 0u && (wi & 31) == lane) {   // the owner retires the entry and looks for its next best
-                sk[wi] = 0u; lk = 0u; li = 0x7fffffff;
+        s_lane[warp][lane] = lk;
+        __syncwarp();
+        int above = 0;
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j) above += s_lane[warp][j] > lk ? 1 : 0;
+        const uint32_t bound = __reduce_min_sync(0xffffffffu, above < a.k ? lk : 0xffffffffu);
+        if (lane == 0) { s_thr[row][sub] = bound; if (sub == 0) s_ncand[row] = 0; }
+        row_barrier(row);
+        const uint32_t thr = max(1u, max(s_thr[row][0], s_thr[row][1]));
 #pragma unroll 4
-                for (int q = qa; q < qb; ++q) { const uint32_t key = sk[32 * q + lane]; if (key > lk) { lk = key; li = 32 * q + lane; } }
-            }
+        for (int q = qa; q < qb; ++q) {
+            const int i = 32 * q + lane;
+            const uint32_t key = sk[i];
+            if (key >= thr) { const int c = atomicAdd(&s_ncand[row], 1); if (c < RG_CAND) { s_ck[row][c] = key; s_ci[row][c] = i; } }
         }
-        if (lane < a.k) { s_ck[row][16 * sub + lane] = myk; s_ci[row][16 * sub + lane] = myi; }
         row_barrier(row);
         if (sub == 0) {
-            // merge by rank: candidate c is the winner number (count of candidates that beat it)
-            const bool valid = lane < 2 * a.k;
-            const int slot = lane < a.k ? lane : 16 + lane - a.k;
-            const uint32_t ck = valid ? s_ck[row][slot] : 0u; const int ci = valid ? s_ci[row][slot] : 0x7fffffff;
-            int rank = 0;
-            for (int j = 0; j < 2 * a.k; ++j) {
-                const int sj = j < a.k ? j : 16 + j - a.k;
-                const uint32_t kj = s_ck[row][sj]; const int ij = s_ci[row][sj];
-                rank += (kj > ck || (kj == ck && ij < ci)) ? 1 : 0;
+            const int n = s_ncand[row];
+            if (n <= RG_CAND) {
+                for (int c = lane; c < n; c += 32) {
+                    const uint32_t ck = s_ck[row][c]; const int ci = s_ci[row][c];
+                    int rank = 0;
+#pragma unroll 4
+                    for (int j = 0; j < n; ++j) { const uint32_t kj = s_ck[row][j]; const int ij = s_ci[row][j]; rank += (kj > ck || (kj == ck && ij < ci)) ? 1 : 0; }
+                    if (rank < a.k) { a.ids[t * ns + rank] = ci; s_sel[row][rank] = __uint_as_float(ck - 1u); }
+                }
+            } else {
+                for (int r = 0; r < a.k; ++r) {
+                    uint32_t bk = 0u; int bi = 0x7fffffff;
+                    for (int q = 0; q < nq; ++q) { const uint32_t key = sk[32 * q + lane]; if (key > bk) { bk = key; bi = 32 * q + lane; } }
+                    const uint32_t m = __reduce_max_sync(0xffffffffu, bk);
+                    const int wi = (int)__reduce_min_sync(0xffffffffu, bk == m ? (uint32_t)bi : 0x7fffffffu);
+                    if (lane == 0) { a.ids[t * ns + r] = wi; s_sel[row][r] = __uint_as_float(m - 1u); sk[wi] = 0u; }
+                    __syncwarp();
+                }
             }
-            if (ck != 0u && rank < a.k) { a.ids[t * ns + rank] = ci; s_sel[row][rank] = __uint_as_float(ck - 1u); }
             __syncwarp();
             float wsum = s_sel[row][0];   // the selected probabilities added in rank order
             for (int r = 1; r < a.k; ++r) wsum = wsum + s_sel[row][r];
