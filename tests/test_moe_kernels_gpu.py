@@ -69,6 +69,24 @@ def test_router_ties_go_to_the_lower_expert_id():
     assert np.array_equal(ids.cpu().numpy(), ids_o) and np.array_equal(bits(y.cpu().numpy()), bits(y_o))
 
 
+@pytest.mark.parametrize("n_expert,k,T", [(100, 10, 1), (512, 15, 3), (300, 3, 9)])
+def test_rows_of_equal_probabilities_take_the_lowest_experts(n_expert, k, T):
+    """More equal candidates than are ranked at once (a row of zeros: all probabilities the same), beside rows of the usual kind, for every number
+    of warps per row."""
+    E, F = 256, 256
+    rng = np.random.default_rng(T)
+    xn = rng.normal(0, 1, size=(T, E)).astype(np.float32); xn[T // 2] = 0.0
+    router = (rng.normal(0, 1, size=(n_expert + 1, E)) / np.sqrt(E)).astype(np.float32)
+    egu = synth.q4k_matrix(n_expert * 2 * F, E, seed=1).reshape(-1); edn = synth.q4k_matrix(n_expert * E, F, seed=2).reshape(-1)
+    sgu = synth.q4k_matrix(2 * F, E, seed=3).reshape(-1); sdn = synth.q4k_matrix(E, F, seed=4).reshape(-1)
+    d = lambda a: torch.from_numpy(a).cuda()
+    ids, w, y = K_.moe_layer(d(xn), d(router), d(egu), d(edn), d(sgu), d(sdn), F, n_expert, k)
+    K_.device_status()
+    ids_o, w_o, y_o, _ = orc.moe_layer(xn, router, egu, edn, sgu, sdn, E, F, n_expert, k)
+    assert list(ids_o[T // 2][:k]) == list(range(k))
+    assert np.array_equal(ids.cpu().numpy(), ids_o) and np.array_equal(bits(w.cpu().numpy()), bits(w_o)) and np.array_equal(bits(y.cpu().numpy()), bits(y_o))
+
+
 def test_unit_form_of_the_expert_gemv_matches_too():
     """The one-warp-per-unit form of the expert GEMVs (taken when the quads' activation buffers do not fit in shared
     memory, or with HIPSTER_B200_MOE_UNITS set) must give the same bits: the switch is read once per process, so the
