@@ -7,6 +7,7 @@
 // last; the output norm, gate and quantiser of all rows in parallel.
 #include "hp_common.cuh"
 #include "kernels.h"
+#include <type_traits>
 
 namespace hp {
 namespace {
@@ -88,37 +89,51 @@ __global__ void __launch_bounds__(PF_ST) k_gdn_pf_scan(GdnPrefillParams a) {
         else cp_async_wait_all();
         __syncthreads();
         const int n = min(PF_CH, a.T - r0);
-        for (int it = 0; it < n; ++it) {
-            const float beta = sg[s][it].x, decay = sg[s][it].y;
-            const float* kk = &sqk[s][it][160 + 20 * ck]; const float* qq = &sqk[s][it][20 * ck];
-            float2 kr[8];
+        // as in k_gdn: the second product of a row runs beside the decay and the first product of the next one, its reduction beside that
+        // one's, and the reads of the next row's k are in flight under both
+        float2 kr[8];
+        float d0 = 0.f, d1 = 0.f, o0 = 0.f, o1 = 0.f;
+        auto ld8 = [&](float2 (&r)[8], const float* p) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) kr[i] = lds_f2(kk + 2 * i);
-            const float v0 = sv[s][it][jl], v1 = sv[s][it][jl + 8];
-            const float2 dc2 = make_float2(decay, decay);
-            float d0 = 0.f, d1 = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                m[0][i] = mul2(m[0][i], dc2); m[1][i] = mul2(m[1][i], dc2);
-                d0 = fmaf(m[0][i].x, kr[i].x, d0); d1 = fmaf(m[1][i].x, kr[i].x, d1);
-                d0 = fmaf(m[0][i].y, kr[i].y, d0); d1 = fmaf(m[1][i].y, kr[i].y, d1);
-            }
-#pragma unroll
-            for (int off = 1; off < 8; off <<= 1) { d0 = d0 + __shfl_xor_sync(0xffffffffu, d0, off); d1 = d1 + __shfl_xor_sync(0xffffffffu, d1, off); }
-            const float e0 = (v0 - d0) * beta, e1 = (v1 - d1) * beta;
-            const float2 dl0 = make_float2(e0, e0), dl1 = make_float2(e1, e1);
-            float o0 = 0.f, o1 = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float2 qv = lds_f2(qq + 2 * i);
-                fma2(m[0][i], dl0, kr[i]); fma2(m[1][i], dl1, kr[i]);
-                o0 = fmaf(m[0][i].x, qv.x, o0); o1 = fmaf(m[1][i].x, qv.x, o1);
-                o0 = fmaf(m[0][i].y, qv.y, o0); o1 = fmaf(m[1][i].y, qv.y, o1);
-            }
+            for (int i = 0; i < 8; ++i) r[i] = lds_f2(p + 2 * i);
+        };
+        auto first = [&](float2 dc2, const float2& k, int i) {   // decay and first product of one column pair
+            m[0][i] = mul2(m[0][i], dc2); m[1][i] = mul2(m[1][i], dc2);
+            d0 = fmaf(m[0][i].x, k.x, d0); d1 = fmaf(m[1][i].x, k.x, d1);
+            d0 = fmaf(m[0][i].y, k.y, d0); d1 = fmaf(m[1][i].y, k.y, d1);
+        };
+        auto put = [&](int it) {
 #pragma unroll
             for (int off = 1; off < 8; off <<= 1) { o0 = o0 + __shfl_xor_sync(0xffffffffu, o0, off); o1 = o1 + __shfl_xor_sync(0xffffffffu, o1, off); }
             if (ck == 0) { float* o = a.o + ((size_t)(r0 + it) * a.n_v + h) * D + j; o[0] = o0 * 0.08838834764831845f; o[8] = o1 * 0.08838834764831845f; }
-        }
+        };
+        ld8(kr, &sqk[s][0][160 + 20 * ck]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) first(make_float2(sg[s][0].y, sg[s][0].y), kr[i], i);
+        auto row = [&](int it, auto last_) {
+            constexpr bool last = decltype(last_)::value;   // of the piece: the state stays as it is behind it
+            float2 qr[8], kn[8];
+            ld8(qr, &sqk[s][it][20 * ck]);
+            if constexpr (!last) ld8(kn, &sqk[s][it + 1][160 + 20 * ck]);
+            const float beta = sg[s][it].x, decay = last ? 1.f : sg[s][it + 1].y, v0 = sv[s][it][jl], v1 = sv[s][it][jl + 8];
+#pragma unroll
+            for (int off = 1; off < 8; off <<= 1) { d0 = d0 + __shfl_xor_sync(0xffffffffu, d0, off); d1 = d1 + __shfl_xor_sync(0xffffffffu, d1, off); }
+            if (it > 0) put(it - 1);
+            const float e0 = (v0 - d0) * beta, e1 = (v1 - d1) * beta;
+            const float2 dl0 = make_float2(e0, e0), dl1 = make_float2(e1, e1), dc2 = make_float2(decay, decay);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { fma2(m[0][i], dl0, kr[i]); fma2(m[1][i], dl1, kr[i]); }
+            o0 = o1 = d0 = d1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                o0 = fmaf(m[0][i].x, qr[i].x, o0); o1 = fmaf(m[1][i].x, qr[i].x, o1);
+                o0 = fmaf(m[0][i].y, qr[i].y, o0); o1 = fmaf(m[1][i].y, qr[i].y, o1);
+                if constexpr (!last) { first(dc2, kn[i], i); kr[i] = kn[i]; }
+            }
+        };
+        for (int it = 0; it + 1 < n; ++it) row(it, std::false_type());
+        row(n - 1, std::true_type());
+        put(n - 1);
         __syncthreads();   // the stage is free again
     }
 #pragma unroll
