@@ -508,15 +508,16 @@ int launch_tc(const TcArgs& a, const XQ8F& x, int grid, cudaStream_t s, bool pdl
 
 size_t gemm_pack_bytes(int R, int K) { return (size_t)((R + 7) / 8 + 15) * (size_t)(K / 256) * 4608; }
 // The cut of the rows into column ranges of ntc tiles of 8, and of the weight tiles into items of G = 8 or 4 (the latter leaves
-// every second tile position empty). An item of 20 blocks takes 36, 56, 72 and 90 us at ntc = 4, 8, 12 and 16: 4.5 us
-// for each of ntc + 4; the cut with the least time over the rounds of the SMs is taken.
+// every second tile position empty). An item of 20 blocks takes 34, 47, 63, 76 and 83 us at ntc = 4, 8, 10, 14 and 16, four fifths of that
+// with G = 4: 5 and 4 for each of ntc + 6; the cut with the least time over the rounds of the SMs is taken (over eight projections and 56 to
+// 512 rows 0.7 % slower than the best cut on average, 8 % at most; with 3 and 2 for each of ntc + 4 1.3 % and 24 %: 2048 x 6144, 304 rows).
 void gemm_cut(int N, int K, int R, int* ntc, int* G) {
     const int t8 = (R + 7) / 8, tiles = (N + 15) / 16, P = gemv_num_parts(N, K / 256);
     long best = 0; *ntc = 0;
     for (int c = 4; c <= 16; c += 2)
         for (int g = 8; g >= 4; g -= 4) {
             const int ncg = (t8 + c - 1) / c;
-            const long cost = ((long)ncg * P * ((tiles + g - 1) / g) + GEMV_NCTA - 1) / GEMV_NCTA * (g == 8 ? (c + 4) * 3 : (c + 4) * 2);
+            const long cost = ((long)ncg * P * ((tiles + g - 1) / g) + GEMV_NCTA - 1) / GEMV_NCTA * (g == 8 ? (c + 6) * 5 : (c + 6) * 4);
             if (!*ntc || cost < best) { best = cost; *ntc = c; *G = g; }
         }
 }
