@@ -1,4 +1,4 @@
-// Q4_K x int8 GEMM for prompt chunks (many rows) on the 5th-generation tensor cores: tcgen05.mma kind::i8 with the
+// Q4_K x int8 GEMM for prompt chunks (many rows) on the 5th-generation tensor cores: tcgen05.mma kind::f8f6f4 with the
 // accumulator in TMEM.
 //
 // The arithmetic is that of the verify GEMV (gemv_q4k.cu) operation by operation: the exact int32 dot of every 32-element
@@ -6,25 +6,29 @@
 // sums of a 16-row tile cut where the GEMV's partition cuts them (K parts, warp boundaries of the tile's CTA) and added
 // in the same order. A row therefore has the same bits whichever of the two kernels computed it.
 //
-// What bounds it: the fp32 update, two conversions and three packed fp32 instructions per two outputs and sub-block. From
-// registers alone a 16x8x32 tile of it takes 15.3 clocks of an SM sub-partition; the int8 mma.sync of the GEMV takes 8.0 and
-// does not overlap with it (23.9 together). In place, at 1965 MHz, this kernel takes 36 clocks per tile at 512 rows of 34816 x 5120 (687
-// us; 40 to 49 for the other projections) and 57 at 32 (68 us), the GEMV 54 at 32 rows (65 us): the rest is TMEM and shared-memory
-// loads, addresses and waits.
+// The dots come as fp32: a nibble q, read as e4m3, is q / 512 (subnormal up to 7), an int8 activation is 16 a + b with |a|, |b| <= 8, both
+// exact in e4m3, and the two products accumulate exactly (at most 16 significant bits). The accumulator holds idot / 512 and the row scales
+// carry the 512. (kind::i8 took one MMA instead of two, but each dot cost a conversion in the update: 34816 x 5120 at 512 rows 692 us, now 611.)
+//
+// What bounds it: the fp32 update, three packed instructions per two outputs and sub-block (12 clocks of an SM sub-partition per 16x8x32
+// tile), which hardly overlaps with what brings its operands into registers: TMEM loads (16x256b fills 64 bytes a clock) and column
+// scales. The loop by itself, two warps per sub-partition, takes 16 clocks per tile; in place, at 1965 MHz, 32 at 512 rows of 34816 x 5120 and 35 to 41 for
+// the other projections. Left out one at a time (611 us): waits of the TMEM slots 17, closing of partial sums 24, MMAs 56, TMEM loads
+// 73, column scales 128.
 // Hence:
-//   * one CTA per SM, M = 128 weight rows (8 tiles of 16), N = 32..128 pass rows, one tcgen05.mma (K = 32) per sub-block,
-//     never accumulating: TMEM only hands the int32 dots over to the update, in slots of 2 or 4 sub-blocks;
+//   * one CTA per SM, M = 128 weight rows (8 tiles of 16), N = 32..128 pass rows, two tcgen05.mma (K = 32) per sub-block: TMEM
+//     only hands the dots over to the update, in slots of 2 or 4 sub-blocks (slots of one, or of half the columns, cost more waits than they
+//     hide: 797 and 619 us);
 //   * 8 update warps (4 TMEM lane quadrants x 2 column halves) read the dots with 16x256b loads, which leave a lane two
 //     rows x two adjacent columns per 16 lanes: one 16-byte read of the scales of the activations serves 4 rows. A step of a
 //     warp is 5 to 8 (column tile, sub-block) pairs whatever N is, all loads in front. (16 warps with steps of half the size
 //     hide more latency but execute the loads and addresses of a step twice, and these compete with the update for the
-//     register ports.)
-//   * 4 conversion warps split the nibbles into u8 (the high ones stay shifted by 4, the scale carries the exact 1/16) in
-//     the K-major, 64-byte-swizzled layout of the tensor core. Rows 2, 3, 6, 7 of a group store their high nibbles first, so
-//     that the 16 lanes of a store phase hit distinct banks;
-//   * the activations are brought into that layout once per call by k_tc_pack (a few microseconds), so that a half-block of
-//     a column range is one bulk copy (8-byte asynchronous copies by two warps took 2800 clocks per half-block);
-//   * one warp streams the weights (2304-byte tile chunks, ring of 4 blocks, primed before the dependency wait), one the
+//     register ports; half a step ahead of the arithmetic: 809 us.)
+//   * 4 conversion warps split the nibbles into bytes in the K-major, 64-byte-swizzled layout of the tensor core. Rows 2, 3, 6, 7 of a
+//     group store their high nibbles first, so that the 16 lanes of a store phase hit distinct banks;
+//   * the activations are brought into that layout, as two planes of e4m3, once per call by k_tc_pack (a few microseconds), so that a
+//     half-block of a column range is one bulk copy (8-byte asynchronous copies by two warps took 2800 clocks per half-block);
+//   * one warp streams the weights (2304-byte tile chunks, ring of 3 blocks, primed before the dependency wait), one the
 //     activations, one thread issues the MMAs.
 // Registers: 512 threads x 128 at launch; the update warps take 184 (8 x 32 threads) from the conversion warps (72) and the
 // last four warps (56): 63488 in all.

@@ -272,9 +272,10 @@ __device__ __forceinline__ float2 gdn_fma2(float2 a, float2 b, float2 c) {   // 
         : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)), "l"(reinterpret_cast<unsigned long long&>(c)));
     return r;
 }
-// Passes over one or two sequences: one wave of a latency-bound kernel. One sequence of 6 rows, 4 replayed: 12.7 us in a captured graph,
-// of 1 row, 1 replayed 7.8, two sequences of 6 rows 16.9 (q and k of the recurrence by 64-bit reads, see lds_f2; by 128-bit ones 12.8, 7.9
-// and 17.0).
+// Passes over one or two sequences: one wave of a latency-bound kernel, its chain the loads, conv and norms, ten rows of the recurrence and two
+// cluster exchanges. One sequence of 6 rows, 4 replayed: 11.5 us in a captured graph, of 1 row, 1 replayed 7.5, two sequences of 6 rows 15.7
+// (with the products of a row one after the other, and q of the replayed rows, 12.7, 7.8 and 16.9). OCC: CTAs per SM. One sequence has 192 CTAs
+// and takes the registers of two per SM (120; at 96 and 80 it spills: 11.7 and 12.1 us), two sequences need three.
 template <int OCC>
 __global__ void __cluster_dims__(GDN_CL, 1, 1) __launch_bounds__(256, OCC) k_gdn(GdnArgs a) {
     constexpr int D = 128, NLD = 8, NCV = 6;   // items per thread: (16 + 3) * 96 <= 8 * 256 raw values, 16 * 96 = 6 * 256 conv outputs
@@ -486,8 +487,8 @@ struct GdnWideSmem {
 // state rows. Every CTA convolves and normalises the head's 128 q and 128 k channels itself (warp w: 32 q channels for w < 4, 32 k
 // channels otherwise) and its own 64 v channels, from raw inputs that arrive by asynchronous copies; both CTAs read the saved rows and
 // the history, so these are rewritten at the end, behind the cluster barrier of the output norm. Sums and their order are those of
-// k_gdn. us in a captured graph, k_gdn in brackets: eight sequences of 3 rows, 2 replayed, 30.5 (43.6; 39.7 with registers for four CTAs per
-// SM), three of them 13.8 (21.7); two sequences of 6 rows, 4 replayed, 17.8 (16.9), one 13.1 (12.7).
+// k_gdn. us in a captured graph: eight sequences of 3 rows, 2 replayed, 29.7 (30.5 with q of the replayed rows; k_gdn's earlier form 43.6, 39.7
+// with registers for four CTAs per SM), three of them 13.3 (21.7); two sequences of 6 rows, 4 replayed, 17.8, one 13.1 (k_gdn 15.7 and 11.5).
 __global__ void __cluster_dims__(GDN_WCL, 1, 1) __launch_bounds__(256, 3) k_gdn_wide(GdnArgs a) {
     constexpr int D = 128;
     extern __shared__ __align__(16) uint8_t gdn_smem[];
