@@ -104,8 +104,21 @@ struct TcArgs {
     const uint8_t* W; const uint8_t* xp; float* y;   // xp: packed activations
     int N, nb, P, R, ldy; size_t part_stride;
     int G, ngrp, ncg;        // tiles of 16 rows per work item (8, or 4 with every second tile position empty), items along M, along the pass rows
+    int nlong, heavy, light; // ranges of NTC column tiles (the others have two less); CTAs with one item more, items of the other CTAs
     int* err;
 };
+// Item `it` of the launch: column range, its first column tile, and part * ngrp + group. Wide ranges go to the CTAs with fewer items first
+// (34816 x 5120 at 304 rows, 38 tiles as 14 + 12 + 12 instead of 3 x 14: 433 -> 410 us, 5120 x 17408 269 -> 248).
+struct TcItem { int cg, c0, rest; bool narrow; };
+__device__ __forceinline__ TcItem tc_item(const TcArgs& a, int it, int ntc) {
+    const int n = gridDim.x, k = it / n, i = it % n, nl = a.nlong * a.ngrp * a.P;
+    int j = i >= a.heavy ? k * (n - a.heavy) + i - a.heavy : a.light + k * a.heavy + i;
+    TcItem v;
+    v.narrow = j >= nl;
+    if (!v.narrow) { v.cg = j % a.nlong; v.rest = j / a.nlong; v.c0 = v.cg * ntc; }
+    else { j -= nl; const int ns = a.ncg - a.nlong; v.cg = a.nlong + j % ns; v.rest = j / ns; v.c0 = a.nlong * ntc + (j % ns) * (ntc - 2); }
+    return v;
+}
 // Units of tile `tile` after which the GEMV's partition closes a partial sum: bit c of the result = after unit c (CB blocks) of the K part
 __device__ __forceinline__ uint64_t tc_cuts(int N, int nb, int P, int tile, int lane) {
     const int tiles = (N + 15) / 16, gc = GEMV_NCTA / P, nbp = nb / P, C = nbp % 2 == 0 ? nbp / 2 : nbp;
@@ -173,7 +186,7 @@ __device__ __forceinline__ void tc_update(float2 (&acc)[4][W], uint32_t ta, uint
 template <int NTC>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
     using Geo = TcGeom<NTC>;
-    constexpr int W = NTC / 2, GB = W == 2 ? 4 : W <= 4 ? 2 : 1, GS = Geo::GS, SLOTS = Geo::SLOTS, BST = Geo::BST;
+    constexpr int GS = Geo::GS, SLOTS = Geo::SLOTS, BST = Geo::BST;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint32_t tmem_ptr;
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -210,7 +223,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
         if (warp == TC_W_TMA) {   // ---- weight stream: one 2304-byte chunk per tile and block
             int k = 0; bool ok = true;
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
-                const int rest = it / a.ncg, grp = rest % a.ngrp, part = rest / a.ngrp, nt = min(G, tiles - grp * G);
+                const int rest = tc_item(a, it, NTC).rest, grp = rest % a.ngrp, part = rest / a.ngrp, nt = min(G, tiles - grp * G);
                 const uint8_t* src = a.W + ((size_t)(grp * G) * nb + (size_t)part * nbp) * 2304;
                 for (int b = 0; b < nbp; ++b, ++k) {
                     const int s = k % TC_RAWS;
@@ -226,9 +239,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
             }
             for (int i = k > TC_RAWS ? k - TC_RAWS : 0; i < k; ++i) tc_wait(raw_full + 8 * (i % TC_RAWS), (i / TC_RAWS) & 1, a.err);   // no copy outlives the CTA
         } else if (warp == TC_W_MMA) {   // ---- MMA issue
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(Geo::N / 8) << 17) | (8u << 24);   // f32 = e4m3 x e4m3, M = 128
             int hb = 0, gr = 0; bool ok = true;
-            for (int it = blockIdx.x; it < items && ok; it += gridDim.x)
+            for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+                const uint32_t idesc = (1u << 4) | ((uint32_t)(tc_item(a, it, NTC).narrow ? NTC - 2 : NTC) << 17) | (8u << 24);   // f32 = e4m3 x e4m3, M = 128
                 for (int h = 0; h < 2 * nbp && ok; ++h, ++hb) {
                     const int as = hb % TC_CNVS, bs = hb % BST;
                     ok = tc_wait(b_full + 8 * bs, (hb / BST) & 1, a.err) && tc_wait(a_full + 8 * as, (hb / TC_CNVS) & 1, a.err);
@@ -252,6 +265,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
                         __syncwarp();
                     }
                 }
+            }
             if (tc_elect()) tc_commit(fin);
             __syncwarp();
             tc_wait(fin, 0, a.err);   // nothing in flight when the accumulator memory is given back
@@ -259,7 +273,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
             pdl_wait();
             int hb = 0, k = 0; bool ok = true;
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
-                const int cg = it % a.ncg, part = it / a.ncg / a.ngrp;
+                const TcItem im = tc_item(a, it, NTC); const int cg = im.cg, part = im.rest / a.ngrp;
                 const uint8_t* src = a.xp + ((size_t)cg * nb + (size_t)part * nbp) * Geo::PACK;
                 for (int b = 0; b < nbp && ok; ++b, ++k, src += Geo::PACK) {
                     const int ss = k % Geo::SCS;
@@ -293,7 +307,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
         auto nib = [](uint32_t v, int sh) { return (v >> sh) & 0x0F0F0F0Fu; };
         int k = 0, hb = 0; bool ok = true;
         for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
-            const int grp = it / a.ncg % a.ngrp, nt = min(G, tiles - grp * G);
+            const int grp = tc_item(a, it, NTC).rest % a.ngrp, nt = min(G, tiles - grp * G);
             for (int b = 0; b < nbp && ok; ++b, ++k) {
                 const int s = k % TC_RAWS, ss = k % Geo::SCS;
                 const uint8_t* raw = smem + s * TC_RAW_BYTES;
@@ -342,12 +356,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
         }
     } else {   // ---- fp32 update: warp = (lane quadrant q, column half); half h of the quadrant holds one tile of 16 rows
         tc_reg_inc<184>();
-        const int q = warp & 3, n0 = (warp >> 2) * W;
+        const int q = warp & 3;
         pdl_wait();
         int k = 0, gr = 0; bool ok = true;
         const int cb1 = nbp % 2 == 0 ? 1 : 0;   // blocks per unit of the GEMV's partition, less 1
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
-            const int cg = it % a.ncg, rest = it / a.ncg, grp = rest % a.ngrp, part = rest / a.ngrp, tile0 = grp * G, tend = min(tiles, tile0 + G);
+        auto item = [&](const TcItem im, auto wt) {
+            constexpr int W = decltype(wt)::value, GB = W <= 2 ? 4 : W <= 4 ? 2 : 1;   // column tiles of this warp, sub-blocks per step
+            const int grp = im.rest % a.ngrp, part = im.rest / a.ngrp, tile0 = grp * G, tend = min(tiles, tile0 + G), n0 = (warp >> 2) * W;
             const int tl[2] = {tile0 + (G == 8 ? 2 * q : q), G == 8 ? tile0 + 2 * q + 1 : tiles};
             const bool has0 = tl[0] < tend, has1 = tl[1] < tend;
             const uint64_t cut[2] = {has0 ? tc_cuts(a.N, nb, a.P, tl[0], lane) : 0, has1 ? tc_cuts(a.N, nb, a.P, tl[1], lane) : 0};
@@ -410,7 +425,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
                         }
                         // element {i, w, e}: row + 8 i, column 2 t + 8 w + e. Other warps wait at the next slot for the one that closes a
                         // tile: whole tiles and ranges without predicates, one pointer per column pair, all loads in front
-                        const int row = tl[h] * 16 + g, col = (cg * NTC + n0) * 8 + 2 * t;
+                        const int row = tl[h] * 16 + g, col = (im.c0 + n0) * 8 + 2 * t;
                         float* yt = y + (size_t)col * ldy + row;
                         const size_t step = (size_t)8 * ldy;
                         auto close = [&](auto live) {
@@ -442,12 +457,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
                                 }
                             }
                         };
-                        if (tl[h] * 16 + 16 <= a.N && (cg * NTC + n0 + W) * 8 <= a.R) close([](int, int, int) { return true; });
+                        if (tl[h] * 16 + 16 <= a.N && (im.c0 + n0 + W) * 8 <= a.R) close([](int, int, int) { return true; });
                         else close([&](int i, int w, int e) { return row + 8 * i < a.N && col + 8 * w + e < a.R; });
                         first[h] = false;
                     }
                 }
             }
+        };
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+            const TcItem im = tc_item(a, it, NTC);
+            if (im.narrow) item(im, std::integral_constant<int, NTC / 2 - 1>()); else item(im, std::integral_constant<int, NTC / 2>());
         }
     }
     tc_fence_before();
@@ -467,18 +486,19 @@ __device__ __forceinline__ void tc_split(uint32_t x, uint32_t& hi, uint32_t& lo)
     }
 }
 // Activations in the order the GEMM copies them: per column range of NTC tiles and block two half-blocks (per 64-element
-// group the swizzled K-major tile of all columns), then the scales. Tiles beyond the rows are zero.
+// group the swizzled K-major tile of all columns), then the scales. Tiles beyond the range and the rows are zero.
 template <int NTC>
-__global__ void __launch_bounds__(256) k_tc_pack(const uint4* __restrict__ xq, const float4* __restrict__ xsc, uint8_t* __restrict__ xp, int nb, int tiles8) {
+__global__ void __launch_bounds__(256) k_tc_pack(const uint4* __restrict__ xq, const float4* __restrict__ xsc, uint8_t* __restrict__ xp, int nb, int tiles8, int nlong) {
     pdl_launch_dependents();
     pdl_wait();
     const int blk = blockIdx.x, cg = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int c0 = cg * NTC - 2 * max(cg - nlong, 0), cend = min(tiles8, c0 + (cg < nlong ? NTC : NTC - 2));
     uint8_t* d = xp + ((size_t)cg * nb + blk) * TcGeom<NTC>::PACK;
     const uint32_t lo = (uint32_t)((((t >> 1) ^ ((g >> 1) & 3)) << 4) + (t & 1) * 8 + g * 64);   // the low sub-block's 8 bytes; the high one's: lo ^ 32
 #pragma unroll
     for (int u = warp; u < NTC * 4; u += 8) {
-        const int n = u >> 2, jj = u & 3, nt = cg * NTC + n;
-        const uint4 v = nt < tiles8 ? xq[((size_t)nt * nb * 4 + (size_t)blk * 4 + jj) * 32 + lane] : make_uint4(0, 0, 0, 0);
+        const int n = u >> 2, jj = u & 3, nt = c0 + n;
+        const uint4 v = nt < cend ? xq[((size_t)nt * nb * 4 + (size_t)blk * 4 + jj) * 32 + lane] : make_uint4(0, 0, 0, 0);
         uint8_t* p = d + (jj >> 1) * TcGeom<NTC>::B_BYTES + (jj & 1) * (2 * NTC * 512) + n * 512;
         uint2 h, l;
         tc_split(v.x, h.x, l.x); tc_split(v.y, h.y, l.y);
@@ -487,8 +507,8 @@ __global__ void __launch_bounds__(256) k_tc_pack(const uint4* __restrict__ xq, c
         *reinterpret_cast<uint2*>(p + (lo ^ 32)) = h; *reinterpret_cast<uint2*>(p + NTC * 512 + (lo ^ 32)) = l;
     }
     for (int n = warp; n < NTC; n += 8) {
-        const int nt = cg * NTC + n;
-        reinterpret_cast<float4*>(d + 2 * TcGeom<NTC>::B_BYTES)[n * 32 + lane] = nt < tiles8 ? xsc[((size_t)nt * nb + blk) * 32 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int nt = c0 + n;
+        reinterpret_cast<float4*>(d + 2 * TcGeom<NTC>::B_BYTES)[n * 32 + lane] = nt < cend ? xsc[((size_t)nt * nb + blk) * 32 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
 
@@ -498,7 +518,7 @@ int launch_tc(const TcArgs& a, const XQ8F& x, int grid, cudaStream_t s, bool pdl
     static bool attr[MAX_DEVICES] = {};   // per device: the opt-in belongs to the device's copy of the kernel
     const int dev = current_device(); if (dev < 0) return HP_ECUDA;
     if (!attr[dev]) { HP_CUDA(cudaFuncSetAttribute(k_gemm_q4k_tc<NTC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); attr[dev] = true; }
-    k_tc_pack<NTC><<<dim3(a.nb, a.ncg), 256, 0, s>>>((const uint4*)x.q, (const float4*)x.sc, (uint8_t*)a.xp, a.nb, (a.R + 7) / 8);
+    k_tc_pack<NTC><<<dim3(a.nb, a.ncg), 256, 0, s>>>((const uint4*)x.q, (const float4*)x.sc, (uint8_t*)a.xp, a.nb, (a.R + 7) / 8, a.nlong);
     HP_CUDA(cudaGetLastError());
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = s;
@@ -511,17 +531,27 @@ int launch_tc(const TcArgs& a, const XQ8F& x, int grid, cudaStream_t s, bool pdl
 }  // namespace
 
 size_t gemm_pack_bytes(int R, int K) { return (size_t)((R + 7) / 8 + 15) * (size_t)(K / 256) * 4608; }
-// The cut of the rows into column ranges of ntc tiles of 8, and of the weight tiles into items of G = 8 or 4 (the latter leaves
-// every second tile position empty). An item of 20 blocks takes 34, 47, 63, 76 and 83 us at ntc = 4, 8, 10, 14 and 16, four fifths of that
-// with G = 4: 5 and 4 for each of ntc + 6; the cut with the least time over the rounds of the SMs is taken (over eight projections and 56 to
-// 512 rows 0.7 % slower than the best cut on average, 8 % at most; with 3 and 2 for each of ntc + 4 1.3 % and 24 %: 2048 x 6144, 304 rows).
+// A cut into ranges of ntc column tiles leaves up to ntc - 1 empty: the number of ranges, not the first, that get two tiles less instead.
+static int tc_narrow(int R, int ntc) {
+    const int t8 = (R + 7) / 8, ncg = (t8 + ntc - 1) / ntc, k = (ncg * ntc - t8) / 2;
+    return k < ncg - 1 ? k : ncg - 1;
+}
+// The cut of the rows into column ranges of ntc tiles of 8, and of the weight tiles into items of G = 8 or 4 (the latter leaves every second
+// tile position empty): the one whose fullest CTA takes the least time. Of an item of 20 blocks that is, at ntc = 4, 8, 10, 14 and 16, 34, 47, 63, 76
+// and 83 us (ntc + 8, from 10 on ntc + 11: half as many sub-blocks per TMEM slot), 1.25 of these units less for a narrow range, four fifths
+// with G = 4. Over eight projections and 18 row counts from 56 to 512 that is 0.4 % slower than the best cut on average, 6 % at most (with ntc + 6,
+// narrow ranges 2 less, 1.0 and 15 %).
 void gemm_cut(int N, int K, int R, int* ntc, int* G) {
     const int t8 = (R + 7) / 8, tiles = (N + 15) / 16, P = gemv_num_parts(N, K / 256);
     long best = 0; *ntc = 0;
     for (int c = 4; c <= 16; c += 2)
         for (int g = 8; g >= 4; g -= 4) {
-            const int ncg = (t8 + c - 1) / c;
-            const long cost = ((long)ncg * P * ((tiles + g - 1) / g) + GEMV_NCTA - 1) / GEMV_NCTA * (g == 8 ? (c + 6) * 5 : (c + 6) * 4);
+            // CTAs with one item more and the others: their items, and at most how many wide ones among these (see tc_item)
+            const long ncg = (t8 + c - 1) / c, per = (long)P * ((tiles + g - 1) / g), nl = (ncg - tc_narrow(R, c)) * per, items = ncg * per;
+            const long n = items < GEMV_NCTA ? items : GEMV_NCTA, full = items / n, heavy = items % n, light = n - heavy, over = nl - full * light;
+            const long wl = (nl + light - 1) / light, wh = heavy && over > 0 ? (over + heavy - 1) / heavy : 0;
+            const long u = 4 * (c + (c > 8 ? 11 : 8)) - 5, cl = full * u + 5 * (wl < full ? wl : full), ch = heavy ? (full + 1) * u + 5 * wh : 0;
+            const long cost = (cl > ch ? cl : ch) * (g == 8 ? 5 : 4);
             if (!*ntc || cost < best) { best = cost; *ntc = c; *G = g; }
         }
 }
@@ -535,6 +565,8 @@ int gemm_q4k_q8_cut(const void* Wt, const XQ8F& x, float* yparts, int N, int K, 
     HP_REQUIRE(a.P > 0, "gemm_q4k_q8: K=%d is too large for the K-part partition", K);
     a.G = G; a.ngrp = ((N + 15) / 16 + G - 1) / G; a.ncg = ((R + 7) / 8 + ntc - 1) / ntc;
     const int items = a.ncg * a.ngrp * a.P, grid = items < GEMV_NCTA ? items : GEMV_NCTA;
+    a.nlong = a.ncg - tc_narrow(R, ntc);
+    a.heavy = a.nlong < a.ncg ? items % grid : 0; a.light = items / grid * (grid - a.heavy);
     switch (ntc) {
         case 4: return launch_tc<4>(a, x, grid, s, pdl);   case 6: return launch_tc<6>(a, x, grid, s, pdl);
         case 8: return launch_tc<8>(a, x, grid, s, pdl);   case 10: return launch_tc<10>(a, x, grid, s, pdl);

@@ -85,6 +85,19 @@ def test_every_cut_gives_the_bits_of_the_gemv(weights, ntc, G):
             assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (N, K, R)   # and nothing beyond column N
 
 
+# rows whose last column ranges are two tiles narrower: one of three, both of the two behind the first, and with more rows left empty than that
+@pytest.mark.gpu
+@pytest.mark.parametrize("ntc,G", CUTS)
+def test_narrow_ranges_give_the_bits_of_the_gemv(weights, ntc, G):
+    for N, K in SHAPES:
+        for R in (24 * ntc - 16, 24 * ntc - 35, 16 * ntc + 1) if N < 30000 else (24 * ntc - 32,):
+            xq = K_.quantize_x_q8(torch.randn((R, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(R)))
+            err = torch.zeros(1, dtype=torch.int32, device="cuda")
+            got, want = run_gemm(weights[N, K], xq, N, K, R, N, (ntc, G), err), run_gemv(weights[N, K], xq, N, K, R, N, err)
+            assert err.item() == 0
+            assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (N, K, R)
+
+
 # the tile-major form of the GEMV on both sides of its row limits (4 rows; three column tiles whose activations leave room for one-block
 # stages only: 20 blocks), against the row-major one
 @pytest.mark.gpu
