@@ -435,34 +435,36 @@ int Engine::ffn_block(const LayerW& L, int R) {
 }
 
 // Qwen4Exp::moe_layer (qwen4exp.cpp:345-354): router -> route -> gate|up for the k+1 slots -> silu*mul+q8 -> down + in-order combine
-// for rows [row0, row0 + R) of the current buffers (R <= MAXR, row0 a multiple of 8)
-int Engine::moe_rows(const LayerW& L, int R, int row0, const int* tok, const int* pos, const int* slot, int* pushed) {
+// for the rows of the current buffers: up to MAXR of a pass, up to PF_MAXR of a prompt chunk
+int Engine::moe_rows(const LayerW& L, int R, const int* tok, const int* pos, const int* slot, int* pushed) {
     const hp_model_cfg& c = c_; const int E = c.n_embd, F = c.expert_ff, ns = c.n_expert_used + 1;
+    const bool chunk = R > MAXR;   // of a prompt: each touched expert streamed once for all its rows
     // synthetic routing (see hp_model_cfg.synth_router_logits): the key of a layer's draws; 0 = the router's own logits
     const int lidx = &L == &mtp_ ? c.n_layer : (int)(&L - layers_.data());
     const uint64_t rkey = c.synth_router_logits ? (splitmix64(c.seed ^ 0x726F75746572ull ^ ((uint64_t)lidx << 40)) | 1ull) : 0ull;
     // the (replicated) shared expert is computed by one GPU per layer, in turn, so that no GPU carries all of them
     const int own_sh = c.ep_world > 1 ? (lidx % c.ep_world == c.ep_rank ? 1 : 0) : 1;
-    MoeRouteParams rp; rp.W = L.router; rp.x = xn_ + (size_t)row0 * E; rp.logits = rlogits_; rp.E = c.n_expert; rp.K = E; rp.k = c.n_expert_used; rp.T = R;
-    rp.ids = moe_ids_ + (size_t)row0 * ns; rp.w = moe_w_ + (size_t)row0 * ns; rp.ticket = route_cnt_; rp.row_tok = tok + row0; rp.row_pos = pos + row0; rp.row_slot = slot + row0; rp.synth_key = rkey;
-    rp.e_lo = e_lo_; rp.e_hi = e_hi_; rp.own_shared = own_sh; rp.segs = moe_segs_; rp.ctl = moe_ctl_; rp.touched = moe_touched_; rp.err = err_;
+    MoeRouteParams rp; rp.W = L.router; rp.x = xn_; rp.logits = chunk ? pf_rlogits_ : rlogits_; rp.E = c.n_expert; rp.K = E; rp.k = c.n_expert_used; rp.T = R;
+    rp.ids = moe_ids_; rp.w = moe_w_; rp.ticket = chunk ? pf_ticket_ : route_cnt_; rp.row_tok = tok; rp.row_pos = pos; rp.row_slot = slot; rp.synth_key = rkey;
+    rp.e_lo = e_lo_; rp.e_hi = e_hi_; rp.own_shared = own_sh; rp.segs = chunk ? nullptr : moe_segs_; rp.ctl = moe_ctl_; rp.touched = moe_touched_; rp.err = err_;
     HP_TRY(moe_route_group(rp, s_));
+    if (chunk) { rp.segs = pf_segs_; HP_TRY(moe_group_rows(rp, s_)); }
     // per-(row, slot) outputs of the experts this GPU owns, grouped by expert so that each touched expert matrix is read
     // once; pairs of experts owned elsewhere stay exact zeros, the exchange fills them in, and the combine runs in slot
     // order (the arithmetic of gemv.hip:1104-1112) on every GPU
     if (c.ep_world > 1) { HP_TRY(ep_ready()); if (!ep_peer_) HP_CUDA(cudaMemsetAsync(moe_v_, 0, (size_t)R * ns * E * 4, s_)); }
     MoeGroupParams g; g.w_gate_up = L.exp_gate_up.wt; g.w_down = L.exp_down.wt; g.sh_gate_up = L.sh_gate_up.wt; g.sh_down = L.sh_down.wt;
     g.E = E; g.F = F; g.nslot = ns; g.T = R; g.e_lo = e_lo_;
-    g.xq = xq_rows(xq_, row0, E); g.xq2 = xq2_; g.v = moe_v_ + (size_t)row0 * ns * E; g.segs = moe_segs_; g.ctl = moe_ctl_; g.err = err_;
+    g.xq = xq_; g.xq2 = chunk ? pf_xq2_ : xq2_; g.v = moe_v_; g.segs = chunk ? pf_segs_ : moe_segs_; g.ctl = moe_ctl_; g.err = err_;
     if (ep_peer_) { g.ep_world = c.ep_world; g.ep_rank = c.ep_rank; g.ep_half = ep_half_; for (int q = 0; q < 8; ++q) { g.ep_x[q] = ep_peer_x_[q]; g.ep_ctl[q] = ep_peer_ctl_[q]; } }
     return moe_experts_grouped(g, s_, pushed);
 }
 int Engine::moe_block(const LayerW& L, int R) {
     if (gemv_only_) return HP_OK;
-    if (pf_on_) return prefill_moe(L, R);
+    if (pf_on_) return moe_rows(L, R, pf_desc_, pf_desc_ + pf_rows_, pf_desc_ + 2 * pf_rows_, nullptr);
     const hp_model_cfg& c = c_; const int lidx = &L == &mtp_ ? c.n_layer : (int)(&L - layers_.data());
     int pushed = 0;
-    HP_TRY(moe_rows(L, R, 0, d_desc_ + D_TOK, d_desc_ + D_POS, d_desc_ + D_SLOT, &pushed));
+    HP_TRY(moe_rows(L, R, d_desc_ + D_TOK, d_desc_ + D_POS, d_desc_ + D_SLOT, &pushed));
     if (c.ep_world > 1) HP_TRY(ep_peer_ ? ep_exchange_peer(R, lidx % c.ep_world, pushed != 0) : ep_exchange(moe_v_, (size_t)R * (c.n_expert_used + 1) * c.n_embd));
     return HP_OK;   // combined in slot order by the norm that follows (norm_in)
 }
@@ -758,12 +760,6 @@ int Engine::prefill_attn(const LayerW& L, uint16_t* kc, uint16_t* vc, size_t kv_
     }
     return lin_parts(L.out_proj, R);
 }
-// the routed experts of a chunk, MAXR rows at a time: the pairs of 32 rows share the expert matrices they touch
-int Engine::prefill_moe(const LayerW& L, int R) {
-    const int PR = pf_rows_;
-    for (int r0 = 0; r0 < R; r0 += MAXR) HP_TRY(moe_rows(L, std::min((int)MAXR, R - r0), r0, pf_desc_, pf_desc_ + PR, pf_desc_ + 2 * PR, nullptr));
-    return HP_OK;
-}
 // Rows [pos0, pos0 + R) of a slot through the trunk (and the K/V rows of the MTP block), committed. tail > 0: the last chunk
 // of a prompt; the head, the hidden rows and the whole MTP block of its last `tail` rows (R - tail a multiple of 8) end up where a
 // pass over just these rows leaves them.
@@ -833,13 +829,15 @@ int Engine::prefill_reserve() {
     auto need = [&](const Lin& l) { if (l.N) planes = std::max(planes, (size_t)l.P * l.N); };
     for (const LayerW& L : layers_) { need(L.in_proj); need(L.out_proj); need(L.down); need(L.gate_up); }
     need(eh_proj_); need(mtp_.in_proj);
-    PassBuf b; float *hin = nullptr, *gdn = nullptr; void* pack = nullptr; int* desc = nullptr;
+    PassBuf b; float *hin = nullptr, *gdn = nullptr; void *pack = nullptr, *segs = nullptr; int* desc = nullptr; float* rlogits = nullptr; XQ8F xq2{nullptr, nullptr};
     std::vector<std::pair<void**, size_t>> at; size_t total = 0;
     auto part = [&](void** p, size_t bytes) { at.emplace_back(p, total); total += (bytes + 255) & ~(size_t)255; };
     part((void**)&b.x, (size_t)PR * E * 4); part((void**)&b.emb, (size_t)PR * E * 4); part((void**)&b.h, (size_t)PR * E * 4); part((void**)&hin, (size_t)PR * E * 4);
     part((void**)&b.big, (size_t)PR * bigw * 4); part((void**)&b.yparts, (size_t)PR * planes * 4);
     const size_t xq_at = total;
     part(&b.xq.q, xq_q_bytes(PR, (int)kmax)); part(&b.xq.sc, xq_sc_floats(PR, (int)kmax) * 4);
+    int* ticket = nullptr;
+    if (c.n_expert) part((void**)&ticket, (size_t)(PR + 7) / 8 * 4);
     const size_t xq_end = total;
     part(&pack, gemm_pack_bytes(PR, (int)kmax));
     if (ngdn()) part((void**)&gdn, gdn_prefill_floats(PR, nq, nv) * 4);
@@ -847,6 +845,7 @@ int Engine::prefill_reserve() {
     if (c.n_expert) {
         const size_t pairs = (size_t)PR * (c.n_expert_used + 1);
         part((void**)&b.xn, (size_t)PR * E * 4); part((void**)&b.moe_v, pairs * E * 4); part((void**)&b.moe_w, pairs * 4); part((void**)&b.moe_ids, pairs * 4);
+        part((void**)&rlogits, (size_t)PR * (c.n_expert + 1) * 4); part(&segs, moe_seg_bytes((int)pairs)); part(&xq2.q, xq_q_bytes((int)pairs, c.expert_ff)); part(&xq2.sc, xq_sc_floats((int)pairs, c.expert_ff) * 4);
     }
     struct Relaxed {   // another thread's capture must not see an allocation of this one
         cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
@@ -863,6 +862,7 @@ int Engine::prefill_reserve() {
     for (auto& [p, off] : at) *p = block + off;
     HP_CUDA(cudaMemsetAsync(block + xq_at, 0, xq_end - xq_at, s_));
     pf_ = b; pf_hin_ = hin; pf_gdn_ = gdn; pf_pack_ = pack; pf_desc_ = desc; pf_rows_ = PR;
+    pf_rlogits_ = rlogits; pf_ticket_ = ticket; pf_segs_ = segs; pf_xq2_ = xq2;
     return HP_OK;
 }
 // Prompt ingestion for one slot (Qwen4Exp::prefill + mtp_catchup, qwen4exp.h:57-60,72-74; Backend::prefill,

@@ -80,8 +80,7 @@ private:
     int prefill_rows(int slot, const int* tokens, int R, int pos0, int with_mtp, int tail);   // a prompt chunk through the GEMM path
     int prefill_attn(const LayerW& L, uint16_t* kc, uint16_t* vc, size_t kv_stride, int R, bool kv_only);
     int prefill_lin(const Lin& l, float* out, int ld, size_t part_stride, int R);
-    int prefill_moe(const LayerW& L, int R);
-    int moe_rows(const LayerW& L, int R, int row0, const int* tok, const int* pos, const int* slot, int* pushed);
+    int moe_rows(const LayerW& L, int R, const int* tok, const int* pos, const int* slot, int* pushed);
     int run_mtp(int R, int ngroups, const float* h_dev, int ldh, bool want_logits, bool kv_only = false);
     int upload_desc();
     int enqueue_round(int S, int n);
@@ -127,6 +126,7 @@ private:
     struct PrefillScope;
     struct PfBatch { int row0, rows, g0, ng; };                   // rows of a chunk that one attention launch takes
     int pf_rows_ = 0, pf_slot_ = 0; bool pf_on_ = false; float *pf_gdn_ = nullptr, *pf_hin_ = nullptr; void* pf_pack_ = nullptr; int *pf_desc_ = nullptr, *pf_hdesc_ = nullptr;
+    float* pf_rlogits_ = nullptr; int* pf_ticket_ = nullptr; void* pf_segs_ = nullptr; XQ8F pf_xq2_{nullptr, nullptr};   // routing and experts of more than MAXR rows
     std::vector<PfBatch> pf_batches_; int pf_nsplit_ = 0;
     void* topk_scratch_ = nullptr; int *d_topk_ids_ = nullptr; float* d_topk_vals_ = nullptr;
     uint16_t* prof_kv_ = nullptr;                                 // K/V rows saved around profile_pass

@@ -127,17 +127,18 @@ int attn_decode_seq(float* qkv, int ld, int R, int pos0, int n_head, int n_kv, i
 // ---- moe.cu ----
 // router (reference f32_gemv, fn.hip:252-277), routing (k_moe_route, fn.hip:167-205) and the grouping of the (row, slot)
 // pairs by expert, in one launch
-constexpr int MOE_MAX_PAIRS = 32 * 16;
+constexpr int MOE_MAX_PAIRS = 32 * 16, MOE_MAX_ROWS = 512;   // (row, slot) pairs of a pass, rows of a prompt chunk
 struct MoeRouteParams {
     const float* W; const float* x; float* logits; int E, K, k, T;   // router [E + 1][K] f32, rows x [T][K], logits [T][E + 1]
     int* ids; float* w;                                               // [T][k + 1]: expert ids (-1 = shared) and combine weights
-    int* ticket;                                                      // five zero-initialised ints (left zero)
+    int* ticket;                                                      // five zero-initialised ints (left zero); (T + 7) / 8 for more than 32 rows
     const int* row_tok = nullptr; const int* row_pos = nullptr; const int* row_slot = nullptr; unsigned long long synth_key = 0;   // synth_key != 0: seeded N(0,1) expert logits per (slot, token, position)
     int e_lo = 0, e_hi = 0, own_shared = 1;                           // experts this GPU owns
     void* segs = nullptr; int* ctl = nullptr; unsigned long long* touched = nullptr;   // grouping outputs (segs == nullptr: no grouping)
     int* err = nullptr;                                               // device status word (bounded waits)
 };
-int moe_route_group(const MoeRouteParams& p, cudaStream_t s);
+int moe_route_group(const MoeRouteParams& p, cudaStream_t s);   // up to 32 rows; without segs up to MOE_MAX_ROWS
+int moe_group_rows(const MoeRouteParams& p, cudaStream_t s);    // the grouping of up to MOE_MAX_ROWS routed rows (ids): segs, ctl, touched
 // Routed experts grouped by expert (see moe.cu). Expert tensors tile-major: gate|up repacked with interleave_half = F.
 struct MoeGroupParams {
     const void* w_gate_up; const void* w_down; const void* sh_gate_up; const void* sh_down;   // this GPU's experts [e_lo, e_hi) and the shared expert
@@ -145,7 +146,7 @@ struct MoeGroupParams {
     int e_lo;                                           // first routed expert this GPU holds (its tensors start there)
     XQ8F xq, xq2;                                       // quantised rows [T] (K = E) in; quantised silu(gate)*up per pair [T * nslot] (K = F) scratch
     float* v;                                           // per-pair outputs [T * nslot][E] (pairs of experts owned elsewhere are not written)
-    void* segs; int* ctl;                               // filled by moe_route_group: MOE_MAX_PAIRS segments of 64 bytes, 4 control ints
+    void* segs; int* ctl;                               // filled by moe_route_group or moe_group_rows: T * nslot segments of 64 bytes at most, 4 control ints
     int* err;
     // Expert parallelism over peer memory (ep_world > 1, optional): the down projection also stores every output it
     // computes into the other ranks' exchange buffers (half (n & 1) of it for exchange number n) and, when the whole grid
@@ -153,7 +154,7 @@ struct MoeGroupParams {
     // [8] = exchanges this rank has completed, [9] = ticket.
     int ep_world = 1, ep_rank = 0; float* ep_x[8] = {}; unsigned* ep_ctl[8] = {}; size_t ep_half = 0;
 };
-size_t moe_seg_bytes();
+size_t moe_seg_bytes(int pairs = MOE_MAX_PAIRS);
 // *pushed (nullable): set to 1 when the down projection delivered its outputs to the peers itself (the quad form), 0 when the
 // caller has to send them
 int moe_experts_grouped(const MoeGroupParams& p, cudaStream_t s, int* pushed = nullptr);   // reference gemv_moe + moe_silu_quant + gemv_moe_down (gemv.h:43-50, fn.hip:206-211)

@@ -46,6 +46,13 @@ def test_prefill_on_both_sides_of_the_gemm_line(n):
     test_prefill_chunks_bit_exact_vs_oracle("tiny", n, {})
 
 
+# experts grouped over a whole chunk: one row beyond a pass, segments that are full and not, a full chunk and a short one behind it, the
+# shared expert behind 1024 others (a bucket of its own beyond the threads of the scan)
+@pytest.mark.parametrize("n,over", [(40, dict(n_expert=1024)), (128, {}), (300, dict(synth_router_logits=1)), (515, dict(max_ctx=640, synth_router_logits=1))])
+def test_prefill_groups_the_experts_of_a_chunk(n, over):
+    test_prefill_chunks_bit_exact_vs_oracle("tiny-moe", n, {"max_ctx": 320, **over})
+
+
 @pytest.mark.parametrize("n", [17, 42])
 def test_prefill_chunks_fill_the_draft_block(n):
     cfg = hb.ModelCfg.preset("tiny", max_ctx=128)
