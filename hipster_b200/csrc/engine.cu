@@ -816,7 +816,7 @@ int Engine::prefill_rows(int slot, const int* tokens, int R, int pos0, int with_
     HP_CUDA(cudaEventElapsedTime(&last_ms_, ev0_, ev1_));
     return check_device_status();
 }
-// Buffers of the prompt chunks (243 MB for the 27B shape), one block that the first prompt of more than 8 tokens takes and the
+// Buffers of the prompt chunks (254 MB for the 27B shape), one block that the first prompt of more than 8 tokens takes and the
 // engine keeps: a model loads with what its passes need. They stay out, and prompts run as 8-row passes with the same results,
 // unless the device has twice their size free: what the caller and the captured rounds still allocate must not fail for
 // the sake of a faster prompt.
@@ -871,7 +871,7 @@ int Engine::prefill_reserve() {
 // otherwise), so that the draft block's KV cache covers the prompt (spec27b.cpp:62-71). Afterwards row 0 of logits /
 // h_nextn / the arg-max ids holds the LAST prompt row.
 // More than 8 tokens run as chunks (prefill_rows): 301 tokens of the 27B shape took 251 ms as 38 verify passes of 8 rows,
-// each of which streams all weights, and take 85 ms as one chunk.
+// each of which streams all weights, and take 75 ms as one chunk.
 int Engine::prefill(int slot, const int* tokens, int n, int pos0, int with_mtp) {
     HP_REQUIRE(slot >= 0 && slot < c_.n_slots && tokens && n >= 1 && pos0 >= 0 && pos0 + n <= c_.max_ctx, "prefill: bad arguments (slot %d, n %d, pos0 %d)", slot, n, pos0);
     HP_REQUIRE(!with_mtp || c_.has_mtp, "model has no MTP block");

@@ -496,7 +496,8 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 1) k_moe_gemv_grouped(MoeGArgs
 // barriers. Per output element the arithmetic is unchanged: one warp, blocks in order along K, no split.
 // Bound by the latency of a warp's serial chain (24 rows, three quads with rings of 3 stages: DRAM 45 and 41 %, issue 54 and 49 %): four quads
 // with rings of 2 hold fewer bytes per warp and as many per SM, and segments of up to 4 columns take fewer instructions: DRAM 48 and 42 %,
-// issue 42 and 34 %, one layer of 24 rows 114 us instead of 125.
+// issue 42 and 34 %, one layer of 24 rows 114 us instead of 125. (With the down projection's rings primed under gate|up and the routing below
+// 110. Five and six quads, or rings of one-block stages: 111 to 119 us against 111 in one run.)
 constexpr int MQ_WARPS = 16, MQ_QUADS = 4, MQ_AUX = 2048;   // bytes after the rings: barriers + the quads' exchange words
 __device__ __forceinline__ void quad_barrier(int quad) { asm volatile("bar.sync %0, 128;" ::"r"(quad + 1) : "memory"); }
 template <int MODE, int SB, int DEPTH>
