@@ -373,14 +373,9 @@ static int lin_class_bit(const Lin& l, const hp_model_cfg& c) {
     return l.N == 2 * c.n_ff ? 16 : l.K == c.n_ff ? 32 : l.N == c.n_vocab ? 64 : l.K == c.n_embd ? 128 : 256;
 }
 // A linear over the rows of a prompt chunk; both kernels give the same bits. The GEMV streams the weights once per 32 rows, large matrices
-// whose activations do not fit once per 16. One line for all projections, where their sum over a 27B layer turns. GEMV against GEMM (us),
-// GDN in-, out-projection, gate|up and down: 32 rows 35 + 17 + 65 + 30 = 146 against 36 + 26 + 68 + 58 = 187; 40 rows 47 + 24 + 87 + 44 =
-// 202 against 44 + 31 + 86 + 73 = 233; 48 rows 51 + 27 + 95 + 49 = 222 against 44 + 31 + 86 + 73 = 234; 64 rows 67 + 33 + 125 + 59 = 284
-// against 54 + 36 + 104 + 85 = 279. Single projections turn elsewhere: in-projection and gate|up below 40 rows, the out-projection between 64
-// and 96, down between 96 and 128. Of the 2048-wide model the GDN in-projection turns at 40 (64 rows 29 and 26), the attention one beyond 96
-// (64 rows 23 and 33), the out-projection between 96 and 128 (64 rows 22 and 35): its chunks of 49 to 80 rows lose some 10 us a layer.
+// whose activations do not fit once per 16: it is the faster one for few rows, and for the longer the more parts K is cut into.
 int Engine::prefill_lin(const Lin& l, float* out, int ld, size_t part_stride, int R) {
-    if (R > 48) return gemm_q4k_q8_parts(l.wt, xq_, out, l.N, l.K, R, ld, part_stride, pf_pack_, err_, s_, pdl_);
+    if (gemm_pays(l.N, l.K, R)) return gemm_q4k_q8_parts(l.wt, xq_, out, l.N, l.K, R, ld, part_stride, pf_pack_, err_, s_, pdl_);
     for (int r0 = 0; r0 < R; r0 += 32)
         HP_TRY(gemv_q4k_q8_parts(l.wt, xq_rows(xq_, r0, l.K), out + (size_t)r0 * ld, l.N, l.K, std::min(32, R - r0), ld, part_stride, err_, s_, pdl_, true));
     return HP_OK;

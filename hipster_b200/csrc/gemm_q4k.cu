@@ -541,19 +541,39 @@ static int tc_narrow(int R, int ntc) {
 // and 83 us (ntc + 8, from 10 on ntc + 11: half as many sub-blocks per TMEM slot), 1.25 of these units less for a narrow range, four fifths
 // with G = 4. Over eight projections and 18 row counts from 56 to 512 that is 0.4 % slower than the best cut on average, 6 % at most (with ntc + 6,
 // narrow ranges 2 less, 1.0 and 15 %).
-void gemm_cut(int N, int K, int R, int* ntc, int* G) {
+struct TcCost { long items, cost; };   // of the fullest CTA: items, and quarters of the units above x (5 or 4)
+static TcCost tc_cost(int N, int K, int R, int c, int g) {
     const int t8 = (R + 7) / 8, tiles = (N + 15) / 16, P = gemv_num_parts(N, K / 256);
+    // CTAs with one item more and the others: their items, and at most how many wide ones among these (see tc_item)
+    const long ncg = (t8 + c - 1) / c, per = (long)P * ((tiles + g - 1) / g), nl = (ncg - tc_narrow(R, c)) * per, items = ncg * per;
+    const long n = items < GEMV_NCTA ? items : GEMV_NCTA, full = items / n, heavy = items % n, light = n - heavy, over = nl - full * light;
+    const long wl = (nl + light - 1) / light, wh = heavy && over > 0 ? (over + heavy - 1) / heavy : 0;
+    const long u = 4 * (c + (c > 8 ? 11 : 8)) - 5, cl = full * u + 5 * (wl < full ? wl : full), ch = heavy ? (full + 1) * u + 5 * wh : 0;
+    return {full + (heavy ? 1 : 0), (cl > ch ? cl : ch) * (g == 8 ? 5 : 4)};
+}
+void gemm_cut(int N, int K, int R, int* ntc, int* G) {
     long best = 0; *ntc = 0;
     for (int c = 4; c <= 16; c += 2)
         for (int g = 8; g >= 4; g -= 4) {
-            // CTAs with one item more and the others: their items, and at most how many wide ones among these (see tc_item)
-            const long ncg = (t8 + c - 1) / c, per = (long)P * ((tiles + g - 1) / g), nl = (ncg - tc_narrow(R, c)) * per, items = ncg * per;
-            const long n = items < GEMV_NCTA ? items : GEMV_NCTA, full = items / n, heavy = items % n, light = n - heavy, over = nl - full * light;
-            const long wl = (nl + light - 1) / light, wh = heavy && over > 0 ? (over + heavy - 1) / heavy : 0;
-            const long u = 4 * (c + (c > 8 ? 11 : 8)) - 5, cl = full * u + 5 * (wl < full ? wl : full), ch = heavy ? (full + 1) * u + 5 * wh : 0;
-            const long cost = (cl > ch ? cl : ch) * (g == 8 ? 5 : 4);
+            const long cost = tc_cost(N, K, R, c, g).cost;
             if (!*ntc || cost < best) { best = cost; *ntc = c; *G = g; }
         }
+}
+// The GEMM against the GEMV in launches of 32 rows, in us. A GEMV launch: 1.2, 0.24 per block of a K part (staging) and 0.52 per block and column
+// tile of its fullest warp; the GEMM: 5.2, 1.9 per item of the fullest CTA and the cost above, and 2 for its second launch, which nothing
+// hides in a prompt (up to 48 rows that decides it: 44 rows of the 27B shape 17.3 and 17.7 ms). Over ten projections and 21 row counts from 33
+// to 192, one by one, the choice is 1.2 % slower than the faster of the two on average, 22 % at most (one line at 48 rows for all projections: 7 and
+// 97 %). 56 rows, 5120 x 17408: 55 us instead of 86; 64 rows, 14336 x 2048: 23 instead of 32. Prompts (ms), one line and this rule: 27B shape, 52 tokens
+// 22.1 and 19.9, 84 tokens 30.7 and 28.0, 130 tokens 44.3 and 42.8; 2048-wide mixture of experts, 60 tokens 13.9 and 13.2.
+bool gemm_pays(int N, int K, int R) {
+    const int tiles = (N + 15) / 16, P = gemv_num_parts(N, K / 256);
+    if (R <= 48 || P <= 0) return false;
+    const int nbp = K / 256 / P, cb = nbp % 2 == 0 ? 2 : 1, gc = GEMV_NCTA / P, cu = (tiles + gc - 1) / gc * (nbp / cb), per_warp = (cu + GEMV_WARPS - 1) / GEMV_WARPS * cb;
+    double gemv = 0;
+    for (int r0 = 0; r0 < R; r0 += 32) gemv += 1.2 + 0.242 * nbp + 0.5165 * per_warp * (((R - r0 < 32 ? R - r0 : 32) + 7) / 8);
+    int c, g; gemm_cut(N, K, R, &c, &g);
+    const TcCost t = tc_cost(N, K, R, c, g);
+    return 0.96 * (7.2 + 1.91 * t.items + 0.00712 * t.cost * nbp) < gemv;
 }
 int gemm_q4k_q8_cut(const void* Wt, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, void* pack, int* err, cudaStream_t s, bool pdl, int ntc, int G) {
     HP_REQUIRE(K > 0 && K % 256 == 0, "gemm_q4k_q8: K=%d must be a positive multiple of 256", K);

@@ -57,6 +57,7 @@ size_t gemv_tiled_bytes(size_t N, int K);
 // gemm_pack_bytes(R, K) bytes, 16-byte aligned
 int gemm_q4k_q8_parts(const void* Wt, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, void* pack, int* err, cudaStream_t s, bool pdl);
 size_t gemm_pack_bytes(int R, int K);
+bool gemm_pays(int N, int K, int R);   // the GEMM is faster than the GEMV in launches of 32 rows
 void gemm_cut(int N, int K, int R, int* ntc, int* G);   // the cut that gemm_q4k_q8_parts takes; _cut: the same call with a given one (ntc = 4, 6 .. 16, G = 8 or 4)
 int gemm_q4k_q8_cut(const void* Wt, const XQ8F& x, float* yparts, int N, int K, int R, int ldy, size_t part_stride, void* pack, int* err, cudaStream_t s, bool pdl, int ntc, int G);
 // interleave_half = F > 0: src is a stack of [gate F rows | up F rows] matrices; gate and up rows of a feature share a tile

@@ -1,5 +1,5 @@
 """hp_prefill over more than one 8-row pass (the chunked GEMM path) against the CPU oracle's 8-row passes, bit for bit: sizes
-around the edges of its row tiles (8), of the GEMV / GEMM rule (32) and of a chunk (512), one and several attention batches per
+around the edges of its row tiles (8), of the GEMV / GEMM rule and of a chunk (512), one and several attention batches per
 chunk and several chunks per prompt; the tail rows, the draft block's cache and hidden rows, the recurrent state (through the
 pass that follows) and pending accepts. (The GEMM's column ranges: test_gemm_gpu.py.)"""
 import numpy as np
@@ -51,6 +51,11 @@ def test_prefill_on_both_sides_of_the_gemm_line(n):
 @pytest.mark.parametrize("n,over", [(40, dict(n_expert=1024)), (128, {}), (300, dict(synth_router_logits=1)), (515, dict(max_ctx=640, synth_router_logits=1))])
 def test_prefill_groups_the_experts_of_a_chunk(n, over):
     test_prefill_chunks_bit_exact_vs_oracle("tiny-moe", n, {"max_ctx": 320, **over})
+
+
+@pytest.mark.parametrize("n", [56, 57, 88, 104, 160])   # all projections in the GEMV, some of them, all in the GEMM
+def test_prefill_around_the_lines_of_its_projections(n):
+    test_prefill_chunks_bit_exact_vs_oracle("tiny", n, dict(max_ctx=192))
 
 
 @pytest.mark.parametrize("n", [17, 42])
