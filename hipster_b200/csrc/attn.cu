@@ -311,6 +311,7 @@ __global__ void __launch_bounds__(256) k_attn_merge(const float* __restrict__ qk
         for (int s = 0; s < n; s += PF) {
 #pragma unroll
             for (int i = 0; i < PF; ++i) {
+                if (i % 4 == 0 && s + i >= n) break;   // nothing left to read ahead either (6 rows at position 500: a layer 31.2 -> 30.0 us)
                 if (s + i < n) { o = fmaf(sw[s + i], pv[i], o); l = fmaf(sw[s + i], sl[s + i], l); }
                 pv[i] = s0 + s + PF + i < nsplit ? po[(size_t)(s0 + s + PF + i) * MAXP * HD] : 0.f;
             }
