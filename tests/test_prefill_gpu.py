@@ -41,7 +41,7 @@ def test_prefill_chunks_bit_exact_vs_oracle(preset, n, over):
     eng.close()
 
 
-@pytest.mark.parametrize("n", [32, 40, 48, 49])   # projections in one and two GEMV launches, and in the GEMM
+@pytest.mark.parametrize("n", [32, 40, 48, 49])   # projections in one and two GEMV launches, and beyond the rows that always take it
 def test_prefill_on_both_sides_of_the_gemm_line(n):
     test_prefill_chunks_bit_exact_vs_oracle("tiny", n, {})
 
