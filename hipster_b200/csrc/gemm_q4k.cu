@@ -8,7 +8,8 @@
 //
 // The dots come as fp32: a nibble q, read as e4m3, is q / 512 (subnormal up to 7), an int8 activation is 16 a + b with |a|, |b| <= 8, both
 // exact in e4m3, and the two products accumulate exactly (at most 16 significant bits). The accumulator holds idot / 512 and the row scales
-// carry the 512. (kind::i8 took one MMA instead of two, but each dot cost a conversion in the update: 34816 x 5120 at 512 rows 692 us, now 611.)
+// carry the 512 (see tc_plain). (kind::i8 took one MMA instead of two, but each dot cost a conversion in the update: 34816 x 5120 at 512 rows 692 us,
+// now 609.)
 //
 // What bounds it: the fp32 update, three packed instructions per two outputs and sub-block (12 clocks of an SM sub-partition per 16x8x32
 // tile), which hardly overlaps with what brings its operands into registers: TMEM loads (16x256b fills 64 bytes a clock) and column
@@ -136,10 +137,18 @@ __device__ __forceinline__ uint64_t tc_cuts(int N, int nb, int P, int tile, int 
     return m;
 }
 
+// The one rounding in front of the fmaf is that of the product (d * sc) * xd, of d / 16 where the GEMV leaves the high nibbles shifted. With xd of this
+// range it is no subnormal number (f16 d: d / 16 is 2^-28 at least) and 512 times (d * sc) * xd no infinity (d * sc is less than 2^22), so the row
+// scales may carry the 512. A launch with other scales (heads whose gates underflow have them; NaN) takes the GEMV's own product, one packed
+// multiplication more per two outputs: in a prompt of the 27B shape two launches of 192, 301 tokens 75.0 -> 75.15 ms. (Left to the tensor core, which
+// then repeats its products up to the GEMV's dot, such a launch takes three to eight times as long.)
+__device__ __forceinline__ bool tc_plain(float xd) { return xd == 0.f || (xd >= 0x1p-98f && xd <= 0x1p96f); }
+
 // One step of an update warp: its W column tiles over GB sub-blocks (row scales 128 float2 apart, one 64-byte group of
-// activation scales per sub-block). H1: the quadrant's second tile exists.
-template <int W, int GB, bool H1>
-__device__ __forceinline__ void tc_update(float2 (&acc)[4][W], uint32_t ta, uint32_t sb_cols, const float4* xs, const float2* rs) {
+// activation scales per sub-block). H1: the quadrant's second tile exists. EXACT: the scale and the dot of the GEMV, d * sc and idot, or (odd
+// sub-block) d / 16 * sc and 16 idot, GB = 1.
+template <int W, int GB, bool H1, bool EXACT>
+__device__ __forceinline__ void tc_update(float2 (&acc)[4][W], uint32_t ta, uint32_t sb_cols, const float4* xs, const float2* rs, bool odd) {
     uint32_t v0[GB][W * 4], v1[H1 ? GB : 1][W * 4];
 #pragma unroll
     for (int b = 0; b < GB; ++b) {
@@ -157,14 +166,22 @@ __device__ __forceinline__ void tc_update(float2 (&acc)[4][W], uint32_t ta, uint
     auto xat = [&](int j) { return xs[(j % W) * 32 + (j / W) * 4]; };
     float4 xb[XA];
 #pragma unroll
-    for (int j = 0; j < XA; ++j) if (W <= 4) xb[j] = xat(j);
+    for (int j = 0; j < XA; ++j) if (W <= 4 && j < NX) xb[j] = xat(j);
     tc_wait_ld();
 #pragma unroll
     for (int b = 0; b < GB; ++b)
 #pragma unroll
         for (int i = 0; i < W * 4; ++i) { tc_after_wait(v0[b][i]); if constexpr (H1) tc_after_wait(v1[b][i]); }
+    const float f = odd ? 8192.f : 512.f;
+    if constexpr (EXACT) {
+        static_assert(GB == 1, "one parity");
+#pragma unroll
+        for (int i = 0; i < (H1 ? 4 : 2); ++i) r[0][i].x *= odd ? 1.f / 8192.f : 1.f / 512.f;
+    }
     auto upd = [&](float2& a, float2 sc, float4 xv, uint32_t i0, uint32_t i1) {
-        fma2(a, mul2(make_float2(sc.x, sc.x), make_float2(xv.x, xv.y)), make_float2(__uint_as_float(i0), __uint_as_float(i1)));
+        float2 dot = make_float2(__uint_as_float(i0), __uint_as_float(i1));
+        if constexpr (EXACT) dot = mul2(dot, make_float2(f, f));
+        fma2(a, mul2(make_float2(sc.x, sc.x), make_float2(xv.x, xv.y)), dot);
         fma2(a, make_float2(sc.y, sc.y), make_float2(xv.z, xv.w));
     };
 #pragma unroll
@@ -360,8 +377,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
         pdl_wait();
         int k = 0, gr = 0; bool ok = true;
         const int cb1 = nbp % 2 == 0 ? 1 : 0;   // blocks per unit of the GEMV's partition, less 1
-        auto item = [&](const TcItem im, auto wt) {
-            constexpr int W = decltype(wt)::value, GB = W <= 2 ? 4 : W <= 4 ? 2 : 1;   // column tiles of this warp, sub-blocks per step
+        auto item = [&](const TcItem im, auto wt, auto exact) {
+            constexpr bool EXACT = decltype(exact)::value;
+            constexpr int W = decltype(wt)::value, GB = EXACT ? 1 : W <= 2 ? 4 : W <= 4 ? 2 : 1;   // column tiles of this warp, sub-blocks per step
             const int grp = im.rest % a.ngrp, part = im.rest / a.ngrp, tile0 = grp * G, tend = min(tiles, tile0 + G), n0 = (warp >> 2) * W;
             const int tl[2] = {tile0 + (G == 8 ? 2 * q : q), G == 8 ? tile0 + 2 * q + 1 : tiles};
             const bool has0 = tl[0] < tend, has1 = tl[1] < tend;
@@ -392,8 +410,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
                         for (int v = 0; v < GS; v += GB) {
                             const int sb = u * GS + v;
                             const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + slot * Geo::SLOT + v * Geo::N + n0 * 8;
-                            if (has1) tc_update<W, GB, true>(acc, ta, Geo::N, xsp + sb * 4, rsp + sb * 128);
-                            else tc_update<W, GB, false>(acc, ta, Geo::N, xsp + sb * 4, rsp + sb * 128);
+                            if (has1) tc_update<W, GB, true, EXACT>(acc, ta, Geo::N, xsp + sb * 4, rsp + sb * 128, sb & 1);
+                            else tc_update<W, GB, false, EXACT>(acc, ta, Geo::N, xsp + sb * 4, rsp + sb * 128, sb & 1);
                         }
                     }
                     tc_fence_before();
@@ -464,10 +482,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
                 }
             }
         };
-        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
-            const TcItem im = tc_item(a, it, NTC);
-            if (im.narrow) item(im, std::integral_constant<int, NTC / 2 - 1>()); else item(im, std::integral_constant<int, NTC / 2>());
+        auto all_items = [&](auto exact) {
+            for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+                const TcItem im = tc_item(a, it, NTC);
+                if (im.narrow) item(im, std::integral_constant<int, NTC / 2 - 1>(), exact); else item(im, std::integral_constant<int, NTC / 2>(), exact);
+            }
+        };
+        const int* flags = reinterpret_cast<const int*>(a.xp + (size_t)a.ncg * nb * Geo::PACK);   // of k_tc_pack; read at once, while the first slots fill
+        int other = 0;
+        for (int i0 = lane; i0 < a.ncg * nb; i0 += 256) {
+#pragma unroll
+            for (int i = 0; i < 256; i += 32) other |= i0 + i < a.ncg * nb ? __ldcg(flags + i0 + i) : 0;
         }
+        if (__any_sync(0xffffffffu, other)) all_items(std::true_type()); else all_items(std::false_type());
     }
     tc_fence_before();
     __syncthreads();
@@ -486,7 +513,8 @@ __device__ __forceinline__ void tc_split(uint32_t x, uint32_t& hi, uint32_t& lo)
     }
 }
 // Activations in the order the GEMM copies them: per column range of NTC tiles and block two half-blocks (per 64-element
-// group the swizzled K-major tile of all columns), then the scales. Tiles beyond the range and the rows are zero.
+// group the swizzled K-major tile of all columns), then the scales. Tiles beyond the range and the rows are zero. Behind all of them an int per
+// range and block: whether one of its scales is beyond tc_plain.
 template <int NTC>
 __global__ void __launch_bounds__(256) k_tc_pack(const uint4* __restrict__ xq, const float4* __restrict__ xsc, uint8_t* __restrict__ xp, int nb, int tiles8, int nlong) {
     pdl_launch_dependents();
@@ -506,10 +534,15 @@ __global__ void __launch_bounds__(256) k_tc_pack(const uint4* __restrict__ xq, c
         tc_split(v.z, h.x, l.x); tc_split(v.w, h.y, l.y);
         *reinterpret_cast<uint2*>(p + (lo ^ 32)) = h; *reinterpret_cast<uint2*>(p + NTC * 512 + (lo ^ 32)) = l;
     }
+    bool other = false;
     for (int n = warp; n < NTC; n += 8) {
         const int nt = c0 + n;
-        reinterpret_cast<float4*>(d + 2 * TcGeom<NTC>::B_BYTES)[n * 32 + lane] = nt < cend ? xsc[((size_t)nt * nb + blk) * 32 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 v = nt < cend ? xsc[((size_t)nt * nb + blk) * 32 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        other |= !tc_plain(v.x) || !tc_plain(v.y);
+        reinterpret_cast<float4*>(d + 2 * TcGeom<NTC>::B_BYTES)[n * 32 + lane] = v;
     }
+    other = __syncthreads_or(other);
+    if (threadIdx.x == 0) reinterpret_cast<int*>(xp + (size_t)gridDim.y * nb * TcGeom<NTC>::PACK)[cg * nb + blk] = other;
 }
 
 template <int NTC>
@@ -530,7 +563,7 @@ int launch_tc(const TcArgs& a, const XQ8F& x, int grid, cudaStream_t s, bool pdl
 
 }  // namespace
 
-size_t gemm_pack_bytes(int R, int K) { return (size_t)((R + 7) / 8 + 15) * (size_t)(K / 256) * 4608; }
+size_t gemm_pack_bytes(int R, int K) { return (size_t)((R + 7) / 8 + 15) * (size_t)(K / 256) * (4608 + 4); }
 // A cut into ranges of ntc column tiles leaves up to ntc - 1 empty: the number of ranges, not the first, that get two tiles less instead.
 static int tc_narrow(int R, int ntc) {
     const int t8 = (R + 7) / 8, ncg = (t8 + ntc - 1) / ntc, k = (ncg * ntc - t8) / 2;

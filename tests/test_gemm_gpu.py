@@ -98,6 +98,29 @@ def test_narrow_ranges_give_the_bits_of_the_gemv(weights, ntc, G):
             assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (N, K, R)
 
 
+# rows from the smallest to the largest of fp32, scales of the weights from subnormal ones up: products of the scales that are subnormal, and dots
+# of few nibbles beside products that leave no factor of 512 to the largest number
+@pytest.mark.gpu
+@pytest.mark.parametrize("ntc,G", CUTS)
+def test_rows_at_the_ends_of_the_range_give_the_bits_of_the_gemv(ntc, G):
+    N, K, R = 400, 768, 8 * ntc + 5
+    g = torch.Generator(device="cuda").manual_seed(ntc)
+    blk = torch.randint(0, 256, (N, K // 256, 144), dtype=torch.uint8, device="cuda", generator=g)
+    blk[N // 2:, :, 16:] *= (torch.rand((N - N // 2, K // 256, 128), device="cuda", generator=g) < 1 / 64).to(torch.uint8)
+    d = torch.randn((N, K // 256, 2), device="cuda", generator=g).mul_(0.01).abs_()
+    d[::3] *= 2.0 ** -12                                          # subnormal f16
+    d[N // 2:, :, 1] = 0
+    blk[..., :4] = d.half().view(torch.uint8)
+    wt = K_.repack_tiled(blk.reshape(-1), N, K, 0)
+    e = torch.linspace(-140, 125, R, device="cuda").round().double()
+    x = (torch.randn((R, K), device="cuda", generator=g).clamp_(-3.9, 3.9).double() * 2.0 ** e[:, None]).float()
+    xq = K_.quantize_x_q8(x); err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got, want = run_gemm(wt, xq, N, K, R, N, (ntc, G), err), run_gemv(wt, xq, N, K, R, N, err)
+    assert err.item() == 0 and torch.isfinite(want).float().mean() > 0.95
+    same = (got.view(torch.int32) == want.view(torch.int32)) | (torch.isnan(got) & torch.isnan(want))
+    assert same.all(), e[(~same).nonzero()[:, 1].unique()].tolist()
+
+
 # the tile-major form of the GEMV on both sides of its row limits (4 rows; three column tiles whose activations leave room for one-block
 # stages only: 20 blocks), against the row-major one
 @pytest.mark.gpu
