@@ -8,8 +8,9 @@ LIB_PATH = os.environ.get("HIPSTER_B200_LIB") or os.path.join(HERE, "libhipster_
 HEADER = os.path.join(HERE, "..", "include", "hipster_b200.h")
 
 _lib = _hot = None
-# the calls whose latency counts go through csrc/pycalls.c, bound to the library that is loaded here
-_HOT = ("hp_quantize_x_q8", "hp_gemv_q4k_q8", "hp_argmax", "hp_accept_greedy", "hp_attn_decode")
+# the calls whose latency counts, with their argument types (p pointer, i int, f float), so that integers pass without a wrapper object
+_TYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "f": ctypes.c_float}
+_HOT = {"hp_quantize_x_q8": "piiippp", "hp_gemv_q4k_q8": "ppppiiiip", "hp_argmax": "piiipppp", "hp_accept_greedy": "ppipp", "hp_attn_decode": "piiiiiipppppipppfpp"}
 
 
 class HipsterError(RuntimeError):
@@ -40,17 +41,22 @@ def lib():
 
 
 def hot():
-    """The calls of _HOT with integers (None: absent) for every argument, without ctypes in between."""
+    """The calls of _HOT with integers (None: absent) for every argument. They go through csrc/pycalls.c, bound to the library that is loaded here;
+    where that module is not there (a package with the library alone, another interpreter than the one it was built for), through ctypes, a
+    microsecond slower each, on function objects of this package's own: those of lib() take whatever ctypes objects a caller passes."""
     global _hot
     if _hot is None:
         L = lib()
         try:
-            from . import _calls
-        except ImportError as e:
-            raise HipsterError(-1, f"{os.path.join(HERE, '_calls')} is missing: build it with `python -m hipster_b200.build` ({e})") from e
-        for name in _HOT:
-            _calls.bind(name, ctypes.cast(getattr(L, name), ctypes.c_void_p).value)
-        _hot = _calls
+            from . import _calls as calls
+        except ImportError:
+            calls = ctypes.CDLL(LIB_PATH)
+            for name, types in _HOT.items():
+                getattr(calls, name).argtypes = [_TYPES[t] for t in types]
+        else:
+            for name in _HOT:
+                calls.bind(name, ctypes.cast(getattr(L, name), ctypes.c_void_p).value)
+        _hot = calls
     return _hot
 
 

@@ -67,6 +67,51 @@ def test_package_imports_on_a_torch_build_without_cuda():
     assert r.returncode == 0 and int(r.stdout) >= 100, r.stderr[-2000:]
 
 
+@pytest.mark.parametrize("native", [True, False])
+def test_short_calls_work_with_and_without_the_native_entry_points(native):
+    """The library alone serves the five calls too, and both forms refuse the same arguments (subprocess: the form is chosen once)."""
+    code = ("import ctypes, sys\n"
+            f"if not {native}: sys.modules['hipster_b200._calls'] = None\n"             # as if it had not been built
+            "import hipster_b200 as hb\n"
+            "from hipster_b200 import _lib\n"
+            "H = _lib.hot(); L = hb.lib()\n"
+            f"assert (H.__class__ is not ctypes.CDLL) == {native}\n"
+            "def refused(f, *a):\n"
+            "    try: f(*a)\n"
+            "    except (TypeError, ctypes.ArgumentError): return True\n"
+            "    return False\n"
+            "for name, types in _lib._HOT.items():\n"
+            "    f = getattr(H, name); null = [None if t == 'p' else 1 for t in types]\n"
+            "    assert f(*null) == 1 and L.hp_last_error(), name\n"                     # refused by the library, before any CUDA call
+            "    assert f(*[v if v is None else 2 ** 32 + 1 for v in null[:-1]], None) == 1, name\n"   # integers wrap as in C
+            "    assert refused(f, *null[:-1]), name\n"
+            "    for i, t in enumerate(types):\n"
+            "        if t == 'i':\n"
+            "            assert refused(f, *null[:i], None, *null[i + 1:]) and refused(f, *null[:i], 1.0, *null[i + 1:]), (name, i)\n"
+            "        if t == 'p': assert refused(f, *null[:i], 1.0, *null[i + 1:]), (name, i)\n"
+            "        if t == 'f': assert refused(f, *null[:i], None, *null[i + 1:]), (name, i)\n"
+            f"if {native}:\n"
+            "    try: H.bind('hp_version', 1)\n"
+            "    except KeyError: print('ok')\n"
+            "else: print('ok')\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("missing", ["headers", "compiler"])
+def test_build_goes_on_without_the_native_entry_points(missing, monkeypatch, tmp_path, capfd):
+    from hipster_b200 import build
+    target = tmp_path / "_calls.so"
+    target.write_bytes(b"of another interpreter")                                         # must not stay behind either
+    monkeypatch.setattr(build, "CALLS", str(target))
+    if missing == "headers":
+        monkeypatch.setattr(build.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+    else:
+        monkeypatch.setattr(build.shutil, "which", lambda name: str(tmp_path / "no-such-compiler"))
+    assert build.build_calls(force=True) is None and not target.exists()
+    assert "ctypes" in capfd.readouterr().err
+
+
 def test_absent_tensors_are_refused_by_the_library(monkeypatch):
     monkeypatch.setattr(K_, "_raw_stream", lambda dev: 0); monkeypatch.setattr(K_, "_device", lambda: 0)   # refused before any CUDA call
     t = lambda *s: torch.zeros(s)  # noqa: E731
