@@ -9,7 +9,8 @@ from ._lib import lib, hot, check, ptr
 
 # The calls below are a few microseconds of device work, so what they spend in Python counts: the handle of the current stream
 # comes without a Stream object around it, the short calls go through native entry points that take addresses as integers (_lib.hot; to
-# a ctypes function an integer would pass as 32 bits, hence the wrapper of _stream), and sizes that depend on shapes alone are computed once.
+# a ctypes function an integer would pass as 32 bits, hence the wrapper of _stream), and sizes that depend on shapes alone are computed once (per
+# type of the numbers, too: a float or a numpy integer that equals an earlier size is still refused by the library's function).
 try:
     _raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
 except AttributeError:   # torch without CUDA: the package still imports, and a call raises torch's own error
@@ -20,17 +21,17 @@ def _stream():
     return ctypes.c_void_p(_raw_stream(_device()))
 
 
-@functools.lru_cache(maxsize=256)
+@functools.lru_cache(maxsize=256, typed=True)
 def _xq8_bytes(R, K):
     return lib().hp_xq8_q_bytes(R, K), lib().hp_xq8_sc_bytes(R, K)
 
 
-@functools.lru_cache(maxsize=256)
+@functools.lru_cache(maxsize=256, typed=True)
 def _argmax_scratch_bytes(R, n):
     return lib().hp_argmax_scratch_bytes(R, n)
 
 
-@functools.lru_cache(maxsize=256)
+@functools.lru_cache(maxsize=256, typed=True)
 def _attn_workspace_bytes(R, n_head, n_kv, max_ctx):
     return lib().hp_attn_workspace_bytes(R, n_head, n_kv, max_ctx)
 
@@ -124,7 +125,7 @@ def attn_decode(qkv, pos0, n_head, n_kv, n_rot, q_norm, k_norm, rope, kc, vc, ma
     q_norm / k_norm bf16 [256] (int16 tensors), rope f32 [max_ctx][n_rot/2][2], kc / vc f16 [n_kv][max_ctx][256] (updated).
     -> (out f32 [R][n_head*256], XQ8 of it or None). Reference: qk_norm_rope_kv + attn_decode_mq (ops.h:71-72,96)."""
     R, ld = qkv.shape[0], qkv.stride(0)
-    ws = torch.empty(_attn_workspace_bytes(R, n_head, n_kv, int(max_ctx)), dtype=torch.uint8, device=qkv.device)
+    ws = torch.empty(_attn_workspace_bytes(R, n_head, n_kv, max_ctx), dtype=torch.uint8, device=qkv.device)
     out = torch.empty((R, n_head * 256), dtype=torch.float32, device=qkv.device)
     xq = XQ8(R, n_head * 256, qkv.device) if want_q8 else None
     check(hot().hp_attn_decode(qkv.data_ptr(), ld, R, int(pos0), n_head, n_kv, n_rot, None if q_norm is None else q_norm.data_ptr(),

@@ -123,6 +123,19 @@ def test_absent_tensors_are_refused_by_the_library(monkeypatch):
             K_.attn_decode(t(1, 2 * 512 + 512), 0, 2, 1, 64, max_ctx=128, **{**args, name: None})
 
 
+def test_sizes_that_were_asked_before_refuse_what_the_library_refuses(monkeypatch):
+    """A number of another type is equal to the one that a size was computed for: it must not find that size."""
+    monkeypatch.setattr(K_, "_raw_stream", lambda dev: 0); monkeypatch.setattr(K_, "_device", lambda: 0)
+    monkeypatch.setattr(K_, "hot", lambda: type("Lib", (), {n: staticmethod(lambda *a: 0) for n in ("hp_argmax", "hp_attn_decode")}))
+    t = torch.zeros(1, 2 * 512 + 512); x = torch.zeros((2, 512))
+    attn = lambda ctx: K_.attn_decode(t, 0, 2, 1, 64, t, t, t, t, t, ctx)  # noqa: E731
+    K_.XQ8(2, 512, "cpu"); K_.argmax(x, 512); attn(128)
+    for other in (float, np.int64):
+        for call in (lambda: K_.XQ8(other(2), 512, "cpu"), lambda: K_.XQ8(2, other(512), "cpu"), lambda: K_.argmax(x, other(512)), lambda: attn(other(128))):
+            with pytest.raises(ctypes.ArgumentError):
+                call()
+
+
 def test_library_functions_take_any_ctypes_object():
     null = ctypes.c_size_t(0)   # an address as a size_t or an int64, as callers with their own bindings pass it
     L = hb.lib()
