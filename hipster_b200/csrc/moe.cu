@@ -272,10 +272,9 @@ struct GroupArgs { const int* ids; int T, ns, e_lo, e_hi, own_shared; MoeSeg* se
 constexpr int GR_THREADS = 1024, GR_PAIRS = 8;   // pairs per thread at most: 512 rows of 16 slots
 __global__ void __launch_bounds__(GR_THREADS) k_moe_group(GroupArgs a) {
     pdl_launch_dependents();
-    __shared__ int scnt[1025], soff[1025], swt[32], s_touched; __shared__ unsigned sbat[1025];   // per bucket: pairs, first segment, batches of 32 rows
+    __shared__ int scnt[1025], soff[1025], swt[32];   // per bucket: pairs, first segment; segments of the warps' buckets
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nown = a.e_hi - a.e_lo, nb = nown + (a.own_shared ? 1 : 0), np = a.T * a.ns;
-    for (int b = tid; b < 1025; b += GR_THREADS) { scnt[b] = 0; sbat[b] = 0u; }
-    if (tid == 0) s_touched = 0;
+    for (int b = tid; b < 1025; b += GR_THREADS) scnt[b] = 0;
     pdl_wait();
     __syncthreads();
     int my_b[GR_PAIRS], my_rank[GR_PAIRS];
@@ -289,7 +288,6 @@ __global__ void __launch_bounds__(GR_THREADS) k_moe_group(GroupArgs a) {
         if (b < 0) continue;
         my_b[i] = b; my_rank[i] = id >= 0 ? atomicAdd(&scnt[b], 1) : t;   // every row has the shared expert
         if (id < 0 && t == 0) scnt[b] = a.T;
-        atomicOr(&sbat[b], 1u << (t >> 5));
     }
     __syncthreads();
     const int c0 = tid < nb ? (scnt[tid] + 7) >> 3 : 0;   // segments of bucket tid; bucket 1024 is appended by the last thread
@@ -297,11 +295,7 @@ __global__ void __launch_bounds__(GR_THREADS) k_moe_group(GroupArgs a) {
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) { const int o = __shfl_up_sync(0xffffffffu, inc, off); if (lane >= off) inc += o; }
     if (lane == 31) swt[warp] = inc;
-    int nt = tid < nb ? __popc(sbat[tid]) : 0;   // touched matrices, counted per 32 rows
-    if (tid == 0 && nb > GR_THREADS) nt += __popc(sbat[GR_THREADS]);
-    nt = __reduce_add_sync(0xffffffffu, nt);
-    if (lane == 0) atomicAdd(&s_touched, nt);
-    __syncthreads();
+    const int touched = __syncthreads_count(c0 > 0) + (nb > GR_THREADS && scnt[GR_THREADS] > 0 ? 1 : 0);
     if (warp == 0) {
         const int wv = swt[lane]; int winc = wv;
 #pragma unroll
@@ -314,7 +308,7 @@ __global__ void __launch_bounds__(GR_THREADS) k_moe_group(GroupArgs a) {
     if (tid == GR_THREADS - 1) {
         soff[GR_THREADS] = ex + c0;
         a.ctl[0] = ex + c0 + (nb > GR_THREADS ? (scnt[GR_THREADS] + 7) >> 3 : 0); a.ctl[1] = 0; a.ctl[2] = 0;
-        if (a.touched) atomicAdd(a.touched, (unsigned long long)s_touched);
+        if (a.touched) atomicAdd(a.touched, (unsigned long long)touched);
     }
     __syncthreads();
 #pragma unroll
@@ -753,7 +747,7 @@ int moe_route_group(const MoeRouteParams& p, cudaStream_t s) {
 size_t moe_seg_bytes(int pairs) { return (size_t)pairs * sizeof(MoeSeg); }
 int moe_group_rows(const MoeRouteParams& p, cudaStream_t s) {
     HP_REQUIRE(p.T >= 1 && p.T <= MOE_MAX_ROWS && p.k >= 1 && p.k <= 15 && p.ids && p.segs && p.ctl && p.e_lo >= 0 && p.e_lo <= p.e_hi && p.e_hi <= p.E && p.E <= 1024, "moe_group_rows: bad arguments");
-    static_assert(MOE_MAX_ROWS * 16 <= GR_THREADS * GR_PAIRS && MOE_MAX_ROWS <= 32 * 32, "pairs per thread, batches of 32 rows per mask");
+    static_assert(MOE_MAX_ROWS * 16 <= GR_THREADS * GR_PAIRS, "pairs per thread");
     GroupArgs a; a.ids = p.ids; a.T = p.T; a.ns = p.k + 1; a.e_lo = p.e_lo; a.e_hi = p.e_hi; a.own_shared = p.own_shared; a.segs = (MoeSeg*)p.segs; a.ctl = p.ctl; a.touched = p.touched;
     HP_CUDA(launch_pdl<8>(k_moe_group, dim3(1), dim3(GR_THREADS), 0, s, a));
     return HP_OK;

@@ -215,8 +215,9 @@ int hp_gdn_state_dev(hp_engine* e, int slot, int gdn_layer, float** ptr_out, siz
  * LM head: the algorithmic bytes of the roofline. */
 int hp_profile_pass(hp_engine* e, int R, int what, int reps, float* ms_out);
 /* More measurement hooks: the number of (layer, expert) matrices touched by the passes since the last call (mixture of
- * experts: the unique expert bytes of the roofline = that count x bytes per expert; 32 rows of a prompt count as a pass); the mean device time in microseconds
- * of one expert-parallel exchange for R rows (0 on a single GPU); the kernels in the last fused round's graph. */
+ * experts: the unique expert bytes of the roofline = that count x bytes per expert; a chunk of a prompt counts each of its
+ * matrices once); the mean device time in microseconds of one expert-parallel exchange for R rows (0 on a single GPU);
+ * the kernels in the last fused round's graph. */
 int hp_moe_touched(hp_engine* e, unsigned long long* n_out);
 int hp_ep_exchange_us(hp_engine* e, int R, int reps, float* us_out);
 /* 1 when the expert-parallel exchange runs over peer memory (every rank mapped every other rank's exchange buffer through

@@ -2,10 +2,13 @@
 for the 24 rows of a configuration-5 verify pass, through the kernel-level C-ABI entry hp_moe_layer: bit for bit against
 the CPU restatement (router GEMV, routing, per-(row, slot) expert GEMVs, SiLU, quantiser, slot-order combine) and,
 for the routing, against the double-precision transcription of fn.hip:167-205."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
+import hipster_b200 as hb
 from hipster_b200 import kernels as K_, synth
 from oracle import orc
 
@@ -100,3 +103,36 @@ def test_unit_form_of_the_expert_gemv_matches_too():
                        env=env, cwd=root, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
     assert "1 passed" in r.stdout
+
+
+class _Route(ctypes.Structure):   # MoeRouteParams of csrc/kernels.h
+    _fields_ = [("W", ctypes.c_void_p), ("x", ctypes.c_void_p), ("logits", ctypes.c_void_p)] + [(n, ctypes.c_int) for n in ("E", "K", "k", "T")] + \
+               [(n, ctypes.c_void_p) for n in ("ids", "w", "ticket", "row_tok", "row_pos", "row_slot")] + [("synth_key", ctypes.c_ulonglong)] + \
+               [(n, ctypes.c_int) for n in ("e_lo", "e_hi", "own_shared")] + [(n, ctypes.c_void_p) for n in ("segs", "ctl", "touched", "err")]
+
+
+# rows of a prompt chunk: one beyond a pass, a ragged last group of eight, the most pairs a thread takes (512 rows of 16 slots), one bucket more than
+# threads, all rows on few experts, and a part of the experts without the shared one
+@pytest.mark.parametrize("T,n_expert,k,lo,hi,shared", [(33, 64, 4, 0, 64, 1), (300, 512, 10, 0, 512, 1), (507, 1024, 15, 0, 1024, 1), (512, 16, 15, 0, 16, 1), (512, 512, 15, 128, 256, 0)])
+def test_chunk_rows_are_grouped_by_expert(T, n_expert, k, lo, hi, shared):
+    rng = np.random.default_rng(T + k)
+    ids = np.full((T, k + 1), -1, dtype=np.int32)
+    for t in range(T):
+        ids[t, :k] = rng.choice(n_expert, size=k, replace=False)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    d_ids, segs, ctl, touched = torch.from_numpy(ids).cuda(), torch.full((T * (k + 1), 16), 0x55, **i32), torch.full((4,), 7, **i32), torch.zeros(1, dtype=torch.int64, device="cuda")
+    p = _Route(E=n_expert, k=k, T=T, ids=d_ids.data_ptr(), e_lo=lo, e_hi=hi, own_shared=shared, segs=segs.data_ptr(), ctl=ctl.data_ptr(), touched=touched.data_ptr())
+    f = getattr(hb.lib(), "_ZN2hp14moe_group_rowsERKNS_14MoeRouteParamsEP11CUstream_st")
+    hb.check(f(ctypes.byref(p), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    flat = ids.reshape(-1)
+    want = {e: np.flatnonzero(flat == e) for e in list(range(lo, hi)) + ([-1] if shared else [])}
+    want = {e: w for e, w in want.items() if len(w)}
+    n = ctl[0].item()
+    assert ctl[:3].tolist() == [sum((len(w) + 7) // 8 for w in want.values()), 0, 0]
+    got, order = {}, []
+    for expert, ncols, *cols in segs[:n, :10].tolist():
+        assert 1 <= ncols <= 8 and (not order or order[-1] == expert or len(got[order[-1]]) == len(want[order[-1]]))
+        got.setdefault(expert, []).extend(cols[:ncols]); order.append(expert)
+    assert sorted(set(order), key=order.index) == list(want)                # in bucket order, the shared expert last
+    assert all(np.array_equal(np.sort(got[e]), want[e]) for e in want)
+    assert touched.item() == len(want)                                      # each matrix of the chunk counts once
