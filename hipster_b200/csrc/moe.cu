@@ -39,6 +39,7 @@ struct RouteArgs {
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 constexpr int RG_THREADS = 512, RG_CAND = 64;   // threads; candidates that are ranked at once
 constexpr int RG_ROUTE_SMEM = 8 * 1024 * 4;   // routing scratch: the probabilities of 8 rows x up to 1024 experts
+constexpr int RG_SMEM_MAX = 204 * 1024;       // staged router and pass rows
 __global__ void __launch_bounds__(RG_THREADS) k_route_group(RouteArgs a) {
     pdl_launch_dependents();
     __shared__ int scnt[1026]; __shared__ int soff[1026]; __shared__ int swt[RG_THREADS / 32]; __shared__ int s_last;
@@ -492,7 +493,7 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 1) k_moe_gemv_grouped(MoeGArgs
 // with rings of 2 hold fewer bytes per warp and as many per SM, and segments of up to 4 columns take fewer instructions: DRAM 48 and 42 %,
 // issue 42 and 34 %, one layer of 24 rows 114 us instead of 125. (With the down projection's rings primed under gate|up and the routing below
 // 110. Five and six quads, or rings of one-block stages: 111 to 119 us against 111 in one run.)
-constexpr int MQ_WARPS = 16, MQ_QUADS = 4, MQ_AUX = 2048;   // bytes after the rings: barriers + the quads' exchange words
+constexpr int MQ_WARPS = 16, MQ_QUADS = 4, MQ_AUX = 2048, MQ_SMEM_MAX = 227 * 1024;   // bytes after the rings: barriers + the quads' exchange words
 __device__ __forceinline__ void quad_barrier(int quad) { asm volatile("bar.sync %0, 128;" ::"r"(quad + 1) : "memory"); }
 template <int MODE, int SB, int DEPTH>
 __global__ void __launch_bounds__(MQ_WARPS * 32, 1) k_moe_gemv_quad(MoeGArgs a) {
@@ -733,14 +734,13 @@ int moe_route_group(const MoeRouteParams& p, cudaStream_t s) {
     // when both fit (K <= 2176); the routing phase needs RG_ROUTE_SMEM bytes of the same buffer
     const size_t wbytes = (size_t)16 * a.K * 4, xbytes = (size_t)8 * a.K * 4;
     a.stage_w = wbytes <= 192 * 1024 && ((uintptr_t)a.W & 15) == 0 ? 1 : 0;
-    a.stage_x = a.stage_w && wbytes + xbytes <= 204 * 1024 && ((uintptr_t)a.x & 15) == 0 ? 1 : 0; a.err = p.err;
+    a.stage_x = a.stage_w && wbytes + xbytes <= RG_SMEM_MAX && ((uintptr_t)a.x & 15) == 0 ? 1 : 0; a.err = p.err;
     size_t smem = a.stage_w ? wbytes + (a.stage_x ? xbytes : 0) : 0;
     if (smem < (size_t)RG_ROUTE_SMEM) smem = RG_ROUTE_SMEM;
-    if (smem > 32 * 1024) {   // the kernel also has ~12 KB of static shared memory: opt in above 48 KB in total
-        static size_t attr[MAX_DEVICES] = {};
-        const int dev = current_device(); if (dev < 0) return HP_ECUDA;
-        if (smem > attr[dev]) { HP_CUDA(cudaFuncSetAttribute(k_route_group, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr[dev] = smem; }
-    }
+    // opted in once, for all sizes: with its 16 KB of static shared memory the smallest launch already stands at the 48 KB that need none
+    static bool attr[MAX_DEVICES] = {};
+    const int dev = current_device(); if (dev < 0) return HP_ECUDA;
+    if (!attr[dev]) { HP_CUDA(cudaFuncSetAttribute(k_route_group, cudaFuncAttributeMaxDynamicSharedMemorySize, RG_SMEM_MAX)); attr[dev] = true; }
     HP_CUDA(launch_pdl<8>(k_route_group, dim3((a.N + 15) / 16, (a.T + 7) / 8), dim3(RG_THREADS), smem, s, a));
     HP_CUDA(cudaGetLastError()); return HP_OK;
 }
@@ -772,9 +772,9 @@ static int launch_grouped_sb(const MoeGArgs& a, bool few, cudaStream_t s) {
 }
 template <int MODE, int SB, int DEPTH>
 static int launch_quad(const MoeGArgs& a, size_t smem, cudaStream_t s) {
-    static size_t attr[MAX_DEVICES] = {};
+    static bool attr[MAX_DEVICES] = {};   // once, for all sizes that take this form: another thread's launch may be of another size
     const int dev = current_device(); if (dev < 0) return HP_ECUDA;
-    if (smem > attr[dev]) { HP_CUDA(cudaFuncSetAttribute(k_moe_gemv_quad<MODE, SB, DEPTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); attr[dev] = smem; }
+    if (!attr[dev]) { HP_CUDA(cudaFuncSetAttribute(k_moe_gemv_quad<MODE, SB, DEPTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, MQ_SMEM_MAX)); attr[dev] = true; }
     HP_CUDA(launch_pdl<8>(k_moe_gemv_quad<MODE, SB, DEPTH>, dim3(GEMV_NCTA), dim3(MQ_WARPS * 32), smem, s, a));
     return HP_OK;
 }
@@ -783,7 +783,7 @@ static int launch_quad(const MoeGArgs& a, size_t smem, cudaStream_t s) {
 static size_t quad_smem(const MoeGArgs& a) { const int sb = a.nb % 2 == 0 ? 2 : 1, depth = sb == 2 ? 2 : 4; return (size_t)MQ_WARPS * depth * sb * 2304 + MQ_AUX + (size_t)MQ_QUADS * a.nb * 2560; }
 static bool quad_form(const MoeGArgs& a) {
     static const bool v1 = getenv("HIPSTER_B200_MOE_UNITS") != nullptr;
-    return !v1 && quad_smem(a) <= 227 * 1024 && a.tiles % MOE_UNIT_TILES == 0;
+    return !v1 && quad_smem(a) <= MQ_SMEM_MAX && a.tiles % MOE_UNIT_TILES == 0;
 }
 template <int MODE>
 static int launch_experts(const MoeGArgs& a, bool few, cudaStream_t s) {
