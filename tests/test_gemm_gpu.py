@@ -98,6 +98,37 @@ def test_narrow_ranges_give_the_bits_of_the_gemv(weights, ntc, G):
             assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (N, K, R)
 
 
+# The GEMM takes each sub-block's integer dot from an fp32 accumulator of the tensor core: the dots that need most of its bits (16: nibbles of
+# 15 against 127, odd ones beside them), one-signed sums and large ones that cancel to a residue. Scales of 1 and no minimum, so that every sum is a
+# whole number below 2^24 and the result exact.
+@pytest.mark.gpu
+@pytest.mark.parametrize("ntc,G", CUTS)
+def test_dots_of_full_width_are_exact(ntc, G):
+    N, K, R = 400, 768, 8 * ntc + 5
+    g = torch.Generator(device="cuda").manual_seed(ntc)
+    ri = lambda hi, *shape: torch.randint(0, hi, shape, device="cuda", generator=g)
+    full, part = torch.full((N, K // 32, 32), 15, device="cuda"), torch.tensor([0, 1, 14, 15], device="cuda")[ri(4, N, K // 32, 32)]
+    one = full.clone(); one.scatter_(2, ri(32, N, K // 32, 1), 14)
+    q = torch.where(ri(2, N, K // 32, 1) == 0, full, torch.where(ri(2, N, K // 32, 1) == 0, one, part))
+    sign = 1 - 2 * ri(2, R, K // 32, 1)
+    flat, near, far = torch.full((R, K // 32, 32), 127, device="cuda"), 119 + ri(3, R, K // 32, 32), torch.tensor([127, 126, 121, 1, 0, -1, -120, -127], device="cuda")[ri(8, R, K // 32, 32)]
+    cancel = flat.clone(); cancel[..., ::2] = -127; cancel.scatter_(2, 1 + 2 * ri(16, R, K // 32, 1), 126)
+    kind = ri(4, R, K // 32, 1)
+    x = sign * torch.where(kind == 0, flat, torch.where(kind == 1, near, torch.where(kind == 2, far, cancel)))
+    x[..., 31] = 127 * sign[..., 0]                              # a largest value of 127: the quantised row is the row itself
+    blk = torch.zeros((N, K // 256, 144), dtype=torch.uint8, device="cuda")
+    blk[..., 1] = 0x3C                                            # d = 1
+    blk[..., 4:8] = 1; blk[..., 12:16] = 1                        # scales of 1, minima of 0
+    qs = q.reshape(N, K // 256, 4, 2, 32)
+    blk[..., 16:] = (qs[..., 0, :] | qs[..., 1, :] << 4).reshape(N, K // 256, 128).to(torch.uint8)
+    wt = K_.repack_tiled(blk.reshape(-1), N, K, 0)
+    xq = K_.quantize_x_q8(x.reshape(R, K).float()); err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got, gemv = run_gemm(wt, xq, N, K, R, N, (ntc, G), err), run_gemv(wt, xq, N, K, R, N, err)
+    want = x.reshape(R, K).double() @ q.reshape(N, K).double().T
+    assert err.item() == 0 and (want.abs() < 2 ** 24).all() and (q * 127).sum(-1).max() == 60960
+    assert torch.equal(gemv.double().sum(0), want) and torch.equal(got.view(torch.int32), gemv.view(torch.int32))
+
+
 # rows from the smallest to the largest of fp32, scales of the weights from subnormal ones up: products of the scales that are subnormal, and dots
 # of few nibbles beside products that leave no factor of 512 to the largest number
 @pytest.mark.gpu

@@ -46,9 +46,11 @@ def test_prefill_on_both_sides_of_the_gemm_line(n):
     test_prefill_chunks_bit_exact_vs_oracle("tiny", n, {})
 
 
-# experts grouped over a whole chunk: one row beyond a pass, segments that are full and not, a full chunk and a short one behind it, the
-# shared expert behind 1024 others (a bucket of its own beyond the threads of the scan)
-@pytest.mark.parametrize("n,over", [(40, dict(n_expert=1024)), (128, {}), (300, dict(synth_router_logits=1)), (515, dict(max_ctx=640, synth_router_logits=1))])
+# experts grouped over a whole chunk: one row beyond a pass, segments that are full and not, two chunks of unequal length, the shared expert behind
+# 1024 others (a bucket of its own beyond the threads of the scan), a full chunk of the most slots per row (512 x 16 pairs) and one with a ragged last
+# group of rows
+@pytest.mark.parametrize("n,over", [(40, dict(n_expert=1024)), (128, {}), (300, dict(synth_router_logits=1)), (515, dict(max_ctx=640, synth_router_logits=1)),
+                                    (512, dict(max_ctx=640, n_expert=64, n_expert_used=15)), (507, dict(max_ctx=640, synth_router_logits=1))])
 def test_prefill_groups_the_experts_of_a_chunk(n, over):
     test_prefill_chunks_bit_exact_vs_oracle("tiny-moe", n, {"max_ctx": 320, **over})
 
