@@ -433,7 +433,7 @@ int Engine::ffn_block(const LayerW& L, int R) {
 // for the rows of the current buffers: up to MAXR of a pass, up to PF_MAXR of a prompt chunk
 int Engine::moe_rows(const LayerW& L, int R, const int* tok, const int* pos, const int* slot, int* pushed) {
     const hp_model_cfg& c = c_; const int E = c.n_embd, F = c.expert_ff, ns = c.n_expert_used + 1;
-    const bool chunk = R > MAXR;   // of a prompt: each touched expert streamed once for all its rows
+    const bool chunk = R > MAXR;   // of a prompt: each touched expert read from memory once for all its rows
     // synthetic routing (see hp_model_cfg.synth_router_logits): the key of a layer's draws; 0 = the router's own logits
     const int lidx = &L == &mtp_ ? c.n_layer : (int)(&L - layers_.data());
     const uint64_t rkey = c.synth_router_logits ? (splitmix64(c.seed ^ 0x726F75746572ull ^ ((uint64_t)lidx << 40)) | 1ull) : 0ull;

@@ -1,7 +1,7 @@
 // Q4_K x int8 GEMM for prompt chunks (many rows) on the 5th-generation tensor cores: tcgen05.mma kind::f8f6f4 with the
 // accumulator in TMEM.
 //
-// The arithmetic is that of the verify GEMV (gemv_q4k.cu) operation by operation: the exact int32 dot of every 32-element
+// The arithmetic is that of the verify GEMV (gemv_q4k.cu) operation by operation: the exact integer dot of every 32-element
 // sub-block, then acc = fmaf((d*sc) * xd, (float)idot, acc); acc = fmaf(-(dmin*mn), xs, acc) in block order, with the
 // sums of a 16-row tile cut where the GEMV's partition cuts them (K parts, warp boundaries of the tile's CTA) and added
 // in the same order. A row therefore has the same bits whichever of the two kernels computed it.
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gemm_q4k_tc(const TcArgs a) {
             for (int i = nh > BST ? nh - BST : 0; i < nh; ++i) tc_wait(b_full + 8 * (i % BST), (i / BST) & 1, a.err);
             if (k) { const int i = k - 1; tc_wait(sc_full + 8 * (i % Geo::SCS), (i / Geo::SCS) & 1, a.err); }
         }
-    } else if (warp >= TC_W_CNV) {   // ---- weights: row scales, nibbles -> u8
+    } else if (warp >= TC_W_CNV) {   // ---- weights: row scales, nibbles -> bytes
         tc_reg_dec<72>();
         const int cw = warp - TC_W_CNV, ct = cw * 32 + lane;
         const int sh_a = sel ? 4 : 0, sh_b = 4 - sh_a;   // nibbles of the first store; the second takes the others

@@ -172,9 +172,13 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // round: its CTAs sit beside the gate|up GEMV's and start the moment it ends) and attention gain, while programmatic
 // edges on the row norms and the GDN kernel cost ~0.1 ms per round each, so while a stream is being captured the default
 // mask switches those and the bookkeeping classes off. HIPSTER_B200_PDL_OFF=<mask> overrides both. Work in front of the wait
-// may read only what nobody writes while the library runs: the engine's own weights. What a caller hands to a public entry
-// point is read behind it, since the kernels in front (and the caller's) may trigger before they have waited themselves
-// (or behind a memset: hp_moe_layer's router rows).
+// may read what nobody writes while the library runs (the engine's own weights), and what was complete before the kernel directly in front
+// was released, if that kernel triggers behind its own wait. Two kernels rely on the latter: k_attn_split (older keys, row groups) follows
+// k_qk_norm_rope_kv or, over further rows of it, k_attn_merge, which cannot start before all splits in front of it have triggered behind their
+// wait; k_moe_gemv_quad<1> (segments, the caller's weights) follows either form of the gate|up projection. The triggers of k_qk_norm_rope_kv,
+// k_attn_split, k_moe_gemv_quad<0> and k_moe_gemv_grouped therefore stay behind their waits. Everything else that a caller hands to a public
+// entry point is read behind the wait, since the kernels in front (and the caller's) may trigger before they have waited themselves (or behind
+// a memset: hp_moe_layer's router rows).
 inline int pdl_off_mask(cudaStream_t s) {
     static const int env = [] { const char* e = getenv("HIPSTER_B200_PDL_OFF"); return e ? atoi(e) : -1; }();
     if (env >= 0) return env;

@@ -118,7 +118,9 @@ struct AttnParams {
 };
 size_t attn_partial_floats(int ngroups, int n_kv, int nsplit_max);
 int attn_rope_kv(const AttnParams& p, int rows, cudaStream_t s);          // reference k_qk_norm_rope_kv (ops.hip:363-411)
-int attn_decode(const AttnParams& p, int rows, int ngroups, cudaStream_t s);   // reference attn_decode_mq (ops.h:72)
+// reference attn_decode_mq (ops.h:72). Directly behind attn_rope_kv of these rows, or behind attn_decode of other rows of the same call of it: keys
+// that are older than all rows of the launch, and the row groups, are read ahead of the dependency wait
+int attn_decode(const AttnParams& p, int rows, int ngroups, cudaStream_t s);
 
 // one sequence of R <= 8 rows at positions pos0.., descriptors and partials in caller-provided workspace
 size_t attn_seq_workspace_bytes(int R, int n_head, int n_kv, int max_ctx);
