@@ -132,9 +132,10 @@ def test_dots_of_full_width_are_exact(ntc, G):
 # rows from the smallest to the largest of fp32, scales of the weights from subnormal ones up: products of the scales that are subnormal, and dots
 # of few nibbles beside products that leave no factor of 512 to the largest number
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,K", [(400, 768), (2100, 17408)])
 @pytest.mark.parametrize("ntc,G", CUTS)
-def test_rows_at_the_ends_of_the_range_give_the_bits_of_the_gemv(ntc, G):
-    N, K, R = 400, 768, 8 * ntc + 5
+def test_rows_at_the_ends_of_the_range_give_the_bits_of_the_gemv(ntc, G, N, K):
+    R = 8 * ntc + 5
     g = torch.Generator(device="cuda").manual_seed(ntc)
     blk = torch.randint(0, 256, (N, K // 256, 144), dtype=torch.uint8, device="cuda", generator=g)
     blk[N // 2:, :, 16:] *= (torch.rand((N - N // 2, K // 256, 128), device="cuda", generator=g) < 1 / 64).to(torch.uint8)
