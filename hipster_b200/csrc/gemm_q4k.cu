@@ -9,7 +9,7 @@
 // The dots come as fp32: a nibble q, read as e4m3, is q / 512 (subnormal up to 7), an int8 activation is 16 a + b with |a|, |b| <= 8, both
 // exact in e4m3, and the two products accumulate exactly (at most 16 significant bits). The accumulator holds idot / 512 and the row scales
 // carry the 512 (see tc_plain). (kind::i8 took one MMA instead of two, but each dot cost a conversion in the update: 34816 x 5120 at 512 rows 692 us,
-// now 609.)
+// now 610.)
 //
 // What bounds it: the fp32 update, three packed instructions per two outputs and sub-block (12 clocks of an SM sub-partition per 16x8x32
 // tile), which hardly overlaps with what brings its operands into registers: TMEM loads (16x256b fills 64 bytes a clock) and column
@@ -140,8 +140,9 @@ __device__ __forceinline__ uint64_t tc_cuts(int N, int nb, int P, int tile, int 
 // The one rounding in front of the fmaf is that of the product (d * sc) * xd, of d / 16 where the GEMV leaves the high nibbles shifted. With xd of this
 // range it is no subnormal number (f16 d: d / 16 is 2^-28 at least) and 512 times (d * sc) * xd no infinity (d * sc is less than 2^22), so the row
 // scales may carry the 512. A launch with other scales (heads whose gates underflow have them; NaN) takes the GEMV's own product, one packed
-// multiplication more per two outputs: in a prompt of the 27B shape two launches of 192, 301 tokens 75.0 -> 75.15 ms. (Left to the tensor core, which
-// then repeats its products up to the GEMV's dot, such a launch takes three to eight times as long.)
+// multiplication more per two outputs: in a prompt of the 27B shape two launches of 192. Prompts against a kernel without these loops (which also shift
+// the registers of the common ones): 27B shape 52 tokens 19.7 -> 19.5 ms, 130 tokens 42.7 -> 42.2, 301 tokens 75.1 -> 75.3, 2048-wide experts 200 tokens
+// 24.4 -> 24.6. (Left to the tensor core, which then repeats its products up to the GEMV's dot, such a launch takes three to eight times as long.)
 __device__ __forceinline__ bool tc_plain(float xd) { return xd == 0.f || (xd >= 0x1p-98f && xd <= 0x1p96f); }
 
 // One step of an update warp: its W column tiles over GB sub-blocks (row scales 128 float2 apart, one 64-byte group of
